@@ -9,10 +9,11 @@
 // (re and im parts of a_lm as separate coordinates) A^T = w S E and
 // S^T = (1/w) E^-1 A, w = 4 pi / npix, E = 1 for m = 0 and 1/2 for m >= 1
 // (the synthesis counts the m >= 1 terms twice), so
-//   f_bar = w S sum_{j=0}^{niter} (I - A S)^j (E a_bar),
-// evaluated as x <- b + x - A S x (niter times, from x = b = E a_bar) with
-// the same synthesis, aliasing fold and analysis kernels as the forward
-// refinement.  Reference: the transforms are those of src/cat2anlm.jl:257-357
+//   f_bar = S sum_{j=0}^{niter} (I - A S)^j (w E a_bar),
+// evaluated as x <- b + x - A S x (niter times, from x = b = w E a_bar).  That
+// is the forward refinement a <- a0 + a - A S a with b for its first pass a0,
+// so it runs through the same Gram form (or, without Gram tables, the same
+// synthesis, aliasing fold and analysis over every ring).  Reference: the transforms are those of src/cat2anlm.jl:257-357
 // (cat2amln, field2anlm_v2) around src/healpix_helpers.jl:50-56 (map2alm).
 #include <algorithm>
 #include <cmath>
@@ -21,20 +22,15 @@
 
 namespace sfb {
 
-// alm[lm][c] *= 1/2 for m >= 1 (E above); lm = l (l+1)/2 + m
-__global__ void k_halve_m(double *alm, int64_t lmsize, int64_t ncol) {
+// alm[lm][c] *= s (m = 0) or s / 2 (m >= 1) (w E above); lm = l (l+1)/2 + m
+__global__ void k_halve_m(double *alm, int64_t lmsize, int64_t ncol, double s) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= lmsize * ncol) return;
     const int64_t lm = i / ncol;
     int l = (int)((sqrt(8.0 * (double)lm + 1.0) - 1.0) * 0.5);
     while ((int64_t)(l + 1) * (l + 2) / 2 <= lm) ++l;
     while ((int64_t)l * (l + 1) / 2 > lm) --l;
-    if (lm - (int64_t)l * (l + 1) / 2 >= 1) alm[i] *= 0.5;
-}
-
-__global__ void k_scale(double *x, int64_t n, double s) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        x[i] *= s;
+    alm[i] *= lm - (int64_t)l * (l + 1) / 2 >= 1 ? 0.5 * s : s;
 }
 
 // Transpose of the radial projection a_nlm = s sum_b c[pair(n,l)][b] A_b[lm]:
@@ -112,16 +108,10 @@ __global__ void k_deposit_adjoint(const double *__restrict__ rtp, int64_t ngal, 
     dw[i] += acc;
 }
 
-void launch_halve_m(double *alm, int64_t lmsize, int64_t ncol, cudaStream_t st) {
+void launch_halve_m(double *alm, int64_t lmsize, int64_t ncol, double s, cudaStream_t st) {
     const int64_t n = lmsize * ncol;
     if (n <= 0) return;
-    k_halve_m<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(alm, lmsize, ncol);
-    note_launch();
-}
-
-void launch_scale(double *x, int64_t n, double s, cudaStream_t st) {
-    if (n <= 0) return;
-    k_scale<<<(unsigned)std::min<int64_t>((n + 255) / 256, 4096), 256, 0, st>>>(x, n, s);
+    k_halve_m<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(alm, lmsize, ncol, s);
     note_launch();
 }
 

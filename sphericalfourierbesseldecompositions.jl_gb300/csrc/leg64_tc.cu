@@ -1,0 +1,567 @@
+// FP64 Legendre and Gram contractions on the tensor cores (tcgen05), many
+// columns: the analysis, the synthesis and the Gram update of the FP64
+// transform, as error-free products of 8-bit digits.
+//
+// GB300 does about 2 FP64 FMA per clock and SM, so a tiled FP64 GEMM of these
+// contractions is bound by the FP64 pipe at 0.6 TFMA/s.  The BF16 tensor cores
+// do 4096 MAC per clock and SM; 28 of them per FP64 product leave 146.  Each
+// operand value is rounded to a 55-bit integer on a scale common to its whole
+// K range (per data column, per table row) and written as seven signed 8-bit
+// digits, which BF16 holds exactly (Ozaki, Ogita, Oishi, Rump, Numer.
+// Algorithms 59, 2012).  The digit products of level v = a + b (v = 0..6, 28
+// of the 49 products; the others are below 2^-56 of the scales) are summed in
+// one FP32 TMEM accumulator per level.  A product is at most 2^14, so the sum
+// of level v over 256 values of K is at most (v + 1) 2^22: levels 0..3 are
+// exact whatever the tensor cores' accumulation order or rounding, and a
+// rounding in level v >= 4 is below 2^-56 of the scales.  K is therefore
+// worked in blocks of SBK chunks; after each the levels are joined as a 62-bit
+// integer, rounded once to FP64 and added to the output.  The result is as
+// close to the exact sum as an FP64 accumulation (the whole FP64 field2anlm
+// against 64-bit references: 3.6e-15 before, 3.5e-15 now).
+//
+// MMA shape: M = 128 data columns, N = table rows (<= 64 a tile), K = 16 a
+// step.  Data digit a multiplies the table digits 0..6-a in as few MMAs as N <=
+// 256 allows (their planes are stored back to back, and level v is TMEM
+// columns [v LS, (v + 1) LS)).  Warps 0-7 read FP64 columns, form the digits
+// with integer operations and store them as K-major core matrices; the table
+// digits arrive by bulk copy; warp 8 issues the MMAs.  7 x 64 TMEM columns and
+// five 42 KB stages: one CTA per SM.  Bound: MMA issue (896 cycles a chunk of
+// 16 x 64 x 128) beside the digit forming (about 640).
+//
+// Measured at 128 columns, nside 128, lmax 82 (one refinement pass of a 64-map
+// adjoint): analysis 800 -> 33 us; see the per-kernel table in the design notes.
+#include <cuda_bf16.h>
+
+#include <algorithm>
+#include <cmath>
+#include <cstdlib>
+
+#include "sfb_internal.h"
+#include "tc_common.cuh"
+
+namespace sfb {
+namespace t64 {
+
+using namespace tc;
+
+constexpr int ND = 7;                                  // digits, and levels kept
+constexpr int KC = 16;                                 // K per chunk (one MMA K step)
+constexpr int MTILE = 128;                             // data columns per CTA
+constexpr int NT = 64;                                 // table rows per CTA
+constexpr int SBK = 16;                                // chunks per exact K block (256 values)
+constexpr int NPROD = 256;
+constexpr int NTH = NPROD + 32;
+constexpr int NSTAGE = 5;
+constexpr uint32_t PLANE_A = MTILE * KC * 2;
+constexpr uint32_t STAGE_BYTES = ND * (PLANE_A + NT * KC * 2);
+constexpr uint32_t TMEM_COLS = 512;
+constexpr size_t SMEM = NSTAGE * (size_t)STAGE_BYTES + 256;
+
+__device__ __forceinline__ int rows_of(int m, int par, int lmax) {
+    return (m + par <= lmax) ? (lmax - m - par) / 2 + 1 : 0;
+}
+__host__ __device__ __forceinline__ int ls_of(int n, int tile) {      // padded table rows of a tile
+    const int left = n - tile * NT;
+    return left >= NT ? NT : (left + 15) & ~15;
+}
+__device__ __forceinline__ uint32_t core_off(int row, int k) {
+    return (uint32_t)((((row >> 3) * (KC / 8) + (k >> 3)) << 7) + ((row & 7) << 4) + ((k & 7) << 1));
+}
+
+// x on the unit 2^(emax - 1077): a 55-bit integer plus sign, rounded to nearest
+// (emax: exponent field of the column's largest magnitude, |x| < 2^(emax - 1022))
+__device__ __forceinline__ int64_t fixed55(double x, int emax) {
+    const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
+    int e = (int)(hi >> 20) & 0x7ff;
+    uint64_t mant = ((uint64_t)((hi & 0xfffffu) | (e ? 0x100000u : 0u)) << 32) | lo;
+    e = max(e, 1);
+    const int s = min(emax - e, 63);
+    const int64_t q = (int64_t)((((mant << 3) >> s) + 1) >> 1);
+    return (int32_t)hi < 0 ? -q : q;
+}
+
+// The digits of two integers as bf16x2 words, most significant first.  With 128 added to the six lower
+// digits the bytes of the sum are the digits plus 128; a byte becomes a float through the mantissa of 2^23.
+__device__ __forceinline__ void digits2(int64_t q0, int64_t q1, uint32_t (&w)[ND]) {
+    constexpr int64_t BIAS = 0x0000808080808080LL;
+    q0 += BIAS;
+    q1 += BIAS;
+    auto top = [](int64_t q) { return __int_as_float(0x4B400000 + (int)(q >> 48)) - 12582912.0f; };
+    auto dig = [](int64_t q, int s) {
+        const uint32_t half = s >= 4 ? (uint32_t)((uint64_t)q >> 32) : (uint32_t)q;
+        return __uint_as_float(__byte_perm(half, 0x4B000000u, 0x7650u | (uint32_t)(s & 3))) - 8388736.0f;
+    };
+    w[0] = bf16x2(top(q0), top(q1));
+#pragma unroll
+    for (int s = 5; s >= 0; --s) w[6 - s] = bf16x2(dig(q0, s), dig(q1, s));
+}
+
+// sum_v L_v 2^(-8 v), times 2^(S + 40), rounded to FP64
+__device__ __forceinline__ double join_levels(const float (&L)[ND], int S) {
+    auto i64 = [](float v) { return (int64_t)__float2int_rn(v); };
+    const int64_t H = (((((i64(L[0]) << 8) + i64(L[1])) << 8) + i64(L[2])) << 8) + i64(L[3]);
+    const int64_t W = (((i64(L[4]) << 8) + i64(L[5])) << 8) + i64(L[6]);
+    const int64_t T = (H << 16) + ((W + 128) >> 8);
+    if (T == 0) return 0.0;
+    const uint64_t a = T < 0 ? (uint64_t)(-T) : (uint64_t)T;
+    const int lz = __clzll((long long)a);
+    const uint64_t frac = (((a << lz) >> 1) + 512u) >> 10;            // 2^52 <= frac <= 2^53
+    const int ef = 11 - lz + S + 52 + 1023;                            // exponent field of frac 2^(11 - lz + S)
+    double v;
+    if (ef >= 1 && ef <= 2045)
+        v = __longlong_as_double((long long)(((uint64_t)(ef - 1) << 52) + frac));
+    else
+        v = ldexp((double)a, S);
+    return T < 0 ? -v : v;
+}
+
+struct Smem {
+    unsigned char *base;
+    uint64_t *full_a, *full_b, *empty, *done;
+    uint32_t *slot;
+    int *bad;
+    __device__ __forceinline__ unsigned char *stage(int s) const { return base + s * STAGE_BYTES; }
+};
+
+__device__ __forceinline__ uint32_t setup(Smem &c, unsigned char *base) {
+    c.base = base;
+    c.full_a = reinterpret_cast<uint64_t *>(base + NSTAGE * STAGE_BYTES);
+    c.full_b = c.full_a + NSTAGE;
+    c.empty = c.full_b + NSTAGE;
+    c.done = c.empty + NSTAGE;
+    c.slot = reinterpret_cast<uint32_t *>(c.done + 1);
+    c.bad = reinterpret_cast<int *>(c.slot + 1);
+    if ((threadIdx.x >> 5) == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(c.slot)),
+                     "r"(TMEM_COLS)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < NSTAGE; ++i) {
+            mbar_init(&c.full_a[i], NPROD / 32);
+            mbar_init(&c.full_b[i], 1);
+            mbar_init(&c.empty[i], 1);
+        }
+        mbar_init(c.done, 1);
+        *c.bad = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    fence_before();
+    __syncthreads();
+    fence_after();
+    return *c.slot;
+}
+
+// the products of one chunk: data digit a with the table digits 0..6-a, level a + b
+__device__ __forceinline__ void issue(uint32_t tmem, uint32_t sa, uint32_t sb, int LS, bool first) {
+    const uint32_t sbo = (KC / 8) * 128;
+    const uint32_t planeB = (uint32_t)LS * KC * 2;
+    const int per = 256 / LS;                             // table digits one MMA can take
+    for (int a = 0; a < ND; ++a) {
+        const uint64_t ad = smem_desc(sa + a * PLANE_A, 128, sbo);
+        for (int b = 0; b < ND - a; b += per) {
+            const int nb = min(per, ND - a - b);
+            mma_bf16(tmem + (uint32_t)(LS * (a + b)), ad, smem_desc(sb + b * planeB, 128, sbo),
+                     idesc_bf16(MTILE, LS * nb), (first && a == 0) ? 0u : 1u);
+        }
+    }
+}
+
+// One CTA: data columns [128 blockIdx.x, +128) x table rows of one tile of block z = (m, parity).
+// LMROWS: the data rows are coefficients l = m + parity + 2 k (synthesis, Gram); else rings k (analysis).
+// Tiles blockIdx.y < ny0 use task 0, the others task 1 (the Gram update and the aliased rings' synthesis of
+// one refinement pass share a launch: both read the current coefficients).
+template <bool LMROWS>
+__global__ void __launch_bounds__(NTH, 1) k_leg64(const double *__restrict__ data, int64_t ncol, int lmax, int nrn,
+                                                  int klim, const int *__restrict__ nzr, Task64 t0, Task64 t1, int ny0,
+                                                  int *err) {
+    extern __shared__ __align__(1024) unsigned char smem[];
+    __shared__ uint32_t red[2][MTILE];
+    const int z = blockIdx.z, m = z >> 1, par = z & 1;
+    const bool first_task = (int)blockIdx.y < ny0;
+    const Task64 &t = first_task ? t0 : t1;
+    const int tile = first_task ? blockIdx.y : blockIdx.y - ny0;
+    const int nrows = rows_of(m, par, lmax);
+    const int N = t.n_is_rows ? nrows : t.nout;                  // table rows of the block
+    const int nwrite = t.n_is_rows ? nrows : t.nlim;             // rows written
+    if (tile * NT >= nwrite || (nrows == 0 && t.n_is_rows)) return;
+    const int K = LMROWS ? nrows : min(klim, nrn);               // data rows
+    const int64_t col0 = (int64_t)blockIdx.x * MTILE;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int c = tid & (MTILE - 1), kh = (tid >> 7) & 1;
+    const bool prod = tid < NPROD, cok = prod && col0 + c < ncol;
+    const double *D = LMROWS ? data + col0 + c
+                             : data + ((int64_t)(par * (lmax + 1) + m) * nrn) * ncol + col0 + c;
+    auto row_at = [&](int k) -> int64_t {
+        if constexpr (LMROWS) {
+            const int l = m + par + 2 * k;
+            return ((int64_t)l * (l + 1) / 2 + m) * ncol;
+        }
+        return (int64_t)k * ncol;
+    };
+    int kbeg = 0, kend = K;
+    if (!LMROWS && nzr) {                     // zero spectra outside the ring pairs [nzr[0], nzr[1]]
+        kbeg = nzr[0];
+        kend = min(K, nzr[1] + 1);
+        if (kbeg >= kend) kbeg = kend = 0;
+    }
+    // chunks with a non-zero table digit (the products with the others are exactly zero)
+    int lo = kbeg / KC, hi = (kend + KC - 1) / KC - 1;
+    if (t.live) {
+        const int2 lv = t.live[(int64_t)z * t.ntile + tile];
+        lo = max(lo, lv.x);
+        hi = min(hi, lv.y);
+    }
+    if (hi < lo && t.mode == 1) return;       // nothing to add
+    const int nch = hi < lo ? 0 : hi - lo + 1;
+    const int LS = ls_of(N, tile);
+    const int nKtab = ((LMROWS ? nrows : nrn) + KC - 1) / KC;    // chunks of the table's block
+    const uint16_t *tab = t.dig + t.off[z] + (int64_t)tile * nKtab * ND * NT * KC + (int64_t)lo * ND * LS * KC;
+    const uint32_t bytesB = (uint32_t)ND * LS * KC * 2;
+
+    // largest magnitude of every column (the high word orders the magnitudes by exponent)
+    uint32_t mx = 0;
+    if (cok) {
+#pragma unroll 8
+        for (int k = kbeg + kh; k < kend; k += 2) {
+            const double v = D[row_at(k)];
+            mx = max(mx, ((uint32_t)__double2hiint(v) & 0x7fffffffu) | (__double2loint(v) != 0 ? 1u : 0u));
+        }
+    }
+    if (prod) red[kh][c] = mx;
+    Smem cs;
+    const uint32_t tmem = setup(cs, smem);    // includes a __syncthreads
+    const uint32_t cmx = max(red[0][c], red[1][c]);
+    const int emax = max(1, (int)(cmx >> 20));
+    const bool zero = cmx == 0 || emax == 2047;                  // no digits: zero or non-finite columns
+
+    double pre[2][8];
+    auto load = [&](int kc, double (&buf)[8]) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int k = (lo + kc) * KC + 8 * kh + j;
+            buf[j] = (cok && !zero && k >= kbeg && k < kend) ? D[row_at(k)] : 0.0;
+        }
+    };
+    if (prod) {
+        if (nch > 0) load(0, pre[0]);
+        if (nch > 1) load(1, pre[1]);
+    }
+    auto chunk = [&](int kc, double (&cur)[8]) -> bool {
+        const int s = kc % NSTAGE;
+        if (kc >= NSTAGE) {
+            if (*(volatile int *)cs.bad) return false;
+            if (!mbar_wait(&cs.empty[s], (uint32_t)((kc / NSTAGE - 1) & 1))) {
+                atomicExch(cs.bad, 1);
+                return false;
+            }
+        }
+        unsigned char *sa = cs.stage(s);
+        if (tid == 0) {
+            mbar_expect_tx(&cs.full_b[s], bytesB);
+            bulk_g2s(sa + ND * PLANE_A, tab + (int64_t)kc * ND * LS * KC, bytesB, &cs.full_b[s]);
+        }
+        uint32_t w[ND][4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            uint32_t v[ND];
+            digits2(fixed55(cur[2 * j], emax), fixed55(cur[2 * j + 1], emax), v);
+#pragma unroll
+            for (int q = 0; q < ND; ++q) w[q][j] = v[q];
+        }
+        const uint32_t off = core_off(c, 8 * kh);
+#pragma unroll
+        for (int q = 0; q < ND; ++q)
+            *reinterpret_cast<uint4 *>(sa + q * PLANE_A + off) = make_uint4(w[q][0], w[q][1], w[q][2], w[q][3]);
+        if (kc + 2 < nch) load(kc + 2, cur);
+        fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&cs.full_a[s]);
+        return true;
+    };
+
+    const int nsb = max(1, (nch + SBK - 1) / SBK);
+    for (int sb = 0; sb < nsb; ++sb) {
+        const int k0 = sb * SBK, k1 = min(nch, k0 + SBK);
+        if (!prod) {
+            if (lane == 0) {
+                int kc = k0;
+                for (; kc < k1; ++kc) {
+                    const int s = kc % NSTAGE;
+                    const uint32_t ph = (uint32_t)((kc / NSTAGE) & 1);
+                    if (*(volatile int *)cs.bad) break;
+                    if (!mbar_wait(&cs.full_a[s], ph) || !mbar_wait(&cs.full_b[s], ph)) {
+                        atomicExch(cs.bad, 1);
+                        break;
+                    }
+                    fence_after();
+                    const uint32_t sa = smem_u32(cs.stage(s));
+                    issue(tmem, sa, sa + ND * PLANE_A, LS, kc == k0);
+                    mma_commit(&cs.empty[s]);
+                }
+                if (kc < k1) atomicExch(cs.bad, 1);
+                mma_commit(cs.done);          // arrives once every MMA issued above has completed
+            }
+            __syncwarp();
+        } else {
+            for (int kc = k0; kc < k1; kc += 2) {         // k0 is even: chunk parity = buffer
+                if (!chunk(kc, pre[0])) break;
+                if (kc + 1 < k1 && !chunk(kc + 1, pre[1])) break;
+            }
+        }
+        bool ok = mbar_wait(cs.done, (uint32_t)(sb & 1));
+        fence_after();
+        ok = __syncthreads_and(ok) && !*(volatile int *)cs.bad;
+        if (!ok) {
+            if (tid == 0) atomicOr(err, ERR_TC_TIMEOUT);
+            break;                                        // uniform: every thread saw the same value
+        }
+        if (prod) {
+            // warp w: TMEM lanes 32 (w % 4).. (columns), table rows [32 (w / 4), +32) of the tile
+            const int lq = warp & 3, hg = warp >> 2;
+            const uint32_t lane_base = (uint32_t)(lq * 32) << 16;
+            const int cl = lq * 32 + lane;
+            const int64_t cc = col0 + cl;
+            const uint32_t lmx = max(red[0][cl], red[1][cl]);
+            const int lemax = max(1, (int)(lmx >> 20));
+            for (int g = 0; g < 4; ++g) {
+                const int i0 = 32 * hg + 8 * g;
+                if (i0 >= LS || tile * NT + i0 >= nwrite) break;              // warp-uniform
+                float v[ND][8];
+#pragma unroll
+                for (int q = 0; q < ND; ++q) tmem_ld8(tmem + lane_base + (uint32_t)(q * LS + i0), v[q]);
+                if (cc < ncol) {
+                    double old[8];
+                    int ex[8];
+                    auto at = [&](int i) -> int64_t {
+                        const int n = tile * NT + i0 + i;
+                        if (t.n_is_rows) {
+                            const int l = m + par + 2 * n;
+                            return ((int64_t)l * (l + 1) / 2 + m) * ncol + cc;
+                        }
+                        return ((int64_t)(par * (lmax + 1) + m) * t.nout + n) * ncol + cc;
+                    };
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const int n = tile * NT + i0 + i;
+                        old[i] = 0.0;
+                        ex[i] = 0;
+                        if (n < nwrite) {
+                            ex[i] = t.ex[(int64_t)z * t.exs + n];
+                            if (sb > 0 || t.mode == 1) old[i] = t.out[at(i)];
+                            else if (t.mode == 2) old[i] = t.a0[at(i)];
+                        }
+                    }
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const int n = tile * NT + i0 + i;
+                        if (n >= nwrite) continue;
+                        double val;
+                        if (lemax == 2047) {                  // non-finite data: the plain FP64 sum
+                            val = 0.0;
+                            if (sb == 0)
+                                for (int k = kbeg; k < kend; ++k)
+                                    val = fma(t.tab64[t.tab64_off[z] + n * t.sn + k * t.sk],
+                                              data[(D - data) - (col0 + c) + cc + row_at(k)], val);
+                        } else if (nch == 0) {
+                            val = 0.0;
+                        } else {
+                            const float L[ND] = {v[0][i], v[1][i], v[2][i], v[3][i], v[4][i], v[5][i], v[6][i]};
+                            val = join_levels(L, lemax + ex[i] - 1076);
+                        }
+                        t.out[at(i)] = t.mode == 2 ? old[i] - val : (sb > 0 || t.mode == 1) ? old[i] + val : val;
+                    }
+                }
+            }
+        }
+        fence_before();
+        __syncthreads();                                      // TMEM is read before the next block's MMAs
+        fence_after();
+    }
+    fence_before();
+    __syncthreads();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
+}
+
+// ---- tables ---------------------------------------------------------------------------------------------------
+// kind 0: analysis (N = rows li, K = rings), 1: synthesis (N = rings, K = rows), 2: Gram (N = K = rows);
+// element (n, k) of block z at off64[z] + n sn + k sk.
+__device__ __forceinline__ void dims(int kind, int z, int lmax, int nrn, int &N, int &K) {
+    const int nrows = rows_of(z >> 1, z & 1, lmax);
+    N = kind == 1 ? nrn : nrows;
+    K = kind == 0 ? nrn : nrows;
+}
+
+// exponent E of every table row, |v| < 2^E (one warp per row)
+__global__ void k64_rowexp(int kind, const double *__restrict__ tab, const int64_t *__restrict__ off64, int64_t sn,
+                           int64_t sk, int lmax, int nrn, int exs, int16_t *__restrict__ ex) {
+    const int z = blockIdx.y, lane = threadIdx.x & 31;
+    int N, K;
+    dims(kind, z, lmax, nrn, N, K);
+    for (int n = blockIdx.x * 8 + (threadIdx.x >> 5); n < N; n += gridDim.x * 8) {
+        double mx = 0.0;
+        for (int k = lane; k < K; k += 32) mx = fmax(mx, fabs(tab[off64[z] + n * sn + k * sk]));
+        for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        if (lane == 0) ex[(int64_t)z * exs + n] = (int16_t)(mx > 0.0 && isfinite(mx) ? ilogb(mx) + 1 : 0);
+    }
+}
+
+// one block per (tile and chunk, z): the digit planes and the live chunk range of the tile
+__global__ void __launch_bounds__(256) k64_build(int kind, const double *__restrict__ tab,
+                                                 const int64_t *__restrict__ off64, int64_t sn, int64_t sk, int lmax,
+                                                 int nrn, int exs, const int16_t *__restrict__ ex, int ntile,
+                                                 int nkmax, const int64_t *__restrict__ off,
+                                                 uint16_t *__restrict__ dig, int2 *__restrict__ live) {
+    const int z = blockIdx.y, tile = blockIdx.x / nkmax, kc = blockIdx.x % nkmax;
+    int N, K;
+    dims(kind, z, lmax, nrn, N, K);
+    const int nK = (K + KC - 1) / KC;
+    if (tile * NT >= N || kc >= nK) return;
+    const int LS = ls_of(N, tile);
+    uint16_t *base = dig + off[z] + (int64_t)tile * nK * ND * NT * KC + (int64_t)kc * ND * LS * KC;
+    int any = 0;
+    for (int e = threadIdx.x; e < LS * KC; e += blockDim.x) {
+        const int nn = sn == 1 ? e % LS : e / KC, k = sn == 1 ? e / LS : e % KC;
+        const int n = tile * NT + nn, kk = kc * KC + k;
+        int64_t q = 0;
+        if (n < N && kk < K)
+            q = llrint(ldexp(tab[off64[z] + n * sn + kk * sk], 55 - (int)ex[(int64_t)z * exs + n]));
+        any |= q != 0;
+        uint32_t w[ND];
+        digits2(q, 0, w);
+#pragma unroll
+        for (int d = 0; d < ND; ++d) base[(int64_t)d * LS * KC + (core_off(nn, k) >> 1)] = (uint16_t)(w[d] & 0xffffu);
+    }
+    if (__syncthreads_or(any) && threadIdx.x == 0) {
+        atomicMin(&live[(int64_t)z * ntile + tile].x, kc);
+        atomicMax(&live[(int64_t)z * ntile + tile].y, kc);
+    }
+}
+
+__global__ void k64_fill(int2 *r, int64_t n) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        r[i] = make_int2(0x7fffffff, -1);
+}
+
+}  // namespace t64
+
+// Digit tables of the plan, built at the first FP64 transform of many columns.  14 bytes a table element
+// against 8 in FP64: above a sixteenth of the free device memory (or SFBGPU_TC64=0) the plan keeps the
+// FP64 units instead (state -1).
+bool ensure_tc64(Plan &p, cudaStream_t st) {
+    if (p.tc64_state) return p.tc64_state > 0;
+    p.tc64_state = -1;
+    if (const char *e = std::getenv("SFBGPU_TC64"))
+        if (e[0] == '0') return false;
+    const int nz = 2 * (p.lmax + 1);
+    const int nrows0 = p.lmax / 2 + 1;
+    std::vector<int64_t> off[3];
+    size_t bytes[3] = {};
+    int exs[3], ntile[3], nkmax[3];
+    const int nkind = p.d_gram64 ? 3 : 2;
+    size_t total = 0;
+    for (int kind = 0; kind < nkind; ++kind) {
+        const int Nmax = kind == 1 ? (int)p.nrn : nrows0, Kmax = kind == 0 ? (int)p.nrn : nrows0;
+        exs[kind] = Nmax;
+        ntile[kind] = (Nmax + t64::NT - 1) / t64::NT;
+        nkmax[kind] = (Kmax + t64::KC - 1) / t64::KC;
+        int64_t o = 0;
+        for (int z = 0; z < nz; ++z) {
+            const int m = z >> 1, par = z & 1;
+            const int nr = (m + par <= p.lmax) ? (p.lmax - m - par) / 2 + 1 : 0;
+            const int N = kind == 1 ? (int)p.nrn : nr, K = kind == 0 ? (int)p.nrn : nr;
+            off[kind].push_back(o);
+            const int64_t nK = (K + t64::KC - 1) / t64::KC;
+            if (nr == 0) continue;
+            for (int t = 0; t * t64::NT < N; ++t) o += nK * t64::ND * t64::ls_of(N, t) * t64::KC;
+        }
+        bytes[kind] = (size_t)o * 2;
+        total += bytes[kind];
+    }
+    size_t fr = 0, tot = 0;
+    if (cudaMemGetInfo(&fr, &tot) != cudaSuccess || total > fr / 16) {
+        cudaGetLastError();
+        return false;
+    }
+    for (int kind = 0; kind < nkind; ++kind) {
+        // one allocation: [digits][offsets][live ranges][exponents], each part 256-byte aligned
+        auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
+        const size_t b0 = up(bytes[kind] + 16), b1 = up(nz * sizeof(int64_t)),
+                     b2 = up((size_t)nz * ntile[kind] * sizeof(int2)), b3 = up((size_t)nz * exs[kind] * sizeof(int16_t));
+        unsigned char *d = nullptr;
+        if (cudaMalloc(&d, b0 + b1 + b2 + b3) != cudaSuccess) {
+            cudaGetLastError();
+            return false;                     // the tables made so far stay owned by the plan
+        }
+        p.device_bytes += (int64_t)(b0 + b1 + b2 + b3);
+        Task64 &t = p.t64[kind];
+        p.t64_mem[kind] = d;
+        t.dig = reinterpret_cast<uint16_t *>(d);
+        t.off = reinterpret_cast<int64_t *>(d + b0);
+        t.live = reinterpret_cast<int2 *>(d + b0 + b1);
+        t.ex = reinterpret_cast<int16_t *>(d + b0 + b1 + b2);
+        t.exs = exs[kind];
+        t.ntile = ntile[kind];
+        t.n_is_rows = kind != 1;
+        t.nout = (int)p.nrn;
+        t.tab64 = kind == 2 ? p.d_gram64 : p.d_lam;
+        t.tab64_off = kind == 2 ? p.d_gram_off : p.d_lam_off;
+        t.sn = kind == 0 ? p.nrn : 1;
+        t.sk = kind == 0 ? 1 : kind == 1 ? p.nrn : p.gram_rows;
+        if (cudaMemcpyAsync(d + b0, off[kind].data(), nz * sizeof(int64_t), cudaMemcpyHostToDevice, st) != cudaSuccess ||
+            cudaStreamSynchronize(st) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        const int64_t nl = (int64_t)nz * ntile[kind];
+        t64::k64_fill<<<(unsigned)((nl + 255) / 256), 256, 0, st>>>(const_cast<int2 *>(t.live), nl);
+        t64::k64_rowexp<<<dim3(16, (unsigned)nz), 256, 0, st>>>(kind, t.tab64, t.tab64_off, t.sn, t.sk, p.lmax,
+                                                               (int)p.nrn, t.exs, const_cast<int16_t *>(t.ex));
+        t64::k64_build<<<dim3((unsigned)(ntile[kind] * nkmax[kind]), (unsigned)nz), 256, 0, st>>>(
+            kind, t.tab64, t.tab64_off, t.sn, t.sk, p.lmax, (int)p.nrn, t.exs, t.ex, t.ntile, nkmax[kind], t.off,
+            const_cast<uint16_t *>(t.dig), const_cast<int2 *>(t.live));
+        note_launch();
+        note_launch();
+        note_launch();
+    }
+    if (cudaGetLastError() != cudaSuccess) return false;
+    p.tc64_state = 1;
+    return true;
+}
+
+static dim3 grid64(const Plan &p, int64_t ncol, int ny) {
+    return dim3((unsigned)((ncol + t64::MTILE - 1) / t64::MTILE), (unsigned)ny, (unsigned)(2 * (p.lmax + 1)));
+}
+
+void launch_leg_analysis64(const Plan &p, const double *F, int64_t ncol, double *A, bool accumulate, cudaStream_t st,
+                           int rlim, const int *nzr) {
+    Task64 t = p.t64[0];
+    t.out = A;
+    t.mode = accumulate ? 1 : 0;
+    set_smem(t64::k_leg64<false>, t64::SMEM);
+    t64::k_leg64<false><<<grid64(p, ncol, t.ntile), t64::NTH, t64::SMEM, st>>>(F, ncol, p.lmax, (int)p.nrn, rlim, nzr,
+                                                                              t, t, t.ntile, p.d_err);
+    note_launch();
+}
+
+// G of the rings r < rlim (G may be null) and, with Anew, the Gram update Anew = A0 - D A.
+void launch_leg_synthesis64(const Plan &p, const double *A, int64_t ncol, double *G, cudaStream_t st, int rlim,
+                            const double *A0, double *Anew) {
+    Task64 g = p.t64[2], s = p.t64[1];
+    g.out = Anew;
+    g.a0 = A0;
+    g.mode = 2;
+    s.out = G;
+    s.mode = 0;
+    s.nlim = rlim;
+    const int ny0 = Anew ? g.ntile : 0, ny1 = G && rlim > 0 ? (rlim + t64::NT - 1) / t64::NT : 0;
+    if (ny0 + ny1 == 0) return;
+    set_smem(t64::k_leg64<true>, t64::SMEM);
+    t64::k_leg64<true><<<grid64(p, ncol, ny0 + ny1), t64::NTH, t64::SMEM, st>>>(A, ncol, p.lmax, (int)p.nrn, 0, nullptr,
+                                                                               g, s, ny0, p.d_err);
+    note_launch();
+}
+
+}  // namespace sfb

@@ -415,6 +415,10 @@ void launch_leg_analysis(const Plan &p, const double *F, int64_t ncol, double *A
     }
     const int maxrows = p.lmax / 2 + 1;
     if (rlim < 0 || rlim > p.nrn) rlim = (int)p.nrn;
+    if (p.precision == SFB_FP64 && p.tc64_state > 0) {
+        launch_leg_analysis64(p, F, ncol, A, accumulate, st, rlim, nzr);
+        return;
+    }
     dim3 grid((unsigned)((ncol + BN - 1) / BN), (unsigned)((maxrows + BM - 1) / BM), (unsigned)(2 * (p.lmax + 1)));
     if (p.precision == SFB_MIXED)
         k_leg_analysis<float><<<grid, 256, 0, st>>>(p.d_lam32, p.d_lam_off, p.lmax, (int)p.nrn, (const float *)F,
@@ -436,6 +440,10 @@ void launch_leg_synthesis(const Plan &p, const double *A, int64_t ncol, double *
     }
     if (rlim < 0 || rlim > p.nrn) rlim = (int)p.nrn;
     if (rlim == 0) return;
+    if (p.precision == SFB_FP64 && p.tc64_state > 0) {
+        launch_leg_synthesis64(p, A, ncol, G, st, rlim, nullptr, nullptr);
+        return;
+    }
     dim3 grid((unsigned)((ncol + BN - 1) / BN), (unsigned)((rlim + BM - 1) / BM), (unsigned)(2 * (p.lmax + 1)));
     if (p.precision == SFB_MIXED)
         k_leg_synthesis<float><<<grid, 256, 0, st>>>(p.d_lam32, p.d_lam_off, p.lmax, (int)p.nrn, (const float *)A,
@@ -728,6 +736,80 @@ __global__ void __launch_bounds__(256) k_fold_alias(const RingGeom *__restrict__
     }
 }
 
+// The same aliased-ring fold in FP64 (F = 0, rings r < ral): residue buckets, one ring at a time.  Block:
+// parity, FC complex columns, rpb rings; shared memory holds the ring's G rows and the buckets.  Bound: the
+// G rows read and R rows written, once each; k_fold_cols above reads every aliased G term from memory for
+// every m' and took 91 us a pass (101 maps, 41 rings, lmax 82) against 9 us here.
+template <int FC>
+__global__ void __launch_bounds__(256) k_fold_alias64(const RingGeom *__restrict__ rings, int nrn, int ral, int rpb,
+                                                      int nbk, int lmax, double w, const double *__restrict__ G,
+                                                      int64_t ncplx, double *__restrict__ R) {
+    extern __shared__ double2 fsm64[];
+    const int par = blockIdx.y, tid = threadIdx.x;
+    const int64_t c0 = (int64_t)blockIdx.x * FC;
+    const int r0 = blockIdx.z * rpb, r1 = min(ral, r0 + rpb);
+    const int L1 = lmax + 1;
+    const int64_t ld = 2 * ncplx;
+    double2 *P = fsm64;                               // [nbk][FC], nbk = the longest of the rings
+    double2 *Gs = fsm64 + (int64_t)nbk * FC;          // [L1][FC] the ring's G rows
+    for (int r = r0; r < r1; ++r) {
+        const RingGeom g = rings[r];
+        const int n = min(g.nph, nbk);
+        const bool odd = g.phi0_den != 0;
+        const double f = w * (double)n * g.cfold;
+        __syncthreads();
+#pragma unroll 4
+        for (int i = tid; i < L1 * FC; i += 256) {
+            const int m = i / FC, cc = i - m * FC;
+            Gs[i] = c0 + cc < ncplx ? *reinterpret_cast<const double2 *>(
+                                          G + ((int64_t)(par * L1 + m) * nrn + r) * ld + 2 * (c0 + cc))
+                                    : make_double2(0.0, 0.0);
+        }
+        __syncthreads();
+        for (int i = tid; i < n * FC; i += 256) {
+            const int k = i / FC, cc = i - k * FC;
+            double sx = 0.0, sy = 0.0;
+            int t = 0;
+            for (int m = k; m <= lmax; m += n, ++t) {
+                const double2 v = Gs[m * FC + cc];
+                const bool neg = odd && (t & 1);
+                sx += neg ? -v.x : v.x;
+                if (m != 0) sy += neg ? -v.y : v.y;
+            }
+            P[i] = make_double2(sx, sy);
+        }
+        __syncthreads();
+        for (int i = tid; i < L1 * FC; i += 256) {
+            const int mp = i / FC, cc = i - mp * FC;
+            if (c0 + cc >= ncplx) continue;
+            const int k = mp % n, kk = (n - k) % n;
+            const double2 p1 = P[k * FC + cc];
+            double2 p2 = P[kk * FC + cc];
+            if (kk == 0) p2.x -= Gs[cc].x;            // without the m = 0 term
+            const bool n1 = odd && ((mp / n) & 1), n2 = odd && (((kk + mp) / n) & 1);
+            const double sx = (n1 ? -p1.x : p1.x) + (n2 ? -p2.x : p2.x);
+            const double sy = (n1 ? -p1.y : p1.y) - (n2 ? -p2.y : p2.y);
+            *reinterpret_cast<double2 *>(R + ((int64_t)(par * L1 + mp) * nrn + r) * ld + 2 * (c0 + cc)) =
+                make_double2(-f * sx, -f * sy);
+        }
+    }
+}
+
+template <int FC>
+static bool fold_alias64(const Plan &p, const double *G, int64_t ncplx, double *R, int rlim, cudaStream_t st) {
+    int nbk = 1;
+    for (int r = 0; r < rlim; ++r) nbk = std::max(nbk, p.h_rings[r].nph);
+    const size_t smem = ((size_t)nbk + (size_t)(p.lmax + 1)) * FC * sizeof(double2);
+    if (smem > 100 * 1024) return false;              // two CTAs per SM
+    const int rpb = 4;
+    set_smem(k_fold_alias64<FC>, smem);
+    k_fold_alias64<FC><<<dim3((unsigned)((ncplx + FC - 1) / FC), 2, (unsigned)((rlim + rpb - 1) / rpb)), 256, smem,
+                         st>>>(p.d_rings, (int)p.nrn, rlim, rpb, nbk, p.lmax, 4.0 * M_PI / (double)p.npix, G, ncplx,
+                               R);
+    note_launch();
+    return true;
+}
+
 // Few columns: one thread per (parity, m', ring, complex column), same sums.
 __device__ __forceinline__ double resid_of(const double *F, int64_t off, double f, double s) {
     return (F ? F[off] : 0.0) - f * s;
@@ -790,6 +872,10 @@ bool launch_gram_update_fp64(const Plan &p, const double *Acur, const double *A0
     case 4: k_gram_update_fp64<4><<<grid, 128, 0, st>>>(p.d_gram64, p.d_gram_off, p.gram_rows, p.lmax, Acur, A0, Anew); break;
     case 8: k_gram_update_fp64<8><<<grid, 128, 0, st>>>(p.d_gram64, p.d_gram_off, p.gram_rows, p.lmax, Acur, A0, Anew); break;
     default: {
+        if (p.tc64_state > 0) {
+            launch_leg_synthesis64(p, Acur, ncol, nullptr, st, 0, A0, Anew);
+            return true;
+        }
         dim3 wg((unsigned)((ncol + BN - 1) / BN), (unsigned)((maxrows + BM - 1) / BM), (unsigned)(2 * (p.lmax + 1)));
         k_gram_update_wide<<<wg, 256, 0, st>>>(p.d_gram64, p.d_gram_off, p.gram_rows, p.lmax, Acur, A0, ncol, Anew);
         break;
@@ -839,7 +925,11 @@ void launch_fold_residual(const Plan &p, const double *F, const double *G, int64
         return;
     }
     if (!F && ncplx > 4) {
-        // FP64 Gram refinement, many columns: the aliased-ring term over rings r < rlim
+        // FP64 Gram refinement, many columns: the aliased-ring term over rings r < rlim (eight columns a
+        // block are the 128-byte rows of G; two where longer rings fill the shared memory)
+        if (rlim > 0 && rlim <= p.ral &&
+            (fold_alias64<8>(p, G, ncplx, R, rlim, st) || fold_alias64<2>(p, G, ncplx, R, rlim, st)))
+            return;
         dim3 grid((unsigned)((ncplx + 127) / 128), (unsigned)(2 * (p.lmax + 1)),
                   (unsigned)((rlim + FOLD_RC - 1) / FOLD_RC));
         const double w = 4.0 * M_PI / (double)p.npix;

@@ -322,6 +322,18 @@ struct ShtWork {
     DevBuf<double> *f, *g, *r, *alm;
 };
 
+// One FP64 Gram refinement step's products of the current coefficients: G on the aliased rings and
+// Anew = A0 - D A (many columns: one tensor-core launch).
+void synthesis_and_gram64(const Plan &p, const double *A, const double *A0, int64_t ncol, double *G, double *Anew,
+                          cudaStream_t st) {
+    if (p.tc64_state > 0 && ncol > 8) {
+        launch_leg_synthesis64(p, A, ncol, G, st, p.ral, A0, Anew);
+        return;
+    }
+    if (p.ral > 0) launch_leg_synthesis(p, A, ncol, G, st, p.ral);
+    launch_gram_update_fp64(p, A, A0, ncol, Anew, st);
+}
+
 // fp64_out: the FP64 a_lm (alm) is wanted besides the double-float copy (almdf, mixed precision); the
 // Gram refinement carries only the double-float one and converts at the end when asked.
 // ring_live / nlive (mixed precision): rings marked 0 hold zeros in maps [0, nlive), left unwritten by the
@@ -333,6 +345,7 @@ int sht_analysis(sfb_plan *h, const double *maps, int64_t nm, cudaStream_t st, b
     const ShtWork own{&p.fbuf, &p.gbuf, &p.rbuf, &p.alm};
     if (!ws) ws = &own;
     DevBuf<double> &fbuf = *ws->f, &gbuf = *ws->g, &rbuf = *ws->r, &alm = *ws->alm;
+    if (p.precision == SFB_FP64 && 2 * nm > 8) ensure_tc64(p, st);
     auto stage = [&](int s) { return stage_override >= 0 ? stage_override : s; };
     if (p.precision == SFB_MIXED && maps_are_fp64) {
         SFB_TRY(grow(p, p.maps32, (size_t)(nm * p.npix)));
@@ -454,8 +467,7 @@ int sht_analysis(sfb_plan *h, const double *maps, int64_t nm, cudaStream_t st, b
             const int nxt = cur ^ 1;
             {
                 Stage s(h, stage(SFB_STAGE_LEG_SYNTHESIS), st);
-                if (p.ral > 0) launch_leg_synthesis(p, Ab[cur], ncol, gbuf.ptr, st, p.ral);
-                launch_gram_update_fp64(p, Ab[cur], a0, ncol, Ab[nxt], st);
+                synthesis_and_gram64(p, Ab[cur], a0, ncol, gbuf.ptr, Ab[nxt], st);
             }
             if (p.ral > 0) {
                 {
@@ -484,6 +496,22 @@ int sht_analysis(sfb_plan *h, const double *maps, int64_t nm, cudaStream_t st, b
         analysis(rbuf.ptr, true);
     }
     SFB_CUDA_TRY(cudaGetLastError());
+    return SFB_OK;
+}
+
+// The transforms that have no other device check (FP64 map2alm, anlm2field, the adjoints): the error word is
+// cleared before and read after, for a tensor-core wait that gave up.
+int clear_err(Plan &p, cudaStream_t st) {
+    SFB_CUDA_TRY(cudaMemsetAsync(p.d_err, 0, sizeof(int), st));
+    return SFB_OK;
+}
+int check_tc(Plan &p, cudaStream_t st, int *err_out = nullptr) {
+    int err = 0;
+    SFB_CUDA_TRY(cudaMemcpyAsync(&err, p.d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
+    SFB_CUDA_TRY(cudaStreamSynchronize(st));
+    SFB_CUDA_TRY(cudaGetLastError());
+    if (err_out) *err_out = err;
+    if (err & ERR_TC_TIMEOUT) return fail(SFB_ETIMEOUT, "tensor-core kernel: bounded mbarrier wait expired");
     return SFB_OK;
 }
 
@@ -520,8 +548,8 @@ int reference_alm(sfb_plan *h, const double *ref, int64_t nref, double *ralm, cu
     return SFB_OK;
 }
 
-// Transpose of sht_analysis in FP64 (adjoint.cu): abar [lmsize][2 nm] on the device becomes E abar;
-// maps_out [nm][npix] FP64 receives w S sum_j (I - A S)^j E abar.
+// Transpose of sht_analysis in FP64 (adjoint.cu): abar [lmsize][2 nm] on the device becomes b = w E abar;
+// maps_out [nm][npix] FP64 receives S sum_j (I - A S)^j b.
 int sht_analysis_adjoint(sfb_plan *h, double *abar, int64_t nm, double *maps_out, cudaStream_t st) {
     Plan &p = h->p;
     const int32_t prec = p.precision;
@@ -533,25 +561,40 @@ int sht_analysis_adjoint(sfb_plan *h, double *abar, int64_t nm, double *maps_out
     } restore{p, prec};
     const int64_t ncol = 2 * nm;
     const size_t fsz = (size_t)2 * (p.lmax + 1) * p.nrn * ncol;
+    const size_t na = (size_t)p.lmsize * ncol;
+    if (ncol > 8) ensure_tc64(p, st);
     SFB_TRY(grow(p, p.gbuf, fsz));
-    SFB_TRY(grow(p, p.alm, (size_t)p.lmsize * ncol));
-    launch_halve_m(abar, p.lmsize, ncol, st);
-    double *x = p.alm.ptr;
-    SFB_CUDA_TRY(cudaMemcpyAsync(x, abar, (size_t)p.lmsize * ncol * sizeof(double), cudaMemcpyDeviceToDevice, st));
-    if (p.niter > 0) {
+    launch_halve_m(abar, p.lmsize, ncol, 4.0 * M_PI / (double)p.npix, st);
+    const double *x = abar;
+    if (p.niter > 0 && p.d_gram64) {
+        // x <- b - D x - A_al(Fold(S_al x)): the forward's Gram refinement with b for its first pass
+        SFB_TRY(grow(p, p.alm, 2 * na));
+        SFB_TRY(grow(p, p.rbuf, fsz));
+        for (int it = 0; it < p.niter; ++it) {
+            double *nxt = p.alm.ptr + (it & 1) * na;
+            synthesis_and_gram64(p, x, abar, ncol, p.gbuf.ptr, nxt, st);
+            if (p.ral > 0) {
+                launch_fold_residual(p, nullptr, p.gbuf.ptr, ncol, p.rbuf.ptr, st, nullptr, p.ral);
+                launch_leg_analysis(p, p.rbuf.ptr, ncol, nxt, true, st, p.ral);
+            }
+            x = nxt;
+        }
+    } else if (p.niter > 0) {
+        SFB_TRY(grow(p, p.alm, na));
         SFB_TRY(grow(p, p.fbuf, fsz));
         SFB_TRY(grow(p, p.rbuf, fsz));
+        SFB_CUDA_TRY(cudaMemcpyAsync(p.alm.ptr, abar, na * sizeof(double), cudaMemcpyDeviceToDevice, st));
         SFB_CUDA_TRY(cudaMemsetAsync(p.fbuf.ptr, 0, fsz * sizeof(double), st));     // F = 0: the fold gives -A S x
-    }
-    for (int it = 0; it < p.niter; ++it) {
-        launch_leg_synthesis(p, x, ncol, p.gbuf.ptr, st);
-        launch_fold_residual(p, p.fbuf.ptr, p.gbuf.ptr, ncol, p.rbuf.ptr, st);
-        launch_leg_analysis(p, p.rbuf.ptr, ncol, x, true, st);                     // x - A S x
-        launch_axpy(x, abar, p.lmsize * ncol, st);                                   // + b
+        for (int it = 0; it < p.niter; ++it) {
+            launch_leg_synthesis(p, p.alm.ptr, ncol, p.gbuf.ptr, st);
+            launch_fold_residual(p, p.fbuf.ptr, p.gbuf.ptr, ncol, p.rbuf.ptr, st);
+            launch_leg_analysis(p, p.rbuf.ptr, ncol, p.alm.ptr, true, st);             // x - A S x
+            launch_axpy(p.alm.ptr, abar, p.lmsize * ncol, st);                           // + b
+        }
+        x = p.alm.ptr;
     }
     launch_leg_synthesis(p, x, ncol, p.gbuf.ptr, st);
     launch_ring_synthesis(p, p.gbuf.ptr, nm, maps_out, st);
-    launch_scale(maps_out, nm * p.npix, 4.0 * M_PI / (double)p.npix, st);
     SFB_CUDA_TRY(cudaGetLastError());
     return SFB_OK;
 }
@@ -1031,7 +1074,7 @@ void sfb_plan_destroy(sfb_plan *h) {
                     p.d_dtw_off, p.d_dtimg, p.d_dtimg_off, p.d_gramts, p.d_gramts_off, p.d_gram64, p.d_gram_off, p.d_cls_rings, p.d_cls_off, p.d_aimg_off, p.aimg.ptr, p.d_lam, p.d_lam32, p.d_lamtc, p.d_lamtc_off, p.d_lamts, p.d_lamts_off, p.d_lamtc_live, p.d_dft_dead, p.d_lam_off, p.d_spl_off, p.d_spl_x, p.d_spl_y, p.d_spl_ypp,
                     p.d_pair_l, p.d_pair_n, p.d_out_pair, p.d_out_lm, p.d_coef, p.d_coefT, p.d_proj_tiles, p.d_err,
                     p.maps.ptr, p.fbuf.ptr, p.gbuf.ptr, p.rbuf.ptr, p.alm.ptr, p.scratch.ptr, p.scratch2.ptr, p.dep.ptr, p.maps32.ptr,
-                    p.ref.ptr, p.rf.ptr, p.rg.ptr, p.rr.ptr, p.ralm.ptr, p.almdf2.ptr, p.adf0.ptr, p.ecoef.ptr, p.erow.ptr, p.almdf.ptr, p.nzr64.ptr, h->d_pair_index, h->d_noff};
+                    p.ref.ptr, p.rf.ptr, p.rg.ptr, p.rr.ptr, p.ralm.ptr, p.almdf2.ptr, p.adf0.ptr, p.ecoef.ptr, p.erow.ptr, p.almdf.ptr, p.nzr64.ptr, p.t64_mem[0], p.t64_mem[1], p.t64_mem[2], h->d_pair_index, h->d_noff};
     for (void *q : ptrs)
         if (q) cudaFree(q);
     if (h->aux) sfb_plan_destroy(h->aux);
@@ -1297,11 +1340,11 @@ int sfb_map2alm_adjoint(sfb_plan *h, const double *abar, int64_t nmaps, double *
     SFB_TRY(grow(p, p.scratch, A.size()));
     SFB_TRY(grow(p, p.maps, (size_t)nmaps * p.npix));
     SFB_CUDA_TRY(cudaMemcpyAsync(p.scratch.ptr, A.data(), A.size() * sizeof(double), cudaMemcpyHostToDevice, st));
+    SFB_TRY(clear_err(p, st));
     SFB_TRY(sht_analysis_adjoint(h, p.scratch.ptr, nmaps, p.maps.ptr, st));
     SFB_CUDA_TRY(cudaMemcpyAsync(maps_out, p.maps.ptr, (size_t)nmaps * p.npix * sizeof(double), cudaMemcpyDeviceToHost,
                                  st));
-    SFB_CUDA_TRY(cudaStreamSynchronize(st));
-    return SFB_OK;
+    return check_tc(p, st);
 }
 
 int sfb_cat2amln_vjp(sfb_plan *h, const double *rtp, int64_t ngal, double nbar, const double *abar, double *dw_out) {
@@ -1334,6 +1377,7 @@ int sfb_cat2amln_vjp(sfb_plan *h, const double *rtp, int64_t ngal, double nbar, 
     SFB_CUDA_TRY(cudaMemcpyAsync(&err, p.d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
     SFB_CUDA_TRY(cudaMemcpyAsync(dw_out, d_dw, ngal * sizeof(double), cudaMemcpyDeviceToHost, st));
     SFB_CUDA_TRY(cudaStreamSynchronize(st));
+    if (err & ERR_TC_TIMEOUT) return fail(SFB_ETIMEOUT, "tensor-core kernel: bounded mbarrier wait expired");
     if (err & ERR_NONFINITE_INPUT) return fail(SFB_ENONFINITE, "non-finite galaxy coordinate");
     if (err & ERR_THETA_RANGE) return fail(SFB_ERANGE, "galaxy theta outside [0, pi]");
     return SFB_OK;
@@ -1380,6 +1424,7 @@ static int field2anlm_vjp_impl(sfb_plan *h, const double *abar, int64_t nr, doub
     double *d_ab = p.scratch.ptr, *d_g = d_ab + 2 * p.nlmsize, *d_A = d_g + p.npairs * nr;
     double *d_f = d_A + p.lmsize * 2 * cs;
     SFB_CUDA_TRY(cudaMemcpyAsync(d_ab, abar, 2 * p.nlmsize * sizeof(double), cudaMemcpyHostToDevice, st));
+    SFB_TRY(clear_err(p, st));
     launch_gtab(p, nr, rmin, dr, 1, d_g, st);                // g_nl(r_s) r_s^2 dr, the field2anlm weights
     SFB_TRY(grow(p, p.scratch2, (size_t)cs * p.npairs));
     SFB_TRY(grow(p, p.maps, (size_t)cs * p.npix));
@@ -1403,8 +1448,7 @@ static int field2anlm_vjp_impl(sfb_plan *h, const double *abar, int64_t nr, doub
     SFB_CUDA_TRY(cudaGetLastError());
     if (resident)
         SFB_CUDA_TRY(cudaMemcpyAsync(df_out, d_f, (size_t)nr * p.npix * es, cudaMemcpyDeviceToHost, st));
-    SFB_CUDA_TRY(cudaStreamSynchronize(st));
-    return SFB_OK;
+    return check_tc(p, st);
 }
 
 int sfb_field2anlm_vjp(sfb_plan *h, const double *abar, int64_t nr, double rmin, double rmax, double *df_out) {
@@ -1424,10 +1468,11 @@ static int sfb_map2alm_impl(sfb_plan *h, const double *maps, int64_t nmaps, doub
     cudaStream_t st = h->stream;
     SFB_TRY(grow(p, p.maps, (size_t)nmaps * p.npix));
     SFB_CUDA_TRY(cudaMemcpyAsync(p.maps.ptr, maps, (size_t)nmaps * p.npix * sizeof(double), cudaMemcpyHostToDevice, st));
+    SFB_TRY(clear_err(p, st));
     SFB_TRY(sht_analysis(h, p.maps.ptr, nmaps, st));
     std::vector<double> A((size_t)p.lmsize * 2 * nmaps);
     SFB_CUDA_TRY(cudaMemcpyAsync(A.data(), p.alm.ptr, A.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
-    SFB_CUDA_TRY(cudaStreamSynchronize(st));
+    SFB_TRY(check_tc(p, st));
     for (int64_t b = 0; b < nmaps; ++b)
         for (int64_t lm = 0; lm < p.lmsize; ++lm) {
             alm_out[(b * p.lmsize + lm) * 2] = A[(size_t)lm * 2 * nmaps + 2 * b];
@@ -1458,6 +1503,7 @@ static int sfb_field2anlm_impl(sfb_plan *h, const void *f, int32_t dtype, int64_
     if (resident) SFB_CUDA_TRY(cudaMemcpyAsync(d_f, f, (size_t)nr * p.npix * es, cudaMemcpyHostToDevice, st));
     launch_gtab(p, nr, rmin, dr, 1, d_g, st);
     SFB_CUDA_TRY(cudaMemsetAsync(d_acc, 0, 2 * p.nlmsize * sizeof(double), st));
+    SFB_TRY(clear_err(p, st));
     SFB_TRY(grow(p, p.scratch2, (size_t)cs * p.npairs));
     const bool mixed = p.precision == SFB_MIXED;
     for (int64_t s0 = 0; s0 < nr; s0 += cs) {
@@ -1488,7 +1534,6 @@ static int sfb_field2anlm_impl(sfb_plan *h, const void *f, int32_t dtype, int64_
         launch_project_shells_g(p, p.scratch2.ptr, nsc, p.alm.ptr, 2 * nsc, d_out, st);
         launch_axpy(d_acc, d_out, 2 * p.nlmsize, st);  // d_acc += d_out
     }
-    SFB_CUDA_TRY(cudaMemsetAsync(p.d_err, 0, sizeof(int), st));
     SFB_TRY(finish(h, d_acc, st));
     SFB_CUDA_TRY(cudaMemcpyAsync(anlm_out, d_acc, 2 * p.nlmsize * sizeof(double), cudaMemcpyDeviceToHost, st));
     SFB_CUDA_TRY(cudaStreamSynchronize(st));
@@ -1515,6 +1560,8 @@ static int sfb_anlm2field_impl(sfb_plan *h, const double *anlm, int64_t nr, doub
     SFB_TRY(grow(p, p.gbuf, fsz));
     SFB_TRY(grow(p, p.alm, (size_t)p.lmsize * 2 * cs));
     SFB_TRY(grow(p, p.maps, (size_t)cs * p.npix));
+    SFB_TRY(clear_err(p, st));
+    if (2 * cs > 8) ensure_tc64(p, st);
     for (int64_t s0 = 0; s0 < nr; s0 += cs) {
         const int64_t nsc = std::min(cs, nr - s0);
         SFB_CUDA_TRY(cudaMemcpy2DAsync(p.scratch2.ptr, nsc * sizeof(double), d_g + s0, nr * sizeof(double),
@@ -1527,8 +1574,7 @@ static int sfb_anlm2field_impl(sfb_plan *h, const double *anlm, int64_t nr, doub
     }
     SFB_CUDA_TRY(cudaGetLastError());
     SFB_CUDA_TRY(cudaMemcpyAsync(f_out, d_f, (size_t)nr * p.npix * sizeof(double), cudaMemcpyDeviceToHost, st));
-    SFB_CUDA_TRY(cudaStreamSynchronize(st));
-    return SFB_OK;
+    return check_tc(p, st);
 }
 
 // The plan's auxiliary FP64 transform at lmax 2 lmax (same nside and niter): one radial
@@ -1575,6 +1621,7 @@ static int window_a00(sfb_plan *h, const double *win, int64_t nr, double *w00) {
     SFB_TRY(grow(q, q.scratch, (size_t)(nr * q.npix)));
     SFB_CUDA_TRY(cudaMemcpyAsync(q.scratch.ptr, win, (size_t)nr * q.npix * sizeof(double), cudaMemcpyHostToDevice,
                                  st));
+    SFB_TRY(clear_err(q, st));
     for (int64_t s0 = 0; s0 < nr; s0 += cs) {
         const int64_t nsc = std::min(cs, nr - s0);
         SFB_TRY(grow(q, q.maps, (size_t)nsc * q.npix));
@@ -1582,9 +1629,7 @@ static int window_a00(sfb_plan *h, const double *win, int64_t nr, double *w00) {
         SFB_TRY(sht_analysis(ax, q.maps.ptr, nsc, st));
         launch_extract_a00(q.alm.ptr, 2 * nsc, nsc, w00 + s0, st);
     }
-    SFB_CUDA_TRY(cudaStreamSynchronize(st));
-    SFB_CUDA_TRY(cudaGetLastError());
-    return SFB_OK;
+    return check_tc(q, st);
 }
 
 int sfb_win_lnn(sfb_plan *h, const double *win, int64_t nr, double rmin, double rmax, const int64_t *lnn,
@@ -1657,6 +1702,7 @@ int sfb_calc_wmix(sfb_plan *h, const double *win, int64_t nr, double rmin, doubl
             st = fail(SFB_ECUDA, "calc_wmix: window copy failed");
             break;
         }
+        if ((st = clear_err(q, as)) != SFB_OK) break;
         for (int64_t s0 = 0; s0 < nr && st == SFB_OK; s0 += cs) {
             const int64_t nsc = std::min(cs, nr - s0);
             if ((st = grow(q, q.maps, (size_t)nsc * q.npix)) != SFB_OK) break;
@@ -1670,10 +1716,7 @@ int sfb_calc_wmix(sfb_plan *h, const double *win, int64_t nr, double rmin, doubl
             }
         }
         if (st != SFB_OK) break;
-        if (cudaStreamSynchronize(as) != cudaSuccess) {
-            st = fail(SFB_ECUDA, cudaGetErrorString(cudaGetLastError()));
-            break;
-        }
+        if ((st = check_tc(q, as)) != SFB_OK) break;
         cudaStream_t ms = h->stream;
         const double dr = (rmax - rmin) / (double)nr;
         launch_gtab(p, nr, rmin, dr, 0, d_g, ms);

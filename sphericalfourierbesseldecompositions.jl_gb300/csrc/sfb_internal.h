@@ -61,6 +61,25 @@ struct DevBuf {
     size_t n = 0;  // elements
 };
 
+// One operand table of the FP64 tensor-core contractions (leg64_tc.cu) and, at a launch, what is done with
+// the product: the digit planes of block z at off[z], row exponents, live chunk ranges, and the same table in
+// FP64 (element (n, k) at tab64_off[z] + n sn + k sk).
+struct Task64 {
+    const uint16_t *dig = nullptr;
+    const int64_t *off = nullptr;
+    const int16_t *ex = nullptr;       // [z][exs]
+    const int2 *live = nullptr;        // [z][ntile]
+    int exs = 0, ntile = 0;
+    int n_is_rows = 0;                 // table rows are coefficients l = m + parity + 2 n (else rings)
+    int nout = 0, nlim = 0;            // rings of the output's layout, and those written
+    const double *tab64 = nullptr;
+    const int64_t *tab64_off = nullptr;
+    int64_t sn = 0, sk = 0;
+    double *out = nullptr;
+    const double *a0 = nullptr;
+    int mode = 0;                      // 0: out = product, 1: out += product, 2: out = a0 - product
+};
+
 struct Plan {
     int device = 0;
     // modes
@@ -163,6 +182,11 @@ struct Plan {
     DevBuf<double> ecoef;           // Gram refinement: column exponents of both a_lm sets (ints)
     DevBuf<double> erow;            // ring DFT row exponents [2][nrn][nmaps] (int)
     DevBuf<double> maps32;          // FP32 copy of FP64 maps (mixed precision, spline / dense-window paths)
+    // digit tables of the FP64 tensor-core contractions (analysis, synthesis, Gram): 0 not made yet, 1 made,
+    // -1 not used (memory); made by ensure_tc64
+    Task64 t64[3];
+    void *t64_mem[3] = {};
+    int tc64_state = 0;
     DevBuf<double> nzr64;           // FP64 many-column transform: first / last ring pair with data (2 ints)
     int64_t device_bytes = 0;
 };
@@ -245,6 +269,13 @@ void launch_leg_synthesis(const Plan &p, const double *A, int64_t ncol, double *
 // FP64 Gram refinement step (any column count); false when the plan has no Gram tables
 bool launch_gram_update_fp64(const Plan &p, const double *Acur, const double *A0, int64_t ncol, double *Anew,
                              cudaStream_t st);
+// FP64 contractions of many columns on the tensor cores (leg64_tc.cu).  ensure_tc64 makes the plan's digit
+// tables (once); false: the plan keeps the FP64 units.  The launches need a plan whose tables are made.
+bool ensure_tc64(Plan &p, cudaStream_t st);
+void launch_leg_analysis64(const Plan &p, const double *F, int64_t ncol, double *A, bool accumulate, cudaStream_t st,
+                           int rlim, const int *nzr);
+void launch_leg_synthesis64(const Plan &p, const double *A, int64_t ncol, double *G, cudaStream_t st, int rlim,
+                            const double *A0, double *Anew);
 // rlim: only rings r < rlim (-1: all); F == nullptr (Gram refinement): R = -w n cfold Fold(G)
 void launch_fold_residual(const Plan &p, const double *F, const double *G, int64_t ncol, double *R, cudaStream_t st,
                           int *Ecol = nullptr, int rlim = -1);
@@ -292,8 +323,8 @@ void launch_gram_update(const Plan &p, const double *A, const float2 *Adf, const
 int build_gram_tables(Plan &p, cudaStream_t st);
 void launch_df_to_fp64(const float2 *a, int64_t n, double *out, cudaStream_t st);
 // adjoint (adjoint.cu)
-void launch_halve_m(double *alm, int64_t lmsize, int64_t ncol, cudaStream_t st);
-void launch_scale(double *x, int64_t n, double s, cudaStream_t st);
+// alm[lm][c] *= s (m = 0) or s / 2 (m >= 1)
+void launch_halve_m(double *alm, int64_t lmsize, int64_t ncol, double s, cudaStream_t st);
 void launch_proj_adjoint(const Plan &p, const double *abar, const int32_t *pair_index, const int64_t *noff, int64_t b0,
                          int64_t nbc, double s, double *Abar, cudaStream_t st);
 void launch_deposit_adjoint(const Plan &p, const double *rtp, int64_t ngal, const double *Dbar, int64_t b0,

@@ -1,0 +1,95 @@
+"""The FP64 contractions on the tensor cores (many columns) at the edges of
+their tiles, against the oracle's map2alm and against the plan's FP64 units
+(SFBGPU_TC64=0).
+
+Tolerance: a value is held to half a unit of 2^-55 of its column's (table
+row's) largest magnitude, and the level sums lose less than that again, so a
+sum over K values is off by at most about K 2^-54 max|F| max|lambda|.  For
+N(0, 1) maps max|F| is about 4 rms and a coefficient is about sqrt(K) times
+the product of the rms values: sqrt(1024) * 16 * 2^-54 = 3e-14 of max|a| a
+pass, 1e-13 over the four passes of niter = 3."""
+
+import numpy as np
+import pytest
+
+import sfbgpu
+from helpers import record, rel_err
+from oracle.sht import SHT
+from sfbgpu.cat2anlm import map2alm, map2alm_adjoint
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-13
+
+
+def _modes(lmax, nside):
+    return sfbgpu.AnlmModes.from_nmax_lmax(1, lmax, 500.0, 1000.0, nside=nside, cache=True)
+
+
+def _maps(nmaps, nside, seed):
+    return np.random.default_rng(seed).normal(size=(nmaps, 12 * nside * nside))
+
+
+# lmax: 16-row padding (30: 16 rows, 31, 32: 17), the 64-row tile (126: 64 rows, 128: 65); nmaps: a
+# partial 128-column tile, a whole one, one column more; nside 8: one 16-ring chunk, 12: a ragged one
+@pytest.mark.parametrize("nside,lmax,nmaps,niter", [(8, 16, 5, 0), (8, 15, 7, 3), (12, 30, 5, 3), (16, 31, 64, 3),
+                                                    (16, 32, 65, 0), (32, 63, 9, 3), (64, 126, 6, 0),
+                                                    (64, 128, 6, 3)])
+def test_edges_vs_oracle(nside, lmax, nmaps, niter):
+    a = _modes(lmax, nside)
+    f = _maps(nmaps, nside, lmax)
+    ref = SHT(nside, lmax).map2alm(f, niter=niter)
+    ref = np.stack([ref[:, l, m] for l in range(lmax + 1) for m in range(l + 1)], axis=1)
+    e = rel_err(map2alm(f, a, niter=niter, radial="spline"), ref)
+    record(f"fp64_tc_map2alm_{nside}_{lmax}_{nmaps}_{niter}", e)
+    assert e < TOL
+
+
+# more than 256 ring pairs (the sum runs in exact blocks of 256), more than 64 and 128 rows
+@pytest.mark.parametrize("nside,lmax,nmaps", [(128, 256, 5), (160, 140, 5), (256, 300, 6)])
+def test_long_sums_vs_fp64_units(nside, lmax, nmaps, monkeypatch):
+    f = _maps(nmaps, nside, 3)
+    got = map2alm(f, _modes(lmax, nside), radial="spline")
+    monkeypatch.setenv("SFBGPU_TC64", "0")
+    ref = map2alm(f, _modes(lmax, nside), radial="spline")
+    e = rel_err(got, ref)
+    record(f"fp64_tc_long_{nside}_{lmax}", e)
+    assert e < TOL
+
+
+@pytest.mark.parametrize("nside,lmax,nmaps,niter", [(16, 24, 9, 3), (16, 40, 65, 0), (32, 60, 33, 3), (16, 60, 6, 2)])
+def test_adjoint_vs_fp64_units(nside, lmax, nmaps, niter, monkeypatch):
+    """(16, 60): most rings alias, so the refinement runs over every ring."""
+    rng = np.random.default_rng(7)
+    n = (lmax + 1) * (lmax + 2) // 2
+    y = rng.normal(size=(nmaps, n)) + 1j * rng.normal(size=(nmaps, n))
+    got = map2alm_adjoint(y, _modes(lmax, nside), niter=niter, radial="spline")
+    monkeypatch.setenv("SFBGPU_TC64", "0")
+    ref = map2alm_adjoint(y, _modes(lmax, nside), niter=niter, radial="spline")
+    e = rel_err(got, ref)
+    record(f"fp64_tc_adjoint_{nside}_{lmax}_{nmaps}", e)
+    assert e < TOL
+
+
+@pytest.mark.parametrize("scale", [1e-25, 1e30])
+def test_scales(scale):
+    """Magnitudes far from one (the ring transform's odd factors run in double-float, which bounds them)."""
+    a = _modes(24, 16)
+    f = _maps(6, 16, 5)
+    one = map2alm(f, a, radial="spline")
+    e = rel_err(map2alm(f * scale, a, radial="spline") / scale, one)
+    assert e < 1e-13
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_nonfinite_and_zero_maps(bad, monkeypatch):
+    """A non-finite map spoils its own coefficients, as on the FP64 units, and no other map's."""
+    f = _maps(9, 16, 6)
+    f[3, 100] = bad
+    f[5] = 0.0
+    got = map2alm(f, _modes(24, 16), radial="spline")
+    monkeypatch.setenv("SFBGPU_TC64", "0")
+    ref = map2alm(f, _modes(24, 16), radial="spline")
+    assert np.array_equal(np.isfinite(got), np.isfinite(ref)) and not np.isfinite(got[3]).any()
+    ok = [i for i in range(9) if i != 3]
+    assert rel_err(got[ok], ref[ok]) < TOL
+    assert not np.any(got[5])
