@@ -19,14 +19,15 @@
 // close to the exact sum as an FP64 accumulation (the whole FP64 field2anlm
 // against 64-bit references: 3.6e-15 before, 3.5e-15 now).
 //
-// MMA shape: M = 128 data columns, N = table rows (<= 64 a tile), K = 16 a
+// MMA shape: M = 128 data columns, N = table rows (<= 32 a tile), K = 16 a
 // step.  Data digit a multiplies the table digits 0..6-a in as few MMAs as N <=
 // 256 allows (their planes are stored back to back, and level v is TMEM
 // columns [v LS, (v + 1) LS)).  Warps 0-7 read FP64 columns, form the digits
 // with integer operations and store them as K-major core matrices; the table
-// digits arrive by bulk copy; warp 8 issues the MMAs.  7 x 64 TMEM columns and
-// five 42 KB stages: one CTA per SM.  Bound: MMA issue (896 cycles a chunk of
-// 16 x 64 x 128) beside the digit forming (about 640).
+// digits arrive by bulk copy; warp 8 issues the MMAs.  7 x 32 TMEM columns and
+// three 35 KB stages: two CTAs per SM, one working while the other starts or
+// ends (one CTA of 64 rows a SM was slower at every size: field_f64's four
+// analyses 150 us against 117, an lmax 189 call 22.4 ms against 21.5).
 //
 // Measured at 128 columns, nside 128, lmax 82 (one refinement pass of a 64-map
 // adjoint): analysis 800 -> 33 us; see the per-kernel table in the design notes.
@@ -47,14 +48,14 @@ using namespace tc;
 constexpr int ND = 7;                                  // digits, and levels kept
 constexpr int KC = 16;                                 // K per chunk (one MMA K step)
 constexpr int MTILE = 128;                             // data columns per CTA
-constexpr int NT = 64;                                 // table rows per CTA
+constexpr int NT = 32;                                 // table rows per CTA
 constexpr int SBK = 16;                                // chunks per exact K block (256 values)
 constexpr int NPROD = 256;
 constexpr int NTH = NPROD + 32;
-constexpr int NSTAGE = 5;
 constexpr uint32_t PLANE_A = MTILE * KC * 2;
+constexpr int NSTAGE = 3;
 constexpr uint32_t STAGE_BYTES = ND * (PLANE_A + NT * KC * 2);
-constexpr uint32_t TMEM_COLS = 512;
+constexpr uint32_t TMEM_COLS = 256;                    // 7 x 32 levels
 constexpr size_t SMEM = NSTAGE * (size_t)STAGE_BYTES + 256;
 
 __device__ __forceinline__ int rows_of(int m, int par, int lmax) {
@@ -66,6 +67,15 @@ __host__ __device__ __forceinline__ int ls_of(int n, int tile) {      // padded 
 }
 __device__ __forceinline__ uint32_t core_off(int row, int k) {
     return (uint32_t)((((row >> 3) * (KC / 8) + (k >> 3)) << 7) + ((row & 7) << 4) + ((k & 7) << 1));
+}
+
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, float (&v)[4]) {
+    uint32_t r[4];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(taddr));
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = __uint_as_float(r[i]);
 }
 
 // x on the unit 2^(emax - 1077): a 55-bit integer plus sign, rounded to nearest
@@ -96,23 +106,23 @@ __device__ __forceinline__ void digits2(int64_t q0, int64_t q1, uint32_t (&w)[ND
     for (int s = 5; s >= 0; --s) w[6 - s] = bf16x2(dig(q0, s), dig(q1, s));
 }
 
-// sum_v L_v 2^(-8 v), times 2^(S + 40), rounded to FP64
+// sum_v L_v 2^(-8 v), times 2^(S + 40), rounded to FP64 (integer operations: the FP64 pipe would take 16
+// cycles a warp for each one)
 __device__ __forceinline__ double join_levels(const float (&L)[ND], int S) {
-    auto i64 = [](float v) { return (int64_t)__float2int_rn(v); };
-    const int64_t H = (((((i64(L[0]) << 8) + i64(L[1])) << 8) + i64(L[2])) << 8) + i64(L[3]);
-    const int64_t W = (((i64(L[4]) << 8) + i64(L[5])) << 8) + i64(L[6]);
-    const int64_t T = (H << 16) + ((W + 128) >> 8);
-    if (T == 0) return 0.0;
+    auto i = [](float v) { return __float2int_rn(v); };
+    auto wide = [](int a, int b, int64_t c) { return (int64_t)a * b + c; };
+    const int64_t H = wide(i(L[0]), 1 << 24, wide(i(L[1]), 1 << 16, wide(i(L[2]), 1 << 8, (int64_t)i(L[3]))));
+    const int64_t W = wide(i(L[4]), 1 << 16, wide(i(L[5]), 1 << 8, (int64_t)(i(L[6]) + 128)));
+    const int64_t T = (H << 16) + (W >> 8);
+    const uint32_t sign = (uint32_t)((uint64_t)T >> 32) & 0x80000000u;
     const uint64_t a = T < 0 ? (uint64_t)(-T) : (uint64_t)T;
     const int lz = __clzll((long long)a);
     const uint64_t frac = (((a << lz) >> 1) + 512u) >> 10;            // 2^52 <= frac <= 2^53
     const int ef = 11 - lz + S + 52 + 1023;                            // exponent field of frac 2^(11 - lz + S)
-    double v;
-    if (ef >= 1 && ef <= 2045)
-        v = __longlong_as_double((long long)(((uint64_t)(ef - 1) << 52) + frac));
-    else
-        v = ldexp((double)a, S);
-    return T < 0 ? -v : v;
+    if (a == 0) return 0.0;
+    if (ef < 1 || ef > 2045) return ldexp(sign ? -(double)a : (double)a, S);
+    const uint32_t hi = (uint32_t)(frac >> 32) + ((uint32_t)(ef - 1) << 20);
+    return __hiloint2double((int)(hi | sign), (int)(uint32_t)frac);
 }
 
 struct Smem {
@@ -173,7 +183,7 @@ __device__ __forceinline__ void issue(uint32_t tmem, uint32_t sa, uint32_t sb, i
 // Tiles blockIdx.y < ny0 use task 0, the others task 1 (the Gram update and the aliased rings' synthesis of
 // one refinement pass share a launch: both read the current coefficients).
 template <bool LMROWS>
-__global__ void __launch_bounds__(NTH, 1) k_leg64(const double *__restrict__ data, int64_t ncol, int lmax, int nrn,
+__global__ void __launch_bounds__(NTH, 2) k_leg64(const double *__restrict__ data, int64_t ncol, int lmax, int nrn,
                                                   int klim, const int *__restrict__ nzr, Task64 t0, Task64 t1, int ny0,
                                                   int *err) {
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -196,9 +206,9 @@ __global__ void __launch_bounds__(NTH, 1) k_leg64(const double *__restrict__ dat
     auto row_at = [&](int k) -> int64_t {
         if constexpr (LMROWS) {
             const int l = m + par + 2 * k;
-            return ((int64_t)l * (l + 1) / 2 + m) * ncol;
+            return (int64_t)((uint64_t)(uint32_t)(l * (l + 1) / 2 + m) * (uint32_t)ncol);
         }
-        return (int64_t)k * ncol;
+        return (int64_t)((uint64_t)(uint32_t)k * (uint32_t)ncol);
     };
     int kbeg = 0, kend = K;
     if (!LMROWS && nzr) {                     // zero spectra outside the ring pairs [nzr[0], nzr[1]]
@@ -318,32 +328,31 @@ __global__ void __launch_bounds__(NTH, 1) k_leg64(const double *__restrict__ dat
             break;                                        // uniform: every thread saw the same value
         }
         if (prod) {
-            // warp w: TMEM lanes 32 (w % 4).. (columns), table rows [32 (w / 4), +32) of the tile
+            // warp w: TMEM lanes 32 (w % 4).. (columns), table rows [NT/2 (w / 4), +NT/2) of the tile
             const int lq = warp & 3, hg = warp >> 2;
             const uint32_t lane_base = (uint32_t)(lq * 32) << 16;
             const int cl = lq * 32 + lane;
             const int64_t cc = col0 + cl;
             const uint32_t lmx = max(red[0][cl], red[1][cl]);
             const int lemax = max(1, (int)(lmx >> 20));
-            for (int g = 0; g < 4; ++g) {
-                const int i0 = 32 * hg + 8 * g;
+            for (int g = 0; g < NT / 8; ++g) {
+                const int i0 = NT / 2 * hg + 4 * g;
                 if (i0 >= LS || tile * NT + i0 >= nwrite) break;              // warp-uniform
-                float v[ND][8];
+                float v[ND][4];
 #pragma unroll
-                for (int q = 0; q < ND; ++q) tmem_ld8(tmem + lane_base + (uint32_t)(q * LS + i0), v[q]);
+                for (int q = 0; q < ND; ++q) tmem_ld4(tmem + lane_base + (uint32_t)(q * LS + i0), v[q]);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                 if (cc < ncol) {
-                    double old[8];
-                    int ex[8];
-                    auto at = [&](int i) -> int64_t {
-                        const int n = tile * NT + i0 + i;
-                        if (t.n_is_rows) {
-                            const int l = m + par + 2 * n;
-                            return ((int64_t)l * (l + 1) / 2 + m) * ncol + cc;
-                        }
-                        return ((int64_t)(par * (lmax + 1) + m) * t.nout + n) * ncol + cc;
+                    double old[4];
+                    int ex[4];
+                    auto at = [&](int i) -> int64_t {                   // row index < 2^31
+                        const int n = tile * NT + i0 + i, l = m + par + 2 * n;
+                        const uint32_t row = t.n_is_rows ? (uint32_t)(l * (l + 1) / 2 + m)
+                                                         : (uint32_t)((par * (lmax + 1) + m) * t.nout + n);
+                        return (int64_t)((uint64_t)row * (uint32_t)ncol) + cc;
                     };
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) {
+                    for (int i = 0; i < 4; ++i) {
                         const int n = tile * NT + i0 + i;
                         old[i] = 0.0;
                         ex[i] = 0;
@@ -354,7 +363,7 @@ __global__ void __launch_bounds__(NTH, 1) k_leg64(const double *__restrict__ dat
                         }
                     }
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) {
+                    for (int i = 0; i < 4; ++i) {
                         const int n = tile * NT + i0 + i;
                         if (n >= nwrite) continue;
                         double val;
@@ -457,6 +466,7 @@ bool ensure_tc64(Plan &p, cudaStream_t st) {
         if (e[0] == '0') return false;
     const int nz = 2 * (p.lmax + 1);
     const int nrows0 = p.lmax / 2 + 1;
+    constexpr int NT = t64::NT;
     std::vector<int64_t> off[3];
     size_t bytes[3] = {};
     int exs[3], ntile[3], nkmax[3];
@@ -465,7 +475,7 @@ bool ensure_tc64(Plan &p, cudaStream_t st) {
     for (int kind = 0; kind < nkind; ++kind) {
         const int Nmax = kind == 1 ? (int)p.nrn : nrows0, Kmax = kind == 0 ? (int)p.nrn : nrows0;
         exs[kind] = Nmax;
-        ntile[kind] = (Nmax + t64::NT - 1) / t64::NT;
+        ntile[kind] = (Nmax + NT - 1) / NT;
         nkmax[kind] = (Kmax + t64::KC - 1) / t64::KC;
         int64_t o = 0;
         for (int z = 0; z < nz; ++z) {
@@ -475,7 +485,7 @@ bool ensure_tc64(Plan &p, cudaStream_t st) {
             off[kind].push_back(o);
             const int64_t nK = (K + t64::KC - 1) / t64::KC;
             if (nr == 0) continue;
-            for (int t = 0; t * t64::NT < N; ++t) o += nK * t64::ND * t64::ls_of(N, t) * t64::KC;
+            for (int t = 0; t * NT < N; ++t) o += nK * t64::ND * t64::ls_of(N, t) * t64::KC;
         }
         bytes[kind] = (size_t)o * 2;
         total += bytes[kind];

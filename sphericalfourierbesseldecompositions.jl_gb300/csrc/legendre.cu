@@ -616,6 +616,11 @@ __global__ void __launch_bounds__(128) k_fold_cols(const RingGeom *__restrict__ 
 // (i = tid + 256 q) in registers instead of shared memory (a smaller footprint, more CTAs per SM).
 constexpr int FOLD_MXQ = 8;
 
+// a / n as the high word of a product, exact for a n < 2^32 (n >= 2): the folds divide every m by the ring's
+// length, and an integer division costs them about twenty instructions
+__device__ __forceinline__ uint32_t recip32(int n) { return (uint32_t)(0x100000000ull / (uint32_t)n) + 1u; }
+__device__ __forceinline__ int div32(int a, uint32_t inv) { return (int)__umulhi((uint32_t)a, inv); }
+
 template <int FC, bool MXREG>
 __global__ void __launch_bounds__(256) k_fold_alias(const RingGeom *__restrict__ rings, int nrn, int ral, int rpb,
                                                     int nbk, int lmax, double w, const float *__restrict__ G,
@@ -654,6 +659,7 @@ __global__ void __launch_bounds__(256) k_fold_alias(const RingGeom *__restrict__
     for (int r = r0; r < r1; ++r) {
         const RingGeom g = rings[r];
         const int n = min(g.nph, nbk);
+        const uint32_t inv = recip32(n);
         const bool odd = g.phi0_den != 0;
         const float f = (float)(w * (double)n * g.cfold);
         __syncthreads();
@@ -689,13 +695,13 @@ __global__ void __launch_bounds__(256) k_fold_alias(const RingGeom *__restrict__
             const int mp = i / FC, cc = i - mp * FC;
             const int64_t c = c0 + cc;
             if (c >= ncplx) continue;
-            const int k = mp % n;
-            const int kk = (n - k) % n;
+            const int dq = div32(mp, inv), k = mp - dq * n;
+            const int kk = k == 0 ? 0 : n - k;
             const float2 p1 = P[k * FC + cc];
             float2 p2 = P[kk * FC + cc];
             if (kk == 0) p2.x -= Gs[cc].x;                  // P' excludes m = 0
-            const float s1 = (odd && ((mp / n) & 1)) ? -1.f : 1.f;
-            const float s2 = (odd && (((kk + mp) / n) & 1)) ? -1.f : 1.f;
+            const float s1 = (odd && (dq & 1)) ? -1.f : 1.f;
+            const float s2 = (odd && ((dq + (k != 0)) & 1)) ? -1.f : 1.f;          // (kk + mp) / n = dq + (k != 0)
             const float sx = s1 * p1.x + s2 * p2.x, sy = s1 * p1.y - s2 * p2.y;
             const float rx = -f * sx, ry = -f * sy;
             const int64_t off = ((int64_t)(par * L1 + mp) * nrn + r) * ld + 2 * c;
@@ -737,9 +743,9 @@ __global__ void __launch_bounds__(256) k_fold_alias(const RingGeom *__restrict__
 }
 
 // The same aliased-ring fold in FP64 (F = 0, rings r < ral): residue buckets, one ring at a time.  Block:
-// parity, FC complex columns, rpb rings; shared memory holds the ring's G rows and the buckets.  Bound: the
-// G rows read and R rows written, once each; k_fold_cols above reads every aliased G term from memory for
-// every m' and took 91 us a pass (101 maps, 41 rings, lmax 82) against 9 us here.
+// parity, FC complex columns, rpb rings; shared memory holds the ring's G rows and the buckets, the next
+// ring's rows are on their way in registers.  Bound: the latency of the steps of one ring; k_fold_cols above
+// reads every aliased G term from memory for every m' (91 us a pass at 101 maps, 41 rings, lmax 82).
 template <int FC>
 __global__ void __launch_bounds__(256) k_fold_alias64(const RingGeom *__restrict__ rings, int nrn, int ral, int rpb,
                                                       int nbk, int lmax, double w, const double *__restrict__ G,
@@ -752,20 +758,33 @@ __global__ void __launch_bounds__(256) k_fold_alias64(const RingGeom *__restrict
     const int64_t ld = 2 * ncplx;
     double2 *P = fsm64;                               // [nbk][FC], nbk = the longest of the rings
     double2 *Gs = fsm64 + (int64_t)nbk * FC;          // [L1][FC] the ring's G rows
+    constexpr int PF = 4;
+    double2 gv[PF];
+    auto at = [&](int i, int r) {
+        const int m = i / FC, cc = i - m * FC;
+        return c0 + cc < ncplx ? *reinterpret_cast<const double2 *>(
+                                     G + ((int64_t)(par * L1 + m) * nrn + r) * ld + 2 * (c0 + cc))
+                               : make_double2(0.0, 0.0);
+    };
+    auto load_ring = [&](int r) {
+#pragma unroll
+        for (int q = 0; q < PF; ++q)
+            if (tid + q * 256 < L1 * FC) gv[q] = at(tid + q * 256, r);
+    };
+    if (r0 < r1) load_ring(r0);
     for (int r = r0; r < r1; ++r) {
         const RingGeom g = rings[r];
         const int n = min(g.nph, nbk);
+        const uint32_t inv = recip32(n);
         const bool odd = g.phi0_den != 0;
         const double f = w * (double)n * g.cfold;
         __syncthreads();
-#pragma unroll 4
-        for (int i = tid; i < L1 * FC; i += 256) {
-            const int m = i / FC, cc = i - m * FC;
-            Gs[i] = c0 + cc < ncplx ? *reinterpret_cast<const double2 *>(
-                                          G + ((int64_t)(par * L1 + m) * nrn + r) * ld + 2 * (c0 + cc))
-                                    : make_double2(0.0, 0.0);
-        }
+#pragma unroll
+        for (int q = 0; q < PF; ++q)
+            if (tid + q * 256 < L1 * FC) Gs[tid + q * 256] = gv[q];
+        for (int i = tid + PF * 256; i < L1 * FC; i += 256) Gs[i] = at(i, r);
         __syncthreads();
+        if (r + 1 < r1) load_ring(r + 1);
         for (int i = tid; i < n * FC; i += 256) {
             const int k = i / FC, cc = i - k * FC;
             double sx = 0.0, sy = 0.0;
@@ -782,11 +801,11 @@ __global__ void __launch_bounds__(256) k_fold_alias64(const RingGeom *__restrict
         for (int i = tid; i < L1 * FC; i += 256) {
             const int mp = i / FC, cc = i - mp * FC;
             if (c0 + cc >= ncplx) continue;
-            const int k = mp % n, kk = (n - k) % n;
+            const int q = div32(mp, inv), k = mp - q * n, kk = k == 0 ? 0 : n - k;
             const double2 p1 = P[k * FC + cc];
             double2 p2 = P[kk * FC + cc];
             if (kk == 0) p2.x -= Gs[cc].x;            // without the m = 0 term
-            const bool n1 = odd && ((mp / n) & 1), n2 = odd && (((kk + mp) / n) & 1);
+            const bool n1 = odd && (q & 1), n2 = odd && ((q + (kk != 0)) & 1);       // (kk + mp) / n = q + (k != 0)
             const double sx = (n1 ? -p1.x : p1.x) + (n2 ? -p2.x : p2.x);
             const double sy = (n1 ? -p1.y : p1.y) - (n2 ? -p2.y : p2.y);
             *reinterpret_cast<double2 *>(R + ((int64_t)(par * L1 + mp) * nrn + r) * ld + 2 * (c0 + cc)) =
@@ -801,7 +820,7 @@ static bool fold_alias64(const Plan &p, const double *G, int64_t ncplx, double *
     for (int r = 0; r < rlim; ++r) nbk = std::max(nbk, p.h_rings[r].nph);
     const size_t smem = ((size_t)nbk + (size_t)(p.lmax + 1)) * FC * sizeof(double2);
     if (smem > 100 * 1024) return false;              // two CTAs per SM
-    const int rpb = 4;
+    const int rpb = 3;
     set_smem(k_fold_alias64<FC>, smem);
     k_fold_alias64<FC><<<dim3((unsigned)((ncplx + FC - 1) / FC), 2, (unsigned)((rlim + rpb - 1) / rpb)), 256, smem,
                          st>>>(p.d_rings, (int)p.nrn, rlim, rpb, nbk, p.lmax, 4.0 * M_PI / (double)p.npix, G, ncplx,
