@@ -66,8 +66,8 @@ __global__ void k_proj_adjoint(const double *__restrict__ abar, const double *__
 // the deposit keys them.
 __global__ void k_deposit_adjoint(const double *__restrict__ rtp, int64_t ngal, int64_t nside, int64_t npix,
                                   double rmin, double rmax, double inv_width, int pieces, int deg, int64_t nbasis,
-                                  const double *__restrict__ Dbar, int64_t b0, int64_t nbc, double *__restrict__ dw,
-                                  int *err) {
+                                  const double *__restrict__ Dbar, int64_t sb, int64_t sp, int64_t b0, int64_t nbc,
+                                  double *__restrict__ dw, int *err) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= ngal) return;
     const double r = rtp[3 * i], th = rtp[3 * i + 1], ph = rtp[3 * i + 2];
@@ -83,7 +83,7 @@ __global__ void k_deposit_adjoint(const double *__restrict__ rtp, int64_t ngal, 
     double acc = 0.0;
     if (r < rmin || r > rmax) {
         const int64_t b = nbasis - 2 + (r < rmin ? 0 : 1);
-        if (b >= b0 && b < b0 + nbc) acc = Dbar[(b - b0) * npix + pix];
+        if (b >= b0 && b < b0 + nbc) acc = Dbar[(b - b0) * sb + pix * sp];
     } else {
         const double u = (r - rmin) * inv_width;
         int slot = (int)u;
@@ -102,7 +102,7 @@ __global__ void k_deposit_adjoint(const double *__restrict__ rtp, int64_t ngal, 
                 p1 = v;
             }
             const int64_t b = bs + k;
-            if (b >= b0 && b < b0 + nbc) acc = fma(v, Dbar[(b - b0) * npix + pix], acc);
+            if (b >= b0 && b < b0 + nbc) acc = fma(v, Dbar[(b - b0) * sb + pix * sp], acc);
         }
     }
     dw[i] += acc;
@@ -124,12 +124,12 @@ void launch_proj_adjoint(const Plan &p, const double *abar, const int32_t *pair_
     note_launch();
 }
 
-void launch_deposit_adjoint(const Plan &p, const double *rtp, int64_t ngal, const double *Dbar, int64_t b0,
-                            int64_t nbc, double *dw, cudaStream_t st) {
+void launch_deposit_adjoint(const Plan &p, const double *rtp, int64_t ngal, const double *Dbar, int64_t sb, int64_t sp,
+                            int64_t b0, int64_t nbc, double *dw, cudaStream_t st) {
     if (ngal <= 0) return;
     k_deposit_adjoint<<<(unsigned)((ngal + 255) / 256), 256, 0, st>>>(
         rtp, ngal, p.nside, p.npix, p.rmin, p.rmax, (double)p.pieces / (p.rmax - p.rmin), p.pieces, p.degree,
-        p.nbasis, Dbar, b0, nbc, dw, p.d_err);
+        p.nbasis, Dbar, sb, sp, b0, nbc, dw, p.d_err);
     note_launch();
 }
 

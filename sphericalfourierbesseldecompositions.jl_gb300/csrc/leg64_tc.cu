@@ -31,153 +31,18 @@
 //
 // Measured at 128 columns, nside 128, lmax 82 (one refinement pass of a 64-map
 // adjoint): analysis 800 -> 33 us; see the per-kernel table in the design notes.
-#include <cuda_bf16.h>
-
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
 
-#include "sfb_internal.h"
-#include "tc_common.cuh"
+#include "digit64.cuh"
 
 namespace sfb {
 namespace t64 {
 
-using namespace tc;
-
-constexpr int ND = 7;                                  // digits, and levels kept
-constexpr int KC = 16;                                 // K per chunk (one MMA K step)
-constexpr int MTILE = 128;                             // data columns per CTA
-constexpr int NT = 32;                                 // table rows per CTA
-constexpr int SBK = 16;                                // chunks per exact K block (256 values)
-constexpr int NPROD = 256;
-constexpr int NTH = NPROD + 32;
-constexpr uint32_t PLANE_A = MTILE * KC * 2;
-constexpr int NSTAGE = 3;
-constexpr uint32_t STAGE_BYTES = ND * (PLANE_A + NT * KC * 2);
-constexpr uint32_t TMEM_COLS = 256;                    // 7 x 32 levels
-constexpr size_t SMEM = NSTAGE * (size_t)STAGE_BYTES + 256;
-
 __device__ __forceinline__ int rows_of(int m, int par, int lmax) {
     return (m + par <= lmax) ? (lmax - m - par) / 2 + 1 : 0;
 }
-__host__ __device__ __forceinline__ int ls_of(int n, int tile) {      // padded table rows of a tile
-    const int left = n - tile * NT;
-    return left >= NT ? NT : (left + 15) & ~15;
-}
-__device__ __forceinline__ uint32_t core_off(int row, int k) {
-    return (uint32_t)((((row >> 3) * (KC / 8) + (k >> 3)) << 7) + ((row & 7) << 4) + ((k & 7) << 1));
-}
-
-__device__ __forceinline__ void tmem_ld4(uint32_t taddr, float (&v)[4]) {
-    uint32_t r[4];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(taddr));
-#pragma unroll
-    for (int i = 0; i < 4; ++i) v[i] = __uint_as_float(r[i]);
-}
-
-// x on the unit 2^(emax - 1077): a 55-bit integer plus sign, rounded to nearest
-// (emax: exponent field of the column's largest magnitude, |x| < 2^(emax - 1022))
-__device__ __forceinline__ int64_t fixed55(double x, int emax) {
-    const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
-    int e = (int)(hi >> 20) & 0x7ff;
-    uint64_t mant = ((uint64_t)((hi & 0xfffffu) | (e ? 0x100000u : 0u)) << 32) | lo;
-    e = max(e, 1);
-    const int s = min(emax - e, 63);
-    const int64_t q = (int64_t)((((mant << 3) >> s) + 1) >> 1);
-    return (int32_t)hi < 0 ? -q : q;
-}
-
-// The digits of two integers as bf16x2 words, most significant first.  With 128 added to the six lower
-// digits the bytes of the sum are the digits plus 128; a byte becomes a float through the mantissa of 2^23.
-__device__ __forceinline__ void digits2(int64_t q0, int64_t q1, uint32_t (&w)[ND]) {
-    constexpr int64_t BIAS = 0x0000808080808080LL;
-    q0 += BIAS;
-    q1 += BIAS;
-    auto top = [](int64_t q) { return __int_as_float(0x4B400000 + (int)(q >> 48)) - 12582912.0f; };
-    auto dig = [](int64_t q, int s) {
-        const uint32_t half = s >= 4 ? (uint32_t)((uint64_t)q >> 32) : (uint32_t)q;
-        return __uint_as_float(__byte_perm(half, 0x4B000000u, 0x7650u | (uint32_t)(s & 3))) - 8388736.0f;
-    };
-    w[0] = bf16x2(top(q0), top(q1));
-#pragma unroll
-    for (int s = 5; s >= 0; --s) w[6 - s] = bf16x2(dig(q0, s), dig(q1, s));
-}
-
-// sum_v L_v 2^(-8 v), times 2^(S + 40), rounded to FP64 (integer operations: the FP64 pipe would take 16
-// cycles a warp for each one)
-__device__ __forceinline__ double join_levels(const float (&L)[ND], int S) {
-    auto i = [](float v) { return __float2int_rn(v); };
-    auto wide = [](int a, int b, int64_t c) { return (int64_t)a * b + c; };
-    const int64_t H = wide(i(L[0]), 1 << 24, wide(i(L[1]), 1 << 16, wide(i(L[2]), 1 << 8, (int64_t)i(L[3]))));
-    const int64_t W = wide(i(L[4]), 1 << 16, wide(i(L[5]), 1 << 8, (int64_t)(i(L[6]) + 128)));
-    const int64_t T = (H << 16) + (W >> 8);
-    const uint32_t sign = (uint32_t)((uint64_t)T >> 32) & 0x80000000u;
-    const uint64_t a = T < 0 ? (uint64_t)(-T) : (uint64_t)T;
-    const int lz = __clzll((long long)a);
-    const uint64_t frac = (((a << lz) >> 1) + 512u) >> 10;            // 2^52 <= frac <= 2^53
-    const int ef = 11 - lz + S + 52 + 1023;                            // exponent field of frac 2^(11 - lz + S)
-    if (a == 0) return 0.0;
-    if (ef < 1 || ef > 2045) return ldexp(sign ? -(double)a : (double)a, S);
-    const uint32_t hi = (uint32_t)(frac >> 32) + ((uint32_t)(ef - 1) << 20);
-    return __hiloint2double((int)(hi | sign), (int)(uint32_t)frac);
-}
-
-struct Smem {
-    unsigned char *base;
-    uint64_t *full_a, *full_b, *empty, *done;
-    uint32_t *slot;
-    int *bad;
-    __device__ __forceinline__ unsigned char *stage(int s) const { return base + s * STAGE_BYTES; }
-};
-
-__device__ __forceinline__ uint32_t setup(Smem &c, unsigned char *base) {
-    c.base = base;
-    c.full_a = reinterpret_cast<uint64_t *>(base + NSTAGE * STAGE_BYTES);
-    c.full_b = c.full_a + NSTAGE;
-    c.empty = c.full_b + NSTAGE;
-    c.done = c.empty + NSTAGE;
-    c.slot = reinterpret_cast<uint32_t *>(c.done + 1);
-    c.bad = reinterpret_cast<int *>(c.slot + 1);
-    if ((threadIdx.x >> 5) == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(c.slot)),
-                     "r"(TMEM_COLS)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    if (threadIdx.x == 0) {
-        for (int i = 0; i < NSTAGE; ++i) {
-            mbar_init(&c.full_a[i], NPROD / 32);
-            mbar_init(&c.full_b[i], 1);
-            mbar_init(&c.empty[i], 1);
-        }
-        mbar_init(c.done, 1);
-        *c.bad = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    fence_before();
-    __syncthreads();
-    fence_after();
-    return *c.slot;
-}
-
-// the products of one chunk: data digit a with the table digits 0..6-a, level a + b
-__device__ __forceinline__ void issue(uint32_t tmem, uint32_t sa, uint32_t sb, int LS, bool first) {
-    const uint32_t sbo = (KC / 8) * 128;
-    const uint32_t planeB = (uint32_t)LS * KC * 2;
-    const int per = 256 / LS;                             // table digits one MMA can take
-    for (int a = 0; a < ND; ++a) {
-        const uint64_t ad = smem_desc(sa + a * PLANE_A, 128, sbo);
-        for (int b = 0; b < ND - a; b += per) {
-            const int nb = min(per, ND - a - b);
-            mma_bf16(tmem + (uint32_t)(LS * (a + b)), ad, smem_desc(sb + b * planeB, 128, sbo),
-                     idesc_bf16(MTILE, LS * nb), (first && a == 0) ? 0u : 1u);
-        }
-    }
-}
-
 // One CTA: data columns [128 blockIdx.x, +128) x table rows of one tile of block z = (m, parity).
 // LMROWS: the data rows are coefficients l = m + parity + 2 k (synthesis, Gram); else rings k (analysis).
 // Tiles blockIdx.y < ny0 use task 0, the others task 1 (the Gram update and the aliased rings' synthesis of
@@ -228,7 +93,6 @@ __global__ void __launch_bounds__(NTH, 2) k_leg64(const double *__restrict__ dat
     const int LS = ls_of(N, tile);
     const int nKtab = ((LMROWS ? nrows : nrn) + KC - 1) / KC;    // chunks of the table's block
     const uint16_t *tab = t.dig + t.off[z] + (int64_t)tile * nKtab * ND * NT * KC + (int64_t)lo * ND * LS * KC;
-    const uint32_t bytesB = (uint32_t)ND * LS * KC * 2;
 
     // largest magnitude of every column (the high word orders the magnitudes by exponent)
     uint32_t mx = 0;
@@ -258,71 +122,12 @@ __global__ void __launch_bounds__(NTH, 2) k_leg64(const double *__restrict__ dat
         if (nch > 0) load(0, pre[0]);
         if (nch > 1) load(1, pre[1]);
     }
-    auto chunk = [&](int kc, double (&cur)[8]) -> bool {
-        const int s = kc % NSTAGE;
-        if (kc >= NSTAGE) {
-            if (*(volatile int *)cs.bad) return false;
-            if (!mbar_wait(&cs.empty[s], (uint32_t)((kc / NSTAGE - 1) & 1))) {
-                atomicExch(cs.bad, 1);
-                return false;
-            }
-        }
-        unsigned char *sa = cs.stage(s);
-        if (tid == 0) {
-            mbar_expect_tx(&cs.full_b[s], bytesB);
-            bulk_g2s(sa + ND * PLANE_A, tab + (int64_t)kc * ND * LS * KC, bytesB, &cs.full_b[s]);
-        }
-        uint32_t w[ND][4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            uint32_t v[ND];
-            digits2(fixed55(cur[2 * j], emax), fixed55(cur[2 * j + 1], emax), v);
-#pragma unroll
-            for (int q = 0; q < ND; ++q) w[q][j] = v[q];
-        }
-        const uint32_t off = core_off(c, 8 * kh);
-#pragma unroll
-        for (int q = 0; q < ND; ++q)
-            *reinterpret_cast<uint4 *>(sa + q * PLANE_A + off) = make_uint4(w[q][0], w[q][1], w[q][2], w[q][3]);
-        if (kc + 2 < nch) load(kc + 2, cur);
-        fence_proxy_async();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&cs.full_a[s]);
-        return true;
-    };
+    auto fix = [&](double v) { return fixed55(v, emax); };
 
     const int nsb = max(1, (nch + SBK - 1) / SBK);
     for (int sb = 0; sb < nsb; ++sb) {
         const int k0 = sb * SBK, k1 = min(nch, k0 + SBK);
-        if (!prod) {
-            if (lane == 0) {
-                int kc = k0;
-                for (; kc < k1; ++kc) {
-                    const int s = kc % NSTAGE;
-                    const uint32_t ph = (uint32_t)((kc / NSTAGE) & 1);
-                    if (*(volatile int *)cs.bad) break;
-                    if (!mbar_wait(&cs.full_a[s], ph) || !mbar_wait(&cs.full_b[s], ph)) {
-                        atomicExch(cs.bad, 1);
-                        break;
-                    }
-                    fence_after();
-                    const uint32_t sa = smem_u32(cs.stage(s));
-                    issue(tmem, sa, sa + ND * PLANE_A, LS, kc == k0);
-                    mma_commit(&cs.empty[s]);
-                }
-                if (kc < k1) atomicExch(cs.bad, 1);
-                mma_commit(cs.done);          // arrives once every MMA issued above has completed
-            }
-            __syncwarp();
-        } else {
-            for (int kc = k0; kc < k1; kc += 2) {         // k0 is even: chunk parity = buffer
-                if (!chunk(kc, pre[0])) break;
-                if (kc + 1 < k1 && !chunk(kc + 1, pre[1])) break;
-            }
-        }
-        bool ok = mbar_wait(cs.done, (uint32_t)(sb & 1));
-        fence_after();
-        ok = __syncthreads_and(ok) && !*(volatile int *)cs.bad;
+        const bool ok = run_block(cs, tmem, k0, k1, nch, sb, LS, tab, pre, load, fix);
         if (!ok) {
             if (tid == 0) atomicOr(err, ERR_TC_TIMEOUT);
             break;                                        // uniform: every thread saw the same value
@@ -339,9 +144,7 @@ __global__ void __launch_bounds__(NTH, 2) k_leg64(const double *__restrict__ dat
                 const int i0 = NT / 2 * hg + 4 * g;
                 if (i0 >= LS || tile * NT + i0 >= nwrite) break;              // warp-uniform
                 float v[ND][4];
-#pragma unroll
-                for (int q = 0; q < ND; ++q) tmem_ld4(tmem + lane_base + (uint32_t)(q * LS + i0), v[q]);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                load_levels(tmem + lane_base + (uint32_t)i0, LS, v);
                 if (cc < ncol) {
                     double old[4];
                     int ex[4];
@@ -377,7 +180,7 @@ __global__ void __launch_bounds__(NTH, 2) k_leg64(const double *__restrict__ dat
                             val = 0.0;
                         } else {
                             const float L[ND] = {v[0][i], v[1][i], v[2][i], v[3][i], v[4][i], v[5][i], v[6][i]};
-                            val = join_levels(L, lemax + ex[i] - 1076);
+                            val = round_int(join_int(L), lemax + ex[i] - 1076);
                         }
                         t.out[at(i)] = t.mode == 2 ? old[i] - val : (sb > 0 || t.mode == 1) ? old[i] + val : val;
                     }
@@ -388,10 +191,7 @@ __global__ void __launch_bounds__(NTH, 2) k_leg64(const double *__restrict__ dat
         __syncthreads();                                      // TMEM is read before the next block's MMAs
         fence_after();
     }
-    fence_before();
-    __syncthreads();
-    if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
+    release(tmem);
 }
 
 // ---- tables ---------------------------------------------------------------------------------------------------

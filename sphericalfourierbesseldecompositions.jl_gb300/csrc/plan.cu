@@ -549,8 +549,10 @@ int reference_alm(sfb_plan *h, const double *ref, int64_t nref, double *ralm, cu
 }
 
 // Transpose of sht_analysis in FP64 (adjoint.cu): abar [lmsize][2 nm] on the device becomes b = w E abar;
-// maps_out [nm][npix] FP64 receives S sum_j (I - A S)^j b.
-int sht_analysis_adjoint(sfb_plan *h, double *abar, int64_t nm, double *maps_out, cudaStream_t st) {
+// maps_out [nm][npix] FP64 receives S sum_j (I - A S)^j b.  With pix_ld the maps may come pixel-major instead:
+// map b, pixel x at pix_out[x pix_ld + b] (float or double); *pixmajor says whether they did.
+int sht_analysis_adjoint(sfb_plan *h, double *abar, int64_t nm, double *maps_out, cudaStream_t st,
+                         void *pix_out = nullptr, int64_t pix_ld = 0, bool pix_f32 = false, bool *pixmajor = nullptr) {
     Plan &p = h->p;
     const int32_t prec = p.precision;
     p.precision = SFB_FP64;
@@ -594,7 +596,9 @@ int sht_analysis_adjoint(sfb_plan *h, double *abar, int64_t nm, double *maps_out
         x = p.alm.ptr;
     }
     launch_leg_synthesis(p, x, ncol, p.gbuf.ptr, st);
-    launch_ring_synthesis(p, p.gbuf.ptr, nm, maps_out, st);
+    const bool pm = pix_out && nm > 4 && launch_ring_synthesis64(p, p.gbuf.ptr, nm, pix_out, pix_ld, true, pix_f32, st);
+    if (pixmajor) *pixmajor = pm;
+    if (!pm) launch_ring_synthesis(p, p.gbuf.ptr, nm, maps_out, st);
     SFB_CUDA_TRY(cudaGetLastError());
     return SFB_OK;
 }
@@ -1074,7 +1078,7 @@ void sfb_plan_destroy(sfb_plan *h) {
                     p.d_dtw_off, p.d_dtimg, p.d_dtimg_off, p.d_gramts, p.d_gramts_off, p.d_gram64, p.d_gram_off, p.d_cls_rings, p.d_cls_off, p.d_aimg_off, p.aimg.ptr, p.d_lam, p.d_lam32, p.d_lamtc, p.d_lamtc_off, p.d_lamts, p.d_lamts_off, p.d_lamtc_live, p.d_dft_dead, p.d_lam_off, p.d_spl_off, p.d_spl_x, p.d_spl_y, p.d_spl_ypp,
                     p.d_pair_l, p.d_pair_n, p.d_out_pair, p.d_out_lm, p.d_coef, p.d_coefT, p.d_proj_tiles, p.d_err,
                     p.maps.ptr, p.fbuf.ptr, p.gbuf.ptr, p.rbuf.ptr, p.alm.ptr, p.scratch.ptr, p.scratch2.ptr, p.dep.ptr, p.maps32.ptr,
-                    p.ref.ptr, p.rf.ptr, p.rg.ptr, p.rr.ptr, p.ralm.ptr, p.almdf2.ptr, p.adf0.ptr, p.ecoef.ptr, p.erow.ptr, p.almdf.ptr, p.nzr64.ptr, p.t64_mem[0], p.t64_mem[1], p.t64_mem[2], h->d_pair_index, h->d_noff};
+                    p.ref.ptr, p.rf.ptr, p.rg.ptr, p.rr.ptr, p.ralm.ptr, p.almdf2.ptr, p.adf0.ptr, p.ecoef.ptr, p.erow.ptr, p.almdf.ptr, p.nzr64.ptr, p.t64_mem[0], p.t64_mem[1], p.t64_mem[2], p.ring64_mem[0], p.ring64_mem[1], p.ring64.ptr, h->d_pair_index, h->d_noff};
     for (void *q : ptrs)
         if (q) cudaFree(q);
     if (h->aux) sfb_plan_destroy(h->aux);
@@ -1370,8 +1374,10 @@ int sfb_cat2amln_vjp(sfb_plan *h, const double *rtp, int64_t ngal, double nbar, 
     for (int64_t b0 = 0; b0 < p.nbasis; b0 += nbc) {
         const int64_t nb = std::min(nbc, p.nbasis - b0);
         launch_proj_adjoint(p, d_ab, h->d_pair_index, h->d_noff, b0, nb, scale, d_A, st);
-        SFB_TRY(sht_analysis_adjoint(h, d_A, nb, p.maps.ptr, st));
-        launch_deposit_adjoint(p, d_rtp, ngal, p.maps.ptr, b0, nb, d_dw, st);
+        // pixel-major: a galaxy reads the basis functions of its piece from one place
+        bool pm = false;
+        SFB_TRY(sht_analysis_adjoint(h, d_A, nb, p.maps.ptr, st, p.maps.ptr, nb, false, &pm));
+        launch_deposit_adjoint(p, d_rtp, ngal, p.maps.ptr, pm ? 1 : p.npix, pm ? nb : 1, b0, nb, d_dw, st);
     }
     int err = 0;
     SFB_CUDA_TRY(cudaMemcpyAsync(&err, p.d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -1434,10 +1440,16 @@ static int field2anlm_vjp_impl(sfb_plan *h, const double *abar, int64_t nr, doub
                                        nsc * sizeof(double), p.npairs, cudaMemcpyDeviceToDevice, st));
         // Abar_s[lm] = sum_n g_nl(r_s) r_s^2 dr abar_nlm (the transpose of the radial sum)
         launch_shell_alm_g(p, h->d_pair_index, h->d_noff, p.scratch2.ptr, nsc, d_ab, d_A, 2 * nsc, st);
-        SFB_TRY(sht_analysis_adjoint(h, d_A, nsc, p.maps.ptr, st));
         // shells s0 .. s0+nsc of df: (ir, p) at ir + nr p (resident) or ir - s0 + nsc p (staging)
         const int64_t ld = resident ? nr : nsc, off = resident ? s0 : 0;
-        if (dtype == SFB_F32)
+        const bool f32 = dtype == SFB_F32;
+        bool pm = false;
+        SFB_TRY(sht_analysis_adjoint(h, d_A, nsc, p.maps.ptr, st,
+                                     f32 ? (void *)(reinterpret_cast<float *>(d_f) + off) : (void *)(d_f + off), ld, f32,
+                                     &pm));
+        if (pm) {
+            // already in place
+        } else if (f32)
             launch_transpose_ld(p.maps.ptr, p.npix, nsc, p.npix, reinterpret_cast<float *>(d_f) + off, ld, st);
         else
             launch_transpose_ld(p.maps.ptr, p.npix, nsc, p.npix, d_f + off, ld, st);
@@ -1568,9 +1580,11 @@ static int sfb_anlm2field_impl(sfb_plan *h, const double *anlm, int64_t nr, doub
                                        nsc * sizeof(double), p.npairs, cudaMemcpyDeviceToDevice, st));
         launch_shell_alm_g(p, h->d_pair_index, h->d_noff, p.scratch2.ptr, nsc, d_a, p.alm.ptr, 2 * nsc, st);
         launch_leg_synthesis(p, p.alm.ptr, 2 * nsc, p.gbuf.ptr, st);
-        launch_ring_synthesis(p, p.gbuf.ptr, nsc, p.maps.ptr, st);
-        // f[s0+s + nr p] = maps[s][p]
-        launch_transpose_ld(p.maps.ptr, p.npix, nsc, p.npix, d_f + s0, nr, st);
+        // f[s0+s + nr p], written so by the tensor-core transform; else transposed from maps[s][p]
+        if (!(nsc > 4 && launch_ring_synthesis64(p, p.gbuf.ptr, nsc, d_f + s0, nr, true, false, st))) {
+            launch_ring_synthesis(p, p.gbuf.ptr, nsc, p.maps.ptr, st);
+            launch_transpose_ld(p.maps.ptr, p.npix, nsc, p.npix, d_f + s0, nr, st);
+        }
     }
     SFB_CUDA_TRY(cudaGetLastError());
     SFB_CUDA_TRY(cudaMemcpyAsync(f_out, d_f, (size_t)nr * p.npix * sizeof(double), cudaMemcpyDeviceToHost, st));

@@ -396,14 +396,19 @@ static void ring_analysis_t(const Plan &p, const TI *maps, int64_t nmaps, T *F, 
     }
 }
 
-void launch_ring_analysis(const Plan &p, const double *maps, int64_t nmaps, double *F, cudaStream_t st, int *nzr) {
+// More than four FP64 maps go through the tensor cores (a row tile of them takes 64 maps; four maps or fewer
+// are the reference maps of the mixed transform and small map2alm batches, which the FFT does sooner).
+constexpr int64_t RING64_MIN = 5;
+
+void launch_ring_analysis(Plan &p, const double *maps, int64_t nmaps, double *F, cudaStream_t st, int *nzr) {
     if (p.precision == SFB_MIXED)
         ring_analysis_t<float, float, float2>(p, (const float *)maps, nmaps, (float *)F, p.d_twtab32, p.d_wphase32, st);
-    else
+    else if (nmaps < RING64_MIN || !launch_ring_analysis64(p, maps, nmaps, F, st, nzr))
         ring_analysis_t<double, double, double2>(p, maps, nmaps, F, p.d_twtab, p.d_wphase, st, nzr);
 }
 
-void launch_ring_synthesis(const Plan &p, const double *G, int64_t nmaps, double *maps, cudaStream_t st) {
+void launch_ring_synthesis(Plan &p, const double *G, int64_t nmaps, double *maps, cudaStream_t st) {
+    if (nmaps >= RING64_MIN && launch_ring_synthesis64(p, G, nmaps, maps, p.npix, false, false, st)) return;
     const int ns = (int)p.nside;
     const bool pow2 = (ns & (ns - 1)) == 0;
     struct Group { int r0, nr; size_t n; bool two; } groups[2] = {

@@ -187,6 +187,14 @@ struct Plan {
     Task64 t64[3];
     void *t64_mem[3] = {};
     int tc64_state = 0;
+    // FP64 ring transforms on the tensor cores (ring64_tc.cu), [0] analysis, [1] synthesis: digit tables
+    // (state as tc64_state), integers of the folded rings per map (ring64_row values a row)
+    int ring64_state[2] = {0, 0}, ring64_ew = 0;
+    int64_t ring64_row = 0;
+    void *ring64_mem[2] = {};
+    uint16_t *ring64_dig[2] = {};
+    int64_t *ring64_off[2] = {}, *ring64_qoff[2] = {};
+    DevBuf<double> ring64;
     DevBuf<double> nzr64;           // FP64 many-column transform: first / last ring pair with data (2 ints)
     int64_t device_bytes = 0;
 };
@@ -258,9 +266,13 @@ void launch_wmix(const Plan &p, const int64_t *noff, const double *gtab, int64_t
 // Exclusive prefix sum of n int32 counters in place; tile_sums holds scan_tile_count(n) ints.
 int64_t scan_tile_count(int64_t n);
 void launch_exclusive_scan(int32_t *data, int64_t n, int32_t *tile_sums, cudaStream_t st);
-void launch_ring_analysis(const Plan &p, const double *maps, int64_t nmaps, double *F, cudaStream_t st,
-                          int *nzr = nullptr);
-void launch_ring_synthesis(const Plan &p, const double *G, int64_t nmaps, double *maps, cudaStream_t st);
+void launch_ring_analysis(Plan &p, const double *maps, int64_t nmaps, double *F, cudaStream_t st, int *nzr = nullptr);
+void launch_ring_synthesis(Plan &p, const double *G, int64_t nmaps, double *maps, cudaStream_t st);
+// The same for many FP64 maps on the tensor cores (ring64_tc.cu); false: nothing was launched (no tables or no
+// memory for them).  Synthesis: out[map ld + pixel], or pixel-major out[pixel ld + map] of double or float.
+bool launch_ring_analysis64(Plan &p, const double *maps, int64_t nmaps, double *F, cudaStream_t st, int *nzr);
+bool launch_ring_synthesis64(Plan &p, const double *G, int64_t nmaps, void *out, int64_t ld, bool pixmajor, bool f32,
+                             cudaStream_t st);
 // rlim: rings r < rlim (analysis: the sum; synthesis: the rings formed); -1 = all.
 // nzr (many columns): the analysis sums over the ring pairs [nzr[0], nzr[1]] only.
 void launch_leg_analysis(const Plan &p, const double *F, int64_t ncol, double *A, bool accumulate,
@@ -327,8 +339,9 @@ void launch_df_to_fp64(const float2 *a, int64_t n, double *out, cudaStream_t st)
 void launch_halve_m(double *alm, int64_t lmsize, int64_t ncol, double s, cudaStream_t st);
 void launch_proj_adjoint(const Plan &p, const double *abar, const int32_t *pair_index, const int64_t *noff, int64_t b0,
                          int64_t nbc, double s, double *Abar, cudaStream_t st);
-void launch_deposit_adjoint(const Plan &p, const double *rtp, int64_t ngal, const double *Dbar, int64_t b0,
-                            int64_t nbc, double *dw, cudaStream_t st);
+// Dbar: map b, pixel x at (b - b0) sb + x sp
+void launch_deposit_adjoint(const Plan &p, const double *rtp, int64_t ngal, const double *Dbar, int64_t sb, int64_t sp,
+                            int64_t b0, int64_t nbc, double *dw, cudaStream_t st);
 std::vector<int3> project_tiles(const std::vector<int32_t> &pair_index, int lmax, int nmax);
 void launch_transpose(const double *in, int64_t rows, int64_t cols, double *out, cudaStream_t st);
 void launch_check_finite(const double *x, int64_t n, int *err, cudaStream_t st);

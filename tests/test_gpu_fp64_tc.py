@@ -1,6 +1,6 @@
-"""The FP64 contractions on the tensor cores (many columns) at the edges of
-their tiles, against the oracle's map2alm and against the plan's FP64 units
-(SFBGPU_TC64=0).
+"""The FP64 contractions on the tensor cores (many columns, Legendre and ring
+transforms) at the edges of their tiles, against the oracle's map2alm and against the plan's FP64 units
+(SFBGPU_TC64=0, SFBGPU_RING64=0).
 
 Tolerance: a value is held to half a unit of 2^-55 of its column's (table
 row's) largest magnitude, and the level sums lose less than that again, so a
@@ -93,3 +93,57 @@ def test_nonfinite_and_zero_maps(bad, monkeypatch):
     ok = [i for i in range(9) if i != 3]
     assert rel_err(got[ok], ref[ok]) < TOL
     assert not np.any(got[5])
+
+
+# rings from 4 pixels on (nside 2), an nside that is no power of two, n/4 at and next to multiples of the
+# 16-value chunk and the 32-value tile, more than 192 values (two exact blocks), 2 lmax above and below the
+# ring lengths, a partial and a whole tile of 64 maps and one map more
+@pytest.mark.parametrize("nside,lmax,nmaps", [(2, 3, 5), (2, 8, 5), (3, 4, 6), (5, 14, 9), (15, 30, 64), (16, 31, 65),
+                                              (17, 33, 7), (31, 64, 5), (32, 20, 33), (33, 62, 5), (64, 63, 5),
+                                              (192, 60, 5), (256, 127, 5)])
+def test_rings_vs_fft(nside, lmax, nmaps, monkeypatch):
+    f = _maps(nmaps, nside, 11)
+    f[1] = 0.0
+    f[2, : 6 * nside * nside] = 0.0                   # rings without data in some maps
+    f[3, 5 * nside * nside] += 1e6                    # a spike
+    y = np.random.default_rng(12).normal(size=(nmaps, (lmax + 1) * (lmax + 2) // 2, 2)) @ np.array([1.0, 1j])
+    y[1] = 0.0
+    a = _modes(lmax, nside)
+    got = map2alm(f, a, niter=0, radial="spline"), map2alm_adjoint(y, a, niter=0, radial="spline")
+    monkeypatch.setenv("SFBGPU_RING64", "0")
+    b = _modes(lmax, nside)
+    ref = map2alm(f, b, niter=0, radial="spline"), map2alm_adjoint(y, b, niter=0, radial="spline")
+    for g, r, what in zip(got, ref, ("analysis", "synthesis")):
+        for k in range(nmaps):                        # each map on its own scale
+            e = float(np.max(np.abs(g[k] - r[k])) / max(np.max(np.abs(r[k])), 1e-300))
+            record(f"fp64_ring_{what}_{nside}_{lmax}_map{k}", e)
+            assert e < TOL, (what, k, e)
+
+
+def test_pixel_major_fields_vs_fft(monkeypatch):
+    """anlm2field and the field gradient (FP64 and FP32) write their fields straight from the ring transform."""
+    rng = np.random.default_rng(13)
+    out = []
+    for v in ("1", "0"):
+        monkeypatch.setenv("SFBGPU_RING64", v)
+        a = sfbgpu.AnlmModes(0.03, 500.0, 1000.0, nside=16)
+        wm = sfbgpu.ConfigurationSpaceModes(a.rmin, a.rmax, 37, 16)
+        n = sfbgpu.getnlmsize(a)
+        c = np.random.default_rng(14).normal(size=(n, 2)) @ np.array([1.0, 1j])
+        out.append([sfbgpu.anlm2field(c, wm, a)] + [sfbgpu.cat2anlm.field2anlm_vjp(c, wm, a, dtype=d)
+                                                    for d in (np.float64, np.float32)])
+    for g, r in zip(*out):
+        assert g.shape == r.shape and g.dtype == r.dtype
+        assert rel_err(g, r) < (TOL if g.dtype == np.float64 else 1e-6)
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_rings_nonfinite(bad, monkeypatch):
+    f = _maps(6, 16, 15)
+    f[2, 40] = bad
+    y = np.ones((6, 25 * 26 // 2), complex)
+    y[4, 7] = bad
+    a = _modes(24, 16)
+    g = map2alm(f, a, radial="spline"), map2alm_adjoint(y, a, radial="spline")
+    assert not np.isfinite(g[0][2]).any() and np.isfinite(np.delete(g[0], 2, 0)).all()
+    assert not np.isfinite(g[1][4]).any() and np.isfinite(np.delete(g[1], 4, 0)).all()
