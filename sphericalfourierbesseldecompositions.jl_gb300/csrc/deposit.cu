@@ -361,69 +361,118 @@ __global__ void k_deposit_scatter_mixed(const double *__restrict__ wgt, int64_t 
     sorted[pos] = make_float4(x.x, x.y, w.hi, w.lo);
 }
 
-// Legendre moments sum_i w_i P_k(x_i), k <= deg, of the galaxies g0..g1-1 of one bin.
+// Legendre moments sum_i w_i P_k(x_i), k <= deg, of the galaxies g0..g1-1 of one bin, in FP64.  The
+// recurrence runs on the monic polynomials r_{k+1} = x r_k - k^2/(4k^2 - 1) r_{k-1}, weighted from the start
+// (three FP64 operations a degree and galaxy instead of four; the FP64 pipe bounds this), and each sum is
+// scaled by P_k's leading coefficient once.
+constexpr double monic_lead(int k) {
+    double c = 1.0;
+    for (int j = 1; j <= k; ++j) c *= (2.0 * j - 1.0) / j;
+    return c;
+}
+
 template <int MAXDEG>
 __device__ __forceinline__ void bin_moments(const double2 *__restrict__ sorted, int64_t g0, int64_t g1, int deg,
                                             double (&acc)[MAXDEG + 1]) {
 #pragma unroll
     for (int k = 0; k <= MAXDEG; ++k) acc[k] = 0.0;
+    double2 nxt = g0 < g1 ? sorted[g0] : make_double2(0.0, 0.0);
     for (int64_t g = g0; g < g1; ++g) {
-        const double2 xw = sorted[g];
-        const double x = xw.x, w = xw.y;
-        double p0 = 1.0, p1 = x;
-        acc[0] += w;
-        if (MAXDEG >= 1) acc[1] += w * x;
+        const double2 xw = nxt;
+        if (g + 1 < g1) nxt = sorted[g + 1];
+        const double x = xw.x;
+        double p0 = xw.y, p1 = xw.y * x;
+        acc[0] += p0;
+        if (MAXDEG >= 1) acc[1] += p1;
 #pragma unroll
         for (int k = 1; k < MAXDEG; ++k) {
             if (k >= deg) break;
-            // (k+1) P_{k+1} = (2k+1) x P_k - k P_{k-1}; coefficients fold to constants
-            const double p2 = ((double)(2 * k + 1) / (k + 1)) * x * p1 - ((double)k / (k + 1)) * p0;
-            acc[k + 1] += w * p2;
+            const double p2 = fma(x, p1, -((double)(k * k) / (4.0 * k * k - 1.0)) * p0);
+            acc[k + 1] += p2;
             p0 = p1;
             p1 = p2;
         }
     }
+#pragma unroll
+    for (int k = 2; k <= MAXDEG; ++k) acc[k] *= monic_lead(k);
 }
 
 __device__ __forceinline__ int64_t basis_of(int slot, int k, int pieces, int deg, int64_t nbasis) {
     return slot < pieces ? (int64_t)slot * (deg + 1) + k : nbasis - 2 + (slot - pieces);
 }
 
-// One thread per (slot, pixel): Legendre moments of its galaxies, minus
-// mu_b ref[pix] when ref is given.
-template <int MAXDEG, typename TM>
-__global__ void k_deposit_moments(const int32_t *__restrict__ offset, const double2 *__restrict__ sorted,
-                                  int64_t npix, int pieces, int deg, int64_t nbasis, const double *__restrict__ ref,
-                                  const double *__restrict__ mu, TM *__restrict__ maps) {
-    const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t nkeys = (int64_t)(pieces + 2) * npix;
-    if (idx >= nkeys) return;
-    const int slot = (int)(idx / npix);
-    const int64_t pix = idx - (int64_t)slot * npix;
-    const int64_t g0 = offset[idx];
-    const int64_t g1 = offset[idx + 1];         // offset[nkeys] = number of keyed galaxies
-    const double rv = ref ? ref[pix] : 0.0;
-    if (slot >= pieces) {       // constant extrapolation maps (r < rmin, r > rmax)
-        double s = 0.0;
-        for (int64_t g = g0; g < g1; ++g) s += sorted[g].y;
-        const int64_t b = nbasis - 2 + (slot - pieces);
-        if (ref) s -= mu[b] * rv;
-        maps[b * npix + pix] = (TM)s;
-        return;
-    }
-    double acc[MAXDEG + 1];
-    bin_moments<MAXDEG>(sorted, g0, g1, deg, acc);
-    const int64_t b0 = (int64_t)slot * (deg + 1);
-    TM *base = maps + b0 * npix + pix;
-#pragma unroll
-    for (int k = 0; k <= MAXDEG; ++k) {
-        if (k <= deg) {
-            const double v = ref ? acc[k] - mu[b0 + k] * rv : acc[k];
-            base[(int64_t)k * npix] = (TM)v;
+// Order the block's 128 bins by decreasing galaxy count (a counting sort in shared memory), so the threads of
+// a warp walk bins of nearly equal length: the position of this thread's bin in that order.
+__device__ __forceinline__ int rank_bins(int cnt, int *hist) {
+    const int t = threadIdx.x;
+    if (t < 64) hist[t] = 0;
+    __syncthreads();
+    const int key = 63 - min(cnt, 63);                 // longest bins first
+    atomicAdd(&hist[key], 1);
+    __syncthreads();
+    if (t < 32) {
+        const int h0 = hist[2 * t], h1 = hist[2 * t + 1];
+        int sc = h0 + h1;
+        for (int off = 1; off < 32; off <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, sc, off);
+            if (t >= off) sc += v;
         }
+        const int base = sc - (h0 + h1);
+        hist[2 * t] = base;
+        hist[2 * t + 1] = base + h0;
     }
+    __syncthreads();
+    return atomicAdd(&hist[key], 1);
 }
 
+// FP64: one thread per (slot, pixel) bin, the bins handed out by decreasing count, the results written with
+// consecutive threads on consecutive pixels.  Bound: the FP64 pipe, 72 operations a galaxy at degree 24 (with
+// four operations a degree and unsorted bins 274 us for 6e5 galaxies at nside 128; 151 so).
+template <int MAXDEG>
+__global__ void __launch_bounds__(128) k_deposit_moments(const int32_t *__restrict__ offset,
+                                                         const double2 *__restrict__ sorted, int64_t npix, int pieces,
+                                                         int deg, int64_t nbasis, double *__restrict__ maps) {
+    extern __shared__ double out_s[];                  // [deg + 1][128]
+    __shared__ int hist[64];
+    __shared__ int perm[128];
+    const int t = threadIdx.x;
+    const int64_t nkeys = (int64_t)(pieces + 2) * npix;
+    const int64_t bt = (int64_t)blockIdx.x * 128 + t;
+    const int cnt = bt < nkeys ? offset[bt + 1] - offset[bt] : 0;        // offset[nkeys] = number of keyed galaxies
+    const int slot = bt < nkeys ? (int)(bt / npix) : 0;
+    const int64_t pix = bt - (int64_t)slot * npix;
+    const int64_t b0 = slot < pieces ? (int64_t)slot * (deg + 1) : nbasis - 2 + (slot - pieces);
+    const int nk = slot < pieces ? deg + 1 : 1;        // one constant map for r < rmin, one for r > rmax
+    double *base = maps + b0 * npix + pix;
+    if (!__syncthreads_or(cnt != 0)) {
+        if (bt < nkeys)
+            for (int k = 0; k < nk; ++k) base[(int64_t)k * npix] = 0.0;
+        return;
+    }
+    perm[rank_bins(cnt, hist)] = t;
+    __syncthreads();
+    {
+        const int q = perm[t];
+        const int64_t b = (int64_t)blockIdx.x * 128 + q;
+        if (b < nkeys) {
+            const int64_t g0 = offset[b], g1 = offset[b + 1];
+            if (b / npix >= pieces) {
+                double s = 0.0;
+                for (int64_t g = g0; g < g1; ++g) s += sorted[g].y;
+                out_s[q] = s;
+            } else {
+                double acc[MAXDEG + 1];
+                bin_moments<MAXDEG>(sorted, g0, g1, deg, acc);
+#pragma unroll
+                for (int k = 0; k <= MAXDEG; ++k)
+                    if (k <= deg) out_s[k * 128 + q] = acc[k];
+            }
+        }
+    }
+    __syncthreads();
+    if (bt < nkeys)
+        for (int k = 0; k < nk; ++k) base[(int64_t)k * npix] = out_s[k * 128 + t];
+}
 
 // One step of the basis recurrence on q_k = w P_k(x):
 // (k+1) q_{k+1} = (2k+1) x q_k - k q_{k-1}, the ratios as double-float
@@ -559,24 +608,7 @@ __global__ void __launch_bounds__(128) k_deposit_moments_bal(const int32_t *__re
         for (int k = 0; k <= deg; ++k) z[(int64_t)k * npix] = make_float2(0.f, 0.f);
         return;
     }
-    if (t < 64) hist[t] = 0;
-    __syncthreads();
-    const int key = 63 - min(cnt, 63);                 // longest bins first
-    atomicAdd(&hist[key], 1);
-    __syncthreads();
-    if (t < 32) {
-        const int h0 = hist[2 * t], h1 = hist[2 * t + 1];
-        int sc = h0 + h1;
-        for (int off = 1; off < 32; off <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, sc, off);
-            if (t >= off) sc += v;
-        }
-        const int base = sc - (h0 + h1);
-        hist[2 * t] = base;
-        hist[2 * t + 1] = base + h0;
-    }
-    __syncthreads();
-    perm[atomicAdd(&hist[key], 1)] = t;
+    perm[rank_bins(cnt, hist)] = t;
     __syncthreads();
     const int q = perm[t];
     const int64_t b = B0 + q;
@@ -717,24 +749,7 @@ __global__ void __launch_bounds__(128, 8) k_deposit_moments_sm(const int32_t *__
         for (int k = 0; k <= deg; ++k) z[(int64_t)k * npix] = make_float2(0.f, 0.f);
         return;
     }
-    if (t < 64) hist[t] = 0;
-    __syncthreads();
-    const int key = 63 - min(cnt, 63);                 // longest bins first
-    atomicAdd(&hist[key], 1);
-    __syncthreads();
-    if (t < 32) {
-        const int h0 = hist[2 * t], h1 = hist[2 * t + 1];
-        int sc = h0 + h1;
-        for (int off = 1; off < 32; off <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, sc, off);
-            if (t >= off) sc += v;
-        }
-        const int base = sc - (h0 + h1);
-        hist[2 * t] = base;
-        hist[2 * t + 1] = base + h0;
-    }
-    __syncthreads();
-    const int walker = atomicAdd(&hist[key], 1);       // the thread that walks this thread's bin
+    const int walker = rank_bins(cnt, hist);           // the thread that walks this thread's bin
     perm[walker] = t;
     __syncthreads();
     const uint32_t acc0 = (uint32_t)__cvta_generic_to_shared(acc_s);
@@ -884,9 +899,8 @@ __global__ void k_weight_map_mixed(const int32_t *__restrict__ offset, const flo
 
 // FP64 path: double (x, w); mixed: double-float pairs and the count map as cdf
 template <int MAXDEG>
-static void launch_moments(const Plan &p, const int32_t *counts, const void *sorted, const double *ref,
-                           const double *mu, const float2 *cdf, const float2 *mudf, double *maps, cudaStream_t st,
-                           const int *ring_live) {
+static void launch_moments(const Plan &p, const int32_t *counts, const void *sorted, const float2 *cdf,
+                           const float2 *mudf, double *maps, cudaStream_t st, const int *ring_live) {
     const int64_t nkeys = (int64_t)(p.pieces + 2) * p.npix;
     const unsigned blocks = (unsigned)((nkeys + 127) / 128);
     const float4 *s4 = static_cast<const float4 *>(sorted);
@@ -907,10 +921,12 @@ static void launch_moments(const Plan &p, const int32_t *counts, const void *sor
     } else if (p.precision == SFB_MIXED)
         k_deposit_moments_df<MAXDEG><<<blocks, 128, 0, st>>>(counts, s4, p.npix, p.pieces, p.degree, p.nbasis, cdf,
                                                              mudf, mf);
-    else
-        k_deposit_moments<MAXDEG, double><<<blocks, 128, 0, st>>>(counts, static_cast<const double2 *>(sorted),
-                                                                  p.npix, p.pieces, p.degree, p.nbasis, ref, mu,
-                                                                  maps);
+    else {
+        const size_t smem = (size_t)(p.degree + 1) * 128 * sizeof(double);
+        set_smem(k_deposit_moments<MAXDEG>, smem);
+        k_deposit_moments<MAXDEG><<<blocks, 128, smem, st>>>(counts, static_cast<const double2 *>(sorted), p.npix,
+                                                             p.pieces, p.degree, p.nbasis, maps);
+    }
     note_launch();
 }
 
@@ -1039,8 +1055,8 @@ int deposit_sorted(Plan &p, const double *rtp, const double *w, int64_t ngal, do
     // moments in FP64 (FP64 path) or double-float (mixed); stored in the transform's precision
     const bool skip_empty = split && ring_live && p.npix >= 128 && p.degree <= 31;   // the balanced kernel
     by_degree(p.degree, [&](auto D) {
-        launch_moments<decltype(D)::value>(p, counts, sorted, split ? ref : nullptr, mu, split ? cdf : nullptr, mudf,
-                                           maps, st, skip_empty ? live : nullptr);
+        launch_moments<decltype(D)::value>(p, counts, sorted, split ? cdf : nullptr, mudf, maps, st,
+                                           skip_empty ? live : nullptr);
     });
     if (skip_empty) *ring_live = live;
     SFB_CUDA_TRY(cudaGetLastError());
