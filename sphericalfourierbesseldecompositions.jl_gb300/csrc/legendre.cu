@@ -905,12 +905,12 @@ bool launch_gram_update_fp64(const Plan &p, const double *Acur, const double *A0
 }
 
 void launch_fold_residual(const Plan &p, const double *F, const double *G, int64_t ncol, double *R,
-                          cudaStream_t st, int *Ecol, int rlim) {
+                          cudaStream_t st, int *Ecol, int rlim, bool ecol_preset) {
     const int64_t ncplx = ncol / 2;
     if (rlim < 0 || rlim > p.nrn) rlim = (int)p.nrn;
     if (p.precision == SFB_MIXED && ncplx > 4) {
         // 0x80 bytes: every exponent word starts at -2139062144, below any scale exponent
-        if (Ecol) cudaMemsetAsync(Ecol, 0x80, (size_t)2 * (p.lmax + 1) * ncol * sizeof(int), st);
+        if (Ecol && !ecol_preset) cudaMemsetAsync(Ecol, 0x80, (size_t)2 * (p.lmax + 1) * ncol * sizeof(int), st);
         if (!F && rlim > 0 && rlim <= p.ral) {
             // aliased rings of the Gram refinement: residue buckets (shared memory within limits)
             constexpr int FC = 8;
@@ -919,8 +919,11 @@ void launch_fold_residual(const Plan &p, const double *F, const double *G, int64
             const bool mxreg = (p.lmax + 1) * FC <= 256 * FOLD_MXQ;
             const size_t smem = ((size_t)nbk + (mxreg ? 1 : 2) * (size_t)(p.lmax + 1)) * FC * sizeof(float2);
             if (smem <= 200 * 1024) {
-                const int rpb = 8;
-                dim3 grid((unsigned)((ncplx + FC - 1) / FC), 2, (unsigned)((rlim + rpb - 1) / rpb));
+                // rings per block: eight, whose loads follow one another, or fewer where that would leave SMs
+                // without a block (nside 32, 53 maps: 13 us at eight, 5 at one)
+                const int64_t gx = (ncplx + FC - 1) / FC;
+                const int rpb = (int)std::max<int64_t>(1, std::min<int64_t>(8, 2 * gx * rlim / 608));
+                dim3 grid((unsigned)gx, 2, (unsigned)((rlim + rpb - 1) / rpb));
                 const double w = 4.0 * M_PI / (double)p.npix;
                 if (mxreg) {
                     set_smem(k_fold_alias<FC, true>, smem);

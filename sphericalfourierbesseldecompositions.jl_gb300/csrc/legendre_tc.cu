@@ -424,31 +424,41 @@ __global__ void __launch_bounds__(NTH, 2) k_leg_analysis_tc(const __nv_bfloat16 
 // Synthesis: grid (column tiles, ring tiles of NT <= NMAX, blocks z); warps
 // 0-7 produce, warp 8 issues the MMAs.
 //
-// Update mode (Adfnew != nullptr): the table holds D = M - I, M the Gram
-// matrices of the alias-free rings; "rings" r are output rows li (nrn = rows of
-// the largest block), and the epilogue writes, instead of G,
+// Update mode (tiles blockIdx.y < ny0, table gram): the table holds D = M - I, M
+// the Gram matrices of the alias-free rings; "rings" r are output rows li (nrn =
+// rows of the largest block), and the epilogue writes, instead of G,
 //   Anew[l(r)] = A0[l(r)] - sum_li D[r][li] Acur[l(li)]
-// (= Acur + (A0 - M Acur)) in double-float and, when Anew is given, in FP64.
-// |D| is the polar rings' share of the quadrature, so the product's FP32
-// accumulation error is that share of |Acur|, not all of it.
-__global__ void __launch_bounds__(NTH, 2) k_leg_synthesis_tc(const __nv_bfloat16 *__restrict__ lamts,
-                                                             const int64_t *__restrict__ lamts_off, int lmax, int nrn,
-                                                             int NT, const float2 *__restrict__ Adf, int64_t ncol,
-                                                             float *__restrict__ G, const double *__restrict__ Acur,
-                                                             const float2 *__restrict__ A0, double *__restrict__ Anew,
+// (= Acur + (A0 - M Acur)) in double-float.  |D| is the polar rings' share of the
+// quadrature, so the product's FP32 accumulation error is that share of |Acur|,
+// not all of it.  A refinement pass runs both modes in one launch (both read the
+// current coefficients): the short tiles of one fill the tail of the other
+// (separate launches: six per call, 62 us at nside 32, 1100 at nside 256; joined:
+// three, 34 and 1023).
+struct SynTable {
+    const __nv_bfloat16 *tab;
+    const int64_t *off;
+    const int2 *live;
+    int nrn, NT;
+};
+__global__ void __launch_bounds__(NTH, 2) k_leg_synthesis_tc(SynTable gram, SynTable syn, int ny0, int lmax,
+                                                             const float2 *__restrict__ Adf, int64_t ncol,
+                                                             float *__restrict__ G, const float2 *__restrict__ A0,
                                                              float2 *__restrict__ Adfnew, const int *__restrict__ Ein,
-                                                             int *__restrict__ Eout, const int2 *__restrict__ live,
-                                                             int *err) {
+                                                             int *__restrict__ Eout, int *err) {
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ float red[2][MTILE];
     const int z = blockIdx.z;
     const int m = z >> 1, par = z & 1;
     const int nrows = rows_of(m, par, lmax);
-    const int nt = blockIdx.y;
+    const bool upd = (int)blockIdx.y < ny0;
+    const int nt = upd ? blockIdx.y : blockIdx.y - ny0;
+    const __nv_bfloat16 *lamts = upd ? gram.tab : syn.tab;
+    const int64_t *lamts_off = upd ? gram.off : syn.off;
+    const int2 *live = upd ? gram.live : syn.live;
+    const int nrn = upd ? gram.nrn : syn.nrn, NT = upd ? gram.NT : syn.NT;
     const int r0 = nt * NT;
     const int64_t col0 = (int64_t)blockIdx.x * MTILE;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const bool upd = Adfnew != nullptr;
     if (upd && r0 >= nrows) return;          // no output row of this block in the tile
     float *Gz = upd ? nullptr : G + ((int64_t)(par * (lmax + 1) + m) * nrn) * ncol;
     // live: the row chunks [lv.x, lv.y] of this ring tile whose lambda slices are not all zero (the
@@ -592,7 +602,6 @@ __global__ void __launch_bounds__(NTH, 2) k_leg_synthesis_tc(const __nv_bfloat16
                     const float e = ((a0[i].x - (s - z2)) + (-hi - z2)) + (a0[i].y - lo);
                     const float nh = s + e, nl = e - (nh - s);
                     Adfnew[o] = make_float2(nh, nl);
-                    if (Anew) Anew[o] = (double)nh + (double)nl;
                     umx = fmaxf(umx, fabsf(nh));
                 }
             }
@@ -920,16 +929,22 @@ void launch_build_lamts(const Plan &p, const int *Es, cudaStream_t st) {
 }
 
 void launch_leg_synthesis_tc(const Plan &p, const float2 *Adf, int64_t ncol, float *G, cudaStream_t st, int rlim,
-                             const int *Ein) {
+                             const int *Ein, const float2 *A0, float2 *Adfnew, int *Eout) {
     const int NT = tc_synth_nt(p);
     if (rlim < 0 || rlim > p.nrn) rlim = (int)p.nrn;
+    const tc::SynTable syn{(const __nv_bfloat16 *)p.d_lamts, p.d_lamts_off, p.d_lamts_live, (int)p.nrn, NT};
+    tc::SynTable gram{};
+    int ny0 = 0;
+    if (Adfnew) {
+        gram = {(const __nv_bfloat16 *)p.d_gramts, p.d_gramts_off, nullptr, p.gram_rows, tc_synth_nt(p.gram_rows)};
+        ny0 = (p.gram_rows + gram.NT - 1) / gram.NT;
+    }
     set_smem(tc::k_leg_synthesis_tc, tc::LEG_SMEM);
     // ring tiles covering the first rlim rings (a tile's rings past rlim are computed as well)
-    dim3 grid((unsigned)((ncol + tc::MTILE - 1) / tc::MTILE), (unsigned)((rlim + NT - 1) / NT),
+    dim3 grid((unsigned)((ncol + tc::MTILE - 1) / tc::MTILE), (unsigned)(ny0 + (rlim + NT - 1) / NT),
               (unsigned)(2 * (p.lmax + 1)));
-    tc::k_leg_synthesis_tc<<<grid, tc::NTH, tc::LEG_SMEM, st>>>((const __nv_bfloat16 *)p.d_lamts, p.d_lamts_off,
-                                                               p.lmax, (int)p.nrn, NT, Adf, ncol, G, nullptr, nullptr,
-                                                               nullptr, nullptr, Ein, nullptr, p.d_lamts_live, p.d_err);
+    tc::k_leg_synthesis_tc<<<grid, tc::NTH, tc::LEG_SMEM, st>>>(gram, syn, ny0, p.lmax, Adf, ncol, G, A0, Adfnew, Ein,
+                                                               Eout, p.d_err);
     note_launch();
 }
 
@@ -946,18 +961,6 @@ void launch_df_to_fp64(const float2 *a, int64_t n, double *out, cudaStream_t st)
     if (n <= 0) return;
     const int64_t blocks = std::min<int64_t>((n + 255) / 256, 152 * 16);
     tc::k_df_to_fp64<<<(unsigned)blocks, 256, 0, st>>>(a, n, out);
-    note_launch();
-}
-
-void launch_gram_update(const Plan &p, const double *A, const float2 *Adf, const float2 *A0, int64_t ncol,
-                        double *Anew, float2 *Adfnew, cudaStream_t st, const int *Ein, int *Eout) {
-    const int NT = tc_synth_nt(p.gram_rows);
-    set_smem(tc::k_leg_synthesis_tc, tc::LEG_SMEM);
-    dim3 grid((unsigned)((ncol + tc::MTILE - 1) / tc::MTILE), (unsigned)((p.gram_rows + NT - 1) / NT),
-              (unsigned)(2 * (p.lmax + 1)));
-    tc::k_leg_synthesis_tc<<<grid, tc::NTH, tc::LEG_SMEM, st>>>((const __nv_bfloat16 *)p.d_gramts, p.d_gramts_off,
-                                                               p.lmax, p.gram_rows, NT, Adf, ncol, nullptr, A, A0,
-                                                               Anew, Adfnew, Ein, Eout, nullptr, p.d_err);
     note_launch();
 }
 

@@ -404,48 +404,52 @@ int sht_analysis(sfb_plan *h, const double *maps, int64_t nm, cudaStream_t st, b
         // Gram refinement: a <- a + (a0 - M a) - A_al(Fold(S_al a)) = a0 - D a - A_al(Fold(S_al a)),
         // M the Gram matrix of the alias-free rings (fold = identity there), D = M - I as the
         // tables store it, S_al / A_al the synthesis and analysis over the aliased rings r < ral.
-        // Each pass writes the other (A, Adf) buffer; the last one lands in the plan's.
+        // The first pass lands in adf0 (the a0 of every step); step it writes almdf or almdf2, the last one almdf.
         SFB_TRY(grow(p, p.almdf2, (size_t)p.lmsize * ncol));
         SFB_TRY(grow(p, p.adf0, (size_t)p.lmsize * ncol));
-        // column exponents of each (A, Adf) set, written by whichever kernel completes the set
+        // Column exponents of every coefficient set and fold residual, raised by whichever kernels write them:
+        // up to 17 arrays preset by one clear (0x80 bytes: below any scale exponent), reused after that.
         const int64_t nE = 2 * (p.lmax + 1) * ncol;
-        SFB_TRY(grow(p, p.ecoef, (size_t)nE + 1));
-        double *Ab[2] = {nullptr, nullptr};          // FP64 a_lm: formed once at the end (fp64_out)
-        float2 *Db[2] = {adf, reinterpret_cast<float2 *>(p.almdf2.ptr)};
-        int *Eb[2] = {reinterpret_cast<int *>(p.ecoef.ptr), reinterpret_cast<int *>(p.ecoef.ptr) + nE};
-        const float2 *a0 = reinterpret_cast<const float2 *>(p.adf0.ptr);
-        int cur = p.niter & 1;
-        // 0x80 bytes: every exponent word starts below any scale exponent (atomicMax)
-        SFB_CUDA_TRY(cudaMemsetAsync(Eb[cur], 0x80, (size_t)nE * sizeof(int), st));
+        const int nset = std::min(2 * p.niter + 1, 17);
+        SFB_TRY(grow(p, p.ecoef, (size_t)(nset * nE / 2 + 1)));
+        SFB_CUDA_TRY(cudaMemsetAsync(p.ecoef.ptr, 0x80, (size_t)(nset * nE) * sizeof(int), st));
+        int used = 0;
+        auto next_set = [&](int *&e) -> int {
+            e = reinterpret_cast<int *>(p.ecoef.ptr) + (used % nset) * nE;
+            if (used++ >= nset) SFB_CUDA_TRY(cudaMemsetAsync(e, 0x80, (size_t)nE * sizeof(int), st));
+            return SFB_OK;
+        };
+        float2 *a0 = reinterpret_cast<float2 *>(p.adf0.ptr), *cur = a0;
+        int *ecur = nullptr, *enxt = nullptr, *efold = nullptr;
+        SFB_TRY(next_set(ecur));
         {
-            Stage s(h, stage(SFB_STAGE_LEG_ANALYSIS), st);
-            launch_leg_analysis_tc(p, (const float2 *)fbuf.ptr, ncol, Ab[cur], Db[cur], ecol, false, st, false, -1,
-                                   Eb[cur], nzr);
+            Stage s(h, SFB_STAGE_LEG_ANALYSIS, st);
+            launch_leg_analysis_tc(p, (const float2 *)fbuf.ptr, ncol, nullptr, cur, ecol, false, st, false, -1, ecur,
+                                   nzr);
         }
-        SFB_CUDA_TRY(cudaMemcpyAsync(p.adf0.ptr, Db[cur], (size_t)p.lmsize * ncol * sizeof(float2),
-                                     cudaMemcpyDeviceToDevice, st));
         for (int it = 0; it < p.niter; ++it) {
-            const int nxt = cur ^ 1;
-            SFB_CUDA_TRY(cudaMemsetAsync(Eb[nxt], 0x80, (size_t)nE * sizeof(int), st));
+            float2 *nxt = reinterpret_cast<float2 *>((p.niter - 1 - it) & 1 ? p.almdf2.ptr : p.almdf.ptr);
+            SFB_TRY(next_set(enxt));
             {
-                Stage s(h, stage(SFB_STAGE_LEG_SYNTHESIS), st);
-                if (p.ral > 0) launch_leg_synthesis_tc(p, Db[cur], ncol, (float *)gbuf.ptr, st, p.ral, Eb[cur]);
+                Stage s(h, SFB_STAGE_LEG_SYNTHESIS, st);
                 // the update records the column exponents of its output; the aliased analysis raises
                 // them where it adds (its CTAs without live chunks leave the update's values)
-                launch_gram_update(p, Ab[cur], Db[cur], a0, ncol, Ab[nxt], Db[nxt], st, Eb[cur], Eb[nxt]);
+                launch_leg_synthesis_tc(p, cur, ncol, (float *)gbuf.ptr, st, p.ral, ecur, a0, nxt, enxt);
             }
             if (p.ral > 0) {
+                SFB_TRY(next_set(efold));
                 {
-                    Stage s(h, stage(SFB_STAGE_FOLD), st);
-                    launch_fold_residual(p, nullptr, gbuf.ptr, ncol, rbuf.ptr, st, ecol, p.ral);
+                    Stage s(h, SFB_STAGE_FOLD, st);
+                    launch_fold_residual(p, nullptr, gbuf.ptr, ncol, rbuf.ptr, st, efold, p.ral, true);
                 }
-                Stage s(h, stage(SFB_STAGE_LEG_ANALYSIS), st);
-                launch_leg_analysis_tc(p, (const float2 *)rbuf.ptr, ncol, Ab[nxt], Db[nxt], ecol, true, st, true,
-                                       p.ral, Eb[nxt]);
+                Stage s(h, SFB_STAGE_LEG_ANALYSIS, st);
+                launch_leg_analysis_tc(p, (const float2 *)rbuf.ptr, ncol, nullptr, nxt, efold, true, st, true, p.ral,
+                                       enxt);
             }
             cur = nxt;
+            ecur = enxt;
         }
-        if (fp64_out) launch_df_to_fp64(Db[cur], p.lmsize * ncol, alm.ptr, st);
+        if (fp64_out) launch_df_to_fp64(cur, p.lmsize * ncol, alm.ptr, st);
         SFB_CUDA_TRY(cudaGetLastError());
         return SFB_OK;
     }

@@ -289,8 +289,9 @@ void launch_leg_analysis64(const Plan &p, const double *F, int64_t ncol, double 
 void launch_leg_synthesis64(const Plan &p, const double *A, int64_t ncol, double *G, cudaStream_t st, int rlim,
                             const double *A0, double *Anew);
 // rlim: only rings r < rlim (-1: all); F == nullptr (Gram refinement): R = -w n cfold Fold(G)
+// Ecol: preset here below every exponent, unless ecol_preset (the caller did)
 void launch_fold_residual(const Plan &p, const double *F, const double *G, int64_t ncol, double *R, cudaStream_t st,
-                          int *Ecol = nullptr, int rlim = -1);
+                          int *Ecol = nullptr, int rlim = -1, bool ecol_preset = false);
 void launch_radial_coeffs(const Plan &p, const double *gl_x, const double *pq, int Q, double *coef,
                           cudaStream_t st);
 void launch_project_poly(const Plan &p, const double *A, int64_t ldA, double scale, int window_kind,
@@ -325,13 +326,11 @@ void launch_build_lamts(const Plan &p, const int *Es, cudaStream_t st);
 int build_live_ranges(Plan &p, cudaStream_t st);
 // rlim: ring tiles covering the first rlim rings only (-1: all)
 // Ein (optional): the column exponents of Adf per block z, as the analysis wrote them
+// Adfnew: also the Gram refinement step over the alias-free rings, Adfnew = A0 - D A (= A + (A0 - M A)) per
+// block, in the same launch, raising Eout by its column exponents
 void launch_leg_synthesis_tc(const Plan &p, const float2 *Adf, int64_t ncol, float *G, cudaStream_t st,
-                             int rlim = -1, const int *Ein = nullptr);
-// Gram refinement step of the mixed transform (alias-free rings):
-//   Anew = A + (A0 - M A) per block, A in FP64 (A) and double-float (Adf)
-void launch_gram_update(const Plan &p, const double *A, const float2 *Adf, const float2 *A0, int64_t ncol,
-                        double *Anew, float2 *Adfnew, cudaStream_t st, const int *Ein = nullptr,
-                        int *Eout = nullptr);
+                             int rlim = -1, const int *Ein = nullptr, const float2 *A0 = nullptr,
+                             float2 *Adfnew = nullptr, int *Eout = nullptr);
 int build_gram_tables(Plan &p, cudaStream_t st);
 void launch_df_to_fp64(const float2 *a, int64_t n, double *out, cudaStream_t st);
 // adjoint (adjoint.cu)
