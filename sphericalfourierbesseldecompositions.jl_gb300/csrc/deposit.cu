@@ -263,10 +263,13 @@ __global__ void k_deposit_keys_fallback(const double *__restrict__ rtp, int64_t 
 }
 
 // Exclusive scan, tile pass: each block scans SCAN_TILE counters in place and
-// writes its total.
+// writes its total; the block that finishes last (counted in *done, zero on
+// entry) scans the totals, so that step costs no launch of its own.
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_tiles(int32_t *__restrict__ data, int64_t n,
-                                                             int32_t *__restrict__ tile_sums) {
+                                                             int32_t *__restrict__ tile_sums, int *done) {
     __shared__ int32_t warp_tot[SCAN_THREADS / 32];
+    __shared__ int32_t carry;
+    __shared__ bool last;
     const int64_t base = (int64_t)blockIdx.x * SCAN_TILE + (int64_t)threadIdx.x * SCAN_ITEMS;
     int32_t v[SCAN_ITEMS];
     int32_t s = 0;
@@ -301,30 +304,40 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_tiles(int32_t *__restrict
         if (idx < n) data[idx] = run;
         run += v[j];
     }
-    if (threadIdx.x == SCAN_THREADS - 1) tile_sums[blockIdx.x] = run;
-}
-
-// Scan of the tile totals by one block (serial over chunks of 1024).
-__global__ void k_scan_sums(int32_t *__restrict__ sums, int64_t n) {
-    __shared__ int32_t buf[1024];
-    __shared__ int32_t carry;
-    if (threadIdx.x == 0) carry = 0;
+    if (threadIdx.x == SCAN_THREADS - 1) {
+        tile_sums[blockIdx.x] = run;
+        __threadfence();
+        last = atomicAdd(done, 1) == (int)gridDim.x - 1;
+        carry = 0;
+    }
     __syncthreads();
-    for (int64_t c0 = 0; c0 < n; c0 += 1024) {
-        const int64_t idx = c0 + threadIdx.x;
-        const int32_t v = idx < n ? sums[idx] : 0;
-        buf[threadIdx.x] = v;
-        __syncthreads();
-        for (int off = 1; off < 1024; off <<= 1) {
-            const int32_t t = threadIdx.x >= off ? buf[threadIdx.x - off] : 0;
-            __syncthreads();
-            buf[threadIdx.x] += t;
-            __syncthreads();
+    if (!last) return;
+    __threadfence();
+    for (int64_t c0 = 0; c0 < gridDim.x; c0 += SCAN_TILE) {
+        const int64_t b0 = c0 + (int64_t)threadIdx.x * SCAN_ITEMS;
+        s = 0;
+#pragma unroll
+        for (int j = 0; j < SCAN_ITEMS; ++j) {
+            v[j] = b0 + j < gridDim.x ? __ldcg(tile_sums + b0 + j) : 0;
+            s += v[j];
         }
-        const int32_t excl = buf[threadIdx.x] - v + carry;
-        if (idx < n) sums[idx] = excl;
+        inc = s;
+        for (int off = 1; off < 32; off <<= 1) {
+            const int32_t t = __shfl_up_sync(0xffffffffu, inc, off);
+            if (lane >= off) inc += t;
+        }
         __syncthreads();
-        if (threadIdx.x == 1023) carry = excl + v;
+        if (lane == 31) warp_tot[wid] = inc;
+        __syncthreads();
+        run = carry + inc - s;
+        for (int w = 0; w < wid; ++w) run += warp_tot[w];
+#pragma unroll
+        for (int j = 0; j < SCAN_ITEMS; ++j) {
+            if (b0 + j < gridDim.x) tile_sums[b0 + j] = run;
+            run += v[j];
+        }
+        __syncthreads();
+        if (threadIdx.x == SCAN_THREADS - 1) carry = run;
         __syncthreads();
     }
 }
@@ -807,12 +820,15 @@ constexpr int STATS_STRIDE = 32;
 // 32 bins (one warp per block): S[b] += <D_b, ref>, Q[slot] += <ref, ref>,
 // with ref as the double-float pairs cdf.  A slot-uniform warp reduces
 // through shared memory in double-float (lane k sums column k) and adds the
-// column sums in FP64; a warp that straddles two slots adds per thread.
+// column sums in FP64; a warp that straddles two slots adds per thread.  The
+// block that finishes last (*done zero on entry) forms mu[b] = S[b] / Q[slot(b)]
+// (0 where the sampled reference map is zero) and the same as a double-float pair.
 template <int MAXDEG>
 __global__ void __launch_bounds__(32) k_deposit_stats(const int32_t *__restrict__ offset,
                                                       const float4 *__restrict__ sorted, int64_t npix, int pieces,
                                                       int deg, int64_t nbasis, const float2 *__restrict__ cdf,
-                                                      double *__restrict__ S, double *__restrict__ Q) {
+                                                      double *S, double *Q, double *__restrict__ mu,
+                                                      float2 *__restrict__ mudf, int *done) {
     __shared__ float2 red[32][MAXDEG + 3];
     const int lane = threadIdx.x;
     const int64_t idx = (int64_t)blockIdx.x * STATS_STRIDE * 32 + lane;
@@ -833,8 +849,7 @@ __global__ void __launch_bounds__(32) k_deposit_stats(const int32_t *__restrict_
     const unsigned full = 0xffffffffu;
     const int slot0 = __shfl_sync(full, slot, 0);
     auto to_d = [](dfl a) { return (double)a.hi + (double)a.lo; };
-    if (__all_sync(full, slot == slot0)) {
-        if (slot0 < 0) return;
+    if (__all_sync(full, slot == slot0)) {          // (a group is never without a valid bin)
 #pragma unroll
         for (int k = 0; k <= MAXDEG; ++k)
             if (k < nk) {
@@ -856,31 +871,42 @@ __global__ void __launch_bounds__(32) k_deposit_stats(const int32_t *__restrict_
             if (k < nk) atomicAdd(S + basis_of(slot, k, pieces, deg, nbasis), to_d(df_mul(acc[k], rv)));
         atomicAdd(Q + slot, to_d(df_mul(rv, rv)));
     }
-}
-
-// mu[b] = S[b] / Q[slot(b)] (0 where the sampled reference map is zero), and
-// the same as a double-float pair in mudf.
-__global__ void k_mean_finalize(const double *S, const double *Q, int pieces, int deg, int64_t nbasis, double *mu,
-                                float2 *mudf) {
-    const int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= nbasis) return;
+    __threadfence();
+    __syncwarp();
+    int last = 0;
+    if (lane == 0) last = atomicAdd(done, 1) == (int)gridDim.x - 1;
+    if (!__shfl_sync(full, last, 0)) return;
+    __threadfence();
     const int64_t npoly = (int64_t)pieces * (deg + 1);
-    const int slot = b < npoly ? (int)(b / (deg + 1)) : pieces + (int)(b - npoly);
-    const double v = Q[slot] > 0.0 ? S[b] / Q[slot] : 0.0;
-    mu[b] = v;
-    const float h = (float)v;
-    mudf[b] = make_float2(h, (float)(v - (double)h));
+    for (int64_t b = lane; b < nbasis; b += 32) {
+        const int sl = b < npoly ? (int)(b / (deg + 1)) : pieces + (int)(b - npoly);
+        const double q = __ldcg(Q + sl), v = q > 0.0 ? __ldcg(S + b) / q : 0.0;
+        mu[b] = v;
+        const float h = (float)v;
+        mudf[b] = make_float2(h, (float)(v - (double)h));
+    }
 }
 
 // Weighted galaxy count per pixel over all radial slots (the reference map of
 // the mixed deposit), in double-float from the sorted pairs, stored as the
 // FP64 value hi + lo (exact) and as the pair itself.
 // ring_live[ring] is set to 1 for every ring holding a galaxy (preset to 0).
+// The window's reference map W01 goes beside C (C[npix + pix]) and, for a
+// separable window, as a double-float map to mask_df.
 __global__ void k_weight_map_mixed(const int32_t *__restrict__ offset, const float4 *__restrict__ sorted,
                                    int64_t nside, int64_t npix, int nslots, double *__restrict__ C,
-                                   float2 *__restrict__ cdf, int *__restrict__ ring_live) {
+                                   float2 *__restrict__ cdf, int *__restrict__ ring_live,
+                                   const double *__restrict__ W01, float2 *__restrict__ mask_df) {
     const int64_t pix = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (pix >= npix) return;
+    if (W01) {
+        const double v = W01[pix];
+        C[npix + pix] = v;
+        if (mask_df) {
+            const float h = (float)v;
+            mask_df[pix] = make_float2(h, (float)(v - (double)h));
+        }
+    }
     dfl s = {0.f, 0.f};
     bool any = false;
     for (int sl = 0; sl < nslots; ++sl) {
@@ -932,11 +958,11 @@ static void launch_moments(const Plan &p, const int32_t *counts, const void *sor
 
 template <int MAXDEG>
 static void launch_stats(const Plan &p, const int32_t *counts, const float4 *sorted, const float2 *cdf, double *S,
-                         double *Q, cudaStream_t st) {
+                         double *Q, double *mu, float2 *mudf, int *done, cudaStream_t st) {
     const int64_t nkeys = (int64_t)(p.pieces + 2) * p.npix;
     const int64_t blocks = (nkeys + 32 * STATS_STRIDE - 1) / (32 * STATS_STRIDE);
     k_deposit_stats<MAXDEG><<<(unsigned)blocks, 32, 0, st>>>(counts, sorted, p.npix, p.pieces, p.degree, p.nbasis,
-                                                              cdf, S, Q);
+                                                              cdf, S, Q, mu, mudf, done);
     note_launch();
 }
 
@@ -951,11 +977,9 @@ static void by_degree(int deg, F &&f) {
 
 int64_t scan_tile_count(int64_t n) { return (n + SCAN_TILE - 1) / SCAN_TILE; }
 
-void launch_exclusive_scan(int32_t *data, int64_t n, int32_t *tile_sums, cudaStream_t st) {
+void launch_exclusive_scan(int32_t *data, int64_t n, int32_t *tile_sums, int *done, cudaStream_t st) {
     const int64_t ntiles = scan_tile_count(n);
-    k_scan_tiles<<<(unsigned)ntiles, SCAN_THREADS, 0, st>>>(data, n, tile_sums);
-    note_launch();
-    k_scan_sums<<<1, 1024, 0, st>>>(tile_sums, ntiles);
+    k_scan_tiles<<<(unsigned)ntiles, SCAN_THREADS, 0, st>>>(data, n, tile_sums, done);
     note_launch();
     k_scan_add<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(data, n, tile_sums);
     note_launch();
@@ -963,38 +987,40 @@ void launch_exclusive_scan(int32_t *data, int64_t n, int32_t *tile_sums, cudaStr
 
 int deposit_sorted(Plan &p, const double *rtp, const double *w, int64_t ngal, double *maps, double *ref,
                    double *mu, cudaEvent_t ref_ready, cudaStream_t st, const cudaEvent_t *chunk_ready,
-                   int nchunks, const int **ring_live) {
+                   int nchunks, const int **ring_live, const double *w01, float2 *mask_df, cudaEvent_t mu_ready) {
     const bool mixed = p.precision == SFB_MIXED;
     if (ring_live) *ring_live = nullptr;
     const int64_t nkeys = (int64_t)(p.pieces + 2) * p.npix;
     const int64_t nscan = nkeys + 1;            // one extra counter: its exclusive prefix is the total
     const int64_t ntiles = (nscan + SCAN_TILE - 1) / SCAN_TILE;
-    // workspace: counters/offsets [nscan] int32, tile sums [ntiles] int32, key, rank and the FP64-pixel
-    // list [ngal] int32 (+ its count), local coordinate [ngal] double (mixed: float2), sorted (x, w) [ngal]
-    // double2 (mixed: float4), S [nbasis], Q [pieces + 2], mudf [nbasis] float2, cdf [npix] float2
-    const int64_t ints = nscan + ntiles + 3 * ngal + 1;
-    const int64_t off_x = (ints + 1) / 2;
+    // workspace: first what one clear presets to zero: counters/offsets [nscan] int32, three block counters and
+    // the length of the FP64-pixel list, ring_live [nrings] int32, S [nbasis], Q [pieces + 2]; then mudf [nbasis]
+    // float2, cdf [npix] float2, local coordinate [ngal] double (mixed: float2), sorted (x, w) [ngal] double2
+    // (mixed: float4), tile sums [ntiles], key, rank and the FP64-pixel list [ngal] int32
+    const int64_t nrings = 4 * p.nside - 1;
+    const int64_t off_S = (nscan + 4 + nrings + 1) / 2;
+    const int64_t off_mudf = off_S + p.nbasis + p.pieces + 2, off_cdf = off_mudf + p.nbasis;
+    const int64_t off_x = off_cdf + p.npix;
     int64_t off_sorted = off_x + ngal;
     off_sorted += off_sorted & 1;
-    const int64_t off_stats = off_sorted + 2 * ngal + 2;
-    const int64_t off_cdf = off_stats + 2 * p.nbasis + p.pieces + 2;
-    const int64_t nrings = 4 * p.nside - 1;
-    const int64_t off_live = off_cdf + p.npix;               // ring_live [nrings] int
-    SFB_TRY(grow(p, p.dep, (size_t)(off_live + (nrings + 1) / 2)));
+    const int64_t off_int = off_sorted + 2 * ngal;
+    SFB_TRY(grow(p, p.dep, (size_t)(off_int + (ntiles + 3 * ngal + 1) / 2)));
     int32_t *counts = reinterpret_cast<int32_t *>(p.dep.ptr);
-    int32_t *tsum = counts + nscan;
-    int32_t *key = tsum + ntiles;
-    int32_t *rank = key + ngal;
-    int32_t *fb_list = rank + ngal;
-    int32_t *fb_count = fb_list + ngal;
+    int *scan_done = counts + nscan, *stats_done = scan_done + 1;
+    int32_t *fb_count = scan_done + 2;
+    int *live = scan_done + 4;
+    double *S = p.dep.ptr + off_S, *Q = S + p.nbasis;
+    float2 *mudf = reinterpret_cast<float2 *>(p.dep.ptr + off_mudf);
+    float2 *cdf = reinterpret_cast<float2 *>(p.dep.ptr + off_cdf);
     double *xloc = p.dep.ptr + off_x;
     float2 *xdf = reinterpret_cast<float2 *>(xloc);
     void *sorted = p.dep.ptr + off_sorted;
     float4 *sorted4 = static_cast<float4 *>(sorted);
-    float2 *cdf = reinterpret_cast<float2 *>(p.dep.ptr + off_cdf);
-    int *live = reinterpret_cast<int *>(p.dep.ptr + off_live);
-    SFB_CUDA_TRY(cudaMemsetAsync(counts, 0, (size_t)nscan * sizeof(int32_t), st));
-    SFB_CUDA_TRY(cudaMemsetAsync(fb_count, 0, sizeof(int32_t), st));
+    int32_t *tsum = reinterpret_cast<int32_t *>(p.dep.ptr + off_int);
+    int32_t *key = tsum + ntiles;
+    int32_t *rank = key + ngal;
+    int32_t *fb_list = rank + ngal;
+    SFB_CUDA_TRY(cudaMemsetAsync(p.dep.ptr, 0, (size_t)off_mudf * sizeof(double), st));
     const double inv_width = (double)p.pieces / (p.rmax - p.rmin);
     RadialKeyParams rk;
     rk.ord_rmin = ord_of(p.rmin);
@@ -1025,7 +1051,7 @@ int deposit_sorted(Plan &p, const double *rtp, const double *w, int64_t ngal, do
         k_deposit_keys_fallback<<<304, 256, 0, st>>>(rtp, p.nside, p.npix, counts, key, rank, fb_list, fb_count);
         note_launch();
     }
-    launch_exclusive_scan(counts, nscan, tsum, st);
+    launch_exclusive_scan(counts, nscan, tsum, scan_done, st);
     if (ngal > 0) {
         if (mixed)
             k_deposit_scatter_mixed<<<(unsigned)((ngal + 255) / 256), 256, 0, st>>>(w, ngal, key, rank, xdf, counts,
@@ -1037,20 +1063,15 @@ int deposit_sorted(Plan &p, const double *rtp, const double *w, int64_t ngal, do
     }
     if (p.degree > 63) return fail(SFB_ENOTSUP, "radial degree above 63 is not supported by the sorted deposit");
     const bool split = ref != nullptr && mixed;
-    float2 *mudf = reinterpret_cast<float2 *>(p.dep.ptr + off_stats + p.nbasis + p.pieces + 2);
     if (split) {
-        SFB_CUDA_TRY(cudaMemsetAsync(live, 0, (size_t)nrings * sizeof(int), st));
         k_weight_map_mixed<<<(unsigned)((p.npix + 255) / 256), 256, 0, st>>>(counts, sorted4, p.nside, p.npix,
-                                                                            p.pieces + 2, ref, cdf, live);
+                                                                            p.pieces + 2, ref, cdf, live, w01, mask_df);
         note_launch();
         if (ref_ready) SFB_CUDA_TRY(cudaEventRecord(ref_ready, st));
-        double *S = p.dep.ptr + off_stats;
-        double *Q = S + p.nbasis;
-        SFB_CUDA_TRY(cudaMemsetAsync(S, 0, (size_t)(p.nbasis + p.pieces + 2) * sizeof(double), st));
-        by_degree(p.degree, [&](auto D) { launch_stats<decltype(D)::value>(p, counts, sorted4, cdf, S, Q, st); });
-        k_mean_finalize<<<(unsigned)((p.nbasis + 127) / 128), 128, 0, st>>>(S, Q, p.pieces, p.degree, p.nbasis, mu,
-                                                                           mudf);
-        note_launch();
+        by_degree(p.degree, [&](auto D) {
+            launch_stats<decltype(D)::value>(p, counts, sorted4, cdf, S, Q, mu, mudf, stats_done, st);
+        });
+        if (mu_ready) SFB_CUDA_TRY(cudaEventRecord(mu_ready, st));
     }
     // moments in FP64 (FP64 path) or double-float (mixed); stored in the transform's precision
     const bool skip_empty = split && ring_live && p.npix >= 128 && p.degree <= 31;   // the balanced kernel

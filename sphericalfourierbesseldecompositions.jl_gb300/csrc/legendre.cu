@@ -310,23 +310,45 @@ static bool narrow_dispatch(const Plan &p, const T *lam, const T *in, int64_t nc
     }
 }
 
-// FP64 Gram refinement step for few columns (the narrow transforms):
-//   Anew[l(r)] = A0[l(r)] - sum_li D_z[r][li] Acur[l(li)]   (= Acur + (A0 - M_z Acur))
-// one thread per (block z, output row r, column); D_z = M_z - I from the plan's
-// FP64 Gram tables (element [li][r] at gram_off[z] + li R + r).
+// FP64 refinement step for few columns (the narrow transforms), one launch: blocks x < ng do the Gram update
+//   Anew[l(r)] = A0[l(r)] - sum_li D_z[r][li] Acur[l(li)]   (= Acur + (A0 - M_z Acur)),
+// one thread per (block z, output row r, column), D_z = M_z - I from the plan's FP64 Gram tables (element [li][r]
+// at gram_off[z] + li R + r); the others form G on the rings r < ral, one thread per (block z, ring).
 template <int NC>
-__global__ void __launch_bounds__(128) k_gram_update_fp64(const double *__restrict__ gram,
-                                                          const int64_t *__restrict__ gram_off, int R, int lmax,
-                                                          const double *__restrict__ Acur,
-                                                          const double *__restrict__ A0, double *__restrict__ Anew) {
+__global__ void __launch_bounds__(128) k_refine_narrow64(const double *__restrict__ gram,
+                                                         const int64_t *__restrict__ gram_off, int R,
+                                                         const double *__restrict__ lam,
+                                                         const int64_t *__restrict__ lam_off, int nrn, int ral, int ng,
+                                                         int lmax, const double *__restrict__ Acur,
+                                                         const double *__restrict__ A0, double *__restrict__ Anew,
+                                                         double *__restrict__ G) {
     const int z = blockIdx.y;
     const int m = z >> 1, par = z & 1;
     const int nrows = nrows_of(m, par, lmax);
+    if ((int)blockIdx.x >= ng) {
+        const int r = ((int)blockIdx.x - ng) * 128 + threadIdx.x;
+        if (r >= ral) return;
+        const double *L = lam + lam_off[z] + r;
+        double acc[NC] = {};
+#pragma unroll 4
+        for (int li = 0; li < nrows; ++li) {
+            const double l = L[(int64_t)li * nrn];
+            const int ll = m + par + 2 * li;
+            const double *a = Acur + ((int64_t)ll * (ll + 1) / 2 + m) * NC;
+#pragma unroll
+            for (int c = 0; c < NC; ++c) acc[c] = fma(l, a[c], acc[c]);
+        }
+        double *g = G + (((int64_t)(par * (lmax + 1) + m) * nrn) + r) * NC;
+#pragma unroll
+        for (int c = 0; c < NC; ++c) g[c] = acc[c];
+        return;
+    }
     const int idx = blockIdx.x * 128 + threadIdx.x;
     const int r = idx / NC, c = idx - r * NC;
     if (r >= nrows) return;
     const double *M = gram + gram_off[z] + r;
     double acc = 0.0;
+#pragma unroll 4
     for (int li = 0; li < nrows; ++li) {
         const int l = m + par + 2 * li;
         acc = fma(M[(int64_t)li * R], Acur[((int64_t)l * (l + 1) / 2 + m) * NC + c], acc);
@@ -334,6 +356,22 @@ __global__ void __launch_bounds__(128) k_gram_update_fp64(const double *__restri
     const int l = m + par + 2 * r;
     const int64_t o = ((int64_t)l * (l + 1) / 2 + m) * NC + c;
     Anew[o] = A0[o] - acc;
+}
+
+bool launch_refine_narrow64(const Plan &p, const double *A, const double *A0, int64_t ncol, double *G, double *Anew,
+                            cudaStream_t st) {
+    if (!p.d_gram64 || p.precision != SFB_FP64 || (ncol != 2 && ncol != 4 && ncol != 8)) return false;
+    const int maxrows = p.lmax / 2 + 1, ng = (int)((maxrows * ncol + 127) / 128);
+    const dim3 grid((unsigned)(ng + (p.ral + 127) / 128), (unsigned)(2 * (p.lmax + 1)));
+    auto go = [&](auto kernel) {
+        kernel<<<grid, 128, 0, st>>>(p.d_gram64, p.d_gram_off, p.gram_rows, p.d_lam, p.d_lam_off, (int)p.nrn, p.ral, ng,
+                                     p.lmax, A, A0, Anew, G);
+    };
+    if (ncol == 2) go(k_refine_narrow64<2>);
+    else if (ncol == 4) go(k_refine_narrow64<4>);
+    else go(k_refine_narrow64<8>);
+    note_launch();
+    return true;
 }
 
 // Many columns: the same update as a tiled GEMM per block z (output rows r x
@@ -884,22 +922,13 @@ __global__ void __launch_bounds__(256) k_fold_residual_narrow(const RingGeom *ri
 bool launch_gram_update_fp64(const Plan &p, const double *Acur, const double *A0, int64_t ncol, double *Anew,
                              cudaStream_t st) {
     if (!p.d_gram64) return false;
+    if (p.tc64_state > 0) {
+        launch_leg_synthesis64(p, Acur, ncol, nullptr, st, 0, A0, Anew);
+        return true;
+    }
     const int maxrows = p.lmax / 2 + 1;
-    dim3 grid((unsigned)((maxrows * ncol + 127) / 128), (unsigned)(2 * (p.lmax + 1)));
-    switch (ncol) {
-    case 2: k_gram_update_fp64<2><<<grid, 128, 0, st>>>(p.d_gram64, p.d_gram_off, p.gram_rows, p.lmax, Acur, A0, Anew); break;
-    case 4: k_gram_update_fp64<4><<<grid, 128, 0, st>>>(p.d_gram64, p.d_gram_off, p.gram_rows, p.lmax, Acur, A0, Anew); break;
-    case 8: k_gram_update_fp64<8><<<grid, 128, 0, st>>>(p.d_gram64, p.d_gram_off, p.gram_rows, p.lmax, Acur, A0, Anew); break;
-    default: {
-        if (p.tc64_state > 0) {
-            launch_leg_synthesis64(p, Acur, ncol, nullptr, st, 0, A0, Anew);
-            return true;
-        }
-        dim3 wg((unsigned)((ncol + BN - 1) / BN), (unsigned)((maxrows + BM - 1) / BM), (unsigned)(2 * (p.lmax + 1)));
-        k_gram_update_wide<<<wg, 256, 0, st>>>(p.d_gram64, p.d_gram_off, p.gram_rows, p.lmax, Acur, A0, ncol, Anew);
-        break;
-    }
-    }
+    dim3 wg((unsigned)((ncol + BN - 1) / BN), (unsigned)((maxrows + BM - 1) / BM), (unsigned)(2 * (p.lmax + 1)));
+    k_gram_update_wide<<<wg, 256, 0, st>>>(p.d_gram64, p.d_gram_off, p.gram_rows, p.lmax, Acur, A0, ncol, Anew);
     note_launch();
     return true;
 }

@@ -105,7 +105,7 @@ struct sfb_plan {
     // side stream for the FP64 reference-map transform of the mixed path,
     // forked / joined with the call's stream through events
     cudaStream_t side = nullptr;
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_mu = nullptr;
     // host entry: the catalogue copy runs on the side stream in NCOPY chunks
     static constexpr int NCOPY = 4;
     cudaEvent_t ev_copy[NCOPY] = {};
@@ -323,13 +323,14 @@ struct ShtWork {
 };
 
 // One FP64 Gram refinement step's products of the current coefficients: G on the aliased rings and
-// Anew = A0 - D A (many columns: one tensor-core launch).
+// Anew = A0 - D A (one launch for many columns on the tensor cores, and for 2, 4 or 8).
 void synthesis_and_gram64(const Plan &p, const double *A, const double *A0, int64_t ncol, double *G, double *Anew,
                           cudaStream_t st) {
     if (p.tc64_state > 0 && ncol > 8) {
         launch_leg_synthesis64(p, A, ncol, G, st, p.ral, A0, Anew);
         return;
     }
+    if (launch_refine_narrow64(p, A, A0, ncol, G, Anew, st)) return;
     if (p.ral > 0) launch_leg_synthesis(p, A, ncol, G, st, p.ral);
     launch_gram_update_fp64(p, A, A0, ncol, Anew, st);
 }
@@ -456,22 +457,20 @@ int sht_analysis(sfb_plan *h, const double *maps, int64_t nm, cudaStream_t st, b
     if (!tc && p.d_gram64 && p.niter > 0) {
         // FP64 Gram refinement: the same identity as above, in FP64 (narrow kernels for 2, 4 or 8
         // columns: reference maps, small map2alm batches; tiled GEMMs for more, the first pass over
-        // the ring pairs with data).  alm holds [current | next | first pass].
+        // the ring pairs with data).  alm holds [result | other | first pass]; step it writes one of the
+        // first two, the last step the first.
         const int64_t na = p.lmsize * ncol;
         SFB_TRY(grow(p, alm, (size_t)(3 * na)));
-        double *Ab[2] = {alm.ptr, alm.ptr + na};
-        double *a0 = alm.ptr + 2 * na;
-        int cur = p.niter & 1;
+        double *a0 = alm.ptr + 2 * na, *cur = a0;
         {
             Stage s(h, stage(SFB_STAGE_LEG_ANALYSIS), st);
-            launch_leg_analysis(p, fbuf.ptr, ncol, Ab[cur], false, st, -1, nzr);
+            launch_leg_analysis(p, fbuf.ptr, ncol, cur, false, st, -1, nzr);
         }
-        SFB_CUDA_TRY(cudaMemcpyAsync(a0, Ab[cur], (size_t)na * sizeof(double), cudaMemcpyDeviceToDevice, st));
         for (int it = 0; it < p.niter; ++it) {
-            const int nxt = cur ^ 1;
+            double *nxt = alm.ptr + ((p.niter - 1 - it) & 1) * na;
             {
                 Stage s(h, stage(SFB_STAGE_LEG_SYNTHESIS), st);
-                synthesis_and_gram64(p, Ab[cur], a0, ncol, gbuf.ptr, Ab[nxt], st);
+                synthesis_and_gram64(p, cur, a0, ncol, gbuf.ptr, nxt, st);
             }
             if (p.ral > 0) {
                 {
@@ -479,7 +478,7 @@ int sht_analysis(sfb_plan *h, const double *maps, int64_t nm, cudaStream_t st, b
                     launch_fold_residual(p, nullptr, gbuf.ptr, ncol, rbuf.ptr, st, nullptr, p.ral);
                 }
                 Stage s(h, stage(SFB_STAGE_LEG_ANALYSIS), st);
-                launch_leg_analysis(p, rbuf.ptr, ncol, Ab[nxt], true, st, p.ral);
+                launch_leg_analysis(p, rbuf.ptr, ncol, nxt, true, st, p.ral);
             }
             cur = nxt;
         }
@@ -519,9 +518,9 @@ int check_tc(Plan &p, cudaStream_t st, int *err_out = nullptr) {
     return SFB_OK;
 }
 
-int finish(sfb_plan *h, const double *out_dev, cudaStream_t st) {
+int finish(sfb_plan *h, const double *out_dev, cudaStream_t st, bool checked = false) {
     Plan &p = h->p;
-    {
+    if (!checked) {
         Stage s(h, SFB_STAGE_OTHER, st);
         launch_check_finite(out_dev, 2 * p.nlmsize, p.d_err, st);
     }
@@ -537,19 +536,16 @@ int finish(sfb_plan *h, const double *out_dev, cudaStream_t st) {
     return SFB_OK;
 }
 
-// FP64 a_lm of nref reference maps (mixed precision's mean terms), into
-// ralm[lmsize][2 nref].
-int reference_alm(sfb_plan *h, const double *ref, int64_t nref, double *ralm, cudaStream_t st) {
+// FP64 a_lm of nref reference maps (mixed precision's mean terms), into the first lmsize rows of p.ralm
+// ([lmsize][2 nref]).
+int reference_alm(sfb_plan *h, const double *ref, int64_t nref, cudaStream_t st) {
     Plan &p = h->p;
     const int32_t prec = p.precision;
     p.precision = SFB_FP64;
     const ShtWork ws{&p.rf, &p.rg, &p.rr, &p.ralm};
     const int rc = sht_analysis(h, ref, nref, st, false, SFB_STAGE_OTHER, &ws);
     p.precision = prec;
-    SFB_TRY(rc);
-    SFB_CUDA_TRY(cudaMemcpyAsync(ralm, p.ralm.ptr, (size_t)2 * nref * p.lmsize * sizeof(double),
-                                 cudaMemcpyDeviceToDevice, st));
-    return SFB_OK;
+    return rc;
 }
 
 // Transpose of sht_analysis in FP64 (adjoint.cu): abar [lmsize][2 nm] on the device becomes b = w E abar;
@@ -644,23 +640,23 @@ int cat2amln_dev(sfb_plan *h, const double *rtp, const double *w, int64_t ngal, 
         const bool split = p.precision == SFB_MIXED && wk != SFB_WINDOW_ZERO;
         const double *W01 = wk == SFB_WINDOW_SEPARABLE ? win->mask : win->dense;
         const int64_t cp = wk == SFB_WINDOW_DENSE ? chunk_pairs(p) : 0;
-        double *Cmap = nullptr, *ralm = nullptr, *mu = nullptr, *nu = nullptr, *smean = nullptr;
+        double *Cmap = nullptr, *mu = nullptr, *nu = nullptr, *smean = nullptr;
+        const double *ralm = nullptr;             // FP64 a_lm of (C, W01), [lmsize][4]
         if (split) {
-            // [C][W01][ralm: lmsize x (C, W01) complex][mu][nu][per-pair mean parts]
-            SFB_TRY(grow(p, p.ref, (size_t)(2 * p.npix + 4 * p.lmsize + p.nbasis + cp + p.npairs)));
+            // [C][W01][mu][nu][per-pair mean parts]
+            SFB_TRY(grow(p, p.ref, (size_t)(2 * p.npix + p.nbasis + cp + p.npairs)));
             Cmap = p.ref.ptr;
-            ralm = Cmap + 2 * p.npix;
-            mu = ralm + 4 * p.lmsize;
+            mu = Cmap + 2 * p.npix;
             nu = mu + p.nbasis;
             smean = nu + cp;
-            SFB_CUDA_TRY(cudaMemcpyAsync(Cmap + p.npix, W01, p.npix * sizeof(double), cudaMemcpyDeviceToDevice, st));
         }
         SFB_TRY(grow(p, p.maps, (size_t)nm * p.npix));
         const int *ring_live = nullptr;          // rings the deposit wrote (mixed precision)
+        float2 *mask_df = nullptr;               // the mask as a map of the mixed transform (the deposit writes it)
         if (wk == SFB_WINDOW_SEPARABLE) {
             Stage s(h, SFB_STAGE_OTHER, st);
-            if (p.precision == SFB_MIXED)
-                launch_to_df(win->mask, p.npix, reinterpret_cast<float2 *>(p.maps.ptr) + p.nbasis * p.npix, st);
+            if (split)
+                mask_df = reinterpret_cast<float2 *>(p.maps.ptr) + p.nbasis * p.npix;
             else
                 SFB_CUDA_TRY(cudaMemcpyAsync(p.maps.ptr + p.nbasis * p.npix, win->mask, p.npix * sizeof(double),
                                              cudaMemcpyDeviceToDevice, st));
@@ -668,13 +664,16 @@ int cat2amln_dev(sfb_plan *h, const double *rtp, const double *w, int64_t ngal, 
         {
             Stage s(h, SFB_STAGE_DEPOSIT, st);
             SFB_TRY(deposit_sorted(p, rtp, w, ngal, p.maps.ptr, Cmap, mu, split ? h->ev_fork : nullptr, st,
-                                   chunk_ready, nchunks, &ring_live));
+                                   chunk_ready, nchunks, &ring_live, W01, mask_df, split ? h->ev_mu : nullptr));
         }
         if (split) {
             // the FP64 transform of (C, W01) runs on the side stream, in its own workspace, beside
             // the rest of the deposit and the main transform; the projection waits for it
             SFB_CUDA_TRY(cudaStreamWaitEvent(h->side, h->ev_fork, 0));
-            SFB_TRY(reference_alm(h, Cmap, 2, ralm, h->side));
+            SFB_TRY(reference_alm(h, Cmap, 2, h->side));
+            ralm = p.ralm.ptr;
+            SFB_CUDA_TRY(cudaStreamWaitEvent(h->side, h->ev_mu, 0));
+            launch_mean_proj(p, mu, smean, h->side);
             SFB_CUDA_TRY(cudaEventRecord(h->ev_join, h->side));
         }
         // the mixed projection reads the double-float a_lm only
@@ -685,8 +684,8 @@ int cat2amln_dev(sfb_plan *h, const double *rtp, const double *w, int64_t ngal, 
             Stage s(h, SFB_STAGE_PROJECT, st);
             if (p.precision == SFB_MIXED)
                 launch_project_mixed(p, reinterpret_cast<const float2 *>(p.almdf.ptr), 2 * nm, p.d_coefT, h->d_noff,
-                                     h->d_pair_index, scale, mu, smean, split ? ralm : nullptr, wk, win->w_ln, out,
-                                     st);
+                                     h->d_pair_index, scale, smean, ralm, wk, win->w_ln, out,
+                                     wk == SFB_WINDOW_DENSE ? nullptr : p.d_err, st);
             else
                 launch_project_poly(p, p.alm.ptr, 2 * nm, scale, wk, win->w_ln, p.nbasis, nullptr, 0, out, st);
         }
@@ -718,12 +717,14 @@ int cat2amln_dev(sfb_plan *h, const double *rtp, const double *w, int64_t ngal, 
         }
     }
     SFB_CUDA_TRY(cudaGetLastError());
+    // the mixed projection has checked what it wrote, unless a dense window was subtracted from it
+    const bool checked = p.radial_mode == SFB_RADIAL_POLY && p.precision == SFB_MIXED && wk != SFB_WINDOW_DENSE;
     if (defer_finish) {
         Stage s(h, SFB_STAGE_OTHER, st);
-        launch_check_finite(out, 2 * p.nlmsize, p.d_err, st);
+        if (!checked) launch_check_finite(out, 2 * p.nlmsize, p.d_err, st);
         return SFB_OK;
     }
-    return finish(h, out, st);
+    return finish(h, out, st, checked);
 }
 
 int check_plan(const sfb_plan *h) {
@@ -851,6 +852,7 @@ int sfb_plan_create(const sfb_plan_desc *d, sfb_plan **out) {
             cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking) != cudaSuccess ||
             cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
             cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming) != cudaSuccess ||
+            cudaEventCreateWithFlags(&h->ev_mu, cudaEventDisableTiming) != cudaSuccess ||
             cudaStreamCreateWithFlags(&p.dft_side, cudaStreamNonBlocking) != cudaSuccess ||
             cudaEventCreateWithFlags(&p.dft_fork, cudaEventDisableTiming) != cudaSuccess ||
             cudaEventCreateWithFlags(&p.dft_join, cudaEventDisableTiming) != cudaSuccess ||
@@ -1092,6 +1094,7 @@ void sfb_plan_destroy(sfb_plan *h) {
     if (h->side) cudaStreamDestroy(h->side);
     if (h->ev_fork) cudaEventDestroy(h->ev_fork);
     if (h->ev_join) cudaEventDestroy(h->ev_join);
+    if (h->ev_mu) cudaEventDestroy(h->ev_mu);
     if (p.dft_side) cudaStreamDestroy(p.dft_side);
     if (p.dft_fork) cudaEventDestroy(p.dft_fork);
     if (p.dft_join) cudaEventDestroy(p.dft_join);

@@ -592,7 +592,7 @@ __global__ void __launch_bounds__(32 * KS) k_project_mixed(const float2 *__restr
                                                               const double *__restrict__ smean,
                                                               const double *__restrict__ ralm, int window_kind,
                                                               const double *__restrict__ w_ln,
-                                                              double *__restrict__ out) {
+                                                              double *__restrict__ out, int *err) {
     __shared__ float4 part[KS - 1][PJ_NPT][32];
     const int3 t = tiles[blockIdx.x];
     const int l = t.x, m0 = t.y, n0 = t.z & 0xffff, npt = t.z >> 16;
@@ -655,6 +655,7 @@ __global__ void __launch_bounds__(32 * KS) k_project_mixed(const float2 *__restr
         const int64_t o = noff[n1] + lm;
         out[2 * o] = vr;
         out[2 * o + 1] = vi;
+        if (err && !(isfinite(vr) && isfinite(vi))) atomicOr(err, ERR_NONFINITE_OUTPUT);
     }
 }
 
@@ -673,18 +674,18 @@ std::vector<int3> project_tiles(const std::vector<int32_t> &pair_index, int lmax
     return t;
 }
 
-void launch_project_mixed(const Plan &p, const float2 *Adf, int64_t ldA, const float2 *CT,
-                          const int64_t *noff, const int32_t *pair_index, double scale, const double *mu,
-                          double *smean, const double *ralm, int window_kind, const double *w_ln, double *out,
-                          cudaStream_t st) {
-    if (ralm) {
-        k_mean_proj<<<(unsigned)((p.npairs + 3) / 4), 128, 0, st>>>(p.d_coef, p.npairs, p.nbasis, mu, smean);
-        note_launch();
-    }
+void launch_mean_proj(const Plan &p, const double *mu, double *smean, cudaStream_t st) {
+    k_mean_proj<<<(unsigned)((p.npairs + 3) / 4), 128, 0, st>>>(p.d_coef, p.npairs, p.nbasis, mu, smean);
+    note_launch();
+}
+
+void launch_project_mixed(const Plan &p, const float2 *Adf, int64_t ldA, const float2 *CT, const int64_t *noff,
+                          const int32_t *pair_index, double scale, const double *smean, const double *ralm,
+                          int window_kind, const double *w_ln, double *out, int *err, cudaStream_t st) {
     if (p.n_proj_tiles <= 0) return;
     k_project_mixed<PJ_KS><<<(unsigned)p.n_proj_tiles, 32 * PJ_KS, 0, st>>>(
         Adf, ldA, p.nbasis, CT, (int)p.nmax, p.lmax, p.d_proj_tiles, noff, pair_index, scale, smean, ralm, window_kind,
-        w_ln, out);
+        w_ln, out, err);
     note_launch();
 }
 

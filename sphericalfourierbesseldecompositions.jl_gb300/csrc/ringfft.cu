@@ -11,6 +11,8 @@
 // aliasing (bin m mod n) and the ring phase e^{-i m phi0}, which is the exact
 // ring sum that libsharp's map2alm performs (reference call site
 // src/healpix_helpers.jl:55).
+#include <algorithm>
+
 #include "sfb_internal.h"
 
 namespace sfb {
@@ -384,16 +386,23 @@ static void ring_analysis_t(const Plan &p, const TI *maps, int64_t nmaps, T *F, 
     struct Group { int r0, nr; size_t n; bool two; } groups[2] = {
         {0, ns - 1, (size_t)(4 * (ns - 1)), true},
         {ns - 1, ns + 1, (size_t)(4 * ns), !pow2}};
-    for (const Group &gr : groups) {
-        if (gr.nr <= 0) continue;
-        const int MT = ring_mt(gr.n, sizeof(cx<T>), gr.two);
-        const size_t smem = ring_smem(gr.n, sizeof(cx<T>), gr.two, MT);
+    auto go = [&](int r0, int nr, size_t n, bool two) {
+        const int MT = (int)std::min<int64_t>(ring_mt(n, sizeof(cx<T>), two), nmaps);
+        const size_t smem = ring_smem(n, sizeof(cx<T>), two, MT);
         set_smem(k_ring_analysis<T, TI, TW>, smem);
-        dim3 grid((unsigned)gr.nr, (unsigned)((nmaps + MT - 1) / MT));
+        dim3 grid((unsigned)nr, (unsigned)((nmaps + MT - 1) / MT));
         k_ring_analysis<T, TI, TW><<<grid, 256, smem, st>>>(p.d_rings, (int)p.nrn, p.lmax, p.npix, maps, nmaps, MT,
-                                                            F, 2 * nmaps, gr.r0, tw, p.d_twoff, wph, nzr);
+                                                            F, 2 * nmaps, r0, tw, p.d_twoff, wph, nzr);
         note_launch();
+    };
+    // two maps or fewer leave most of the chip to the other group: both in one launch (the mixed transform's
+    // reference maps at nside 128: 72 us in two launches)
+    if (nmaps <= 2 && ns > 1 && ring_smem((size_t)(4 * ns), sizeof(cx<T>), true, (int)nmaps) <= 112 * 1024) {
+        go(0, 2 * ns, (size_t)(4 * ns), true);
+        return;
     }
+    for (const Group &gr : groups)
+        if (gr.nr > 0) go(gr.r0, gr.nr, gr.n, gr.two);
 }
 
 // More than four FP64 maps go through the tensor cores (a row tile of them takes 64 maps; four maps or fewer

@@ -225,9 +225,12 @@ void launch_legendre_table(const Plan &p, cudaStream_t st);
 // ring_live (mixed precision with a reference map): receives a device array of 4 nside - 1 ints, 1 for the
 // rings that hold a galaxy; the basis maps are left unwritten on the other rings (they are zero there),
 // and the ring DFT must be given the array (launch_ring_analysis_tc) so that it does not read them.
+// w01 / mask_df (with ref): the window's reference map is copied to ref[npix ..] and, when mask_df is given, laid
+// out there as a double-float map.  mu_ready (if given) is recorded on st once mu is complete.
 int deposit_sorted(Plan &p, const double *rtp, const double *w, int64_t ngal, double *maps, double *ref,
                    double *mu, cudaEvent_t ref_ready, cudaStream_t st, const cudaEvent_t *chunk_ready = nullptr,
-                   int nchunks = 0, const int **ring_live = nullptr);
+                   int nchunks = 0, const int **ring_live = nullptr, const double *w01 = nullptr,
+                   float2 *mask_df = nullptr, cudaEvent_t mu_ready = nullptr);
 
 // 0-based ring (1 .. 4 nside - 1 minus one) of a RING-scheme pixel
 __host__ __device__ __forceinline__ int ring_of_pixel(int64_t nside, int64_t pix) {
@@ -249,10 +252,11 @@ void launch_add_mean(double *A, int64_t ldA, int64_t nmaps, const double *mu, co
 // Mixed-precision radial projection (double-float sums; FP64 mean and window
 // terms), replacing add_mean + project_poly for the data term.
 void launch_coef_df(const Plan &p, const int32_t *pair_index, float2 *CT, cudaStream_t st);
-void launch_project_mixed(const Plan &p, const float2 *Adf, int64_t ldA, const float2 *CT,
-                          const int64_t *noff, const int32_t *pair_index, double scale, const double *mu,
-                          double *smean, const double *ralm, int window_kind, const double *w_ln, double *out,
-                          cudaStream_t st);
+void launch_mean_proj(const Plan &p, const double *mu, double *smean, cudaStream_t st);     // smean of the next
+// err (optional): ERR_NONFINITE_OUTPUT is raised there for a non-finite coefficient
+void launch_project_mixed(const Plan &p, const float2 *Adf, int64_t ldA, const float2 *CT, const int64_t *noff,
+                          const int32_t *pair_index, double scale, const double *smean, const double *ralm,
+                          int window_kind, const double *w_ln, double *out, int *err, cudaStream_t st);
 // maps[j] -= nu[j] ref with nu[j] = <maps[j], ref> / <ref, ref> (FP64, in place).
 void launch_split_mean(double *maps, int64_t nmaps, int64_t npix, const double *ref, double *nu, cudaStream_t st);
 // nzr (FP64): receives the first / last ring pair holding a non-zero value in any map
@@ -263,9 +267,9 @@ constexpr int WMIX_LMAX = 128;
 size_t wmix_smem_bytes(int l, int lp, int64_t nr, int neg_m);
 void launch_wmix(const Plan &p, const int64_t *noff, const double *gtab, int64_t nr, double rmin, double dr,
                  const double *WT, int64_t ldW, int LW, int neg_m, double *out, size_t smem, cudaStream_t st);
-// Exclusive prefix sum of n int32 counters in place; tile_sums holds scan_tile_count(n) ints.
+// Exclusive prefix sum of n int32 counters in place; tile_sums holds scan_tile_count(n) ints, *done is zero.
 int64_t scan_tile_count(int64_t n);
-void launch_exclusive_scan(int32_t *data, int64_t n, int32_t *tile_sums, cudaStream_t st);
+void launch_exclusive_scan(int32_t *data, int64_t n, int32_t *tile_sums, int *done, cudaStream_t st);
 void launch_ring_analysis(Plan &p, const double *maps, int64_t nmaps, double *F, cudaStream_t st, int *nzr = nullptr);
 void launch_ring_synthesis(Plan &p, const double *G, int64_t nmaps, double *maps, cudaStream_t st);
 // The same for many FP64 maps on the tensor cores (ring64_tc.cu); false: nothing was launched (no tables or no
@@ -278,6 +282,9 @@ bool launch_ring_synthesis64(Plan &p, const double *G, int64_t nmaps, void *out,
 void launch_leg_analysis(const Plan &p, const double *F, int64_t ncol, double *A, bool accumulate,
                          cudaStream_t st, int rlim = -1, const int *nzr = nullptr);
 void launch_leg_synthesis(const Plan &p, const double *A, int64_t ncol, double *G, cudaStream_t st, int rlim = -1);
+// Gram update and aliased rings' synthesis of one FP64 refinement step for 2, 4 or 8 columns (else false).
+bool launch_refine_narrow64(const Plan &p, const double *A, const double *A0, int64_t ncol, double *G, double *Anew,
+                            cudaStream_t st);
 // FP64 Gram refinement step (any column count); false when the plan has no Gram tables
 bool launch_gram_update_fp64(const Plan &p, const double *Acur, const double *A0, int64_t ncol, double *Anew,
                              cudaStream_t st);

@@ -103,7 +103,7 @@ int check_args(int64_t nside, const double *win, int64_t nr, double rmin, double
     return SFB_OK;
 }
 
-// Device-pointer core: workspace ws holds [flags ngal + 1][tile sums][max: 1 u64][err: 1 int].
+// Device-pointer core: workspace ws holds [flags ngal + 1][tile sums][max: 1 u64][err: 1 int][scan counter: 1 int].
 int run(int64_t nside, const double *win, int64_t nr, double rmin, double rmax, double dr, const double *rtp,
         int64_t ngal, const double *uniform, uint64_t seed, double *out, int64_t *nkept, char *ws, cudaStream_t st) {
     const int64_t npix = 12 * nside * nside;
@@ -112,14 +112,14 @@ int run(int64_t nside, const double *win, int64_t nr, double rmin, double rmax, 
     const int64_t ntiles = scan_tile_count(ngal + 1);
     unsigned long long *mx = reinterpret_cast<unsigned long long *>(ws + (((ngal + 1 + ntiles) * 4 + 15) / 16) * 16);
     int *err = reinterpret_cast<int *>(mx + 1);
-    SFB_CUDA_TRY(cudaMemsetAsync(mx, 0, sizeof(unsigned long long) + sizeof(int), st));
+    SFB_CUDA_TRY(cudaMemsetAsync(mx, 0, sizeof(unsigned long long) + 2 * sizeof(int), st));
     k_window_max<<<608, 256, 0, st>>>(win, nr * npix, mx, err);
     note_launch();
     k_window_flags<<<(unsigned)((ngal + 255) / 256), 256, 0, st>>>(rtp, ngal, win, nr, nside, rmin, rmax, dr, uniform,
                                                                    seed, mx, flags, err);
     note_launch();
     SFB_CUDA_TRY(cudaMemsetAsync(flags + ngal, 0, sizeof(int32_t), st));
-    launch_exclusive_scan(flags, ngal + 1, tsum, st);
+    launch_exclusive_scan(flags, ngal + 1, tsum, err + 1, st);
     k_window_scatter<<<(unsigned)((ngal + 255) / 256), 256, 0, st>>>(rtp, ngal, flags, out);
     note_launch();
     int32_t h[2] = {0, 0};
