@@ -339,8 +339,9 @@ __global__ void __launch_bounds__(NTHR, 1) k_ring_dft_tc(const float2 *__restric
             const int64_t qo = pair0 + pr;
             if (mm > lmax || qo >= npairs) continue;
             const int oring = cls_rings[rb + (int)(qo / nmaps)];
-            // unread spectra (outside the span of ring pairs with data, or dead) are not written
-            if (span && (oring < span[0] || oring > span[1])) continue;
+            // unread spectra (outside the span of ring pairs with data, or dead) are not written; the analysis
+            // reads the span in whole chunks of 16 ring pairs, so those at its ends are
+            if (span && (oring < (span[0] & ~15) || oring > (span[1] | 15))) continue;
             if (dead && dead[(int64_t)oring * ntn + u]) continue;
             *reinterpret_cast<float4 *>(F + ((int64_t)(sg * L1 + mm) * nrn + oring) * ldF + 2 * (qo % nmaps)) =
                 make_float4(0.f, 0.f, 0.f, 0.f);

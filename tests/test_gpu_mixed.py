@@ -202,3 +202,27 @@ def test_bounded_wait_times_out_and_context_survives():
     rtp, w = catalogue(1000, a.rmin, a.rmax, seed=4)
     out = sfbgpu.cat2amln(rtp, a, 1e-4, None, None, precision="mixed")
     assert np.all(np.isfinite(out))
+
+
+@pytest.mark.parametrize("zlim", [(0.5, 1.0), (-0.3, 0.3), (-1.0, -0.6)])
+def test_partial_sky_after_other_map_counts(zlim):
+    """A partial-sky catalogue on a plan whose buffers hold another transform's
+    spectra (a full-sky field of more shells than the catalogue has maps): the
+    first analysis pass reads whole chunks of ring pairs, so the spectra at the
+    ends of the survey's span must have been written by this call.  Same
+    kernels on the same inputs: the deposit's run-to-run rounding, 1e-9."""
+    def plan():
+        return sfbgpu.AnlmModes(0.05, 500.0, 1000.0, nside=32)
+
+    a = plan()
+    rng = np.random.default_rng(70)
+    n = 20_000
+    r = np.cbrt(a.rmin ** 3 + rng.random(n) * (a.rmax ** 3 - a.rmin ** 3))
+    rtp = np.stack([r, np.arccos(rng.uniform(*zlim, n)), rng.uniform(0, 2 * np.pi, n)])
+    fresh = sfbgpu.cat2amln(rtp, a, 1e-5, None, None, precision="mixed")
+    b = plan()
+    wm = sfbgpu.ConfigurationSpaceModes(b.rmin, b.rmax, 90, 32)
+    f = np.asfortranarray(rng.normal(size=(90, wm.npix)) * 1e3)
+    sfbgpu.field2anlm(f, wm, b, precision="mixed")
+    got = sfbgpu.cat2amln(rtp, b, 1e-5, None, None, precision="mixed")
+    assert rel_err(got, fresh) < 1e-9
