@@ -143,13 +143,24 @@ __device__ __forceinline__ int slot_of(double r, double rmin, double rmax, doubl
     return slot;
 }
 
-// Keys of galaxies [0, ngal) of this chunk (global index gbase + i).  A galaxy
+// Mock of galaxy i (global index): the last j with off[j] <= i.
+__device__ __forceinline__ int mock_of(const Mocks &mk, int64_t i) {
+    int lo = 0, hi = mk.n;
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (mk.off[mid] <= i) lo = mid;
+        else hi = mid;
+    }
+    return lo;
+}
+
+// Keys of galaxies [0, ngal) of this chunk (global index gbase + i); mock j's slots are j (pieces + 2) + ....  A galaxy
 // whose pixel the FP32 evaluation cannot settle goes to fb_list with key
 // -2 - slot, and gets its key and rank from k_deposit_keys_fallback (FP64
 // pixel), so no warp runs the FP64 pixel path for one lane.
 __global__ void k_deposit_keys(const double *__restrict__ rtp, const double *__restrict__ wgt, int64_t ngal,
                                int64_t gbase, int64_t nside, int64_t npix, double rmin, double rmax,
-                               double inv_width, int pieces, int32_t *__restrict__ counts,
+                               double inv_width, int pieces, Mocks mk, int32_t *__restrict__ counts,
                                int32_t *__restrict__ key, int32_t *__restrict__ rank, double *__restrict__ xloc,
                                int32_t *__restrict__ fb_list, int32_t *__restrict__ fb_count, int *err) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -164,7 +175,7 @@ __global__ void k_deposit_keys(const double *__restrict__ rtp, const double *__r
         atomicOr(err, ERR_THETA_RANGE);
     } else {
         const int64_t pix = ang2pix_ring_try(nside, th, ph);
-        const int slot = slot_of(r, rmin, rmax, inv_width, pieces, x);
+        const int slot = slot_of(r, rmin, rmax, inv_width, pieces, x) + mock_of(mk, gbase + i) * (pieces + 2);
         if (pix >= 0) {
             k = (int32_t)(slot * npix + pix);
             rank[i] = atomicAdd(counts + k, 1);
@@ -191,7 +202,7 @@ struct RadialKeyParams {
 
 __global__ void k_deposit_keys_mixed(const double *__restrict__ rtp, const double *__restrict__ wgt, int64_t ngal,
                                      int64_t gbase, int64_t nside, int64_t npix, RadialKeyParams rk, int pieces,
-                                     int32_t *__restrict__ counts, int32_t *__restrict__ key,
+                                     Mocks mk, int32_t *__restrict__ counts, int32_t *__restrict__ key,
                                      int32_t *__restrict__ rank, float2 *__restrict__ xdf,
                                      int32_t *__restrict__ fb_list, int32_t *__restrict__ fb_count, int *err) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -226,6 +237,7 @@ __global__ void k_deposit_keys_mixed(const double *__restrict__ rtp, const doubl
                 if (xx.hi < -1.f || (xx.hi == -1.f && xx.lo < 0.f)) xx = {-1.f, 0.f};
                 x = make_float2(xx.hi, xx.lo);
             }
+            slot += mock_of(mk, gbase + i) * (pieces + 2);
             const long long phabs = __double_as_longlong(ph) & 0x7fffffffffffffffll;
             const int64_t pix = (nside <= (int64_t(1) << 16) && phabs <= ORD_4PI)
                                     ? ang2pix_ring_try32(nside, df_of_bits(th).hi, df_of_bits(ph).hi)
@@ -448,6 +460,9 @@ __global__ void __launch_bounds__(128) k_deposit_moments(const int32_t *__restri
     extern __shared__ double out_s[];                  // [deg + 1][128]
     __shared__ int hist[64];
     __shared__ int perm[128];
+    // grid.y: mocks
+    offset += (int64_t)blockIdx.y * (pieces + 2) * npix;
+    maps += (int64_t)blockIdx.y * nbasis * npix;
     const int t = threadIdx.x;
     const int64_t nkeys = (int64_t)(pieces + 2) * npix;
     const int64_t bt = (int64_t)blockIdx.x * 128 + t;
@@ -540,6 +555,13 @@ template <int MAXDEG>
 __global__ void k_deposit_moments_df(const int32_t *__restrict__ offset, const float4 *__restrict__ sorted,
                                      int64_t npix, int pieces, int deg, int64_t nbasis, const float2 *__restrict__ cdf,
                                      const float2 *__restrict__ mudf, float2 *__restrict__ maps) {
+    // grid.y: mocks
+    offset += (int64_t)blockIdx.y * (pieces + 2) * npix;
+    maps += (int64_t)blockIdx.y * nbasis * npix;
+    if (cdf) {
+        cdf += blockIdx.y * npix;
+        mudf += blockIdx.y * nbasis;
+    }
     const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t nkeys = (int64_t)(pieces + 2) * npix;
     if (idx >= nkeys) return;
@@ -594,6 +616,14 @@ __global__ void __launch_bounds__(128) k_deposit_moments_bal(const int32_t *__re
     __shared__ int hist[64];
     __shared__ int perm[128];
     __shared__ float2 out[(MAXDEG + 1) * 128];
+    // grid.y: mocks
+    offset += (int64_t)blockIdx.y * (pieces + 2) * npix;
+    maps += (int64_t)blockIdx.y * nbasis * npix;
+    if (cdf) {
+        cdf += blockIdx.y * npix;
+        mudf += blockIdx.y * nbasis;
+    }
+    if (ring_live) ring_live += blockIdx.y * (4 * nside - 1);
     const int t = threadIdx.x;
     const int64_t nkeys = (int64_t)(pieces + 2) * npix;
     const int64_t B0 = (int64_t)blockIdx.x * 128;
@@ -737,6 +767,14 @@ __global__ void __launch_bounds__(128, 8) k_deposit_moments_sm(const int32_t *__
     __shared__ int hist[64];
     __shared__ int perm[128];
     __shared__ __align__(16) float2 acc_s[(MAXDEG + 1) * 128];
+    // grid.y: mocks
+    offset += (int64_t)blockIdx.y * (pieces + 2) * npix;
+    maps += (int64_t)blockIdx.y * nbasis * npix;
+    if (cdf) {
+        cdf += blockIdx.y * npix;
+        mudf += blockIdx.y * nbasis;
+    }
+    if (ring_live) ring_live += blockIdx.y * (4 * nside - 1);
     const int t = threadIdx.x;
     const int64_t nkeys = (int64_t)(pieces + 2) * npix;
     const int64_t B0 = (int64_t)blockIdx.x * 128;
@@ -830,6 +868,12 @@ __global__ void __launch_bounds__(32) k_deposit_stats(const int32_t *__restrict_
                                                       double *S, double *Q, double *__restrict__ mu,
                                                       float2 *__restrict__ mudf, int *done) {
     __shared__ float2 red[32][MAXDEG + 3];
+    // grid.y: mocks
+    offset += (int64_t)blockIdx.y * (pieces + 2) * npix;
+    cdf += blockIdx.y * npix;
+    double *const S0 = S, *const Q0 = Q;
+    S += blockIdx.y * nbasis;
+    Q += blockIdx.y * (pieces + 2);
     const int lane = threadIdx.x;
     const int64_t idx = (int64_t)blockIdx.x * STATS_STRIDE * 32 + lane;
     const int64_t nkeys = (int64_t)(pieces + 2) * npix;
@@ -874,16 +918,17 @@ __global__ void __launch_bounds__(32) k_deposit_stats(const int32_t *__restrict_
     __threadfence();
     __syncwarp();
     int last = 0;
-    if (lane == 0) last = atomicAdd(done, 1) == (int)gridDim.x - 1;
+    if (lane == 0) last = atomicAdd(done, 1) == (int)(gridDim.x * gridDim.y) - 1;
     if (!__shfl_sync(full, last, 0)) return;
     __threadfence();
     const int64_t npoly = (int64_t)pieces * (deg + 1);
-    for (int64_t b = lane; b < nbasis; b += 32) {
+    for (int64_t i = lane; i < nbasis * gridDim.y; i += 32) {
+        const int64_t mock = i / nbasis, b = i - mock * nbasis;
         const int sl = b < npoly ? (int)(b / (deg + 1)) : pieces + (int)(b - npoly);
-        const double q = __ldcg(Q + sl), v = q > 0.0 ? __ldcg(S + b) / q : 0.0;
-        mu[b] = v;
+        const double q = __ldcg(Q0 + mock * (pieces + 2) + sl), v = q > 0.0 ? __ldcg(S0 + i) / q : 0.0;
+        mu[i] = v;
         const float h = (float)v;
-        mudf[b] = make_float2(h, (float)(v - (double)h));
+        mudf[i] = make_float2(h, (float)(v - (double)h));
     }
 }
 
@@ -891,22 +936,19 @@ __global__ void __launch_bounds__(32) k_deposit_stats(const int32_t *__restrict_
 // the mixed deposit), in double-float from the sorted pairs, stored as the
 // FP64 value hi + lo (exact) and as the pair itself.
 // ring_live[ring] is set to 1 for every ring holding a galaxy (preset to 0).
-// The window's reference map W01 goes beside C (C[npix + pix]) and, for a
-// separable window, as a double-float map to mask_df.
+// The window's reference map W01 goes behind the count maps.
 __global__ void k_weight_map_mixed(const int32_t *__restrict__ offset, const float4 *__restrict__ sorted,
                                    int64_t nside, int64_t npix, int nslots, double *__restrict__ C,
                                    float2 *__restrict__ cdf, int *__restrict__ ring_live,
-                                   const double *__restrict__ W01, float2 *__restrict__ mask_df) {
+                                   const double *__restrict__ W01) {
     const int64_t pix = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (pix >= npix) return;
-    if (W01) {
-        const double v = W01[pix];
-        C[npix + pix] = v;
-        if (mask_df) {
-            const float h = (float)v;
-            mask_df[pix] = make_float2(h, (float)(v - (double)h));
-        }
-    }
+    // grid.y: mocks
+    if (W01 && blockIdx.y == 0) C[gridDim.y * npix + pix] = W01[pix];
+    offset += (int64_t)blockIdx.y * nslots * npix;
+    C += blockIdx.y * npix;
+    cdf += blockIdx.y * npix;
+    ring_live += blockIdx.y * (4 * nside - 1);
     dfl s = {0.f, 0.f};
     bool any = false;
     for (int sl = 0; sl < nslots; ++sl) {
@@ -925,10 +967,10 @@ __global__ void k_weight_map_mixed(const int32_t *__restrict__ offset, const flo
 
 // FP64 path: double (x, w); mixed: double-float pairs and the count map as cdf
 template <int MAXDEG>
-static void launch_moments(const Plan &p, const int32_t *counts, const void *sorted, const float2 *cdf,
+static void launch_moments(const Plan &p, int nmock, const int32_t *counts, const void *sorted, const float2 *cdf,
                            const float2 *mudf, double *maps, cudaStream_t st, const int *ring_live) {
     const int64_t nkeys = (int64_t)(p.pieces + 2) * p.npix;
-    const unsigned blocks = (unsigned)((nkeys + 127) / 128);
+    const dim3 blocks((unsigned)((nkeys + 127) / 128), (unsigned)nmock);
     const float4 *s4 = static_cast<const float4 *>(sorted);
     float2 *mf = reinterpret_cast<float2 *>(maps);
     bool done = false;
@@ -957,11 +999,11 @@ static void launch_moments(const Plan &p, const int32_t *counts, const void *sor
 }
 
 template <int MAXDEG>
-static void launch_stats(const Plan &p, const int32_t *counts, const float4 *sorted, const float2 *cdf, double *S,
+static void launch_stats(const Plan &p, int nmock, const int32_t *counts, const float4 *sorted, const float2 *cdf, double *S,
                          double *Q, double *mu, float2 *mudf, int *done, cudaStream_t st) {
     const int64_t nkeys = (int64_t)(p.pieces + 2) * p.npix;
     const int64_t blocks = (nkeys + 32 * STATS_STRIDE - 1) / (32 * STATS_STRIDE);
-    k_deposit_stats<MAXDEG><<<(unsigned)blocks, 32, 0, st>>>(counts, sorted, p.npix, p.pieces, p.degree, p.nbasis,
+    k_deposit_stats<MAXDEG><<<dim3((unsigned)blocks, (unsigned)nmock), 32, 0, st>>>(counts, sorted, p.npix, p.pieces, p.degree, p.nbasis,
                                                               cdf, S, Q, mu, mudf, done);
     note_launch();
 }
@@ -985,22 +1027,24 @@ void launch_exclusive_scan(int32_t *data, int64_t n, int32_t *tile_sums, int *do
     note_launch();
 }
 
-int deposit_sorted(Plan &p, const double *rtp, const double *w, int64_t ngal, double *maps, double *ref,
-                   double *mu, cudaEvent_t ref_ready, cudaStream_t st, const cudaEvent_t *chunk_ready,
-                   int nchunks, const int **ring_live, const double *w01, float2 *mask_df, cudaEvent_t mu_ready) {
+int deposit_sorted(Plan &p, const DepositArgs &a, cudaStream_t st, const int **ring_live) {
     const bool mixed = p.precision == SFB_MIXED;
-    if (ring_live) *ring_live = nullptr;
-    const int64_t nkeys = (int64_t)(p.pieces + 2) * p.npix;
+    const double *rtp = a.rtp, *w = a.w;
+    const int64_t ngal = a.ngal, nmock = a.mocks.n;
+    double *ref = a.ref, *mu = a.mu;
+    *ring_live = nullptr;
+    const int64_t nkeys = nmock * (p.pieces + 2) * p.npix;
+    if (nkeys > 0x7fffffff || ngal > 0x7fffffff) return fail(SFB_EINVAL, "catalogue or key range above 2^31 - 1");
     const int64_t nscan = nkeys + 1;            // one extra counter: its exclusive prefix is the total
     const int64_t ntiles = (nscan + SCAN_TILE - 1) / SCAN_TILE;
     // workspace: first what one clear presets to zero: counters/offsets [nscan] int32, three block counters and
-    // the length of the FP64-pixel list, ring_live [nrings] int32, S [nbasis], Q [pieces + 2]; then mudf [nbasis]
-    // float2, cdf [npix] float2, local coordinate [ngal] double (mixed: float2), sorted (x, w) [ngal] double2
+    // the length of the FP64-pixel list, ring_live [nmock][nrings] int32, S [nmock][nbasis], Q [nmock][pieces + 2];
+    // then mudf [nmock][nbasis] float2, cdf [nmock][npix] float2, local coordinate [ngal] double (mixed: float2), sorted (x, w) [ngal] double2
     // (mixed: float4), tile sums [ntiles], key, rank and the FP64-pixel list [ngal] int32
     const int64_t nrings = 4 * p.nside - 1;
-    const int64_t off_S = (nscan + 4 + nrings + 1) / 2;
-    const int64_t off_mudf = off_S + p.nbasis + p.pieces + 2, off_cdf = off_mudf + p.nbasis;
-    const int64_t off_x = off_cdf + p.npix;
+    const int64_t off_S = (nscan + 4 + nmock * nrings + 1) / 2;
+    const int64_t off_mudf = off_S + nmock * (p.nbasis + p.pieces + 2), off_cdf = off_mudf + nmock * p.nbasis;
+    const int64_t off_x = off_cdf + nmock * p.npix;
     int64_t off_sorted = off_x + ngal;
     off_sorted += off_sorted & 1;
     const int64_t off_int = off_sorted + 2 * ngal;
@@ -1009,7 +1053,7 @@ int deposit_sorted(Plan &p, const double *rtp, const double *w, int64_t ngal, do
     int *scan_done = counts + nscan, *stats_done = scan_done + 1;
     int32_t *fb_count = scan_done + 2;
     int *live = scan_done + 4;
-    double *S = p.dep.ptr + off_S, *Q = S + p.nbasis;
+    double *S = p.dep.ptr + off_S, *Q = S + nmock * p.nbasis;
     float2 *mudf = reinterpret_cast<float2 *>(p.dep.ptr + off_mudf);
     float2 *cdf = reinterpret_cast<float2 *>(p.dep.ptr + off_cdf);
     double *xloc = p.dep.ptr + off_x;
@@ -1030,20 +1074,20 @@ int deposit_sorted(Plan &p, const double *rtp, const double *w, int64_t ngal, do
     rk.invw_hi = (float)inv_width;
     rk.invw_lo = (float)(inv_width - (double)rk.invw_hi);
     // keys: in nchunks galaxy ranges, each after its event (the host entry's copy pipeline), or at once
-    const int nck = (chunk_ready && nchunks > 0) ? nchunks : 1;
+    const int nck = (a.chunk_ready && a.nchunks > 0) ? a.nchunks : 1;
     const int64_t per = (ngal + nck - 1) / nck;
     for (int c = 0; c < nck; ++c) {
         const int64_t g0 = c * per, n = std::min<int64_t>(per, ngal - g0);
-        if (chunk_ready && nchunks > 0) SFB_CUDA_TRY(cudaStreamWaitEvent(st, chunk_ready[c], 0));
+        if (a.chunk_ready && a.nchunks > 0) SFB_CUDA_TRY(cudaStreamWaitEvent(st, a.chunk_ready[c], 0));
         if (n <= 0) continue;
         const unsigned nb = (unsigned)((n + 255) / 256);
         if (mixed)
             k_deposit_keys_mixed<<<nb, 256, 0, st>>>(rtp + 3 * g0, w ? w + g0 : nullptr, n, g0, p.nside, p.npix, rk,
-                                                     p.pieces, counts, key + g0, rank + g0, xdf + g0, fb_list,
+                                                     p.pieces, a.mocks, counts, key + g0, rank + g0, xdf + g0, fb_list,
                                                      fb_count, p.d_err);
         else
             k_deposit_keys<<<nb, 256, 0, st>>>(rtp + 3 * g0, w ? w + g0 : nullptr, n, g0, p.nside, p.npix, p.rmin,
-                                               p.rmax, inv_width, p.pieces, counts, key + g0, rank + g0, xloc + g0,
+                                               p.rmax, inv_width, p.pieces, a.mocks, counts, key + g0, rank + g0, xloc + g0,
                                                fb_list, fb_count, p.d_err);
         note_launch();
     }
@@ -1064,19 +1108,19 @@ int deposit_sorted(Plan &p, const double *rtp, const double *w, int64_t ngal, do
     if (p.degree > 63) return fail(SFB_ENOTSUP, "radial degree above 63 is not supported by the sorted deposit");
     const bool split = ref != nullptr && mixed;
     if (split) {
-        k_weight_map_mixed<<<(unsigned)((p.npix + 255) / 256), 256, 0, st>>>(counts, sorted4, p.nside, p.npix,
-                                                                            p.pieces + 2, ref, cdf, live, w01, mask_df);
+        k_weight_map_mixed<<<dim3((unsigned)((p.npix + 255) / 256), (unsigned)nmock), 256, 0, st>>>(
+            counts, sorted4, p.nside, p.npix, p.pieces + 2, ref, cdf, live, a.w01);
         note_launch();
-        if (ref_ready) SFB_CUDA_TRY(cudaEventRecord(ref_ready, st));
+        if (a.ref_ready) SFB_CUDA_TRY(cudaEventRecord(a.ref_ready, st));
         by_degree(p.degree, [&](auto D) {
-            launch_stats<decltype(D)::value>(p, counts, sorted4, cdf, S, Q, mu, mudf, stats_done, st);
+            launch_stats<decltype(D)::value>(p, (int)nmock, counts, sorted4, cdf, S, Q, mu, mudf, stats_done, st);
         });
-        if (mu_ready) SFB_CUDA_TRY(cudaEventRecord(mu_ready, st));
+        if (a.mu_ready) SFB_CUDA_TRY(cudaEventRecord(a.mu_ready, st));
     }
     // moments in FP64 (FP64 path) or double-float (mixed); stored in the transform's precision
-    const bool skip_empty = split && ring_live && p.npix >= 128 && p.degree <= 31;   // the balanced kernel
+    const bool skip_empty = split && p.npix >= 128 && p.degree <= 31;                 // the balanced kernel
     by_degree(p.degree, [&](auto D) {
-        launch_moments<decltype(D)::value>(p, counts, sorted, split ? cdf : nullptr, mudf, maps, st,
+        launch_moments<decltype(D)::value>(p, (int)nmock, counts, sorted, split ? cdf : nullptr, mudf, a.maps, st,
                                            skip_empty ? live : nullptr);
     });
     if (skip_empty) *ring_live = live;

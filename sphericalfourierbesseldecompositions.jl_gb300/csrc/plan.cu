@@ -337,11 +337,11 @@ void synthesis_and_gram64(const Plan &p, const double *A, const double *A0, int6
 
 // fp64_out: the FP64 a_lm (alm) is wanted besides the double-float copy (almdf, mixed precision); the
 // Gram refinement carries only the double-float one and converts at the end when asked.
-// ring_live / nlive (mixed precision): rings marked 0 hold zeros in maps [0, nlive), left unwritten by the
-// deposit (deposit_sorted's ring_live).
+// ring_live / nper (mixed precision): rings marked 0 hold zeros, left unwritten by the deposit (deposit_sorted's
+// ring_live), one array per nper maps.
 int sht_analysis(sfb_plan *h, const double *maps, int64_t nm, cudaStream_t st, bool maps_are_fp64 = false,
                  int stage_override = -1, const ShtWork *ws = nullptr, bool fp64_out = true,
-                 const int *ring_live = nullptr, int64_t nlive = 0) {
+                 const int *ring_live = nullptr, int64_t nper = 1) {
     Plan &p = h->p;
     const ShtWork own{&p.fbuf, &p.gbuf, &p.rbuf, &p.alm};
     if (!ws) ws = &own;
@@ -377,7 +377,7 @@ int sht_analysis(sfb_plan *h, const double *maps, int64_t nm, cudaStream_t st, b
         const bool skip_unread = (nm > 4 && p.d_gramts && p.niter > 0) || p.niter == 0;
         SFB_TRY(launch_ring_analysis_tc(p, reinterpret_cast<const float2 *>(maps), nm,
                                         reinterpret_cast<float2 *>(fbuf.ptr), reinterpret_cast<int *>(p.erow.ptr), nzr,
-                                        st, ring_live, nlive, skip_unread));
+                                        st, ring_live, nper, skip_unread));
     } else {
         // many columns: the FFT records the span of ring pairs with data, over which the
         // first analysis pass sums (the spectra are zero elsewhere)
@@ -611,26 +611,29 @@ int64_t chunk_pairs(const Plan &p) {
     return c;
 }
 
+// a_nlm of mocks.n catalogues (one, or the mocks of a group: mock j's result at out + 2 j nlmsize).
 // defer_finish (batched calls): the device error word is neither cleared nor read here and the
 // call does not wait for the device; the caller clears it once and checks it at the end.
-int cat2amln_dev(sfb_plan *h, const double *rtp, const double *w, int64_t ngal, double nbar, const sfb_window *win,
-                 double *out, cudaStream_t st, const cudaEvent_t *chunk_ready = nullptr, int nchunks = 0,
-                 bool defer_finish = false) {
+int cat2amln_dev(sfb_plan *h, const double *rtp, const double *w, int64_t ngal, const Mocks &mocks, const double *nbar,
+                 const sfb_window *win, double *out, cudaStream_t st, const cudaEvent_t *chunk_ready = nullptr,
+                 int nchunks = 0, bool defer_finish = false) {
     Plan &p = h->p;
     if (ngal < 0) return fail(SFB_EINVAL, "ngal < 0");
     if (!win) return fail(SFB_EINVAL, "window descriptor is NULL");
     if (ngal > 0 && !rtp) return fail(SFB_EINVAL, "rtp is NULL");
-    if (!(std::isfinite(nbar) && nbar != 0.0)) return fail(SFB_ENONFINITE, "nbar must be finite and non-zero");
+    const int nmock = mocks.n;
+    double scale[MOCKS_MAX];
+    for (int j = 0; j < nmock; ++j) {
+        if (!(std::isfinite(nbar[j]) && nbar[j] != 0.0)) return fail(SFB_ENONFINITE, "nbar must be finite and non-zero");
+        scale[j] = 1.0 / (nbar[j] * (4.0 * M_PI / (double)p.npix));
+    }
     const int wk = win->kind;
     if (wk != SFB_WINDOW_ZERO && wk != SFB_WINDOW_SEPARABLE && wk != SFB_WINDOW_DENSE)
         return fail(SFB_EINVAL, "unknown window kind");
     if (wk == SFB_WINDOW_SEPARABLE && !(win->mask && win->w_ln)) return fail(SFB_EINVAL, "separable window needs mask and w_ln");
     if (wk == SFB_WINDOW_DENSE && !win->dense) return fail(SFB_EINVAL, "dense window pointer is NULL");
-    const double dOmega = 4.0 * M_PI / (double)p.npix;
-    const double scale = 1.0 / (nbar * dOmega);
     if (!defer_finish) SFB_CUDA_TRY(cudaMemsetAsync(p.d_err, 0, sizeof(int), st));
     if (p.radial_mode == SFB_RADIAL_POLY) {
-        const int64_t nm = p.nbasis + (wk == SFB_WINDOW_SEPARABLE ? 1 : 0);
         // Mixed precision: the data maps are split into mu_b C + fluctuation
         // with C the weighted galaxy count map, the dense window maps into
         // nu W01 + fluctuation with W01 the window's (l=0, n=1) map; only the
@@ -638,58 +641,70 @@ int cat2amln_dev(sfb_plan *h, const double *rtp, const double *w, int64_t ngal, 
         // (or W01's) a_lm are computed in FP64, so the cancellation between
         // data and window term happens in FP64.
         const bool split = p.precision == SFB_MIXED && wk != SFB_WINDOW_ZERO;
+        // the basis maps of every mock; in FP64 the mask of a separable window is one map more
+        const bool mask_map = wk == SFB_WINDOW_SEPARABLE && !split;
+        const int64_t nb = p.nbasis, nm = nmock * nb + (mask_map ? 1 : 0);
         const double *W01 = wk == SFB_WINDOW_SEPARABLE ? win->mask : win->dense;
         const int64_t cp = wk == SFB_WINDOW_DENSE ? chunk_pairs(p) : 0;
         double *Cmap = nullptr, *mu = nullptr, *nu = nullptr, *smean = nullptr;
-        const double *ralm = nullptr;             // FP64 a_lm of (C, W01), [lmsize][4]
+        const double *ralm = nullptr;             // FP64 a_lm of (C of every mock, W01), [lmsize][2 nmock + 2]
         if (split) {
             // [C][W01][mu][nu][per-pair mean parts]
-            SFB_TRY(grow(p, p.ref, (size_t)(2 * p.npix + p.nbasis + cp + p.npairs)));
+            SFB_TRY(grow(p, p.ref, (size_t)((nmock + 1) * p.npix + nmock * (nb + p.npairs) + cp)));
             Cmap = p.ref.ptr;
-            mu = Cmap + 2 * p.npix;
-            nu = mu + p.nbasis;
+            mu = Cmap + (nmock + 1) * p.npix;
+            nu = mu + nmock * nb;
             smean = nu + cp;
         }
         SFB_TRY(grow(p, p.maps, (size_t)nm * p.npix));
         const int *ring_live = nullptr;          // rings the deposit wrote (mixed precision)
-        float2 *mask_df = nullptr;               // the mask as a map of the mixed transform (the deposit writes it)
-        if (wk == SFB_WINDOW_SEPARABLE) {
+        if (mask_map) {
             Stage s(h, SFB_STAGE_OTHER, st);
-            if (split)
-                mask_df = reinterpret_cast<float2 *>(p.maps.ptr) + p.nbasis * p.npix;
-            else
-                SFB_CUDA_TRY(cudaMemcpyAsync(p.maps.ptr + p.nbasis * p.npix, win->mask, p.npix * sizeof(double),
-                                             cudaMemcpyDeviceToDevice, st));
+            SFB_CUDA_TRY(cudaMemcpyAsync(p.maps.ptr + nmock * nb * p.npix, win->mask, p.npix * sizeof(double),
+                                         cudaMemcpyDeviceToDevice, st));
         }
         {
             Stage s(h, SFB_STAGE_DEPOSIT, st);
-            SFB_TRY(deposit_sorted(p, rtp, w, ngal, p.maps.ptr, Cmap, mu, split ? h->ev_fork : nullptr, st,
-                                   chunk_ready, nchunks, &ring_live, W01, mask_df, split ? h->ev_mu : nullptr));
+            DepositArgs a;
+            a.rtp = rtp;
+            a.w = w;
+            a.ngal = ngal;
+            a.mocks = mocks;
+            a.maps = p.maps.ptr;
+            a.ref = Cmap;
+            a.mu = mu;
+            a.w01 = W01;
+            a.ref_ready = split ? h->ev_fork : nullptr;
+            a.mu_ready = split ? h->ev_mu : nullptr;
+            a.chunk_ready = chunk_ready;
+            a.nchunks = nchunks;
+            SFB_TRY(deposit_sorted(p, a, st, &ring_live));
         }
         if (split) {
             // the FP64 transform of (C, W01) runs on the side stream, in its own workspace, beside
             // the rest of the deposit and the main transform; the projection waits for it
             SFB_CUDA_TRY(cudaStreamWaitEvent(h->side, h->ev_fork, 0));
-            SFB_TRY(reference_alm(h, Cmap, 2, h->side));
+            SFB_TRY(reference_alm(h, Cmap, nmock + 1, h->side));
             ralm = p.ralm.ptr;
             SFB_CUDA_TRY(cudaStreamWaitEvent(h->side, h->ev_mu, 0));
-            launch_mean_proj(p, mu, smean, h->side);
+            launch_mean_proj(p, mu, nmock, smean, h->side);
             SFB_CUDA_TRY(cudaEventRecord(h->ev_join, h->side));
         }
         // the mixed projection reads the double-float a_lm only
-        SFB_TRY(sht_analysis(h, p.maps.ptr, nm, st, false, -1, nullptr, p.precision != SFB_MIXED, ring_live,
-                             p.nbasis));
+        SFB_TRY(sht_analysis(h, p.maps.ptr, nm, st, false, -1, nullptr, p.precision != SFB_MIXED, ring_live, nb));
         if (split) SFB_CUDA_TRY(cudaStreamWaitEvent(st, h->ev_join, 0));
         {
             Stage s(h, SFB_STAGE_PROJECT, st);
             if (p.precision == SFB_MIXED)
                 launch_project_mixed(p, reinterpret_cast<const float2 *>(p.almdf.ptr), 2 * nm, p.d_coefT, h->d_noff,
-                                     h->d_pair_index, scale, smean, ralm, wk, win->w_ln, out,
+                                     h->d_pair_index, nmock, scale, smean, ralm, 2 * (nmock + 1), wk, win->w_ln, out,
                                      wk == SFB_WINDOW_DENSE ? nullptr : p.d_err, st);
             else
-                launch_project_poly(p, p.alm.ptr, 2 * nm, scale, wk, win->w_ln, p.nbasis, nullptr, 0, out, st);
+                for (int j = 0; j < nmock; ++j)
+                    launch_project_poly(p, p.alm.ptr + 2 * nb * j, 2 * nm, scale[j], wk, win->w_ln, nb * (nmock - j),
+                                        nullptr, 0, out + 2 * p.nlmsize * j, st);
         }
-        if (wk == SFB_WINDOW_DENSE) {
+        if (wk == SFB_WINDOW_DENSE) {             // one catalogue at a time
             SFB_TRY(grow(p, p.maps, (size_t)cp * p.npix));
             for (int64_t p0 = 0; p0 < p.npairs; p0 += cp) {
                 const int64_t npc = std::min(cp, p.npairs - p0);
@@ -709,7 +724,7 @@ int cat2amln_dev(sfb_plan *h, const double *rtp, const double *w, int64_t ngal, 
         for (int64_t p0 = 0; p0 < p.npairs; p0 += cp) {
             const int64_t npc = std::min(cp, p.npairs - p0);
             SFB_CUDA_TRY(cudaMemsetAsync(p.maps.ptr, 0, (size_t)npc * p.npix * sizeof(double), st));
-            { Stage s(h, SFB_STAGE_DEPOSIT, st); launch_deposit_spline_chunk(p, rtp, w, ngal, p0, npc, scale, p.maps.ptr, st); }
+            { Stage s(h, SFB_STAGE_DEPOSIT, st); launch_deposit_spline_chunk(p, rtp, w, ngal, p0, npc, scale[0], p.maps.ptr, st); }
             if (wk == SFB_WINDOW_DENSE) launch_subtract_dense_chunk(p, p.maps.ptr, win->dense, p0, npc, st);
             if (wk == SFB_WINDOW_SEPARABLE) launch_subtract_sep_chunk(p, p.maps.ptr, win->mask, win->w_ln, p0, npc, st);
             SFB_TRY(sht_analysis(h, p.maps.ptr, npc, st, true));
@@ -721,10 +736,23 @@ int cat2amln_dev(sfb_plan *h, const double *rtp, const double *w, int64_t ngal, 
     const bool checked = p.radial_mode == SFB_RADIAL_POLY && p.precision == SFB_MIXED && wk != SFB_WINDOW_DENSE;
     if (defer_finish) {
         Stage s(h, SFB_STAGE_OTHER, st);
-        if (!checked) launch_check_finite(out, 2 * p.nlmsize, p.d_err, st);
+        if (!checked) launch_check_finite(out, 2 * p.nlmsize * nmock, p.d_err, st);
         return SFB_OK;
     }
     return finish(h, out, st, checked);
+}
+
+// Mocks of [k, nmocks) that go through the kernels together.  Light mocks leave the chip idle and cost their
+// launches' latencies each; the limit is where one mock's maps fill it anyway (2^25 map pixels a group: twelve of
+// the mocks of nside 64 and 53 basis maps, one of nside 256), and 2^23 galaxies, whose copy the next group's
+// transform has to cover.
+int mock_group(const Plan &p, const int64_t *offsets, int64_t k, int64_t nmocks, int window_kind) {
+    if (p.radial_mode != SFB_RADIAL_POLY || window_kind == SFB_WINDOW_DENSE) return 1;
+    const int64_t most = std::min<int64_t>(
+        {MOCKS_MAX, (int64_t(1) << 25) / (p.nbasis * p.npix), 0x7fffffff / ((p.pieces + 2) * p.npix) - 1, nmocks - k});
+    int n = 1;
+    while (n < most && offsets[k + n + 1] - offsets[k] <= (int64_t(1) << 23)) ++n;
+    return n;
 }
 
 int check_plan(const sfb_plan *h) {
@@ -1153,7 +1181,7 @@ int sfb_cat2amln_device(sfb_plan *h, const double *rtp, const double *weight, in
     SFB_TRY(check_plan(h));
     SFB_TRY(set_device_of(h));
     if (!anlm_out) return fail(SFB_EINVAL, "output is NULL");
-    return cat2amln_dev(h, rtp, weight, ngal, nbar, window, anlm_out, (cudaStream_t)stream);
+    return cat2amln_dev(h, rtp, weight, ngal, Mocks(), &nbar, window, anlm_out, (cudaStream_t)stream);
 }
 
 int sfb_cat2amln(sfb_plan *h, const double *rtp, const double *weight, int64_t ngal, double nbar,
@@ -1206,16 +1234,17 @@ int sfb_cat2amln(sfb_plan *h, const double *rtp, const double *weight, int64_t n
         SFB_CUDA_TRY(cudaMemcpyAsync(d_win, window->dense, (size_t)wlen * sizeof(double), cudaMemcpyHostToDevice, st));
         dw.dense = d_win;
     }
-    SFB_TRY(cat2amln_dev(h, ngal > 0 ? d_rtp : nullptr, d_w, ngal, nbar, &dw, d_out, st, ncopy ? h->ev_copy : nullptr,
-                         ncopy));
+    SFB_TRY(cat2amln_dev(h, ngal > 0 ? d_rtp : nullptr, d_w, ngal, Mocks(), &nbar, &dw, d_out, st,
+                         ncopy ? h->ev_copy : nullptr, ncopy));
     SFB_CUDA_TRY(cudaMemcpyAsync(anlm_out, d_out, 2 * p.nlmsize * sizeof(double), cudaMemcpyDeviceToHost, st));
     SFB_CUDA_TRY(cudaStreamSynchronize(st));
     return SFB_OK;
 }
 
-// Batched catalogues (mock batches): mock k's galaxies go up on a copy stream into one of two
-// staging buffers while mock k - 1 is transformed on the plan's stream; results come back
-// per mock.  The device error word collects every mock's errors and is read once.
+// Batched catalogues (mock batches), in groups of mocks that go through the kernels together: a group's
+// galaxies go up on a copy stream into one of two staging buffers while the group before is transformed on
+// the plan's stream; results come back per group.  The device error word collects every mock's errors and is
+// read once.
 int sfb_cat2amln_batched(sfb_plan *h, const double *rtp, const double *weight, const int64_t *offsets,
                          int64_t nmocks, const double *nbar, const sfb_window *window, double *anlm_out) {
     SFB_TRY(check_plan(h));
@@ -1223,20 +1252,28 @@ int sfb_cat2amln_batched(sfb_plan *h, const double *rtp, const double *weight, c
     if (nmocks < 0 || (nmocks > 0 && (!offsets || !nbar || !anlm_out)) || !window)
         return fail(SFB_EINVAL, "bad batched cat2amln arguments");
     if (nmocks == 0) return SFB_OK;
-    int64_t nmax_gal = 0;
     for (int64_t k = 0; k < nmocks; ++k) {
         const int64_t n = offsets[k + 1] - offsets[k];
         if (offsets[k] < 0 || n < 0) return fail(SFB_EINVAL, "offsets must be non-decreasing from 0");
         if (!(std::isfinite(nbar[k]) && nbar[k] != 0.0)) return fail(SFB_ENONFINITE, "nbar must be finite and non-zero");
-        nmax_gal = std::max(nmax_gal, n);
     }
     if (offsets[nmocks] > 0 && !rtp) return fail(SFB_EINVAL, "rtp is NULL");
     Plan &p = h->p;
+    std::vector<int64_t> first{0};                 // first mock of every group, then nmocks
+    int64_t nmax_gal = 0, most = 0;
+    while (first.back() < nmocks) {
+        const int64_t k = first.back();
+        const int n = mock_group(p, offsets, k, nmocks, window->kind);
+        nmax_gal = std::max(nmax_gal, offsets[k + n] - offsets[k]);
+        most = std::max<int64_t>(most, n);
+        first.push_back(k + n);
+    }
+    const int64_t ngroups = (int64_t)first.size() - 1;
     cudaStream_t st = h->stream;
     const int64_t wlen = window->kind == SFB_WINDOW_SEPARABLE ? p.npix + (int64_t)(p.lmax + 1) * p.nmax
                        : window->kind == SFB_WINDOW_DENSE ? p.npix * (int64_t)(p.lmax + 1) * p.nmax : 0;
-    // [window][2 x (rtp 3 nmax_gal, w nmax_gal, out 2 nlmsize)]
-    const int64_t per_buf = 3 * nmax_gal + (weight ? nmax_gal : 0) + 2 * p.nlmsize;
+    // [window][2 x (rtp 3 nmax_gal, w nmax_gal, out 2 nlmsize per mock)]
+    const int64_t per_buf = 3 * nmax_gal + (weight ? nmax_gal : 0) + 2 * p.nlmsize * most;
     SFB_TRY(grow(p, p.scratch, (size_t)(wlen + 2 * per_buf + 1)));
     double *d_win = p.scratch.ptr;
     sfb_window dw = *window;
@@ -1280,12 +1317,12 @@ int sfb_cat2amln_batched(sfb_plan *h, const double *rtp, const double *weight, c
                          cudaEventRecord(ev[0][sfb_plan::NCOPY], st) != cudaSuccess))
         rc = fail(SFB_ECUDA, "event record failed");
     auto dbuf = [&](int64_t k) { return d_win + wlen + (k & 1) * per_buf; };
-    // copies of mock k into buffer k & 1, once mock k - 2 released it
-    auto enqueue_copy = [&](int64_t k) -> int {
-        const int b = (int)(k & 1);
-        double *d_rtp = dbuf(k);
+    // copies of group g into buffer g & 1, once group g - 2 released it
+    auto enqueue_copy = [&](int64_t g) -> int {
+        const int b = (int)(g & 1);
+        double *d_rtp = dbuf(g);
         double *d_w = weight ? d_rtp + 3 * nmax_gal : nullptr;
-        const int64_t g0 = offsets[k], ngal = offsets[k + 1] - offsets[k];
+        const int64_t g0 = offsets[first[g]], ngal = offsets[first[g + 1]] - g0;
         if (cudaStreamWaitEvent(cs, ev[b][sfb_plan::NCOPY], 0) != cudaSuccess) return fail(SFB_ECUDA, "stream wait failed");
         const int ncopy = sfb_plan::NCOPY;
         const int64_t per = ngal > 0 ? (ngal + ncopy - 1) / ncopy : 0;
@@ -1303,20 +1340,23 @@ int sfb_cat2amln_batched(sfb_plan *h, const double *rtp, const double *weight, c
         return SFB_OK;
     };
     if (rc == SFB_OK) rc = enqueue_copy(0);
-    for (int64_t k = 0; k < nmocks && rc == SFB_OK; ++k) {
-        // the next mock's copy is queued before this mock's result is read back (which blocks the host
-        // for pageable output), so it overlaps this mock's transform
-        if (k + 1 < nmocks && (rc = enqueue_copy(k + 1)) != SFB_OK) break;
-        const int b = (int)(k & 1);
-        double *d_rtp = dbuf(k);
+    for (int64_t g = 0; g < ngroups && rc == SFB_OK; ++g) {
+        // the next group's copy is queued before this group's results are read back (which blocks the host
+        // for pageable output), so it overlaps this group's transform
+        if (g + 1 < ngroups && (rc = enqueue_copy(g + 1)) != SFB_OK) break;
+        const int b = (int)(g & 1);
+        double *d_rtp = dbuf(g);
         double *d_w = weight ? d_rtp + 3 * nmax_gal : nullptr;
         double *d_out = d_rtp + 3 * nmax_gal + (weight ? nmax_gal : 0);
-        const int64_t ngal = offsets[k + 1] - offsets[k];
-        rc = cat2amln_dev(h, ngal > 0 ? d_rtp : nullptr, d_w, ngal, nbar[k], &dw, d_out, st, ev[b],
-                          sfb_plan::NCOPY, true);
+        const int64_t k = first[g], ngal = offsets[first[g + 1]] - offsets[k];
+        Mocks mk;
+        mk.n = (int)(first[g + 1] - k);
+        for (int j = 0; j <= mk.n; ++j) mk.off[j] = (int32_t)(mk.n > 1 ? offsets[k + j] - offsets[k] : 0);
+        rc = cat2amln_dev(h, ngal > 0 ? d_rtp : nullptr, d_w, ngal, mk, nbar + k, &dw, d_out, st, ev[b], sfb_plan::NCOPY,
+                          true);
         if (rc != SFB_OK) break;
         if (cudaEventRecord(ev[b][sfb_plan::NCOPY], st) != cudaSuccess ||
-            cudaMemcpyAsync(anlm_out + 2 * p.nlmsize * k, d_out, 2 * p.nlmsize * sizeof(double),
+            cudaMemcpyAsync(anlm_out + 2 * p.nlmsize * k, d_out, 2 * p.nlmsize * mk.n * sizeof(double),
                             cudaMemcpyDeviceToHost, st) != cudaSuccess)
             rc = fail(SFB_ECUDA, "result copy failed");
     }

@@ -11,6 +11,8 @@
 // constant basis maps.
 #include <vector>
 
+#include <algorithm>
+
 #include "sfb_internal.h"
 
 namespace sfb {
@@ -542,8 +544,11 @@ void launch_coef_df(const Plan &p, const int32_t *pair_index, float2 *CT, cudaSt
 
 // s[pair] = sum_b coef[pair][b] mu_b (FP64): the mean part of every pair, one
 // warp per pair (lanes over b, coalesced rows).
+// (grid.y: mocks, their mu and s one after another)
 __global__ void k_mean_proj(const double *__restrict__ coef, int64_t npairs, int64_t nbasis,
                             const double *__restrict__ mu, double *__restrict__ s) {
+    mu += blockIdx.y * nbasis;
+    s += blockIdx.y * npairs;
     const int64_t pr = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (pr >= npairs) return;
@@ -583,17 +588,28 @@ __device__ __forceinline__ void pj_mac(pacc &a, float2 c, float xh, float xl) {
     a.lo = fmaf(c.y, xh, fmaf(c.x, xl, (a.lo + err) + e));
 }
 
+struct Scales {
+    double v[MOCKS_MAX];
+};
+
+// grid.y: mocks (launch_project_mixed says where each one's data lie)
 template <int KS>
 __global__ void __launch_bounds__(32 * KS) k_project_mixed(const float2 *__restrict__ Adf, int64_t ldA,
                                                               int64_t nbasis, const float2 *__restrict__ CT, int nmax,
                                                               int lmax, const int3 *__restrict__ tiles,
                                                               const int64_t *__restrict__ noff,
-                                                              const int32_t *__restrict__ pair_index, double scale,
-                                                              const double *__restrict__ smean,
-                                                              const double *__restrict__ ralm, int window_kind,
+                                                              const int32_t *__restrict__ pair_index, Scales scales,
+                                                              const double *__restrict__ smean, int64_t npairs,
+                                                              const double *__restrict__ ralm, int64_t ldR,
+                                                              int64_t nlmsize, int window_kind,
                                                               const double *__restrict__ w_ln,
                                                               double *__restrict__ out, int *err) {
     __shared__ float4 part[KS - 1][PJ_NPT][32];
+    const int mock = blockIdx.y;
+    const double scale = scales.v[mock];
+    Adf += (int64_t)mock * 2 * nbasis;
+    smean += mock * npairs;
+    out += (int64_t)mock * 2 * nlmsize;
     const int3 t = tiles[blockIdx.x];
     const int l = t.x, m0 = t.y, n0 = t.z & 0xffff, npt = t.z >> 16;
     const int lane = threadIdx.x & 31, ks = threadIdx.x >> 5;
@@ -644,12 +660,13 @@ __global__ void __launch_bounds__(32 * KS) k_project_mixed(const float2 *__restr
         double vi = scale * ((double)si.hi + (double)si.lo);
         if (ralm) {
             const double mu = scale * smean[pr];
-            vr = fma(mu, ralm[4 * lm], vr);
-            vi = fma(mu, ralm[4 * lm + 1], vi);
+            const double *cm = ralm + ldR * lm + 2 * mock, *wm = ralm + ldR * lm + 2 * gridDim.y;
+            vr = fma(mu, cm[0], vr);
+            vi = fma(mu, cm[1], vi);
             if (window_kind == SFB_WINDOW_SEPARABLE) {
                 const double wl = w_ln[l + (int64_t)(lmax + 1) * n1];
-                vr = fma(-wl, ralm[4 * lm + 2], vr);
-                vi = fma(-wl, ralm[4 * lm + 3], vi);
+                vr = fma(-wl, wm[0], vr);
+                vi = fma(-wl, wm[1], vi);
             }
         }
         const int64_t o = noff[n1] + lm;
@@ -674,18 +691,22 @@ std::vector<int3> project_tiles(const std::vector<int32_t> &pair_index, int lmax
     return t;
 }
 
-void launch_mean_proj(const Plan &p, const double *mu, double *smean, cudaStream_t st) {
-    k_mean_proj<<<(unsigned)((p.npairs + 3) / 4), 128, 0, st>>>(p.d_coef, p.npairs, p.nbasis, mu, smean);
+void launch_mean_proj(const Plan &p, const double *mu, int nmock, double *smean, cudaStream_t st) {
+    k_mean_proj<<<dim3((unsigned)((p.npairs + 3) / 4), (unsigned)nmock), 128, 0, st>>>(p.d_coef, p.npairs, p.nbasis, mu,
+                                                                                     smean);
     note_launch();
 }
 
 void launch_project_mixed(const Plan &p, const float2 *Adf, int64_t ldA, const float2 *CT, const int64_t *noff,
-                          const int32_t *pair_index, double scale, const double *smean, const double *ralm,
-                          int window_kind, const double *w_ln, double *out, int *err, cudaStream_t st) {
+                          const int32_t *pair_index, int nmock, const double *scale, const double *smean,
+                          const double *ralm, int64_t ldR, int window_kind, const double *w_ln, double *out, int *err,
+                          cudaStream_t st) {
     if (p.n_proj_tiles <= 0) return;
-    k_project_mixed<PJ_KS><<<(unsigned)p.n_proj_tiles, 32 * PJ_KS, 0, st>>>(
-        Adf, ldA, p.nbasis, CT, (int)p.nmax, p.lmax, p.d_proj_tiles, noff, pair_index, scale, smean, ralm, window_kind,
-        w_ln, out, err);
+    Scales sc;
+    std::copy(scale, scale + nmock, sc.v);
+    k_project_mixed<PJ_KS><<<dim3((unsigned)p.n_proj_tiles, (unsigned)nmock), 32 * PJ_KS, 0, st>>>(
+        Adf, ldA, p.nbasis, CT, (int)p.nmax, p.lmax, p.d_proj_tiles, noff, pair_index, sc, smean, p.npairs, ralm, ldR,
+        p.nlmsize, window_kind, w_ln, out, err);
     note_launch();
 }
 

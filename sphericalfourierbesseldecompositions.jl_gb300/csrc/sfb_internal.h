@@ -215,22 +215,33 @@ inline void set_smem(K kernel, size_t bytes) {
 // kernels (launch wrappers; all enqueue on `st`)
 // ---------------------------------------------------------------------------
 void launch_legendre_table(const Plan &p, cudaStream_t st);
-// galaxies -> radial-basis x pixel maps (counting sort + register moments); writes every map element
-// Sorted deposit of the catalogue into the basis maps.  With ref (mixed
-// precision only) the weighted count map C is written to ref[npix], the maps
-// hold D_b - mu_b C and mu[nbasis] receives mu_b; ref_ready (if given) is
-// recorded on st once C is complete.
-// chunk_ready / nchunks: the catalogue arrives in nchunks equal galaxy ranges,
-// range c complete when chunk_ready[c] fires (keys wait per range).
-// ring_live (mixed precision with a reference map): receives a device array of 4 nside - 1 ints, 1 for the
-// rings that hold a galaxy; the basis maps are left unwritten on the other rings (they are zero there),
-// and the ring DFT must be given the array (launch_ring_analysis_tc) so that it does not read them.
-// w01 / mask_df (with ref): the window's reference map is copied to ref[npix ..] and, when mask_df is given, laid
-// out there as a double-float map.  mu_ready (if given) is recorded on st once mu is complete.
-int deposit_sorted(Plan &p, const double *rtp, const double *w, int64_t ngal, double *maps, double *ref,
-                   double *mu, cudaEvent_t ref_ready, cudaStream_t st, const cudaEvent_t *chunk_ready = nullptr,
-                   int nchunks = 0, const int **ring_live = nullptr, const double *w01 = nullptr,
-                   float2 *mask_df = nullptr, cudaEvent_t mu_ready = nullptr);
+// Mock catalogues deposited together: mock j is galaxies [off[j], off[j + 1]) of the arrays.
+constexpr int MOCKS_MAX = 16;
+struct Mocks {
+    int n = 1;
+    int32_t off[MOCKS_MAX + 1] = {};
+};
+
+// Sorted deposit of the catalogues into the basis maps, mock j at maps + j nbasis npix; every map element is
+// written.  With ref (mixed precision only) the weighted count map C of mock j is written to ref[j npix ..], the
+// maps hold D_b - mu_b C and mu[j nbasis ..] receives mu_b; w01 (the window's reference map) is copied behind the
+// count maps; ref_ready / mu_ready (if given) are recorded on st once the count maps / mu are complete.
+// chunk_ready / nchunks: the galaxies arrive in nchunks equal ranges, range c complete when chunk_ready[c] fires
+// (keys wait per range).
+// ring_live (mixed precision with a reference map): receives a device array of 4 nside - 1 ints per mock, 1 for
+// the rings that hold a galaxy; the mock's basis maps are left unwritten on the other rings (they are zero
+// there), and the ring DFT must be given the array (launch_ring_analysis_tc) so that it does not read them.
+struct DepositArgs {
+    const double *rtp = nullptr, *w = nullptr;
+    int64_t ngal = 0;
+    Mocks mocks;
+    double *maps = nullptr, *ref = nullptr, *mu = nullptr;
+    const double *w01 = nullptr;
+    cudaEvent_t ref_ready = nullptr, mu_ready = nullptr;
+    const cudaEvent_t *chunk_ready = nullptr;
+    int nchunks = 0;
+};
+int deposit_sorted(Plan &p, const DepositArgs &a, cudaStream_t st, const int **ring_live);
 
 // 0-based ring (1 .. 4 nside - 1 minus one) of a RING-scheme pixel
 __host__ __device__ __forceinline__ int ring_of_pixel(int64_t nside, int64_t pix) {
@@ -252,11 +263,15 @@ void launch_add_mean(double *A, int64_t ldA, int64_t nmaps, const double *mu, co
 // Mixed-precision radial projection (double-float sums; FP64 mean and window
 // terms), replacing add_mean + project_poly for the data term.
 void launch_coef_df(const Plan &p, const int32_t *pair_index, float2 *CT, cudaStream_t st);
-void launch_mean_proj(const Plan &p, const double *mu, double *smean, cudaStream_t st);     // smean of the next
+// smean[j npairs ..] of nmock mocks for the next
+void launch_mean_proj(const Plan &p, const double *mu, int nmock, double *smean, cudaStream_t st);
+// nmock mocks: mock j's columns of Adf start at map j nbasis, its count map is column pair j of ralm [lmsize][ldR]
+// (the window's map is the pair after them), its result out + 2 j nlmsize.
 // err (optional): ERR_NONFINITE_OUTPUT is raised there for a non-finite coefficient
 void launch_project_mixed(const Plan &p, const float2 *Adf, int64_t ldA, const float2 *CT, const int64_t *noff,
-                          const int32_t *pair_index, double scale, const double *smean, const double *ralm,
-                          int window_kind, const double *w_ln, double *out, int *err, cudaStream_t st);
+                          const int32_t *pair_index, int nmock, const double *scale, const double *smean,
+                          const double *ralm, int64_t ldR, int window_kind, const double *w_ln, double *out, int *err,
+                          cudaStream_t st);
 // maps[j] -= nu[j] ref with nu[j] = <maps[j], ref> / <ref, ref> (FP64, in place).
 void launch_split_mean(double *maps, int64_t nmaps, int64_t npix, const double *ref, double *nu, cudaStream_t st);
 // nzr (FP64): receives the first / last ring pair holding a non-zero value in any map
@@ -309,9 +324,10 @@ void launch_to_float(const double *in, int64_t n, float *out, cudaStream_t st);
 void launch_to_df(const double *in, int64_t n, float2 *out, cudaStream_t st);
 // Mixed-precision ring analysis on the tensor cores (double-float maps -> double-float F).
 // nzr[0..1] receives the first and last ring pair holding a non-zero map row.
-// ring_live (optional): rings whose entry is 0 hold zeros in maps [0, nlive) and are not read.
+// ring_live (optional): nper maps share an array of 4 nside - 1 entries (map b the (b / nper)-th); their rings whose
+// entry is 0 hold zeros and are not read.
 int launch_ring_analysis_tc(Plan &p, const float2 *maps, int64_t nmaps, float2 *F, int *erow, int *nzr,
-                            cudaStream_t st, const int *ring_live = nullptr, int64_t nlive = 0,
+                            cudaStream_t st, const int *ring_live = nullptr, int64_t nper = 1,
                             bool skip_unread = false);
 uint2 dft_slices(double v, int EB);
 int64_t dft_image_offsets(const Plan &p, const std::vector<int32_t> &crings, const std::vector<int32_t> &coff,

@@ -81,3 +81,29 @@ def test_batched_band_power_covariance():
     e = rel_err(clnn[0], osfb.amln2clnn(anlm[0], anlm[0], cm.lnn, md))
     record("batched_band_power_vs_oracle", e)
     assert e < 1e-14
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("window", ["separable", "zero", "dense"])
+def test_groups_of_mocks_equal_single_calls(precision, window):
+    """More mocks than one group holds (16), with empty ones at both ends of a
+    group: every row equals its single call.  A mock's maps pass through the
+    same operations in a group, on its own scales, except that the FP64
+    reference maps of a group run on the tensor cores: FP64 rounding, 1e-12,
+    and the deposit's rounding of the mixed records, 1e-9 (as above)."""
+    a = sfbgpu.AnlmModes(0.03, 500.0, 1000.0, nside=16)
+    wm, phi, mask = _window(a)
+    sep = sfbgpu.SeparableArray(phi, mask, "phi", "mask")
+    win = {"zero": None, "separable": sfbgpu.win_rhat_ln(sep, wm, a),
+           "dense": sfbgpu.win_rhat_ln(sep.dense(), wm, a)}[window]
+    veff = sfbgpu.integrate_window(sep, wm)
+    sizes = [0, 900, 3001, 1, 5000, 2047, 2048, 64, 0, 777, 4096, 31, 32, 33, 1500, 0, 0, 2500, 129]
+    cats, ws = _mocks(a, sizes, 47)
+    nbars = [max(n, 1) / veff for n in sizes]
+    batch = sfbgpu.cat2amln_batched(cats, a, nbars, win, ws, precision=precision)
+    for k in range(len(sizes)):
+        single = sfbgpu.cat2amln(cats[k], a, nbars[k], win, ws[k], precision=precision)
+        if not np.any(single):
+            assert not np.any(batch[k])
+            continue
+        assert rel_err(batch[k], single) < (1e-12 if precision == "fp64" else 1e-9), k
