@@ -91,29 +91,9 @@ __device__ __forceinline__ dfl df_renorm(dfl a) {
     return {h, a.lo - (h - a.hi)};
 }
 
-// Double -> double-float by integer operations only (no FP64 instruction, whose
-// rate on this GPU is a small fraction of the FP32 one): hi = d rounded to the
-// nearest FP32 (ties to even, as (float)d), lo = d - hi rounded to FP32, ~48
-// significant bits in all.  Finite d; below the FP32 normal range hi is 0
-// (sign kept), and lo is 0 for |d| < 2^-75.
 __device__ __forceinline__ dfl df_of_bits(double d) {
-    const unsigned long long b = (unsigned long long)__double_as_longlong(d);
-    const unsigned sign = (unsigned)(b >> 32) & 0x80000000u;
-    const int e = (int)((b >> 52) & 0x7ff);
-    const int fe = e - 1023 + 127;
-    if (fe <= 0) return {__uint_as_float(sign), 0.f};
-    if (fe >= 255) return {__uint_as_float(sign | 0x7f800000u), 0.f};
-    const unsigned long long m = b & 0xfffffffffffffull;
-    const unsigned rem = (unsigned)(m & 0x1fffffffu);                 // the 29 bits below FP32
-    const unsigned hb = sign | ((unsigned)fe << 23) | (unsigned)(m >> 29);
-    const bool up = rem > 0x10000000u || (rem == 0x10000000u && (hb & 1u));
-    // a mantissa carry moves into the exponent, as rounding up does
-    const float hi = __uint_as_float(hb + (up ? 1u : 0u));
-    // d - hi = (rem - up 2^29) 2^(e - 1075); exact scale where 2^(e - 1075) is an FP32 normal
-    const int r = (int)rem - (up ? 0x20000000 : 0);
-    const int se = e - 1075 + 127;
-    float lo = se >= 1 ? (float)r * __uint_as_float((unsigned)se << 23) : 0.f;
-    return {hi, sign ? -lo : lo};
+    const float2 v = df_split_bits(d);
+    return {v.x, v.y};
 }
 
 // IEEE order of finite doubles as signed 64-bit integers (-0 and +0 both 0),
@@ -160,7 +140,7 @@ __device__ __forceinline__ int mock_of(const Mocks &mk, int64_t i) {
 // pixel), so no warp runs the FP64 pixel path for one lane.
 __global__ void k_deposit_keys(const double *__restrict__ rtp, const double *__restrict__ wgt, int64_t ngal,
                                int64_t gbase, int64_t nside, int64_t npix, double rmin, double rmax,
-                               double inv_width, int pieces, Mocks mk, int32_t *__restrict__ counts,
+                               double inv_width, int pieces, const __grid_constant__ Mocks mk, int32_t *__restrict__ counts,
                                int32_t *__restrict__ key, int32_t *__restrict__ rank, double *__restrict__ xloc,
                                int32_t *__restrict__ fb_list, int32_t *__restrict__ fb_count, int *err) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -202,7 +182,7 @@ struct RadialKeyParams {
 
 __global__ void k_deposit_keys_mixed(const double *__restrict__ rtp, const double *__restrict__ wgt, int64_t ngal,
                                      int64_t gbase, int64_t nside, int64_t npix, RadialKeyParams rk, int pieces,
-                                     Mocks mk, int32_t *__restrict__ counts, int32_t *__restrict__ key,
+                                     const __grid_constant__ Mocks mk, int32_t *__restrict__ counts, int32_t *__restrict__ key,
                                      int32_t *__restrict__ rank, float2 *__restrict__ xdf,
                                      int32_t *__restrict__ fb_list, int32_t *__restrict__ fb_count, int *err) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -922,13 +902,25 @@ __global__ void __launch_bounds__(32) k_deposit_stats(const int32_t *__restrict_
     if (!__shfl_sync(full, last, 0)) return;
     __threadfence();
     const int64_t npoly = (int64_t)pieces * (deg + 1);
-    for (int64_t i = lane; i < nbasis * gridDim.y; i += 32) {
-        const int64_t mock = i / nbasis, b = i - mock * nbasis;
-        const int sl = b < npoly ? (int)(b / (deg + 1)) : pieces + (int)(b - npoly);
-        const double q = __ldcg(Q0 + mock * (pieces + 2) + sl), v = q > 0.0 ? __ldcg(S0 + i) / q : 0.0;
-        mu[i] = v;
-        const float h = (float)v;
-        mudf[i] = make_float2(h, (float)(v - (double)h));
+    const int64_t nmu = nbasis * gridDim.y;
+    for (int64_t i0 = lane; i0 < nmu; i0 += 8 * 32) {
+        double sv[8], qv[8];                             // eight loads on their way at a time
+#pragma unroll
+        for (int t = 0; t < 8; ++t) {
+            const int64_t i = min(i0 + 32 * t, nmu - 1), mock = i / nbasis, b = i - mock * nbasis;
+            const int sl = b < npoly ? (int)b / (deg + 1) : pieces + (int)(b - npoly);
+            sv[t] = __ldcg(S0 + i);
+            qv[t] = __ldcg(Q0 + mock * (pieces + 2) + sl);
+        }
+#pragma unroll
+        for (int t = 0; t < 8; ++t) {
+            const int64_t i = i0 + 32 * t;
+            if (i >= nmu) break;
+            const double v = qv[t] > 0.0 ? sv[t] / qv[t] : 0.0;
+            mu[i] = v;
+            const float h = (float)v;
+            mudf[i] = make_float2(h, (float)(v - (double)h));
+        }
     }
 }
 

@@ -105,7 +105,7 @@ struct sfb_plan {
     // side stream for the FP64 reference-map transform of the mixed path,
     // forked / joined with the call's stream through events
     cudaStream_t side = nullptr;
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_mu = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_mu = nullptr, ev_dense = nullptr;
     // host entry: the catalogue copy runs on the side stream in NCOPY chunks
     static constexpr int NCOPY = 4;
     cudaEvent_t ev_copy[NCOPY] = {};
@@ -337,11 +337,10 @@ void synthesis_and_gram64(const Plan &p, const double *A, const double *A0, int6
 
 // fp64_out: the FP64 a_lm (alm) is wanted besides the double-float copy (almdf, mixed precision); the
 // Gram refinement carries only the double-float one and converts at the end when asked.
-// ring_live / nper (mixed precision): rings marked 0 hold zeros, left unwritten by the deposit (deposit_sorted's
-// ring_live), one array per nper maps.
+// live (mixed precision): rings that hold zeros, left unwritten by the deposit (deposit_sorted's ring_live).
 int sht_analysis(sfb_plan *h, const double *maps, int64_t nm, cudaStream_t st, bool maps_are_fp64 = false,
                  int stage_override = -1, const ShtWork *ws = nullptr, bool fp64_out = true,
-                 const int *ring_live = nullptr, int64_t nper = 1) {
+                 const LiveRings &live = LiveRings()) {
     Plan &p = h->p;
     const ShtWork own{&p.fbuf, &p.gbuf, &p.rbuf, &p.alm};
     if (!ws) ws = &own;
@@ -377,7 +376,7 @@ int sht_analysis(sfb_plan *h, const double *maps, int64_t nm, cudaStream_t st, b
         const bool skip_unread = (nm > 4 && p.d_gramts && p.niter > 0) || p.niter == 0;
         SFB_TRY(launch_ring_analysis_tc(p, reinterpret_cast<const float2 *>(maps), nm,
                                         reinterpret_cast<float2 *>(fbuf.ptr), reinterpret_cast<int *>(p.erow.ptr), nzr,
-                                        st, ring_live, nper, skip_unread));
+                                        st, live, skip_unread));
     } else {
         // many columns: the FFT records the span of ring pairs with data, over which the
         // first analysis pass sums (the spectra are zero elsewhere)
@@ -643,20 +642,34 @@ int cat2amln_dev(sfb_plan *h, const double *rtp, const double *w, int64_t ngal, 
         const bool split = p.precision == SFB_MIXED && wk != SFB_WINDOW_ZERO;
         // the basis maps of every mock; in FP64 the mask of a separable window is one map more
         const bool mask_map = wk == SFB_WINDOW_SEPARABLE && !split;
-        const int64_t nb = p.nbasis, nm = nmock * nb + (mask_map ? 1 : 0);
         const double *W01 = wk == SFB_WINDOW_SEPARABLE ? win->mask : win->dense;
+        // dense windows: pairs per window transform; where all pairs fit, the mixed path transforms their maps
+        // together with the basis maps
         const int64_t cp = wk == SFB_WINDOW_DENSE ? chunk_pairs(p) : 0;
-        double *Cmap = nullptr, *mu = nullptr, *nu = nullptr, *smean = nullptr;
+        const bool joint = split && cp > 0 && cp >= p.npairs;
+        const int64_t nb = p.nbasis, nm = nmock * nb + (mask_map ? 1 : 0) + (joint ? p.npairs : 0);
+        double *Cmap = nullptr, *mu = nullptr, *nu = nullptr, *smean = nullptr, *refsq = nullptr;
         const double *ralm = nullptr;             // FP64 a_lm of (C of every mock, W01), [lmsize][2 nmock + 2]
         if (split) {
-            // [C][W01][mu][nu][per-pair mean parts]
-            SFB_TRY(grow(p, p.ref, (size_t)((nmock + 1) * p.npix + nmock * (nb + p.npairs) + cp)));
+            // [C][W01][mu][nu][per-pair mean parts][<W01, W01>]
+            SFB_TRY(grow(p, p.ref, (size_t)((nmock + 1) * p.npix + nmock * (nb + p.npairs) + cp + 1)));
             Cmap = p.ref.ptr;
             mu = Cmap + (nmock + 1) * p.npix;
             nu = mu + nmock * nb;
             smean = nu + cp;
+            refsq = smean + nmock * p.npairs;
         }
         SFB_TRY(grow(p, p.maps, (size_t)nm * p.npix));
+        if (split && wk == SFB_WINDOW_DENSE) {
+            // the window's maps do not wait for the catalogue: on the side stream beside the deposit
+            SFB_CUDA_TRY(cudaEventRecord(h->ev_join, st));
+            SFB_CUDA_TRY(cudaStreamWaitEvent(h->side, h->ev_join, 0));
+            launch_ref_square(W01, p.npix, refsq, h->side);
+            if (joint)
+                launch_dense_maps_df(p, win->dense, W01, refsq, 0, p.npairs, nu,
+                                     reinterpret_cast<float2 *>(p.maps.ptr) + nb * p.npix, h->side);
+            SFB_CUDA_TRY(cudaEventRecord(h->ev_dense, h->side));
+        }
         const int *ring_live = nullptr;          // rings the deposit wrote (mixed precision)
         if (mask_map) {
             Stage s(h, SFB_STAGE_OTHER, st);
@@ -691,7 +704,9 @@ int cat2amln_dev(sfb_plan *h, const double *rtp, const double *w, int64_t ngal, 
             SFB_CUDA_TRY(cudaEventRecord(h->ev_join, h->side));
         }
         // the mixed projection reads the double-float a_lm only
-        SFB_TRY(sht_analysis(h, p.maps.ptr, nm, st, false, -1, nullptr, p.precision != SFB_MIXED, ring_live, nb));
+        if (split && wk == SFB_WINDOW_DENSE) SFB_CUDA_TRY(cudaStreamWaitEvent(st, h->ev_dense, 0));
+        const LiveRings live{ring_live, ring_live ? nmock * nb : 0, nb};
+        SFB_TRY(sht_analysis(h, p.maps.ptr, nm, st, false, -1, nullptr, p.precision != SFB_MIXED, live));
         if (split) SFB_CUDA_TRY(cudaStreamWaitEvent(st, h->ev_join, 0));
         {
             Stage s(h, SFB_STAGE_PROJECT, st);
@@ -704,14 +719,23 @@ int cat2amln_dev(sfb_plan *h, const double *rtp, const double *w, int64_t ngal, 
                     launch_project_poly(p, p.alm.ptr + 2 * nb * j, 2 * nm, scale[j], wk, win->w_ln, nb * (nmock - j),
                                         nullptr, 0, out + 2 * p.nlmsize * j, st);
         }
-        if (wk == SFB_WINDOW_DENSE) {             // one catalogue at a time
+        const float2 *adf = reinterpret_cast<const float2 *>(p.almdf.ptr);
+        if (joint) {
+            launch_sub_window_df(p, adf + 2 * nb, 2 * nm, 0, p.npairs, nu, ralm + 2, 4, out, p.d_err, st);
+        } else if (wk == SFB_WINDOW_DENSE) {
             SFB_TRY(grow(p, p.maps, (size_t)cp * p.npix));
             for (int64_t p0 = 0; p0 < p.npairs; p0 += cp) {
                 const int64_t npc = std::min(cp, p.npairs - p0);
+                if (split) {
+                    launch_dense_maps_df(p, win->dense, W01, refsq, p0, npc, nu, reinterpret_cast<float2 *>(p.maps.ptr),
+                                         st);
+                    SFB_TRY(sht_analysis(h, p.maps.ptr, npc, st, false, -1, nullptr, false));
+                    adf = reinterpret_cast<const float2 *>(p.almdf.ptr);
+                    launch_sub_window_df(p, adf, 2 * npc, p0, npc, nu, ralm + 2, 4, out, p.d_err, st);
+                    continue;
+                }
                 launch_gather_dense_chunk(p, p.maps.ptr, win->dense, p0, npc, st);
-                if (split) launch_split_mean(p.maps.ptr, npc, p.npix, W01, nu, st);
-                SFB_TRY(sht_analysis(h, p.maps.ptr, npc, st, true));
-                if (split) launch_add_mean(p.alm.ptr, 2 * npc, npc, nu, ralm + 2, nullptr, 4, p.lmsize, -1, st);
+                SFB_TRY(sht_analysis(h, p.maps.ptr, npc, st));
                 launch_sub_window_chunk(p, p.alm.ptr, 2 * npc, p0, npc, out, st);
             }
         }
@@ -732,8 +756,8 @@ int cat2amln_dev(sfb_plan *h, const double *rtp, const double *w, int64_t ngal, 
         }
     }
     SFB_CUDA_TRY(cudaGetLastError());
-    // the mixed projection has checked what it wrote, unless a dense window was subtracted from it
-    const bool checked = p.radial_mode == SFB_RADIAL_POLY && p.precision == SFB_MIXED && wk != SFB_WINDOW_DENSE;
+    // the mixed projection, or the subtraction of a dense window after it, has checked what it wrote
+    const bool checked = p.radial_mode == SFB_RADIAL_POLY && p.precision == SFB_MIXED;
     if (defer_finish) {
         Stage s(h, SFB_STAGE_OTHER, st);
         if (!checked) launch_check_finite(out, 2 * p.nlmsize * nmock, p.d_err, st);
@@ -881,6 +905,7 @@ int sfb_plan_create(const sfb_plan_desc *d, sfb_plan **out) {
             cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
             cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming) != cudaSuccess ||
             cudaEventCreateWithFlags(&h->ev_mu, cudaEventDisableTiming) != cudaSuccess ||
+            cudaEventCreateWithFlags(&h->ev_dense, cudaEventDisableTiming) != cudaSuccess ||
             cudaStreamCreateWithFlags(&p.dft_side, cudaStreamNonBlocking) != cudaSuccess ||
             cudaEventCreateWithFlags(&p.dft_fork, cudaEventDisableTiming) != cudaSuccess ||
             cudaEventCreateWithFlags(&p.dft_join, cudaEventDisableTiming) != cudaSuccess ||
@@ -1123,6 +1148,7 @@ void sfb_plan_destroy(sfb_plan *h) {
     if (h->ev_fork) cudaEventDestroy(h->ev_fork);
     if (h->ev_join) cudaEventDestroy(h->ev_join);
     if (h->ev_mu) cudaEventDestroy(h->ev_mu);
+    if (h->ev_dense) cudaEventDestroy(h->ev_dense);
     if (p.dft_side) cudaStreamDestroy(p.dft_side);
     if (p.dft_fork) cudaEventDestroy(p.dft_fork);
     if (p.dft_join) cudaEventDestroy(p.dft_join);

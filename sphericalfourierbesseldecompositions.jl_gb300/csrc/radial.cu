@@ -474,33 +474,6 @@ void launch_winweights(const double *weights, int64_t nr, int64_t nside, const d
     note_launch();
 }
 
-__global__ void k_add_mean(double *__restrict__ A, int64_t ldA, int64_t ncol, int64_t nmaps,
-                           const double *__restrict__ mu, const double *__restrict__ rmu,
-                           const double *__restrict__ rset, int64_t ldr, int64_t lmsize, int64_t set_col) {
-    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= lmsize * ncol) return;
-    const int64_t lm = e / ncol, j = e - lm * ncol;
-    if (j < nmaps) {
-        double *a = A + lm * ldA + 2 * j;
-        const double m = mu[j];
-        a[0] = fma(m, rmu[lm * ldr], a[0]);
-        a[1] = fma(m, rmu[lm * ldr + 1], a[1]);
-    } else {
-        double *a = A + lm * ldA + 2 * set_col;
-        a[0] = rset[lm * ldr];
-        a[1] = rset[lm * ldr + 1];
-    }
-}
-
-void launch_add_mean(double *A, int64_t ldA, int64_t nmaps, const double *mu, const double *rmu, const double *rset,
-                     int64_t ldr, int64_t lmsize, int64_t set_col, cudaStream_t st) {
-    const int64_t ncol = nmaps + (set_col >= 0 ? 1 : 0);
-    const int64_t n = lmsize * ncol;
-    if (n <= 0) return;
-    k_add_mean<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(A, ldA, ncol, nmaps, mu, rmu, rset, ldr, lmsize, set_col);
-    note_launch();
-}
-
 // ---- mixed-precision radial projection ---------------------------------------
 // Double-float helpers (FP32 pairs, ~48 significant bits).
 struct df2 {
@@ -710,44 +683,94 @@ void launch_project_mixed(const Plan &p, const float2 *Adf, int64_t ldA, const f
     note_launch();
 }
 
-// One block per map: nu = <m, ref> / <ref, ref>, then m -= nu ref.
-__global__ void __launch_bounds__(512) k_split_mean(double *maps, int64_t npix, const double *__restrict__ ref,
-                                                    double *nu) {
-    __shared__ double red[2][16];
-    double *m = maps + (int64_t)blockIdx.x * npix;
-    double d = 0.0, q = 0.0;
-    for (int64_t p = threadIdx.x; p < npix; p += blockDim.x) {
-        const double r = ref[p];
-        d = fma(m[p], r, d);
-        q = fma(r, r, q);
-    }
-    for (int off = 16; off > 0; off >>= 1) {
-        d += __shfl_xor_sync(0xffffffffu, d, off);
-        q += __shfl_xor_sync(0xffffffffu, q, off);
-    }
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0) {
-        red[0][wid] = d;
-        red[1][wid] = q;
-    }
+// <ref, ref> of one map, by one block
+__global__ void __launch_bounds__(1024) k_ref_square(const double *__restrict__ ref, int64_t npix, double *refsq) {
+    __shared__ double red[32];
+    double q = 0.0;
+#pragma unroll 4
+    for (int64_t p = threadIdx.x; p < npix; p += 1024) q = fma(ref[p], ref[p], q);
+    for (int off = 16; off > 0; off >>= 1) q += __shfl_xor_sync(0xffffffffu, q, off);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = q;
     __syncthreads();
     if (threadIdx.x == 0) {
-        double dd = 0.0, qq = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
-            dd += red[0][w];
-            qq += red[1][w];
-        }
-        red[0][0] = qq > 0.0 ? dd / qq : 0.0;
-        nu[blockIdx.x] = red[0][0];
+        for (int w = 1; w < 32; ++w) q += red[w];
+        *refsq = q;
     }
-    __syncthreads();
-    const double v = red[0][0];
-    for (int64_t p = threadIdx.x; p < npix; p += blockDim.x) m[p] = fma(-v, ref[p], m[p]);
 }
 
-void launch_split_mean(double *maps, int64_t nmaps, int64_t npix, const double *ref, double *nu, cudaStream_t st) {
-    if (nmaps <= 0) return;
-    k_split_mean<<<(unsigned)nmaps, 512, 0, st>>>(maps, npix, ref, nu);
+void launch_ref_square(const double *ref, int64_t npix, double *refsq, cudaStream_t st) {
+    k_ref_square<<<1, 1024, 0, st>>>(ref, npix, refsq);
+    note_launch();
+}
+
+// One block per pair: nu = <W, ref> / <ref, ref>, then the fluctuation W - nu ref as double-float pairs (the
+// split by integer operations).  The window map is read where the caller's array has it, the second time from L2,
+// and written once.  Bound: the FP64 pipe (two operations a pixel) beside HBM (16 bytes); as a gather, an in-place
+// split with three FP64 operations and a conversion pass it took 446 us for 507 maps of nside 64.
+__global__ void __launch_bounds__(512) k_dense_maps_df(const double *__restrict__ dense, int64_t npix, int lmax,
+                                                       const int32_t *__restrict__ pair_n,
+                                                       const int32_t *__restrict__ pair_l, int64_t pair0,
+                                                       const double *__restrict__ ref,
+                                                       const double *__restrict__ refsq, double *__restrict__ nu,
+                                                       float2 *__restrict__ maps) {
+    __shared__ double red[16];
+    const int64_t pr = pair0 + blockIdx.x;
+    const double *W = dense + npix * ((int64_t)pair_l[pr] + (int64_t)(lmax + 1) * (pair_n[pr] - 1));
+    float2 *m = maps + (int64_t)blockIdx.x * npix;
+    double d = 0.0;
+#pragma unroll 8
+    for (int64_t p = threadIdx.x; p < npix; p += 512) d = fma(W[p], ref[p], d);
+    for (int off = 16; off > 0; off >>= 1) d += __shfl_xor_sync(0xffffffffu, d, off);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = d;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 16; ++w) d += red[w];
+        const double q = *refsq;
+        red[0] = q > 0.0 ? d / q : 0.0;
+        nu[blockIdx.x] = red[0];
+    }
+    __syncthreads();
+    const double v = red[0];
+#pragma unroll 8
+    for (int64_t p = threadIdx.x; p < npix; p += 512) {
+        const double x = fma(-v, ref[p], W[p]);
+        // a non-finite value keeps its kind (the split by bits takes finite ones)
+        m[p] = isfinite(x) ? df_split_bits(x) : make_float2((float)x, 0.f);
+    }
+}
+
+void launch_dense_maps_df(const Plan &p, const double *dense, const double *ref, const double *refsq, int64_t pair0,
+                          int64_t npc, double *nu, float2 *maps, cudaStream_t st) {
+    if (npc <= 0) return;
+    k_dense_maps_df<<<(unsigned)npc, 512, 0, st>>>(dense, p.npix, p.lmax, p.d_pair_n, p.d_pair_l, pair0, ref, refsq, nu,
+                                                   maps);
+    note_launch();
+}
+
+// The window's part of every coefficient of the chunk's pairs, from the double-float a_lm (the rows l of pair (n,
+// l) only) and the reference map's FP64 ones.
+__global__ void k_sub_window_df(const int32_t *__restrict__ out_pair, const int32_t *__restrict__ out_lm,
+                                int64_t nlmsize, const float2 *__restrict__ Adf, int64_t ldA, int64_t pair0, int64_t npc,
+                                const double *__restrict__ nu, const double *__restrict__ rref, int64_t ldR,
+                                double *__restrict__ out, int *err) {
+    const int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (o >= nlmsize) return;
+    const int64_t q = (int64_t)out_pair[o] - pair0;
+    if (q < 0 || q >= npc) return;
+    const int64_t lm = out_lm[o];
+    const float4 a = *reinterpret_cast<const float4 *>(Adf + lm * ldA + 2 * q);
+    const double v = nu[q];
+    const double re = out[2 * o] - fma(v, rref[lm * ldR], (double)a.x + (double)a.y);
+    const double im = out[2 * o + 1] - fma(v, rref[lm * ldR + 1], (double)a.z + (double)a.w);
+    out[2 * o] = re;
+    out[2 * o + 1] = im;
+    if (!(isfinite(re) && isfinite(im))) atomicOr(err, ERR_NONFINITE_OUTPUT);
+}
+
+void launch_sub_window_df(const Plan &p, const float2 *Adf, int64_t ldA, int64_t pair0, int64_t npc, const double *nu,
+                          const double *rref, int64_t ldR, double *out, int *err, cudaStream_t st) {
+    k_sub_window_df<<<(unsigned)((p.nlmsize + 127) / 128), 128, 0, st>>>(p.d_out_pair, p.d_out_lm, p.nlmsize, Adf, ldA,
+                                                                        pair0, npc, nu, rref, ldR, out, err);
     note_launch();
 }
 

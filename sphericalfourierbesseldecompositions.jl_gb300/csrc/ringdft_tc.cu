@@ -112,11 +112,11 @@ __device__ __forceinline__ void st_shared_v4(unsigned char *p, const uint32_t (&
 // non-finite value keeps an ordinary exponent, so the value reaches the
 // spectra and the transform's finiteness check.  erow layout [2][nrn][nmaps];
 // nzr[0] / nzr[1] get the first / last ring pair with a non-zero row (preset
-// to a large value / -1).  With ring_live (one array per nper maps), the rows on
-// the rings marked 0 are zero by construction and are not read.
+// to a large value / -1).  With live, rows on the rings marked 0 there are zero by
+// construction and are not read.
 __global__ void __launch_bounds__(128) k_ring_rowexp(const float2 *__restrict__ maps, int64_t npix, int64_t nmaps,
                                                      const RingGeom *__restrict__ rings, int nrn, int *erow,
-                                                     int *nzr, const int *__restrict__ ring_live, int64_t nper,
+                                                     int *nzr, LiveRings live,
                                                      int nrings) {
     const int r = blockIdx.x;
     const int64_t b = (int64_t)blockIdx.y * 4 + (threadIdx.x >> 5);
@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(128) k_ring_rowexp(const float2 *__restrict__ 
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         if (b >= nmaps) break;
-        if (ring_live && !ring_live[(b / nper) * nrings + (h ? nrings - 1 - r : r)]) {
+        if (b < live.n && !live.ring[(b / live.per) * nrings + (h ? nrings - 1 - r : r)]) {
             if (lane == 0) erow[((int64_t)h * nrn + r) * nmaps + b] = ZERO_ROW_E;
             continue;
         }
@@ -707,14 +707,14 @@ uint2 dft_slices(double v, int EB) {
 }
 
 int launch_ring_analysis_tc(Plan &p, const float2 *maps, int64_t nmaps, float2 *F, int *erow, int *nzr,
-                            cudaStream_t st, const int *ring_live, int64_t nper, bool skip_unread) {
+                            cudaStream_t st, const LiveRings &live, bool skip_unread) {
     {
         // nzr[0] = 0x7f7f7f7f (above any ring index), nzr[1] = -1
         cudaMemsetAsync(nzr, 0x7f, sizeof(int), st);
         cudaMemsetAsync(nzr + 1, 0xff, sizeof(int), st);
         dim3 grid((unsigned)p.nrn, (unsigned)((nmaps + 3) / 4));
-        dft::k_ring_rowexp<<<grid, 128, 0, st>>>(maps, p.npix, nmaps, p.d_rings, (int)p.nrn, erow, nzr, ring_live,
-                                                 nper, (int)(4 * p.nside - 1));
+        dft::k_ring_rowexp<<<grid, 128, 0, st>>>(maps, p.npix, nmaps, p.d_rings, (int)p.nrn, erow, nzr, live,
+                                                 (int)(4 * p.nside - 1));
         note_launch();
     }
     set_smem(dft::k_ring_dft_tc<true, true>, dft::SMEM);

@@ -256,10 +256,6 @@ __host__ __device__ __forceinline__ int ring_of_pixel(int64_t nside, int64_t pix
     if (pix >= npix - ncap) return (int)(4 * nside - cap(npix - 1 - pix)) - 1;
     return (int)((pix - ncap) / (4 * nside) + nside) - 1;
 }
-// A[lm][2j + c] += mu[j] * rmu[lm * ldr + c] for j < nmaps; with set_col >= 0
-// also A[lm][2 set_col + c] = rset[lm * ldr + c].
-void launch_add_mean(double *A, int64_t ldA, int64_t nmaps, const double *mu, const double *rmu, const double *rset,
-                     int64_t ldr, int64_t lmsize, int64_t set_col, cudaStream_t st);
 // Mixed-precision radial projection (double-float sums; FP64 mean and window
 // terms), replacing add_mean + project_poly for the data term.
 void launch_coef_df(const Plan &p, const int32_t *pair_index, float2 *CT, cudaStream_t st);
@@ -272,8 +268,15 @@ void launch_project_mixed(const Plan &p, const float2 *Adf, int64_t ldA, const f
                           const int32_t *pair_index, int nmock, const double *scale, const double *smean,
                           const double *ralm, int64_t ldR, int window_kind, const double *w_ln, double *out, int *err,
                           cudaStream_t st);
-// maps[j] -= nu[j] ref with nu[j] = <maps[j], ref> / <ref, ref> (FP64, in place).
-void launch_split_mean(double *maps, int64_t nmaps, int64_t npix, const double *ref, double *nu, cudaStream_t st);
+// Dense window maps of the pairs [pair0, pair0 + npc) for the mixed transform: maps[j] = W_j - nu[j] ref as
+// double-float maps, nu[j] = <W_j, ref> / <ref, ref> (FP64; *refsq holds <ref, ref>, made by launch_ref_square).
+void launch_ref_square(const double *ref, int64_t npix, double *refsq, cudaStream_t st);
+void launch_dense_maps_df(const Plan &p, const double *dense, const double *ref, const double *refsq, int64_t pair0,
+                          int64_t npc, double *nu, float2 *maps, cudaStream_t st);
+// out -= the window coefficients of those pairs: Adf (row lm of ldA, pair j's columns 2 j, 2 j + 1) + nu[j] rref[lm
+// ldR ..]; err as in launch_project_mixed
+void launch_sub_window_df(const Plan &p, const float2 *Adf, int64_t ldA, int64_t pair0, int64_t npc, const double *nu,
+                          const double *rref, int64_t ldR, double *out, int *err, cudaStream_t st);
 // nzr (FP64): receives the first / last ring pair holding a non-zero value in any map
 // (preset by the caller to a large value / -1).
 // Window mixing matrix (wmix.cu): largest lmax it supports, shared memory of one CTA for the
@@ -324,11 +327,14 @@ void launch_to_float(const double *in, int64_t n, float *out, cudaStream_t st);
 void launch_to_df(const double *in, int64_t n, float2 *out, cudaStream_t st);
 // Mixed-precision ring analysis on the tensor cores (double-float maps -> double-float F).
 // nzr[0..1] receives the first and last ring pair holding a non-zero map row.
-// ring_live (optional): nper maps share an array of 4 nside - 1 entries (map b the (b / nper)-th); their rings whose
-// entry is 0 hold zeros and are not read.
+// live (optional): the first n maps have rings that hold zeros and are not read, those whose entry in an array of
+// 4 nside - 1 is 0; per maps share one array (map b the (b / per)-th).
+struct LiveRings {
+    const int *ring = nullptr;
+    int64_t n = 0, per = 1;
+};
 int launch_ring_analysis_tc(Plan &p, const float2 *maps, int64_t nmaps, float2 *F, int *erow, int *nzr,
-                            cudaStream_t st, const int *ring_live = nullptr, int64_t nper = 1,
-                            bool skip_unread = false);
+                            cudaStream_t st, const LiveRings &live = LiveRings(), bool skip_unread = false);
 uint2 dft_slices(double v, int EB);
 int64_t dft_image_offsets(const Plan &p, const std::vector<int32_t> &crings, const std::vector<int32_t> &coff,
                           bool with_polar, std::vector<int64_t> &off, int &max_nch);
@@ -374,6 +380,31 @@ void launch_ang2pix(int64_t nside, const double *theta, const double *phi, int64
 // shared device helpers
 // ---------------------------------------------------------------------------
 #ifdef __CUDACC__
+// Double -> double-float by integer operations only (no FP64 instruction, whose
+// rate on this GPU is a small fraction of the FP32 one): hi = d rounded to the
+// nearest FP32 (ties to even, as (float)d), lo = d - hi rounded to FP32, ~48
+// significant bits in all.  Finite d; below the FP32 normal range hi is 0
+// (sign kept), and lo is 0 for |d| < 2^-75.
+__device__ __forceinline__ float2 df_split_bits(double d) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(d);
+    const unsigned sign = (unsigned)(b >> 32) & 0x80000000u;
+    const int e = (int)((b >> 52) & 0x7ff);
+    const int fe = e - 1023 + 127;
+    if (fe <= 0) return make_float2(__uint_as_float(sign), 0.f);
+    if (fe >= 255) return make_float2(__uint_as_float(sign | 0x7f800000u), 0.f);
+    const unsigned long long m = b & 0xfffffffffffffull;
+    const unsigned rem = (unsigned)(m & 0x1fffffffu);                 // the 29 bits below FP32
+    const unsigned hb = sign | ((unsigned)fe << 23) | (unsigned)(m >> 29);
+    const bool up = rem > 0x10000000u || (rem == 0x10000000u && (hb & 1u));
+    // a mantissa carry moves into the exponent, as rounding up does
+    const float hi = __uint_as_float(hb + (up ? 1u : 0u));
+    // d - hi = (rem - up 2^29) 2^(e - 1075); exact scale where 2^(e - 1075) is an FP32 normal
+    const int r = (int)rem - (up ? 0x20000000 : 0);
+    const int se = e - 1075 + 127;
+    float lo = se >= 1 ? (float)r * __uint_as_float((unsigned)se << 23) : 0.f;
+    return make_float2(hi, sign ? -lo : lo);
+}
+
 // 0-based HEALPix RING pixel of (z = cos theta, phi); the HEALPix paper
 // algorithm (Gorski et al. 2005).  Every operation is an explicitly rounded
 // IEEE op (no FMA contraction) so the integer result matches a plain FP64
