@@ -96,11 +96,14 @@ void launch_transpose(const double *in, int64_t rows, int64_t cols, double *out,
 }
 
 __device__ __forceinline__ float2 convert_elem(float v, float2 *) { return make_float2(v, 0.f); }
+__device__ __forceinline__ float2 convert_elem(double v, float2 *) {
+    return isfinite(v) ? df_split_bits(v) : make_float2((float)v, 0.f);
+}
 template <typename TI, typename TO>
 __device__ __forceinline__ TO convert_elem(TI v, TO *) { return (TO)v; }
 
 // out[c * ldo + r] = in[r * ldi + c] for r < rows, c < cols (converted to TO; float -> double-float
-// pairs with a zero low word).
+// pairs with a zero low word, double -> normalised pairs).
 template <typename TI, typename TO>
 __global__ void k_transpose_ld(const TI *in, int64_t ldi, int64_t rows, int64_t cols, TO *out, int64_t ldo) {
     __shared__ TI tile[32][33];
@@ -127,6 +130,11 @@ static void transpose_ld(const TI *in, int64_t ldi, int64_t rows, int64_t cols, 
     dim3 grid((unsigned)((cols + 31) / 32), (unsigned)std::min<int64_t>((rows + 31) / 32, 65535));
     k_transpose_ld<TI, TO><<<grid, dim3(32, 8), 0, st>>>(in, ldi, rows, cols, out, ldo);
     note_launch();
+}
+
+void launch_transpose_ld(const double *in, int64_t ldi, int64_t rows, int64_t cols, float2 *out, int64_t ldo,
+                         cudaStream_t st) {
+    transpose_ld(in, ldi, rows, cols, out, ldo, st);
 }
 
 void launch_transpose_ld(const double *in, int64_t ldi, int64_t rows, int64_t cols, double *out, int64_t ldo,

@@ -88,6 +88,8 @@ void launch_transpose_ld(const double *in, int64_t ldi, int64_t rows, int64_t co
                          cudaStream_t st);
 void launch_transpose_ld(const float *in, int64_t ldi, int64_t rows, int64_t cols, float2 *out, int64_t ldo,
                          cudaStream_t st);
+void launch_transpose_ld(const double *in, int64_t ldi, int64_t rows, int64_t cols, float2 *out, int64_t ldo,
+                         cudaStream_t st);
 void launch_axpy(double *y, const double *x, int64_t n, cudaStream_t st);
 void launch_winweights(const double *weights, int64_t nr, int64_t nside, const double *rbounds, double rmax,
                        const double *rtp, int64_t ngal, double *w, int *err, cudaStream_t st);
@@ -108,7 +110,9 @@ struct sfb_plan {
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_mu = nullptr, ev_dense = nullptr;
     // host entry: the catalogue copy runs on the side stream in NCOPY chunks
     static constexpr int NCOPY = 4;
-    cudaEvent_t ev_copy[NCOPY] = {};
+    // (a field's copies run in ring groups, NFIELD at most)
+    static constexpr int NFIELD = 8;
+    cudaEvent_t ev_copy[NFIELD] = {};
     int32_t *d_pair_index = nullptr;
     int64_t *d_noff = nullptr;
     // FP64 transform at lmax 2 lmax for the window harmonics of win_lnn (the reference's
@@ -335,12 +339,131 @@ void synthesis_and_gram64(const Plan &p, const double *A, const double *A0, int6
     launch_gram_update_fp64(p, A, A0, ncol, Anew, st);
 }
 
+// Ring groups of a field in pixel-major host memory: `belt` groups of equatorial ring pairs, then the polar rings.
+// A group is a range of ring launch indices and the two pixel ranges (north, south) that hold its rings.
+struct PixGroup {
+    int z0, nz;
+    int64_t p0[2], np[2];
+};
+std::vector<PixGroup> pix_groups(const Plan &p, int belt) {
+    std::vector<PixGroup> v;
+    const int ns = (int)p.nside, nrn = (int)p.nrn;
+    belt = std::min(belt, ns + 1);
+    auto north = [&](int r) { return r < nrn ? p.h_rings[r].start_n : p.h_rings[nrn - 1].start_n + p.h_rings[nrn - 1].nph; };
+    auto add = [&](int z0, int nz, int ra, int rb) {            // ring pairs [ra, rb), the equator without a mirror
+        PixGroup g{z0, nz, {north(ra), 0}, {north(rb) - north(ra), 0}};
+        const int last = std::min(rb, nrn - 1) - 1;              // southernmost pair's mirror is the first ring there
+        if (last >= ra) {
+            g.p0[1] = p.h_rings[last].start_s;
+            g.np[1] = p.h_rings[ra].start_s + p.h_rings[ra].nph - g.p0[1];
+        }
+        v.push_back(g);
+    };
+    for (int i = 0; i < belt; ++i) {
+        const int a = (ns + 1) * i / belt, b = (ns + 1) * (i + 1) / belt;
+        add(a, b - a, ns - 1 + a, ns - 1 + b);
+    }
+    if (ns > 1) add(ns + 1, ns - 1, 0, ns - 1);
+    return v;
+}
+
+// Belt groups of a field of `bytes`: 16 MB each (about 80 us of the copy, a few times what a group's launches cost),
+// four at most; 0: below 8 MB the copy is not worth splitting.
+int belt_groups(int64_t bytes) {
+    return bytes < (8 << 20) ? 0 : (int)std::max<int64_t>(1, std::min<int64_t>(4, bytes >> 24));
+}
+
+// A field [npix][nr] in host memory whose shells are the maps of one transform: the ring stage copies it to `dev` on
+// the side stream one ring group at a time and starts on a group's rings when they have landed.
+struct FieldSrc {
+    const char *host;
+    char *dev;
+    int32_t dtype;
+    int64_t nr;
+};
+
+int copy_group(sfb_plan *h, const FieldSrc &s, const PixGroup &g, cudaEvent_t landed) {
+    const size_t row = (size_t)s.nr * (s.dtype == SFB_F32 ? sizeof(float) : sizeof(double));
+    for (int i = 0; i < 2; ++i)
+        if (g.np[i] > 0)
+            SFB_CUDA_TRY(cudaMemcpyAsync(s.dev + g.p0[i] * row, s.host + g.p0[i] * row, g.np[i] * row,
+                                         cudaMemcpyHostToDevice, h->side));
+    SFB_CUDA_TRY(cudaEventRecord(landed, h->side));
+    return SFB_OK;
+}
+
+// the group's pixels of every shell into the maps [nr][npix] (double-float pairs for the mixed transform, else FP64)
+void lay_out_group(const Plan &p, const FieldSrc &s, const PixGroup &g, bool mixed, double *maps, cudaStream_t st) {
+    for (int i = 0; i < 2; ++i) {
+        if (g.np[i] <= 0) continue;
+        const int64_t p0 = g.p0[i], n = g.np[i];
+        const float *f = reinterpret_cast<const float *>(s.dev) + p0 * s.nr;
+        const double *d = reinterpret_cast<const double *>(s.dev) + p0 * s.nr;
+        float2 *mf = reinterpret_cast<float2 *>(maps) + p0;
+        if (s.dtype == SFB_F32) {
+            if (mixed) launch_transpose_ld(f, s.nr, n, s.nr, mf, p.npix, st);
+            else launch_transpose_ld(f, s.nr, n, s.nr, maps + p0, p.npix, st);
+        } else {
+            if (mixed) launch_transpose_ld(d, s.nr, n, s.nr, mf, p.npix, st);
+            else launch_transpose_ld(d, s.nr, n, s.nr, maps + p0, p.npix, st);
+        }
+    }
+}
+
+// The ring stage of a field transform, beside the field's copy.  Mixed: the equatorial rings (two thirds of the
+// pixels) first, on the DFT's second stream, then the polar ones, which wait for the last third of the copy only.
+// FP64: the polar rings first, then the belt in groups.
+int field_ring_stage(sfb_plan *h, const FieldSrc &s, double *maps, double *F, int *erow, int *nzr, bool skip_unread,
+                     cudaStream_t st) {
+    Plan &p = h->p;
+    const bool mixed = p.precision == SFB_MIXED;
+    const int64_t bytes = p.npix * s.nr * (int64_t)(s.dtype == SFB_F32 ? sizeof(float) : sizeof(double));
+    std::vector<PixGroup> g = pix_groups(p, std::min(belt_groups(bytes), mixed ? 3 : 4));
+    const int n = (int)g.size();
+    const bool polar = p.nside > 1;
+    if (!mixed && polar) std::rotate(g.begin(), g.end() - 1, g.end());
+    if (mixed) SFB_TRY(ring_tc_begin(p, s.nr, nzr, st));
+    SFB_CUDA_TRY(cudaEventRecord(p.dft_fork, st));
+    SFB_CUDA_TRY(cudaStreamWaitEvent(h->side, p.dft_fork, 0));
+    // (group by group, so that the kernels of one run while a copy from pageable memory holds the host)
+    if (mixed) {
+        cudaStream_t eq = p.dft_side;
+        SFB_CUDA_TRY(cudaStreamWaitEvent(eq, p.dft_fork, 0));
+        for (int i = 0; i < n; ++i) {
+            const bool pol = polar && i == n - 1;
+            cudaStream_t q = pol ? st : eq;
+            SFB_TRY(copy_group(h, s, g[i], h->ev_copy[i]));
+            SFB_CUDA_TRY(cudaStreamWaitEvent(q, h->ev_copy[i], 0));
+            lay_out_group(p, s, g[i], true, maps, q);
+            if (pol || i == n - 1 - (polar ? 1 : 0))
+                ring_tc_part(p, reinterpret_cast<const float2 *>(maps), s.nr, reinterpret_cast<float2 *>(F), erow, nzr,
+                             skip_unread, !pol, q);
+        }
+        SFB_CUDA_TRY(cudaEventRecord(p.dft_join, eq));
+        SFB_CUDA_TRY(cudaStreamWaitEvent(st, p.dft_join, 0));
+        return SFB_OK;
+    }
+    bool tc = s.nr >= RING64_MIN;
+    for (int i = 0; i < n; ++i) {
+        SFB_TRY(copy_group(h, s, g[i], h->ev_copy[i]));
+        SFB_CUDA_TRY(cudaStreamWaitEvent(st, h->ev_copy[i], 0));
+        lay_out_group(p, s, g[i], false, maps, st);
+        if (tc && !launch_ring_analysis64(p, maps, s.nr, F, st, nzr, g[i].z0, g[i].nz)) {
+            if (i > 0) return fail(SFB_ENOMEM, "ring transform workspace lost");      // the first group made it
+            tc = false;
+        }
+    }
+    if (!tc) launch_ring_analysis(p, maps, s.nr, F, st, nzr);
+    return SFB_OK;
+}
+
 // fp64_out: the FP64 a_lm (alm) is wanted besides the double-float copy (almdf, mixed precision); the
 // Gram refinement carries only the double-float one and converts at the end when asked.
+// src: the maps are still to be made in `maps` from a field in host memory (field_ring_stage).
 // live (mixed precision): rings that hold zeros, left unwritten by the deposit (deposit_sorted's ring_live).
 int sht_analysis(sfb_plan *h, const double *maps, int64_t nm, cudaStream_t st, bool maps_are_fp64 = false,
                  int stage_override = -1, const ShtWork *ws = nullptr, bool fp64_out = true,
-                 const LiveRings &live = LiveRings()) {
+                 const LiveRings &live = LiveRings(), const FieldSrc *src = nullptr) {
     Plan &p = h->p;
     const ShtWork own{&p.fbuf, &p.gbuf, &p.rbuf, &p.alm};
     if (!ws) ws = &own;
@@ -374,7 +497,11 @@ int sht_analysis(sfb_plan *h, const double *maps, int64_t nm, cudaStream_t st, b
         // the Gram refinement and niter = 0 read the spectra only in the first analysis pass (over the
         // span with data and the live chunks); the full refinement passes fold them over every ring
         const bool skip_unread = (nm > 4 && p.d_gramts && p.niter > 0) || p.niter == 0;
-        SFB_TRY(launch_ring_analysis_tc(p, reinterpret_cast<const float2 *>(maps), nm,
+        if (src)
+            SFB_TRY(field_ring_stage(h, *src, const_cast<double *>(maps), fbuf.ptr, reinterpret_cast<int *>(p.erow.ptr),
+                                     nzr, skip_unread, st));
+        else
+            SFB_TRY(launch_ring_analysis_tc(p, reinterpret_cast<const float2 *>(maps), nm,
                                         reinterpret_cast<float2 *>(fbuf.ptr), reinterpret_cast<int *>(p.erow.ptr), nzr,
                                         st, live, skip_unread));
     } else {
@@ -387,7 +514,8 @@ int sht_analysis(sfb_plan *h, const double *maps, int64_t nm, cudaStream_t st, b
             SFB_CUDA_TRY(cudaMemsetAsync(nzr + 1, 0xff, sizeof(int), st));      // last: -1
         }
         Stage s(h, stage(SFB_STAGE_RING_FFT), st);
-        launch_ring_analysis(p, maps, nm, fbuf.ptr, st, nzr);
+        if (src) SFB_TRY(field_ring_stage(h, *src, const_cast<double *>(maps), fbuf.ptr, nullptr, nzr, false, st));
+        else launch_ring_analysis(p, maps, nm, fbuf.ptr, st, nzr);
     }
     const bool tc = p.precision == SFB_MIXED;
     float2 *adf = reinterpret_cast<float2 *>(p.almdf.ptr);
@@ -547,11 +675,52 @@ int reference_alm(sfb_plan *h, const double *ref, int64_t nref, cudaStream_t st)
     return rc;
 }
 
+// Pixel-major ring synthesis into out[pixel ld + map] of nm maps on the device; with host, which has the same layout,
+// each ring group's pixels go there on the side stream while the next group is formed (the caller's stream waits
+// for the copies at the end).  *done: false when the plan's tensor-core transform is not available (nothing done).
+// *copied: the field is on its way to host.
+int synthesis_pixmajor(sfb_plan *h, const double *G, int64_t nm, void *out, int64_t ld, bool f32, void *host,
+                       cudaStream_t st, bool *done, bool *copied) {
+    Plan &p = h->p;
+    *done = *copied = false;
+    if (nm < RING64_MIN) return SFB_OK;
+    const size_t row = (size_t)ld * (f32 ? sizeof(float) : sizeof(double));
+    const int belt = belt_groups((int64_t)row * p.npix);
+    if (!host || belt == 0) {
+        *done = launch_ring_synthesis64(p, G, nm, out, ld, true, f32, st);
+        return SFB_OK;
+    }
+    const std::vector<PixGroup> gs = pix_groups(p, belt);
+    for (size_t i = 0; i < gs.size(); ++i) {
+        const PixGroup &g = gs[i];
+        if (!launch_ring_synthesis64(p, G, nm, out, ld, true, f32, st, g.z0, g.nz)) {
+            if (i == 0) return SFB_OK;
+            return fail(SFB_ENOMEM, "ring synthesis workspace lost");
+        }
+        SFB_CUDA_TRY(cudaEventRecord(h->ev_copy[i], st));
+    }
+    for (size_t i = 0; i < gs.size(); ++i) {      // (a copy to pageable memory holds the host: every kernel is queued)
+        const PixGroup &g = gs[i];
+        SFB_CUDA_TRY(cudaStreamWaitEvent(h->side, h->ev_copy[i], 0));
+        for (int k = 0; k < 2; ++k)
+            if (g.np[k] > 0)
+                SFB_CUDA_TRY(cudaMemcpyAsync(static_cast<char *>(host) + g.p0[k] * row,
+                                             static_cast<char *>(out) + g.p0[k] * row, g.np[k] * row,
+                                             cudaMemcpyDeviceToHost, h->side));
+    }
+    SFB_CUDA_TRY(cudaEventRecord(h->ev_join, h->side));
+    SFB_CUDA_TRY(cudaStreamWaitEvent(st, h->ev_join, 0));
+    *done = *copied = true;
+    return SFB_OK;
+}
+
 // Transpose of sht_analysis in FP64 (adjoint.cu): abar [lmsize][2 nm] on the device becomes b = w E abar;
 // maps_out [nm][npix] FP64 receives S sum_j (I - A S)^j b.  With pix_ld the maps may come pixel-major instead:
-// map b, pixel x at pix_out[x pix_ld + b] (float or double); *pixmajor says whether they did.
+// map b, pixel x at pix_out[x pix_ld + b] (float or double); *pixmajor says whether they did and, with pix_host,
+// *copied whether they are on their way there.
 int sht_analysis_adjoint(sfb_plan *h, double *abar, int64_t nm, double *maps_out, cudaStream_t st,
-                         void *pix_out = nullptr, int64_t pix_ld = 0, bool pix_f32 = false, bool *pixmajor = nullptr) {
+                         void *pix_out = nullptr, int64_t pix_ld = 0, bool pix_f32 = false, bool *pixmajor = nullptr,
+                         void *pix_host = nullptr, bool *copied = nullptr) {
     Plan &p = h->p;
     const int32_t prec = p.precision;
     p.precision = SFB_FP64;
@@ -595,7 +764,9 @@ int sht_analysis_adjoint(sfb_plan *h, double *abar, int64_t nm, double *maps_out
         x = p.alm.ptr;
     }
     launch_leg_synthesis(p, x, ncol, p.gbuf.ptr, st);
-    const bool pm = pix_out && nm > 4 && launch_ring_synthesis64(p, p.gbuf.ptr, nm, pix_out, pix_ld, true, pix_f32, st);
+    bool pm = false, cp = false;
+    if (pix_out) SFB_TRY(synthesis_pixmajor(h, p.gbuf.ptr, nm, pix_out, pix_ld, pix_f32, pix_host, st, &pm, &cp));
+    if (copied) *copied = cp;
     if (pixmajor) *pixmajor = pm;
     if (!pm) launch_ring_synthesis(p, p.gbuf.ptr, nm, maps_out, st);
     SFB_CUDA_TRY(cudaGetLastError());
@@ -1504,6 +1675,7 @@ static int field2anlm_vjp_impl(sfb_plan *h, const double *abar, int64_t nr, doub
     double *d_f = d_A + p.lmsize * 2 * cs;
     SFB_CUDA_TRY(cudaMemcpyAsync(d_ab, abar, 2 * p.nlmsize * sizeof(double), cudaMemcpyHostToDevice, st));
     SFB_TRY(clear_err(p, st));
+    bool copied = false;
     launch_gtab(p, nr, rmin, dr, 1, d_g, st);                // g_nl(r_s) r_s^2 dr, the field2anlm weights
     SFB_TRY(grow(p, p.scratch2, (size_t)cs * p.npairs));
     SFB_TRY(grow(p, p.maps, (size_t)cs * p.npix));
@@ -1517,9 +1689,10 @@ static int field2anlm_vjp_impl(sfb_plan *h, const double *abar, int64_t nr, doub
         const int64_t ld = resident ? nr : nsc, off = resident ? s0 : 0;
         const bool f32 = dtype == SFB_F32;
         bool pm = false;
+        const bool one = resident && nsc == nr;            // the whole gradient: copied out beside the ring synthesis
         SFB_TRY(sht_analysis_adjoint(h, d_A, nsc, p.maps.ptr, st,
                                      f32 ? (void *)(reinterpret_cast<float *>(d_f) + off) : (void *)(d_f + off), ld, f32,
-                                     &pm));
+                                     &pm, one ? df_out : nullptr, &copied));
         if (pm) {
             // already in place
         } else if (f32)
@@ -1531,7 +1704,7 @@ static int field2anlm_vjp_impl(sfb_plan *h, const double *abar, int64_t nr, doub
                                            p.npix, cudaMemcpyDeviceToHost, st));
     }
     SFB_CUDA_TRY(cudaGetLastError());
-    if (resident)
+    if (resident && !copied)
         SFB_CUDA_TRY(cudaMemcpyAsync(df_out, d_f, (size_t)nr * p.npix * es, cudaMemcpyDeviceToHost, st));
     return check_tc(p, st);
 }
@@ -1585,7 +1758,10 @@ static int sfb_field2anlm_impl(sfb_plan *h, const void *f, int32_t dtype, int64_
     double *d_out = d_g + p.npairs * nr;
     double *d_acc = d_out + 2 * p.nlmsize;
     double *d_f = d_acc + 2 * p.nlmsize;
-    if (resident) SFB_CUDA_TRY(cudaMemcpyAsync(d_f, f, (size_t)nr * p.npix * es, cudaMemcpyHostToDevice, st));
+    // all shells in one transform: the copy runs beside its ring stage
+    const bool one = resident && cs >= nr && belt_groups(nr * p.npix * (int64_t)es) > 0;
+    const FieldSrc src{static_cast<const char *>(f), reinterpret_cast<char *>(d_f), dtype, nr};
+    if (resident && !one) SFB_CUDA_TRY(cudaMemcpyAsync(d_f, f, (size_t)nr * p.npix * es, cudaMemcpyHostToDevice, st));
     launch_gtab(p, nr, rmin, dr, 1, d_g, st);
     SFB_CUDA_TRY(cudaMemsetAsync(d_acc, 0, 2 * p.nlmsize * sizeof(double), st));
     SFB_TRY(clear_err(p, st));
@@ -1598,21 +1774,19 @@ static int sfb_field2anlm_impl(sfb_plan *h, const void *f, int32_t dtype, int64_
             SFB_CUDA_TRY(cudaMemcpy2DAsync(d_f, nsc * es, static_cast<const char *>(f) + s0 * es, nr * es, nsc * es,
                                            p.npix, cudaMemcpyHostToDevice, st));
         const int64_t ld = resident ? nr : nsc, off = resident ? s0 : 0;
-        // maps[s][p] = f[s0+s + nr p]: double-float maps (lo = 0) straight from an FP32 field in mixed
-        // precision, else FP64
-        bool maps64 = true;
-        if (dtype == SFB_F32) {
-            const float *src = reinterpret_cast<const float *>(d_f) + off;
-            if (mixed) {
-                launch_transpose_ld(src, ld, p.npix, nsc, reinterpret_cast<float2 *>(p.maps.ptr), p.npix, st);
-                maps64 = false;
+        // maps[s][p] = f[s0+s + nr p]
+        if (!one) {
+            if (dtype == SFB_F32) {
+                const float *q = reinterpret_cast<const float *>(d_f) + off;
+                if (mixed) launch_transpose_ld(q, ld, p.npix, nsc, reinterpret_cast<float2 *>(p.maps.ptr), p.npix, st);
+                else launch_transpose_ld(q, ld, p.npix, nsc, p.maps.ptr, p.npix, st);
             } else {
-                launch_transpose_ld(src, ld, p.npix, nsc, p.maps.ptr, p.npix, st);
+                const double *q = d_f + off;
+                if (mixed) launch_transpose_ld(q, ld, p.npix, nsc, reinterpret_cast<float2 *>(p.maps.ptr), p.npix, st);
+                else launch_transpose_ld(q, ld, p.npix, nsc, p.maps.ptr, p.npix, st);
             }
-        } else {
-            launch_transpose_ld(d_f + off, ld, p.npix, nsc, p.maps.ptr, p.npix, st);
         }
-        SFB_TRY(sht_analysis(h, p.maps.ptr, nsc, st, maps64));     // FP64 maps are converted in mixed precision
+        SFB_TRY(sht_analysis(h, p.maps.ptr, nsc, st, false, -1, nullptr, true, LiveRings(), one ? &src : nullptr));
         // gtab for this chunk: rows pair, cols nsc (copy sub-block)
         SFB_CUDA_TRY(cudaMemcpy2DAsync(p.scratch2.ptr, nsc * sizeof(double), d_g + s0, nr * sizeof(double),
                                        nsc * sizeof(double), p.npairs, cudaMemcpyDeviceToDevice, st));
@@ -1646,6 +1820,7 @@ static int sfb_anlm2field_impl(sfb_plan *h, const double *anlm, int64_t nr, doub
     SFB_TRY(grow(p, p.alm, (size_t)p.lmsize * 2 * cs));
     SFB_TRY(grow(p, p.maps, (size_t)cs * p.npix));
     SFB_TRY(clear_err(p, st));
+    bool copied = false;
     if (2 * cs > 8) ensure_tc64(p, st);
     for (int64_t s0 = 0; s0 < nr; s0 += cs) {
         const int64_t nsc = std::min(cs, nr - s0);
@@ -1654,13 +1829,16 @@ static int sfb_anlm2field_impl(sfb_plan *h, const double *anlm, int64_t nr, doub
         launch_shell_alm_g(p, h->d_pair_index, h->d_noff, p.scratch2.ptr, nsc, d_a, p.alm.ptr, 2 * nsc, st);
         launch_leg_synthesis(p, p.alm.ptr, 2 * nsc, p.gbuf.ptr, st);
         // f[s0+s + nr p], written so by the tensor-core transform; else transposed from maps[s][p]
-        if (!(nsc > 4 && launch_ring_synthesis64(p, p.gbuf.ptr, nsc, d_f + s0, nr, true, false, st))) {
+        bool pm = false;
+        SFB_TRY(synthesis_pixmajor(h, p.gbuf.ptr, nsc, d_f + s0, nr, false, nsc == nr ? f_out : nullptr, st, &pm, &copied));
+        if (!pm) {
             launch_ring_synthesis(p, p.gbuf.ptr, nsc, p.maps.ptr, st);
             launch_transpose_ld(p.maps.ptr, p.npix, nsc, p.npix, d_f + s0, nr, st);
         }
     }
     SFB_CUDA_TRY(cudaGetLastError());
-    SFB_CUDA_TRY(cudaMemcpyAsync(f_out, d_f, (size_t)nr * p.npix * sizeof(double), cudaMemcpyDeviceToHost, st));
+    if (!copied)
+        SFB_CUDA_TRY(cudaMemcpyAsync(f_out, d_f, (size_t)nr * p.npix * sizeof(double), cudaMemcpyDeviceToHost, st));
     return check_tc(p, st);
 }
 

@@ -71,8 +71,8 @@ __device__ __forceinline__ int64_t fixed53(double x, int emax) {
 __global__ void __launch_bounds__(256) k_fold64(const RingGeom *__restrict__ rings, int ns, int64_t npix,
                                                 const double *__restrict__ maps, int64_t nm,
                                                 const int64_t *__restrict__ qoff, int64_t *__restrict__ Q,
-                                                int *__restrict__ ex, int *nzr) {
-    const int r = blockIdx.y, lane = threadIdx.x & 31;
+                                                int *__restrict__ ex, int *nzr, int z0) {
+    const int r = ring_at(z0 + blockIdx.y, ns), lane = threadIdx.x & 31;
     const int64_t b = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (b >= nm) return;
     const RingGeom g = rings[r];
@@ -132,9 +132,9 @@ __global__ void __launch_bounds__(NTH, 2) k_rdft64(const RingGeom *__restrict__ 
                                                    const int64_t *__restrict__ qoff, const int64_t *__restrict__ Q,
                                                    const int *__restrict__ ex, const uint16_t *__restrict__ dig,
                                                    const int64_t *__restrict__ off, int Ew, double *__restrict__ F,
-                                                   int *err) {
+                                                   int z0, int *err) {
     extern __shared__ __align__(1024) unsigned char smem[];
-    const int r = ring_at(blockIdx.z, ns), cb = blockIdx.y & 3, tile = blockIdx.y >> 2;
+    const int r = ring_at(z0 + blockIdx.z, ns), cb = blockIdx.y & 3, tile = blockIdx.y >> 2;
     const int e = cb & 1, isS = cb >> 1;
     const RingGeom g = rings[r];
     const Ring R = ring_of(g, r, ns);
@@ -237,12 +237,12 @@ __global__ void __launch_bounds__(NTH, 2) k_rsyn64(const RingGeom *__restrict__ 
                                                    const double *__restrict__ G, const uint16_t *__restrict__ dig,
                                                    const int64_t *__restrict__ off, const int64_t *__restrict__ qoff,
                                                    int64_t *__restrict__ Y, int *__restrict__ gex, int kbmax, int sh,
-                                                   int *err) {
+                                                   int z0, int *err) {
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ uint32_t red[2][MTILE];
     __shared__ __align__(8) uint64_t bars[2];
     __shared__ uint32_t slot;
-    const int r = ring_at(blockIdx.z, ns), cb = blockIdx.y, e = cb & 1, isS = cb >> 1;
+    const int r = ring_at(z0 + blockIdx.z, ns), cb = blockIdx.y, e = cb & 1, isS = cb >> 1;
     const RingGeom g = rings[r];
     const Ring R = ring_of(g, r, ns);
     const int K = lmax >= e ? (lmax - e) / 2 + 1 : 0;
@@ -391,8 +391,8 @@ template <typename T, bool PIXMAJOR>
 __global__ void __launch_bounds__(256) k_unfold64(const RingGeom *__restrict__ rings, int ns, int64_t nm,
                                                   const int64_t *__restrict__ qoff, const int64_t *__restrict__ Y,
                                                   const int *__restrict__ gex, int sh, T *__restrict__ out,
-                                                  int64_t ld) {
-    const int r = ring_at(blockIdx.z, ns);
+                                                  int64_t ld, int z0) {
+    const int r = ring_at(z0 + blockIdx.z, ns);
     const RingGeom g = rings[r];
     const Ring R = ring_of(g, r, ns);
     int64_t b;
@@ -579,18 +579,20 @@ static bool ring64_room(Plan &p, int64_t nm, int *&ex) {
     return true;
 }
 
-bool launch_ring_analysis64(Plan &p, const double *maps, int64_t nm, double *F, cudaStream_t st, int *nzr) {
+bool launch_ring_analysis64(Plan &p, const double *maps, int64_t nm, double *F, cudaStream_t st, int *nzr, int z0,
+                            int nz) {
     int *ex = nullptr;
+    if (nz < 0) nz = (int)p.nrn;
     if (!ensure_ring64(p, 0, st) || !ring64_room(p, nm, ex)) return false;
     const int ns = (int)p.nside;
     int64_t *Q = reinterpret_cast<int64_t *>(p.ring64.ptr);
-    r64::k_fold64<<<dim3((unsigned)((nm + 7) / 8), (unsigned)p.nrn), 256, 0, st>>>(p.d_rings, ns, p.npix, maps, nm,
-                                                                                 p.ring64_qoff[0], Q, ex, nzr);
+    r64::k_fold64<<<dim3((unsigned)((nm + 7) / 8), (unsigned)nz), 256, 0, st>>>(p.d_rings, ns, p.npix, maps, nm,
+                                                                             p.ring64_qoff[0], Q, ex, nzr, z0);
     const int ntile = (r64::nfreq(4 * ns, p.lmax, 0) + t64::NT - 1) / t64::NT;
     set_smem(r64::k_rdft64, t64::SMEM);
-    r64::k_rdft64<<<dim3((unsigned)((2 * nm + t64::MTILE - 1) / t64::MTILE), (unsigned)(4 * ntile), (unsigned)p.nrn),
+    r64::k_rdft64<<<dim3((unsigned)((2 * nm + t64::MTILE - 1) / t64::MTILE), (unsigned)(4 * ntile), (unsigned)nz),
                     t64::NTH, t64::SMEM, st>>>(p.d_rings, ns, p.lmax, nm, p.ring64_qoff[0], Q, ex, p.ring64_dig[0],
-                                               p.ring64_off[0], p.ring64_ew, F, p.d_err);
+                                               p.ring64_off[0], p.ring64_ew, F, z0, p.d_err);
     note_launch();
     note_launch();
     return true;
@@ -598,8 +600,9 @@ bool launch_ring_analysis64(Plan &p, const double *maps, int64_t nm, double *F, 
 
 // Ring synthesis into maps out[map ld + pixel] or, pixel-major, out[pixel ld + map] of double or float.
 bool launch_ring_synthesis64(Plan &p, const double *G, int64_t nm, void *out, int64_t ld, bool pixmajor, bool f32,
-                             cudaStream_t st) {
+                             cudaStream_t st, int z0, int nz) {
     int *ex = nullptr;
+    if (nz < 0) nz = (int)p.nrn;
     if (!ensure_ring64(p, 1, st) || !ring64_room(p, nm, ex)) return false;
     const int ns = (int)p.nside;
     int64_t *Y = reinterpret_cast<int64_t *>(p.ring64.ptr);
@@ -610,21 +613,21 @@ bool launch_ring_synthesis64(Plan &p, const double *G, int64_t nm, void *out, in
     while (K >= (64 << sh)) ++sh;
     const size_t smem = (size_t)kb * t64::ND * (t64::PLANE_A + t64::NT * t64::KC * 2);
     set_smem(r64::k_rsyn64, smem);
-    r64::k_rsyn64<<<dim3((unsigned)((2 * nm + t64::MTILE - 1) / t64::MTILE), 4, (unsigned)p.nrn), t64::NTH, smem, st>>>(
-        p.d_rings, ns, p.lmax, nm, G, p.ring64_dig[1], p.ring64_off[1], p.ring64_qoff[1], Y, ex, kb, sh, p.d_err);
+    r64::k_rsyn64<<<dim3((unsigned)((2 * nm + t64::MTILE - 1) / t64::MTILE), 4, (unsigned)nz), t64::NTH, smem, st>>>(
+        p.d_rings, ns, p.lmax, nm, G, p.ring64_dig[1], p.ring64_off[1], p.ring64_qoff[1], Y, ex, kb, sh, z0, p.d_err);
     const int kcmax = ns + 1;
     if (pixmajor) {
-        const dim3 grid((unsigned)((nm + 31) / 32), (unsigned)((kcmax + 31) / 32), (unsigned)p.nrn);
+        const dim3 grid((unsigned)((nm + 31) / 32), (unsigned)((kcmax + 31) / 32), (unsigned)nz);
         if (f32)
             r64::k_unfold64<float, true><<<grid, 256, 0, st>>>(p.d_rings, ns, nm, p.ring64_qoff[1], Y, ex, sh,
-                                                               (float *)out, ld);
+                                                               (float *)out, ld, z0);
         else
             r64::k_unfold64<double, true><<<grid, 256, 0, st>>>(p.d_rings, ns, nm, p.ring64_qoff[1], Y, ex, sh,
-                                                                (double *)out, ld);
+                                                                (double *)out, ld, z0);
     } else {
-        const dim3 grid((unsigned)((nm + 7) / 8), (unsigned)((kcmax + 127) / 128), (unsigned)p.nrn);
+        const dim3 grid((unsigned)((nm + 7) / 8), (unsigned)((kcmax + 127) / 128), (unsigned)nz);
         r64::k_unfold64<double, false><<<grid, 256, 0, st>>>(p.d_rings, ns, nm, p.ring64_qoff[1], Y, ex, sh,
-                                                             (double *)out, ld);
+                                                             (double *)out, ld, z0);
     }
     note_launch();
     note_launch();

@@ -117,8 +117,8 @@ __device__ __forceinline__ void st_shared_v4(unsigned char *p, const uint32_t (&
 __global__ void __launch_bounds__(128) k_ring_rowexp(const float2 *__restrict__ maps, int64_t npix, int64_t nmaps,
                                                      const RingGeom *__restrict__ rings, int nrn, int *erow,
                                                      int *nzr, LiveRings live,
-                                                     int nrings) {
-    const int r = blockIdx.x;
+                                                     int nrings, int r0) {
+    const int r = r0 + blockIdx.x;
     const int64_t b = (int64_t)blockIdx.y * 4 + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     const RingGeom g = rings[r];
@@ -706,111 +706,112 @@ uint2 dft_slices(double v, int EB) {
     return make_uint2((uint32_t)s[0] | ((uint32_t)s[1] << 16), (uint32_t)s[2] | ((uint32_t)s[3] << 16));
 }
 
-int launch_ring_analysis_tc(Plan &p, const float2 *maps, int64_t nmaps, float2 *F, int *erow, int *nzr,
-                            cudaStream_t st, const LiveRings &live, bool skip_unread) {
-    {
-        // nzr[0] = 0x7f7f7f7f (above any ring index), nzr[1] = -1
-        cudaMemsetAsync(nzr, 0x7f, sizeof(int), st);
-        cudaMemsetAsync(nzr + 1, 0xff, sizeof(int), st);
-        dim3 grid((unsigned)p.nrn, (unsigned)((nmaps + 3) / 4));
-        dft::k_ring_rowexp<<<grid, 128, 0, st>>>(maps, p.npix, nmaps, p.d_rings, (int)p.nrn, erow, nzr, live,
-                                                 (int)(4 * p.nside - 1));
-        note_launch();
-    }
+static void ring_rowexp(const Plan &p, const float2 *maps, int64_t nmaps, int *erow, int *nzr, const LiveRings &live,
+                        int r0, int nr, cudaStream_t st) {
+    dft::k_ring_rowexp<<<dim3((unsigned)nr, (unsigned)((nmaps + 3) / 4)), 128, 0, st>>>(
+        maps, p.npix, nmaps, p.d_rings, (int)p.nrn, erow, nzr, live, (int)(4 * p.nside - 1), r0);
+    note_launch();
+}
+
+// with the A image the polar rings take B from the twiddle image as well (SFBGPU_DFT_POLAR_GATHER:
+// from the L1-resident ring tables, gathered by warps 4-7)
+static bool aimg_polar(const Plan &p) { return p.dft_aimg && p.n_polar > 0 && (p.dft_polar_gather || p.dtimg_polar); }
+static bool aimg_eq(const Plan &p) { return p.dft_aimg && p.d_dtimg != nullptr && p.n_eq_cls > 0; }
+
+// The non-zero range's preset, and the A image's per-class chunk offsets and buffer for this map count.
+int ring_tc_begin(Plan &p, int64_t nmaps, int *nzr, cudaStream_t st) {
+    // nzr[0] = 0x7f7f7f7f (above any ring index), nzr[1] = -1
+    cudaMemsetAsync(nzr, 0x7f, sizeof(int), st);
+    cudaMemsetAsync(nzr + 1, 0xff, sizeof(int), st);
     set_smem(dft::k_ring_dft_tc<true, true>, dft::SMEM);
     set_smem(dft::k_ring_dft_tc<false, true>, dft::SMEM);
     set_smem(dft::k_ring_dft_tc<true, false>, dft::SMEM);
     set_smem(dft::k_ring_dft_tc<false, false>, dft::SMEM);
+    if (!aimg_polar(p) && !aimg_eq(p)) return SFB_OK;
+    const int ncls = (int)p.h_cls_off.size() - 1;
+    if (p.aimg_nmaps != nmaps) {
+        p.h_aimg_off.assign(ncls + 1, 0);
+        int64_t o = 0;
+        for (int c = 0; c < ncls; ++c) {
+            p.h_aimg_off[c] = o;
+            const int64_t rings_c = p.h_cls_off[c + 1] - p.h_cls_off[c];
+            const int64_t tiles = (rings_c * nmaps + dft::NPAIR - 1) / dft::NPAIR;
+            const int64_t nph = p.h_rings[p.h_cls_rings[p.h_cls_off[c]]].nph;
+            o += tiles * ((nph + dft::KC - 1) / dft::KC);
+        }
+        p.h_aimg_off[ncls] = o;
+        SFB_CUDA_TRY(cudaMemcpyAsync(p.d_aimg_off, p.h_aimg_off.data(), (size_t)(ncls + 1) * sizeof(int64_t),
+                                     cudaMemcpyHostToDevice, st));
+        p.aimg_nmaps = nmaps;
+    }
+    return grow(p, p.aimg, (size_t)(p.h_aimg_off[ncls] * (4 * dft::PLANE) / sizeof(double)));
+}
+
+// Slicing pass and DFT of the equatorial classes (eq) or the polar rings, after their row exponents.
+static void ring_tc_dft(const Plan &p, const float2 *maps, int64_t nmaps, float2 *F, const int *erow,
+                        const unsigned char *dead, const int *span, bool eq, cudaStream_t st) {
     const unsigned ntn = (unsigned)((p.lmax + 1 + 63) / 64);
     const double wq = 4.0 * M_PI / (double)p.npix;
     const float2 wdf = make_float2((float)wq, (float)(wq - (double)(float)wq));
+    const unsigned mtiles = (unsigned)((nmaps + dft::NPAIR - 1) / dft::NPAIR);
+    const int64_t eq_tiles = ((int64_t)p.eq_max_rings * nmaps + dft::NPAIR - 1) / dft::NPAIR;
+    const unsigned tiles = eq ? (unsigned)eq_tiles : mtiles, ncls = (unsigned)(eq ? p.n_eq_cls : p.n_polar);
+    if (ncls == 0) return;
+    const int c0 = eq ? p.n_polar : 0;
+    const bool ai = eq ? aimg_eq(p) : aimg_polar(p);
+    // imaged classes read B from the image, the others gather it from the ring table
+    const bool img = eq ? p.d_dtimg != nullptr : p.dtimg_polar && !(ai && p.dft_polar_gather);
+    unsigned char *aimg = reinterpret_cast<unsigned char *>(p.aimg.ptr);
+    if (ai) {
+        // chunk groups: the longest ring (4 nside pixels) in groups of SLICE_CPG chunks
+        const unsigned ngrp = (unsigned)((4 * p.nside + dft::KC * dft::SLICE_CPG - 1) / (dft::KC * dft::SLICE_CPG));
+        dft::k_dft_slice_a<<<dim3(tiles, ncls, ngrp), dft::NPROD, 0, st>>>(
+            maps, p.npix, nmaps, p.d_rings, (int)p.nrn, p.d_cls_rings, p.d_cls_off + c0, erow, p.d_aimg_off + c0, aimg);
+        note_launch();
+    }
+    auto go = [&](auto kernel) {
+        kernel<<<dim3(ntn, tiles, ncls), dft::NTHR, dft::SMEM, st>>>(
+            maps, p.npix, nmaps, p.d_rings, (int)p.nrn, p.lmax, p.d_cls_rings, p.d_cls_off + c0, erow, p.d_dtw,
+            p.d_dtw_off, img ? p.d_dtimg : nullptr, img ? p.d_dtimg_off + c0 : nullptr, F, 2 * nmaps, wdf, dead, (int)ntn,
+            span, eq ? 0 : 1, ai ? p.d_aimg_off + c0 : nullptr, ai ? aimg : nullptr, p.d_err);
+    };
+    if (img && ai) go(dft::k_ring_dft_tc<true, true>);
+    else if (ai) go(dft::k_ring_dft_tc<false, true>);
+    else if (img) go(dft::k_ring_dft_tc<true, false>);
+    else go(dft::k_ring_dft_tc<false, false>);
+    note_launch();
+}
+
+// The equatorial rings (eq) or the polar rings of a transform begun with ring_tc_begin, alone: their maps arrive
+// apart (a field that is still being copied).  The span of ring pairs with data is not known yet, so the spectra
+// outside it are written too.
+void ring_tc_part(const Plan &p, const float2 *maps, int64_t nmaps, float2 *F, int *erow, int *nzr, bool skip_unread,
+                  bool eq, cudaStream_t st) {
+    const int r0 = eq ? p.n_polar : 0, nr = eq ? (int)p.nrn - p.n_polar : p.n_polar;
+    if (nr <= 0) return;
+    ring_rowexp(p, maps, nmaps, erow, nzr, LiveRings(), r0, nr, st);
+    ring_tc_dft(p, maps, nmaps, F, erow, skip_unread ? p.d_dft_dead : nullptr, nullptr, eq, st);
+}
+
+int launch_ring_analysis_tc(Plan &p, const float2 *maps, int64_t nmaps, float2 *F, int *erow, int *nzr,
+                            cudaStream_t st, const LiveRings &live, bool skip_unread) {
+    SFB_TRY(ring_tc_begin(p, nmaps, nzr, st));
+    ring_rowexp(p, maps, nmaps, erow, nzr, live, 0, (int)p.nrn, st);
     // skip_unread: the spectra are read only by the first analysis pass, over the span of ring pairs
     // with data and the live chunks, so the others need not be computed or written
     const unsigned char *dead = skip_unread ? p.d_dft_dead : nullptr;
     const int *span = skip_unread ? nzr : nullptr;
-    // imaged classes read B from the image, the others gather it from the ring table
-    const unsigned mtiles = (unsigned)((nmaps + dft::NPAIR - 1) / dft::NPAIR);
-    const int64_t eq_tiles = ((int64_t)p.eq_max_rings * nmaps + dft::NPAIR - 1) / dft::NPAIR;
-    // A-operand image for the imaged launches: per-class chunk offsets for this map count, the
-    // buffer, and the slicing pass (after the row exponents, on the call's stream)
-    // with the A image the polar rings take B from the twiddle image as well (SFBGPU_DFT_POLAR_GATHER:
-    // from the L1-resident ring tables, gathered by warps 4-7)
-    const bool aimg_polar = p.dft_aimg && p.n_polar > 0 && (p.dft_polar_gather || p.dtimg_polar);
-    const bool polar_img = p.dtimg_polar && !(aimg_polar && p.dft_polar_gather);
-    const bool aimg_eq = p.dft_aimg && p.d_dtimg != nullptr && p.n_eq_cls > 0;
     // the equatorial classes (equal CTAs, a partly filled last wave) run on the second stream beside
     // the polar rings (longest first), each class group's slicing pass directly before its DFT, so
     // the slicing of one group overlaps the DFT of the other and the tail of each launch the other
     const bool two = p.dft_side && p.n_polar > 0;
-    cudaStream_t st_eq = two ? p.dft_side : st;
-    if (aimg_polar || aimg_eq) {
-        const int ncls = (int)p.h_cls_off.size() - 1;
-        if (p.aimg_nmaps != nmaps) {
-            p.h_aimg_off.assign(ncls + 1, 0);
-            int64_t o = 0;
-            for (int c = 0; c < ncls; ++c) {
-                p.h_aimg_off[c] = o;
-                const int64_t rings_c = p.h_cls_off[c + 1] - p.h_cls_off[c];
-                const int64_t tiles = (rings_c * nmaps + dft::NPAIR - 1) / dft::NPAIR;
-                const int64_t nph = p.h_rings[p.h_cls_rings[p.h_cls_off[c]]].nph;
-                o += tiles * ((nph + dft::KC - 1) / dft::KC);
-            }
-            p.h_aimg_off[ncls] = o;
-            SFB_CUDA_TRY(cudaMemcpyAsync(p.d_aimg_off, p.h_aimg_off.data(), (size_t)(ncls + 1) * sizeof(int64_t),
-                                         cudaMemcpyHostToDevice, st));
-            p.aimg_nmaps = nmaps;
-        }
-        SFB_TRY(grow(p, p.aimg, (size_t)(p.h_aimg_off[ncls] * (4 * dft::PLANE) / sizeof(double))));
-    }
     if (two) {
         // after the row exponents, the offsets upload and the image's allocation on the call's stream
         cudaEventRecord(p.dft_fork, st);
         cudaStreamWaitEvent(p.dft_side, p.dft_fork, 0);
     }
-    if (aimg_polar || aimg_eq) {
-        unsigned char *aimg = reinterpret_cast<unsigned char *>(p.aimg.ptr);
-        // chunk groups: the longest ring (4 nside pixels) in groups of SLICE_CPG chunks
-        const unsigned ngrp = (unsigned)((4 * p.nside + dft::KC * dft::SLICE_CPG - 1) / (dft::KC * dft::SLICE_CPG));
-        if (aimg_polar) {
-            dft::k_dft_slice_a<<<dim3(mtiles, (unsigned)p.n_polar, ngrp), dft::NPROD, 0, st>>>(
-                maps, p.npix, nmaps, p.d_rings, (int)p.nrn, p.d_cls_rings, p.d_cls_off, erow, p.d_aimg_off, aimg);
-            note_launch();
-        }
-        if (aimg_eq) {
-            dft::k_dft_slice_a<<<dim3((unsigned)eq_tiles, (unsigned)p.n_eq_cls, ngrp), dft::NPROD, 0, st_eq>>>(
-                maps, p.npix, nmaps, p.d_rings, (int)p.nrn, p.d_cls_rings, p.d_cls_off + p.n_polar, erow,
-                p.d_aimg_off + p.n_polar, aimg);
-            note_launch();
-        }
-    }
-    unsigned char *aimg = reinterpret_cast<unsigned char *>(p.aimg.ptr);
-    auto launch = [&](dim3 grid, int c0, bool img, bool ai, int rev, cudaStream_t s) {
-        if (!img && ai)
-            dft::k_ring_dft_tc<false, true><<<grid, dft::NTHR, dft::SMEM, s>>>(
-                maps, p.npix, nmaps, p.d_rings, (int)p.nrn, p.lmax, p.d_cls_rings, p.d_cls_off + c0, erow, p.d_dtw,
-                p.d_dtw_off, nullptr, nullptr, F, 2 * nmaps, wdf, dead, (int)ntn, span, rev, p.d_aimg_off + c0, aimg,
-                p.d_err);
-        else if (img && ai)
-            dft::k_ring_dft_tc<true, true><<<grid, dft::NTHR, dft::SMEM, s>>>(
-                maps, p.npix, nmaps, p.d_rings, (int)p.nrn, p.lmax, p.d_cls_rings, p.d_cls_off + c0, erow, p.d_dtw,
-                p.d_dtw_off, p.d_dtimg, p.d_dtimg_off + c0, F, 2 * nmaps, wdf, dead, (int)ntn, span, rev,
-                p.d_aimg_off + c0, aimg, p.d_err);
-        else if (img)
-            dft::k_ring_dft_tc<true, false><<<grid, dft::NTHR, dft::SMEM, s>>>(
-                maps, p.npix, nmaps, p.d_rings, (int)p.nrn, p.lmax, p.d_cls_rings, p.d_cls_off + c0, erow, p.d_dtw,
-                p.d_dtw_off, p.d_dtimg, p.d_dtimg_off + c0, F, 2 * nmaps, wdf, dead, (int)ntn, span, rev, nullptr,
-                nullptr, p.d_err);
-        else
-            dft::k_ring_dft_tc<false, false><<<grid, dft::NTHR, dft::SMEM, s>>>(
-                maps, p.npix, nmaps, p.d_rings, (int)p.nrn, p.lmax, p.d_cls_rings, p.d_cls_off + c0, erow, p.d_dtw,
-                p.d_dtw_off, nullptr, nullptr, F, 2 * nmaps, wdf, dead, (int)ntn, span, rev, nullptr, nullptr,
-                p.d_err);
-        note_launch();
-    };
-    launch(dim3(ntn, (unsigned)eq_tiles, (unsigned)p.n_eq_cls), p.n_polar, p.d_dtimg != nullptr, aimg_eq, 0,
-           st_eq);
-    if (p.n_polar > 0)
-        launch(dim3(ntn, mtiles, (unsigned)p.n_polar), 0, polar_img, aimg_polar, 1, st);
+    ring_tc_dft(p, maps, nmaps, F, erow, dead, span, true, two ? p.dft_side : st);
+    ring_tc_dft(p, maps, nmaps, F, erow, dead, span, false, st);
     if (two) {
         cudaEventRecord(p.dft_join, p.dft_side);
         cudaStreamWaitEvent(st, p.dft_join, 0);

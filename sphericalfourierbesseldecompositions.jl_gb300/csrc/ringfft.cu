@@ -407,8 +407,6 @@ static void ring_analysis_t(const Plan &p, const TI *maps, int64_t nmaps, T *F, 
 
 // More than four FP64 maps go through the tensor cores (a row tile of them takes 64 maps; four maps or fewer
 // are the reference maps of the mixed transform and small map2alm batches, which the FFT does sooner).
-constexpr int64_t RING64_MIN = 5;
-
 void launch_ring_analysis(Plan &p, const double *maps, int64_t nmaps, double *F, cudaStream_t st, int *nzr) {
     if (p.precision == SFB_MIXED)
         ring_analysis_t<float, float, float2>(p, (const float *)maps, nmaps, (float *)F, p.d_twtab32, p.d_wphase32, st);

@@ -292,9 +292,13 @@ void launch_ring_analysis(Plan &p, const double *maps, int64_t nmaps, double *F,
 void launch_ring_synthesis(Plan &p, const double *G, int64_t nmaps, double *maps, cudaStream_t st);
 // The same for many FP64 maps on the tensor cores (ring64_tc.cu); false: nothing was launched (no tables or no
 // memory for them).  Synthesis: out[map ld + pixel], or pixel-major out[pixel ld + map] of double or float.
-bool launch_ring_analysis64(Plan &p, const double *maps, int64_t nmaps, double *F, cudaStream_t st, int *nzr);
+// Rings: launch indices [z0, z0 + nz) only, z <= nside the equatorial ring pairs nside - 1 + z, then the polar ones
+// from the longest (nz < 0: all 2 nside).  Nothing else is launched for them when it returns true once.
+bool launch_ring_analysis64(Plan &p, const double *maps, int64_t nmaps, double *F, cudaStream_t st, int *nzr, int z0 = 0,
+                            int nz = -1);
 bool launch_ring_synthesis64(Plan &p, const double *G, int64_t nmaps, void *out, int64_t ld, bool pixmajor, bool f32,
-                             cudaStream_t st);
+                             cudaStream_t st, int z0 = 0, int nz = -1);
+constexpr int64_t RING64_MIN = 5;      // maps from which they are used (launch_ring_analysis says why)
 // rlim: rings r < rlim (analysis: the sum; synthesis: the rings formed); -1 = all.
 // nzr (many columns): the analysis sums over the ring pairs [nzr[0], nzr[1]] only.
 void launch_leg_analysis(const Plan &p, const double *F, int64_t ncol, double *A, bool accumulate,
@@ -335,6 +339,9 @@ struct LiveRings {
 };
 int launch_ring_analysis_tc(Plan &p, const float2 *maps, int64_t nmaps, float2 *F, int *erow, int *nzr,
                             cudaStream_t st, const LiveRings &live = LiveRings(), bool skip_unread = false);
+int ring_tc_begin(Plan &p, int64_t nmaps, int *nzr, cudaStream_t st);
+void ring_tc_part(const Plan &p, const float2 *maps, int64_t nmaps, float2 *F, int *erow, int *nzr, bool skip_unread,
+                  bool eq, cudaStream_t st);
 uint2 dft_slices(double v, int EB);
 int64_t dft_image_offsets(const Plan &p, const std::vector<int32_t> &crings, const std::vector<int32_t> &coff,
                           bool with_polar, std::vector<int64_t> &off, int &max_nch);
