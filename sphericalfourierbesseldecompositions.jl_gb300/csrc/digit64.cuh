@@ -22,8 +22,9 @@ constexpr int KC = 16;                                 // K per chunk (one MMA K
 constexpr int MTILE = 128;                             // data columns per CTA
 constexpr int NT = 32;                                 // table rows per CTA
 constexpr int SBK = 16;                                // chunks per exact K block (256 values)
-constexpr int NPROD = 256;
-constexpr int NTH = NPROD + 32;
+// eight warps: a ninth for the MMAs would leave 96 registers a thread at two CTAs per SM instead of 128
+constexpr int NTH = 256;
+constexpr int MMA_WARP = NTH / 32 - 1;
 constexpr uint32_t PLANE_A = MTILE * KC * 2;
 constexpr int NSTAGE = 3;
 constexpr uint32_t STAGE_BYTES = ND * (PLANE_A + NT * KC * 2);
@@ -121,7 +122,7 @@ __device__ __forceinline__ uint32_t setup(Smem &c, unsigned char *base) {
     }
     if (threadIdx.x == 0) {
         for (int i = 0; i < NSTAGE; ++i) {
-            mbar_init(&c.full_a[i], NPROD / 32);
+            mbar_init(&c.full_a[i], NTH / 32);
             mbar_init(&c.full_b[i], 1);
             mbar_init(&c.empty[i], 1);
         }
@@ -150,73 +151,72 @@ __device__ __forceinline__ void issue(uint32_t tmem, uint32_t sa, uint32_t sb, i
     }
 }
 
-// One exact K block, chunks [k0, k1) of nch (k0 even): warps 0-7 turn their values into digits (load(kc,
-// buf): this thread's eight values of chunk kc, row tid % 128, k = 8 (tid / 128)..; fix: a value as the
-// integer), the table digits of chunk kc come from tab + kc ND LS KC, warp 8 issues the MMAs.  pre holds the
-// values of chunks k0 and k0 + 1 on entry.  Returns with every MMA complete; false when a wait gave up.
+// One exact K block, chunks [k0, k1) of nch (k0 even), up to its last MMA's issue: every warp turns its values
+// into digits (load(kc, buf): this thread's eight values of chunk kc, row tid % 128, k = 8 (tid / 128)..; fix: a
+// value as the integer), the table digits of chunk kc come from tab + kc ND LS KC, and the last warp issues a
+// chunk's MMAs once all have written theirs.  pre holds the values of chunks k0 and k0 + 1 on entry.  end_block
+// waits for the MMAs.
 template <typename T, typename Load, typename Fix>
-__device__ __forceinline__ bool run_block(const Smem &cs, uint32_t tmem, int k0, int k1, int nch, int sb, int LS,
+__device__ __forceinline__ void run_block(const Smem &cs, uint32_t tmem, int k0, int k1, int nch, int LS,
                                           const uint16_t *tab, T (&pre)[2][8], const Load &load, const Fix &fix) {
     const int tid = threadIdx.x, lane = tid & 31;
     const uint32_t bytesB = (uint32_t)ND * LS * KC * 2;
-    if (tid >= NPROD) {
+    const uint32_t off = core_off(tid & (MTILE - 1), 8 * (tid >> 7));
+    auto chunk = [&](int kc, T (&cur)[8]) -> bool {
+        const int s = kc % NSTAGE;
+        if (kc >= NSTAGE) {
+            if (*(volatile int *)cs.bad) return false;
+            if (!mbar_wait(&cs.empty[s], (uint32_t)((kc / NSTAGE - 1) & 1))) {
+                atomicExch(cs.bad, 1);
+                return false;
+            }
+        }
+        unsigned char *sa = cs.stage(s);
+        if (tid == 0) {
+            mbar_expect_tx(&cs.full_b[s], bytesB);
+            bulk_g2s(sa + ND * PLANE_A, tab + (int64_t)kc * ND * LS * KC, bytesB, &cs.full_b[s]);
+        }
+        uint32_t w[ND][4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            uint32_t v[ND];
+            digits2(fix(cur[2 * j]), fix(cur[2 * j + 1]), v);
+#pragma unroll
+            for (int q = 0; q < ND; ++q) w[q][j] = v[q];
+        }
+#pragma unroll
+        for (int q = 0; q < ND; ++q)
+            *reinterpret_cast<uint4 *>(sa + q * PLANE_A + off) = make_uint4(w[q][0], w[q][1], w[q][2], w[q][3]);
+        if (kc + 2 < nch) load(kc + 2, cur);
+        fence_proxy_async();
+        __syncwarp();
         if (lane == 0) {
-            int kc = k0;
-            for (; kc < k1; ++kc) {
-                const int s = kc % NSTAGE;
+            mbar_arrive(&cs.full_a[s]);
+            if (tid == 32 * MMA_WARP) {
                 const uint32_t ph = (uint32_t)((kc / NSTAGE) & 1);
-                if (*(volatile int *)cs.bad) break;
                 if (!mbar_wait(&cs.full_a[s], ph) || !mbar_wait(&cs.full_b[s], ph)) {
                     atomicExch(cs.bad, 1);
-                    break;
+                } else {
+                    fence_after();
+                    const uint32_t a = smem_u32(sa);
+                    issue(tmem, a, a + ND * PLANE_A, LS, kc == k0);
+                    mma_commit(&cs.empty[s]);
                 }
-                fence_after();
-                const uint32_t sa = smem_u32(cs.stage(s));
-                issue(tmem, sa, sa + ND * PLANE_A, LS, kc == k0);
-                mma_commit(&cs.empty[s]);
             }
-            if (kc < k1) atomicExch(cs.bad, 1);
-            mma_commit(cs.done);          // arrives once every MMA issued above has completed
         }
         __syncwarp();
-    } else {
-        const uint32_t off = core_off(tid & (MTILE - 1), 8 * (tid >> 7));
-        auto chunk = [&](int kc, T (&cur)[8]) -> bool {
-            const int s = kc % NSTAGE;
-            if (kc >= NSTAGE) {
-                if (*(volatile int *)cs.bad) return false;
-                if (!mbar_wait(&cs.empty[s], (uint32_t)((kc / NSTAGE - 1) & 1))) {
-                    atomicExch(cs.bad, 1);
-                    return false;
-                }
-            }
-            unsigned char *sa = cs.stage(s);
-            if (tid == 0) {
-                mbar_expect_tx(&cs.full_b[s], bytesB);
-                bulk_g2s(sa + ND * PLANE_A, tab + (int64_t)kc * ND * LS * KC, bytesB, &cs.full_b[s]);
-            }
-            uint32_t w[ND][4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                uint32_t v[ND];
-                digits2(fix(cur[2 * j]), fix(cur[2 * j + 1]), v);
-#pragma unroll
-                for (int q = 0; q < ND; ++q) w[q][j] = v[q];
-            }
-#pragma unroll
-            for (int q = 0; q < ND; ++q)
-                *reinterpret_cast<uint4 *>(sa + q * PLANE_A + off) = make_uint4(w[q][0], w[q][1], w[q][2], w[q][3]);
-            if (kc + 2 < nch) load(kc + 2, cur);
-            fence_proxy_async();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&cs.full_a[s]);
-            return true;
-        };
-        for (int kc = k0; kc < k1; kc += 2) {
-            if (!chunk(kc, pre[0])) break;
-            if (kc + 1 < k1 && !chunk(kc + 1, pre[1])) break;
-        }
+        return true;
+    };
+    for (int kc = k0; kc < k1; kc += 2) {
+        if (!chunk(kc, pre[0])) break;
+        if (kc + 1 < k1 && !chunk(kc + 1, pre[1])) break;
     }
+    if (tid == 32 * MMA_WARP) mma_commit(cs.done);          // arrives once every MMA issued above has completed
+    __syncwarp();
+}
+
+// Every MMA of block sb is complete; false when a wait gave up.
+__device__ __forceinline__ bool end_block(const Smem &cs, int sb) {
     const bool ok = mbar_wait(cs.done, (uint32_t)(sb & 1));
     fence_after();
     return __syncthreads_and(ok) && !*(volatile int *)cs.bad;

@@ -22,9 +22,9 @@
 // MMA shape: M = 128 data columns, N = table rows (<= 32 a tile), K = 16 a
 // step.  Data digit a multiplies the table digits 0..6-a in as few MMAs as N <=
 // 256 allows (their planes are stored back to back, and level v is TMEM
-// columns [v LS, (v + 1) LS)).  Warps 0-7 read FP64 columns, form the digits
+// columns [v LS, (v + 1) LS)).  Eight warps read FP64 columns, form the digits
 // with integer operations and store them as K-major core matrices; the table
-// digits arrive by bulk copy; warp 8 issues the MMAs.  7 x 32 TMEM columns and
+// digits arrive by bulk copy; the last warp issues the MMAs.  7 x 32 TMEM columns and
 // three 35 KB stages: two CTAs per SM, one working while the other starts or
 // ends (one CTA of 64 rows a SM was slower at every size: field_f64's four
 // analyses 150 us against 117, an lmax 189 call 22.4 ms against 21.5).
@@ -53,6 +53,7 @@ __global__ void __launch_bounds__(NTH, 2) k_leg64(const double *__restrict__ dat
                                                   int *err) {
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ uint32_t red[2][MTILE];
+    __shared__ int ex_s[NT];
     const int z = blockIdx.z, m = z >> 1, par = z & 1;
     const bool first_task = (int)blockIdx.y < ny0;
     const Task64 &t = first_task ? t0 : t1;
@@ -65,7 +66,7 @@ __global__ void __launch_bounds__(NTH, 2) k_leg64(const double *__restrict__ dat
     const int64_t col0 = (int64_t)blockIdx.x * MTILE;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int c = tid & (MTILE - 1), kh = (tid >> 7) & 1;
-    const bool prod = tid < NPROD, cok = prod && col0 + c < ncol;
+    const bool cok = col0 + c < ncol;
     const double *D = LMROWS ? data + col0 + c
                              : data + ((int64_t)(par * (lmax + 1) + m) * nrn) * ncol + col0 + c;
     auto row_at = [&](int k) -> int64_t {
@@ -94,102 +95,310 @@ __global__ void __launch_bounds__(NTH, 2) k_leg64(const double *__restrict__ dat
     const int nKtab = ((LMROWS ? nrows : nrn) + KC - 1) / KC;    // chunks of the table's block
     const uint16_t *tab = t.dig + t.off[z] + (int64_t)tile * nKtab * ND * NT * KC + (int64_t)lo * ND * LS * KC;
 
-    // largest magnitude of every column (the high word orders the magnitudes by exponent)
-    uint32_t mx = 0;
-    if (cok) {
-#pragma unroll 8
-        for (int k = kbeg + kh; k < kend; k += 2) {
-            const double v = D[row_at(k)];
-            mx = max(mx, ((uint32_t)__double2hiint(v) & 0x7fffffffu) | (__double2loint(v) != 0 ? 1u : 0u));
+    // The column's values: largest magnitude over every chunk (the high word orders the magnitudes by exponent);
+    // those of the first two chunks to be worked stay in registers.
+    double pre[2][8];
+    bool use = cok;
+    auto load_at = [&](int c16, double (&buf)[8]) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int k = c16 * KC + 8 * kh + j;
+            buf[j] = (use && k >= kbeg && k < kend) ? D[row_at(k)] : 0.0;
         }
+    };
+    auto load = [&](int kc, double (&buf)[8]) { load_at(lo + kc, buf); };
+    uint32_t mx = 0;
+    auto top = [&](const double (&buf)[8]) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            mx = max(mx, ((uint32_t)__double2hiint(buf[j]) & 0x7fffffffu) | (__double2loint(buf[j]) != 0 ? 1u : 0u));
+    };
+    if (tid < NT && tile * NT + tid < nwrite) ex_s[tid] = t.ex[(int64_t)z * t.exs + tile * NT + tid];
+    {
+        if (nch > 0) load(0, pre[0]);
+        if (nch > 1) load(1, pre[1]);
+        const int skip0 = nch > 0 ? lo : -1, skip1 = nch > 1 ? lo + 1 : -1;
+        for (int c16 = kbeg / KC; c16 * KC < kend; ++c16) {
+            if (c16 == skip0 || c16 == skip1) continue;
+            double buf[8];
+            load_at(c16, buf);
+            top(buf);
+        }
+        if (nch > 0) top(pre[0]);
+        if (nch > 1) top(pre[1]);
+        red[kh][c] = mx;
     }
-    if (prod) red[kh][c] = mx;
     Smem cs;
     const uint32_t tmem = setup(cs, smem);    // includes a __syncthreads
     const uint32_t cmx = max(red[0][c], red[1][c]);
     const int emax = max(1, (int)(cmx >> 20));
-    const bool zero = cmx == 0 || emax == 2047;                  // no digits: zero or non-finite columns
-
-    double pre[2][8];
-    auto load = [&](int kc, double (&buf)[8]) {
+    if (cmx == 0 || emax == 2047) {           // no digits: zero or non-finite columns
+        use = false;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int k = (lo + kc) * KC + 8 * kh + j;
-            buf[j] = (cok && !zero && k >= kbeg && k < kend) ? D[row_at(k)] : 0.0;
-        }
-    };
-    if (prod) {
-        if (nch > 0) load(0, pre[0]);
-        if (nch > 1) load(1, pre[1]);
+        for (int j = 0; j < 8; ++j) pre[0][j] = pre[1][j] = 0.0;
     }
     auto fix = [&](double v) { return fixed55(v, emax); };
 
+    // warp w of the epilogue: TMEM lanes 32 (w % 4).. (columns), table rows [NT/2 (w / 4), +NT/2) of the tile
+    const int lq = warp & 3, hg = warp >> 2;
+    const uint32_t lane_base = (uint32_t)(lq * 32) << 16;
+    const int cl = lq * 32 + lane;
+    const int64_t cc = col0 + cl;
+    const bool ook = cc < ncol;
+    const uint32_t lmx = max(red[0][cl], red[1][cl]);
+    const int lemax = max(1, (int)(lmx >> 20));
+    const int n0 = tile * NT + NT / 2 * hg;
+    auto at = [&](int i) -> int64_t {                       // output row n0 + i of this lane's column; rows < 2^31
+        const int n = n0 + i, l = m + par + 2 * n;
+        const uint32_t row = t.n_is_rows ? (uint32_t)(l * (l + 1) / 2 + m) : (uint32_t)((par * (lmax + 1) + m) * t.nout + n);
+        return (int64_t)((uint64_t)row * (uint32_t)ncol) + cc;
+    };
     const int nsb = max(1, (nch + SBK - 1) / SBK);
     for (int sb = 0; sb < nsb; ++sb) {
         const int k0 = sb * SBK, k1 = min(nch, k0 + SBK);
-        const bool ok = run_block(cs, tmem, k0, k1, nch, sb, LS, tab, pre, load, fix);
-        if (!ok) {
+        run_block(cs, tmem, k0, k1, nch, LS, tab, pre, load, fix);
+        // what the sums are added to, on its way while the MMAs run
+        double old[NT / 2];
+        const double *base = sb > 0 || t.mode == 1 ? t.out : t.mode == 2 ? t.a0 : nullptr;
+#pragma unroll
+        for (int i = 0; i < NT / 2; ++i) old[i] = (base && ook && n0 + i < nwrite) ? base[at(i)] : 0.0;
+        if (!end_block(cs, sb)) {
             if (tid == 0) atomicOr(err, ERR_TC_TIMEOUT);
             break;                                        // uniform: every thread saw the same value
         }
-        if (prod) {
-            // warp w: TMEM lanes 32 (w % 4).. (columns), table rows [NT/2 (w / 4), +NT/2) of the tile
-            const int lq = warp & 3, hg = warp >> 2;
-            const uint32_t lane_base = (uint32_t)(lq * 32) << 16;
-            const int cl = lq * 32 + lane;
-            const int64_t cc = col0 + cl;
-            const uint32_t lmx = max(red[0][cl], red[1][cl]);
-            const int lemax = max(1, (int)(lmx >> 20));
+        {
+#pragma unroll
             for (int g = 0; g < NT / 8; ++g) {
                 const int i0 = NT / 2 * hg + 4 * g;
                 if (i0 >= LS || tile * NT + i0 >= nwrite) break;              // warp-uniform
                 float v[ND][4];
                 load_levels(tmem + lane_base + (uint32_t)i0, LS, v);
-                if (cc < ncol) {
-                    double old[4];
-                    int ex[4];
-                    auto at = [&](int i) -> int64_t {                   // row index < 2^31
-                        const int n = tile * NT + i0 + i, l = m + par + 2 * n;
-                        const uint32_t row = t.n_is_rows ? (uint32_t)(l * (l + 1) / 2 + m)
-                                                         : (uint32_t)((par * (lmax + 1) + m) * t.nout + n);
-                        return (int64_t)((uint64_t)row * (uint32_t)ncol) + cc;
-                    };
+                if (!ook) continue;
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const int n = tile * NT + i0 + i;
-                        old[i] = 0.0;
-                        ex[i] = 0;
-                        if (n < nwrite) {
-                            ex[i] = t.ex[(int64_t)z * t.exs + n];
-                            if (sb > 0 || t.mode == 1) old[i] = t.out[at(i)];
-                            else if (t.mode == 2) old[i] = t.a0[at(i)];
-                        }
+                for (int i = 0; i < 4; ++i) {
+                    const int n = tile * NT + i0 + i;
+                    if (n >= nwrite) break;
+                    double val = 0.0;
+                    if (lemax == 2047) {                  // non-finite data: the plain FP64 sum
+                        if (sb == 0)
+                            for (int k = kbeg; k < kend; ++k)
+                                val = fma(t.tab64[t.tab64_off[z] + n * t.sn + k * t.sk],
+                                          data[(D - data) - (col0 + c) + cc + row_at(k)], val);
+                    } else if (nch > 0) {
+                        const float L[ND] = {v[0][i], v[1][i], v[2][i], v[3][i], v[4][i], v[5][i], v[6][i]};
+                        val = round_int(join_int(L), lemax + ex_s[i0 + i] - 1076);
                     }
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const int n = tile * NT + i0 + i;
-                        if (n >= nwrite) continue;
-                        double val;
-                        if (lemax == 2047) {                  // non-finite data: the plain FP64 sum
-                            val = 0.0;
-                            if (sb == 0)
-                                for (int k = kbeg; k < kend; ++k)
-                                    val = fma(t.tab64[t.tab64_off[z] + n * t.sn + k * t.sk],
-                                              data[(D - data) - (col0 + c) + cc + row_at(k)], val);
-                        } else if (nch == 0) {
-                            val = 0.0;
-                        } else {
-                            const float L[ND] = {v[0][i], v[1][i], v[2][i], v[3][i], v[4][i], v[5][i], v[6][i]};
-                            val = round_int(join_int(L), lemax + ex[i] - 1076);
-                        }
-                        t.out[at(i)] = t.mode == 2 ? old[i] - val : (sb > 0 || t.mode == 1) ? old[i] + val : val;
-                    }
+                    const double o = old[4 * g + i];
+                    t.out[at(4 * g + i)] = t.mode == 2 ? o - val : base ? o + val : val;
                 }
             }
         }
         fence_before();
         __syncthreads();                                      // TMEM is read before the next block's MMAs
         fence_after();
+    }
+    release(tmem);
+}
+
+// The same for short sums (K <= 16 RES, the refinement passes: rows, or the aliased rings).  The column digits are
+// formed once and stay in shared memory; the table tiles of both tasks (every gridDim.y-th) come past them one
+// after another, the next one's digits copied in during a tile's epilogue.  Of a tile-a-CTA launch half the
+// instructions formed the same digits again for each tile (102 maps, lmax 82: 68 us a refinement's Gram update and
+// aliased synthesis, LATER so).
+constexpr int RES = 3;
+constexpr size_t SMEM_RES = (size_t)RES * ND * (PLANE_A + NT * KC * 2);
+
+struct TileJob {
+    int task, tile, lo, nch, LS, nwrite;
+    const uint16_t *tab;
+};
+
+template <bool LMROWS>
+__global__ void __launch_bounds__(NTH, 2) k_leg64_short(const double *__restrict__ data, int64_t ncol, int lmax,
+                                                        int nrn, int klim, Task64 t0, Task64 t1, int ny0, int ny1,
+                                                        int *err) {
+    extern __shared__ __align__(1024) unsigned char smem[];
+    __shared__ uint32_t red[2][MTILE];
+    __shared__ int ex_s[2][NT];
+    __shared__ __align__(8) uint64_t bars[2];
+    __shared__ uint32_t slot;
+    const int z = blockIdx.z, m = z >> 1, par = z & 1;
+    const int nrows = rows_of(m, par, lmax);
+    const int K = LMROWS ? nrows : min(klim, nrn);
+    const int nK = (K + KC - 1) / KC, nKtab = LMROWS ? nK : (nrn + KC - 1) / KC;
+    const int64_t col0 = (int64_t)blockIdx.x * MTILE;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int c = tid & (MTILE - 1), kh = tid >> 7;
+    const bool cok = col0 + c < ncol;
+    const double *D = LMROWS ? data : data + ((int64_t)(par * (lmax + 1) + m) * nrn) * ncol;
+    auto row_at = [&](int k) -> int64_t {
+        const int l = m + par + 2 * k;
+        const uint32_t row = LMROWS ? (uint32_t)(l * (l + 1) / 2 + m) : (uint32_t)k;
+        return (int64_t)((uint64_t)row * (uint32_t)ncol);
+    };
+    // job i of this block: tiles of task 0, then of task 1; false: nothing to do there
+    auto job_at = [&](int i, TileJob &j) -> bool {
+        j.task = i < ny0 ? 0 : 1;
+        const Task64 &t = j.task ? t1 : t0;
+        j.tile = j.task ? i - ny0 : i;
+        const int N = t.n_is_rows ? nrows : t.nout;
+        j.nwrite = t.n_is_rows ? nrows : t.nlim;
+        if (j.tile * NT >= j.nwrite || (t.n_is_rows && nrows == 0)) return false;
+        int lo = 0, hi = nK - 1;
+        if (t.live) {
+            const int2 lv = t.live[(int64_t)z * t.ntile + j.tile];
+            lo = max(lo, lv.x);
+            hi = min(hi, lv.y);
+        }
+        j.nch = hi < lo ? 0 : hi - lo + 1;
+        j.lo = j.nch ? lo : 0;
+        if (t.mode == 1 && j.nch == 0) return false;
+        j.LS = ls_of(N, j.tile);
+        j.tab = t.dig + t.off[z] + (int64_t)j.tile * nKtab * ND * NT * KC + (int64_t)j.lo * ND * j.LS * KC;
+        return true;
+    };
+    auto next_job = [&](int i, TileJob &j) -> int {          // the first job at or after i, or -1
+        for (; i < ny0 + ny1; i += gridDim.y)
+            if (job_at(i, j)) return i;
+        return -1;
+    };
+    TileJob job;
+    int cur = next_job(blockIdx.y, job);
+    if (cur < 0) return;
+
+    double v[RES][8];
+    uint32_t mx = 0;
+#pragma unroll
+    for (int q = 0; q < RES; ++q)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int k = q * KC + 8 * kh + j;
+            v[q][j] = (cok && k < K) ? D[row_at(k) + col0 + c] : 0.0;
+        }
+#pragma unroll
+    for (int q = 0; q < RES; ++q)
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            mx = max(mx, ((uint32_t)__double2hiint(v[q][j]) & 0x7fffffffu) | (__double2loint(v[q][j]) != 0 ? 1u : 0u));
+    red[kh][c] = mx;
+    uint64_t *full_b = &bars[0], *done = &bars[1];
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&slot)),
+                     "r"(TMEM_COLS)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (tid == 0) {
+        mbar_init(full_b, 1);
+        mbar_init(done, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    fence_before();
+    __syncthreads();
+    fence_after();
+    const uint32_t tmem = slot;
+    unsigned char *sA = smem, *sB = smem + (size_t)RES * ND * PLANE_A;
+    auto fetch = [&](const TileJob &j) {
+        const uint32_t bytes = (uint32_t)j.nch * ND * j.LS * KC * 2;
+        mbar_expect_tx(full_b, bytes);
+        bulk_g2s(sB, j.tab, bytes, full_b);
+    };
+    if (tid == 0 && job.nch > 0) fetch(job);
+    {
+        const uint32_t cmx = max(red[0][c], red[1][c]);
+        const int emax = max(1, (int)(cmx >> 20));
+        const bool dead = cmx == 0 || emax == 2047;              // no digits: zero or non-finite columns
+        const uint32_t off = core_off(c, 8 * kh);
+#pragma unroll
+        for (int q = 0; q < RES; ++q) {
+            if (q >= nK) break;
+            uint32_t w[ND][4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                uint32_t u[ND];
+                digits2(dead ? 0 : fixed55(v[q][2 * j], emax), dead ? 0 : fixed55(v[q][2 * j + 1], emax), u);
+#pragma unroll
+                for (int d = 0; d < ND; ++d) w[d][j] = u[d];
+            }
+#pragma unroll
+            for (int d = 0; d < ND; ++d)
+                *reinterpret_cast<uint4 *>(sA + (q * ND + d) * PLANE_A + off) = make_uint4(w[d][0], w[d][1], w[d][2], w[d][3]);
+        }
+        fence_proxy_async();
+    }
+    // warp w of the epilogue: TMEM lanes 32 (w % 4).. (columns), table rows [NT/2 (w / 4), +NT/2) of the tile
+    const int lq = warp & 3, hg = warp >> 2;
+    const uint32_t lane_base = (uint32_t)(lq * 32) << 16;
+    const int cl = lq * 32 + lane;
+    const int64_t cc = col0 + cl;
+    const bool ook = cc < ncol;
+    const int lemax = max(1, (int)(max(red[0][cl], red[1][cl]) >> 20));
+    int uses = 0;                                             // tiles whose digits were fetched: barrier phases
+    for (int step = 0; cur >= 0; ++step) {
+        const Task64 &t = job.task ? t1 : t0;
+        int *exs = ex_s[step & 1];
+        if (tid < NT && job.tile * NT + tid < job.nwrite) exs[tid] = t.ex[(int64_t)z * t.exs + job.tile * NT + tid];
+        const int n0 = job.tile * NT + NT / 2 * hg;
+        auto at = [&](int i) -> int64_t {                   // output row n0 + i of this lane's column; rows < 2^31
+            const int n = n0 + i, l = m + par + 2 * n;
+            const uint32_t row = t.n_is_rows ? (uint32_t)(l * (l + 1) / 2 + m)
+                                             : (uint32_t)((par * (lmax + 1) + m) * t.nout + n);
+            return (int64_t)((uint64_t)row * (uint32_t)ncol) + cc;
+        };
+        if (step == 0) __syncthreads();                       // every digit is written
+        const uint32_t ph = (uint32_t)(uses & 1);
+        if (job.nch > 0 && tid == 32 * MMA_WARP) {
+            if (mbar_wait(full_b, ph)) {
+                fence_after();
+                for (int q = 0; q < job.nch; ++q)
+                    issue(tmem, smem_u32(sA) + (job.lo + q) * ND * PLANE_A, smem_u32(sB) + q * ND * job.LS * KC * 2, job.LS,
+                          q == 0);
+                mma_commit(done);
+            }                                                 // (else done stays pending and the wait below gives up)
+        }
+        __syncwarp();
+        double old[NT / 2];
+        const double *base = t.mode == 1 ? t.out : t.mode == 2 ? t.a0 : nullptr;
+#pragma unroll
+        for (int i = 0; i < NT / 2; ++i) old[i] = (base && ook && n0 + i < job.nwrite) ? base[at(i)] : 0.0;
+        const bool fin = job.nch == 0 || mbar_wait(done, ph);
+        fence_after();
+        if (!__syncthreads_and(fin)) {
+            if (tid == 0) atomicOr(err, ERR_TC_TIMEOUT);
+            break;
+        }
+        if (job.nch > 0) ++uses;
+        TileJob nxt;
+        const int ni = next_job(cur + gridDim.y, nxt);
+        if (tid == 0 && ni >= 0 && nxt.nch > 0) fetch(nxt);      // the MMAs have read this tile's digits
+#pragma unroll
+        for (int g = 0; g < NT / 8; ++g) {
+            const int i0 = NT / 2 * hg + 4 * g;
+            if (i0 >= job.LS || job.tile * NT + i0 >= job.nwrite) break;          // warp-uniform
+            float L4[ND][4];
+            load_levels(tmem + lane_base + (uint32_t)i0, job.LS, L4);
+            if (!ook) continue;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int n = job.tile * NT + i0 + i;
+                if (n >= job.nwrite) break;
+                double val = 0.0;
+                if (lemax == 2047) {                          // non-finite data: the plain FP64 sum
+                    for (int k = 0; k < K; ++k)
+                        val = fma(t.tab64[t.tab64_off[z] + n * t.sn + k * t.sk], D[row_at(k) + cc], val);
+                } else if (job.nch > 0) {
+                    const float L[ND] = {L4[0][i], L4[1][i], L4[2][i], L4[3][i], L4[4][i], L4[5][i], L4[6][i]};
+                    val = round_int(join_int(L), lemax + exs[i0 + i] - 1076);
+                }
+                const double o = old[4 * g + i];
+                t.out[at(4 * g + i)] = t.mode == 2 ? o - val : base ? o + val : val;
+            }
+        }
+        fence_before();
+        __syncthreads();                                      // TMEM is read before the next tile's MMAs
+        fence_after();
+        cur = ni;
+        job = nxt;
     }
     release(tmem);
 }
@@ -345,11 +554,24 @@ static dim3 grid64(const Plan &p, int64_t ncol, int ny) {
     return dim3((unsigned)((ncol + t64::MTILE - 1) / t64::MTILE), (unsigned)ny, (unsigned)(2 * (p.lmax + 1)));
 }
 
+// blocks a column tile and (m, parity) are split into, so that two CTAs per SM have work
+static unsigned short_split(const Plan &p, int64_t ncol, int ntile) {
+    const int64_t ctas = ((ncol + t64::MTILE - 1) / t64::MTILE) * 2 * (p.lmax + 1);
+    return (unsigned)std::max<int64_t>(1, std::min<int64_t>(ntile, 304 / ctas));
+}
+
 void launch_leg_analysis64(const Plan &p, const double *F, int64_t ncol, double *A, bool accumulate, cudaStream_t st,
                            int rlim, const int *nzr) {
     Task64 t = p.t64[0];
     t.out = A;
     t.mode = accumulate ? 1 : 0;
+    if (!nzr && rlim <= t64::RES * t64::KC) {
+        set_smem(t64::k_leg64_short<false>, t64::SMEM_RES);
+        t64::k_leg64_short<false><<<grid64(p, ncol, (int)short_split(p, ncol, t.ntile)), t64::NTH, t64::SMEM_RES, st>>>(
+            F, ncol, p.lmax, (int)p.nrn, rlim, t, t, t.ntile, 0, p.d_err);
+        note_launch();
+        return;
+    }
     set_smem(t64::k_leg64<false>, t64::SMEM);
     t64::k_leg64<false><<<grid64(p, ncol, t.ntile), t64::NTH, t64::SMEM, st>>>(F, ncol, p.lmax, (int)p.nrn, rlim, nzr,
                                                                               t, t, t.ntile, p.d_err);
@@ -368,6 +590,13 @@ void launch_leg_synthesis64(const Plan &p, const double *A, int64_t ncol, double
     s.nlim = rlim;
     const int ny0 = Anew ? g.ntile : 0, ny1 = G && rlim > 0 ? (rlim + t64::NT - 1) / t64::NT : 0;
     if (ny0 + ny1 == 0) return;
+    if (p.lmax / 2 + 1 <= t64::RES * t64::KC) {
+        set_smem(t64::k_leg64_short<true>, t64::SMEM_RES);
+        t64::k_leg64_short<true><<<grid64(p, ncol, (int)short_split(p, ncol, ny0 + ny1)), t64::NTH, t64::SMEM_RES, st>>>(
+            A, ncol, p.lmax, (int)p.nrn, 0, g, s, ny0, ny1, p.d_err);
+        note_launch();
+        return;
+    }
     set_smem(t64::k_leg64<true>, t64::SMEM);
     t64::k_leg64<true><<<grid64(p, ncol, ny0 + ny1), t64::NTH, t64::SMEM, st>>>(A, ncol, p.lmax, (int)p.nrn, 0, nullptr,
                                                                                g, s, ny0, p.d_err);

@@ -142,15 +142,14 @@ __global__ void __launch_bounds__(NTH, 2) k_rdft64(const RingGeom *__restrict__ 
     if (tile * NT >= nf) return;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int kh = (tid >> 7) & 1;
-    const bool prod = tid < NPROD;
     const int64_t nrow = 2 * nm, R0 = (int64_t)blockIdx.x * MTILE, row = R0 + (tid & (MTILE - 1));
-    const bool rok = prod && row < nrow;
+    const bool rok = row < nrow;
     const int em0 = rok ? ex[(int64_t)r * nm + (row >= nm ? row - nm : row)] : 0;
     const int LS = ls_of(nf, tile);
     // this thread's output row: warps 0-7, TMEM lanes 32 (w % 4).., frequencies [16 (w / 4), +16) of the tile
     const int lq = warp & 3, hg = warp >> 2;
     const int64_t orow = R0 + lq * 32 + lane;
-    const bool ook = prod && orow < nrow;
+    const bool ook = orow < nrow;
     const int par = orow >= nm ? 1 : 0;
     const int64_t ob = orow - par * nm;
     const int64_t L1 = lmax + 1, ld = 2 * nm;
@@ -188,22 +187,19 @@ __global__ void __launch_bounds__(NTH, 2) k_rdft64(const RingGeom *__restrict__ 
             buf[2 * j + 1] = v.y;
         }
     };
-    if (prod) {
-        load(0, pre[0]);
-        if (nch > 1) load(1, pre[1]);
-    }
+    load(0, pre[0]);
+    if (nch > 1) load(1, pre[1]);
     Smem cs;
     const uint32_t tmem = setup(cs, smem);
     const int oem = ook ? ex[(int64_t)r * nm + ob] : 0;
     const int nsb = (nch + SBR - 1) / SBR;
     for (int sb = 0; sb < nsb; ++sb) {
-        const bool ok = run_block(cs, tmem, sb * SBR, min(nch, (sb + 1) * SBR), nch, sb, LS, tab, pre, load,
-                                  [](int64_t v) { return v; });
-        if (!ok) {
+        run_block(cs, tmem, sb * SBR, min(nch, (sb + 1) * SBR), nch, LS, tab, pre, load, [](int64_t v) { return v; });
+        if (!end_block(cs, sb)) {
             if (tid == 0) atomicOr(err, ERR_TC_TIMEOUT);
             break;
         }
-        if (prod) {
+        {
             for (int gq = 0; gq < 4; ++gq) {
                 const int i0 = 16 * hg + 4 * gq;
                 if (i0 >= LS || tile * NT + i0 >= nf) break;                  // warp-uniform
@@ -248,9 +244,8 @@ __global__ void __launch_bounds__(NTH, 2) k_rsyn64(const RingGeom *__restrict__ 
     const int K = lmax >= e ? (lmax - e) / 2 + 1 : 0;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int rl = tid & (MTILE - 1), kh = (tid >> 7) & 1;
-    const bool prod = tid < NPROD;
     const int64_t nrow = 2 * nm, R0 = (int64_t)blockIdx.x * MTILE, row = R0 + rl;
-    const bool rok = prod && row < nrow;
+    const bool rok = row < nrow;
     const int64_t L1 = lmax + 1, ld = 2 * nm;
     const int par = row >= nm ? 1 : 0;
     const double *Gr = G + (par * L1 * 2 * ns + r) * ld + 2 * (row - par * nm) + isS;
@@ -264,7 +259,7 @@ __global__ void __launch_bounds__(NTH, 2) k_rsyn64(const RingGeom *__restrict__ 
             mx = max(mx, ((uint32_t)__double2hiint(v) & 0x7fffffffu) | (__double2loint(v) != 0 ? 1u : 0u));
         }
     }
-    if (prod) red[kh][rl] = mx;
+    red[kh][rl] = mx;
     uint64_t *full_b = &bars[0], *done = &bars[1];
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&slot)),
@@ -298,13 +293,13 @@ __global__ void __launch_bounds__(NTH, 2) k_rsyn64(const RingGeom *__restrict__ 
     const int lq = warp & 3, hg = warp >> 2;
     const int64_t orow = R0 + lq * 32 + lane;
     int64_t *Yo = Y + qoff[r] * nrow + (int64_t)cb * nrow * R.kp + orow * R.kp;
-    const bool ook = prod && orow < nrow;
+    const bool ook = orow < nrow;
     int step = 0;
     bool ok = true;
     for (int k0 = 0; k0 < max(nK, 1) && ok; k0 += kbmax) {
         const int nk = min(kbmax, nK - k0);
         if (tid == 0 && nk > 0) fetch(0, k0, nk);
-        if (prod) {
+        {
             for (int kc = 0; kc < nk; ++kc) {
                 double buf[8];
 #pragma unroll
@@ -334,7 +329,7 @@ __global__ void __launch_bounds__(NTH, 2) k_rsyn64(const RingGeom *__restrict__ 
         for (int t = 0; t < ntile; ++t, ++step) {
             const int LS = ls_of(R.kc, t);
             if (nk > 0) {
-                if (!prod) {
+                if (warp == MMA_WARP) {
                     if (lane == 0) {
                         ok = mbar_wait(full_b, (uint32_t)(step & 1));
                         fence_after();
@@ -355,7 +350,7 @@ __global__ void __launch_bounds__(NTH, 2) k_rsyn64(const RingGeom *__restrict__ 
                 }
                 if (tid == 0 && t + 1 < ntile) fetch(t + 1, k0, nk);      // the MMAs have read this tile's block
             }
-            if (prod) {
+            {
                 for (int gq = 0; gq < 4; ++gq) {
                     const int i0 = 16 * hg + 4 * gq, j0 = t * NT + i0;
                     if (i0 >= LS || j0 >= R.kc) break;                        // warp-uniform
