@@ -93,7 +93,12 @@ __device__ __forceinline__ double round_int(int64_t T, int S) {
     const uint64_t frac = (((a << lz) >> 1) + 512u) >> 10;            // 2^52 <= frac <= 2^53
     const int ef = 11 - lz + S + 52 + 1023;                            // exponent field of frac 2^(11 - lz + S)
     if (a == 0) return 0.0;
-    if (ef < 1 || ef > 2045) return ldexp(sign ? -(double)a : (double)a, S);
+    if (ef < 1 || ef > 2045) {                     // subnormal or overflowing: two scalings of the rounded value
+        auto pow2 = [](int e) { return __hiloint2double((1023 + max(-1022, min(e, 1023))) << 20, 0); };
+        const int e = 11 - lz + S, e1 = e / 2;
+        const double v = (double)(int64_t)frac * pow2(e1) * pow2(e - e1);
+        return sign ? -v : v;
+    }
     const uint32_t hi = (uint32_t)(frac >> 32) + ((uint32_t)(ef - 1) << 20);
     return __hiloint2double((int)(hi | sign), (int)(uint32_t)frac);
 }

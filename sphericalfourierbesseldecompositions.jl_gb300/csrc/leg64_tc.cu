@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(NTH, 2) k_leg64(const double *__restrict__ dat
     }
     auto fix = [&](double v) { return fixed55(v, emax); };
 
-    // warp w of the epilogue: TMEM lanes 32 (w % 4).. (columns), table rows [NT/2 (w / 4), +NT/2) of the tile
+    // warp w of the epilogue: TMEM lanes 32 (w % 4).. (columns), every other group of four table rows of the tile
     const int lq = warp & 3, hg = warp >> 2;
     const uint32_t lane_base = (uint32_t)(lq * 32) << 16;
     const int cl = lq * 32 + lane;
@@ -147,9 +147,8 @@ __global__ void __launch_bounds__(NTH, 2) k_leg64(const double *__restrict__ dat
     const bool ook = cc < ncol;
     const uint32_t lmx = max(red[0][cl], red[1][cl]);
     const int lemax = max(1, (int)(lmx >> 20));
-    const int n0 = tile * NT + NT / 2 * hg;
-    auto at = [&](int i) -> int64_t {                       // output row n0 + i of this lane's column; rows < 2^31
-        const int n = n0 + i, l = m + par + 2 * n;
+    auto at = [&](int i) -> int64_t {                       // output row i of the tile, this lane's column; rows < 2^31
+        const int n = tile * NT + i, l = m + par + 2 * n;
         const uint32_t row = t.n_is_rows ? (uint32_t)(l * (l + 1) / 2 + m) : (uint32_t)((par * (lmax + 1) + m) * t.nout + n);
         return (int64_t)((uint64_t)row * (uint32_t)ncol) + cc;
     };
@@ -157,23 +156,24 @@ __global__ void __launch_bounds__(NTH, 2) k_leg64(const double *__restrict__ dat
     for (int sb = 0; sb < nsb; ++sb) {
         const int k0 = sb * SBK, k1 = min(nch, k0 + SBK);
         run_block(cs, tmem, k0, k1, nch, LS, tab, pre, load, fix);
-        // what the sums are added to, on its way while the MMAs run
-        double old[NT / 2];
+        // what the sums are added to, a group of rows ahead (the first on its way while the MMAs run)
         const double *base = sb > 0 || t.mode == 1 ? t.out : t.mode == 2 ? t.a0 : nullptr;
+        double old[4], nold[4];
+        auto load_old = [&](int i0, double (&o)[4]) {
 #pragma unroll
-        for (int i = 0; i < NT / 2; ++i) old[i] = (base && ook && n0 + i < nwrite) ? base[at(i)] : 0.0;
+            for (int i = 0; i < 4; ++i) o[i] = (base && ook && i0 + i < LS && tile * NT + i0 + i < nwrite) ? base[at(i0 + i)] : 0.0;
+        };
+        load_old(4 * hg, old);
         if (!end_block(cs, sb)) {
             if (tid == 0) atomicOr(err, ERR_TC_TIMEOUT);
             break;                                        // uniform: every thread saw the same value
         }
-        {
-#pragma unroll
-            for (int g = 0; g < NT / 8; ++g) {
-                const int i0 = NT / 2 * hg + 4 * g;
-                if (i0 >= LS || tile * NT + i0 >= nwrite) break;              // warp-uniform
-                float v[ND][4];
-                load_levels(tmem + lane_base + (uint32_t)i0, LS, v);
-                if (!ook) continue;
+#pragma unroll 1
+        for (int i0 = 4 * hg; i0 < LS && tile * NT + i0 < nwrite; i0 += 8) {           // warp-uniform
+            load_old(i0 + 8, nold);
+            float v[ND][4];
+            load_levels(tmem + lane_base + (uint32_t)i0, LS, v);
+            if (ook) {
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const int n = tile * NT + i0 + i;
@@ -188,10 +188,11 @@ __global__ void __launch_bounds__(NTH, 2) k_leg64(const double *__restrict__ dat
                         const float L[ND] = {v[0][i], v[1][i], v[2][i], v[3][i], v[4][i], v[5][i], v[6][i]};
                         val = round_int(join_int(L), lemax + ex_s[i0 + i] - 1076);
                     }
-                    const double o = old[4 * g + i];
-                    t.out[at(4 * g + i)] = t.mode == 2 ? o - val : base ? o + val : val;
+                    t.out[at(i0 + i)] = t.mode == 2 ? old[i] - val : base ? old[i] + val : val;
                 }
             }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) old[i] = nold[i];
         }
         fence_before();
         __syncthreads();                                      // TMEM is read before the next block's MMAs
@@ -204,7 +205,8 @@ __global__ void __launch_bounds__(NTH, 2) k_leg64(const double *__restrict__ dat
 // formed once and stay in shared memory; the table tiles of both tasks (every gridDim.y-th) come past them one
 // after another, the next one's digits copied in during a tile's epilogue.  Of a tile-a-CTA launch half the
 // instructions formed the same digits again for each tile (102 maps, lmax 82: 68 us a refinement's Gram update and
-// aliased synthesis, LATER so).
+// aliased synthesis, 40 so).  Bound: the epilogue's integer operations (about 80 an output), a third of the issue
+// slots at four warps a scheduler.
 constexpr int RES = 3;
 constexpr size_t SMEM_RES = (size_t)RES * ND * (PLANE_A + NT * KC * 2);
 
@@ -326,7 +328,7 @@ __global__ void __launch_bounds__(NTH, 2) k_leg64_short(const double *__restrict
         }
         fence_proxy_async();
     }
-    // warp w of the epilogue: TMEM lanes 32 (w % 4).. (columns), table rows [NT/2 (w / 4), +NT/2) of the tile
+    // warp w of the epilogue: TMEM lanes 32 (w % 4).. (columns), every other group of four table rows of the tile
     const int lq = warp & 3, hg = warp >> 2;
     const uint32_t lane_base = (uint32_t)(lq * 32) << 16;
     const int cl = lq * 32 + lane;
@@ -338,9 +340,8 @@ __global__ void __launch_bounds__(NTH, 2) k_leg64_short(const double *__restrict
         const Task64 &t = job.task ? t1 : t0;
         int *exs = ex_s[step & 1];
         if (tid < NT && job.tile * NT + tid < job.nwrite) exs[tid] = t.ex[(int64_t)z * t.exs + job.tile * NT + tid];
-        const int n0 = job.tile * NT + NT / 2 * hg;
-        auto at = [&](int i) -> int64_t {                   // output row n0 + i of this lane's column; rows < 2^31
-            const int n = n0 + i, l = m + par + 2 * n;
+        auto at = [&](int i) -> int64_t {                   // output row i of the tile, this lane's column; rows < 2^31
+            const int n = job.tile * NT + i, l = m + par + 2 * n;
             const uint32_t row = t.n_is_rows ? (uint32_t)(l * (l + 1) / 2 + m)
                                              : (uint32_t)((par * (lmax + 1) + m) * t.nout + n);
             return (int64_t)((uint64_t)row * (uint32_t)ncol) + cc;
@@ -357,10 +358,14 @@ __global__ void __launch_bounds__(NTH, 2) k_leg64_short(const double *__restrict
             }                                                 // (else done stays pending and the wait below gives up)
         }
         __syncwarp();
-        double old[NT / 2];
         const double *base = t.mode == 1 ? t.out : t.mode == 2 ? t.a0 : nullptr;
+        double old[4], nold[4];                               // what the sums are added to, a group of rows ahead
+        auto load_old = [&](int i0, double (&o)[4]) {
 #pragma unroll
-        for (int i = 0; i < NT / 2; ++i) old[i] = (base && ook && n0 + i < job.nwrite) ? base[at(i)] : 0.0;
+            for (int i = 0; i < 4; ++i)
+                o[i] = (base && ook && i0 + i < job.LS && job.tile * NT + i0 + i < job.nwrite) ? base[at(i0 + i)] : 0.0;
+        };
+        load_old(4 * hg, old);
         const bool fin = job.nch == 0 || mbar_wait(done, ph);
         fence_after();
         if (!__syncthreads_and(fin)) {
@@ -371,28 +376,29 @@ __global__ void __launch_bounds__(NTH, 2) k_leg64_short(const double *__restrict
         TileJob nxt;
         const int ni = next_job(cur + gridDim.y, nxt);
         if (tid == 0 && ni >= 0 && nxt.nch > 0) fetch(nxt);      // the MMAs have read this tile's digits
-#pragma unroll
-        for (int g = 0; g < NT / 8; ++g) {
-            const int i0 = NT / 2 * hg + 4 * g;
-            if (i0 >= job.LS || job.tile * NT + i0 >= job.nwrite) break;          // warp-uniform
+#pragma unroll 1
+        for (int i0 = 4 * hg; i0 < job.LS && job.tile * NT + i0 < job.nwrite; i0 += 8) {         // warp-uniform
+            load_old(i0 + 8, nold);
             float L4[ND][4];
             load_levels(tmem + lane_base + (uint32_t)i0, job.LS, L4);
-            if (!ook) continue;
+            if (ook) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int n = job.tile * NT + i0 + i;
-                if (n >= job.nwrite) break;
-                double val = 0.0;
-                if (lemax == 2047) {                          // non-finite data: the plain FP64 sum
-                    for (int k = 0; k < K; ++k)
-                        val = fma(t.tab64[t.tab64_off[z] + n * t.sn + k * t.sk], D[row_at(k) + cc], val);
-                } else if (job.nch > 0) {
-                    const float L[ND] = {L4[0][i], L4[1][i], L4[2][i], L4[3][i], L4[4][i], L4[5][i], L4[6][i]};
-                    val = round_int(join_int(L), lemax + exs[i0 + i] - 1076);
+                for (int i = 0; i < 4; ++i) {
+                    const int n = job.tile * NT + i0 + i;
+                    if (n >= job.nwrite) break;
+                    double val = 0.0;
+                    if (lemax == 2047) {                      // non-finite data: the plain FP64 sum
+                        for (int k = 0; k < K; ++k)
+                            val = fma(t.tab64[t.tab64_off[z] + n * t.sn + k * t.sk], D[row_at(k) + cc], val);
+                    } else if (job.nch > 0) {
+                        const float L[ND] = {L4[0][i], L4[1][i], L4[2][i], L4[3][i], L4[4][i], L4[5][i], L4[6][i]};
+                        val = round_int(join_int(L), lemax + exs[i0 + i] - 1076);
+                    }
+                    t.out[at(i0 + i)] = t.mode == 2 ? old[i] - val : base ? old[i] + val : val;
                 }
-                const double o = old[4 * g + i];
-                t.out[at(4 * g + i)] = t.mode == 2 ? o - val : base ? o + val : val;
             }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) old[i] = nold[i];
         }
         fence_before();
         __syncthreads();                                      // TMEM is read before the next tile's MMAs

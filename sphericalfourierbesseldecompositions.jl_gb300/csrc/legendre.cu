@@ -858,7 +858,10 @@ static bool fold_alias64(const Plan &p, const double *G, int64_t ncplx, double *
     for (int r = 0; r < rlim; ++r) nbk = std::max(nbk, p.h_rings[r].nph);
     const size_t smem = ((size_t)nbk + (size_t)(p.lmax + 1)) * FC * sizeof(double2);
     if (smem > 100 * 1024) return false;              // two CTAs per SM
-    const int rpb = 3;
+    // rings per block: several only where every SM has blocks enough (at 101 maps and 41 rings: 31 us at three, one
+    // ring's latency chain after another)
+    const int64_t gx = (ncplx + FC - 1) / FC;
+    const int rpb = (int)std::max<int64_t>(1, std::min<int64_t>(4, 2 * gx * rlim / 1216));
     set_smem(k_fold_alias64<FC>, smem);
     k_fold_alias64<FC><<<dim3((unsigned)((ncplx + FC - 1) / FC), 2, (unsigned)((rlim + rpb - 1) / rpb)), 256, smem,
                          st>>>(p.d_rings, (int)p.nrn, rlim, rpb, nbk, p.lmax, 4.0 * M_PI / (double)p.npix, G, ncplx,

@@ -146,7 +146,8 @@ __global__ void __launch_bounds__(NTH, 2) k_rdft64(const RingGeom *__restrict__ 
     const bool rok = row < nrow;
     const int em0 = rok ? ex[(int64_t)r * nm + (row >= nm ? row - nm : row)] : 0;
     const int LS = ls_of(nf, tile);
-    // this thread's output row: warps 0-7, TMEM lanes 32 (w % 4).., frequencies [16 (w / 4), +16) of the tile
+    // this thread's output row: warps 0-7, TMEM lanes 32 (w % 4).., every other group of four
+    // frequencies of the tile
     const int lq = warp & 3, hg = warp >> 2;
     const int64_t orow = R0 + lq * 32 + lane;
     const bool ook = orow < nrow;
@@ -168,8 +169,8 @@ __global__ void __launch_bounds__(NTH, 2) k_rdft64(const RingGeom *__restrict__ 
     };
     if (!__syncthreads_or(em0 != 0)) {           // no data on this ring pair in any of the maps
         if (ook)
-            for (int i = 0; i < 16; ++i) {
-                const int k = tile * NT + 16 * hg + i;
+            for (int i = hg; i < NT; i += 2) {
+                const int k = tile * NT + i;
                 if (k < nf) emit(e + 2 * k, 0.0, false);
             }
         return;
@@ -200,9 +201,8 @@ __global__ void __launch_bounds__(NTH, 2) k_rdft64(const RingGeom *__restrict__ 
             break;
         }
         {
-            for (int gq = 0; gq < 4; ++gq) {
-                const int i0 = 16 * hg + 4 * gq;
-                if (i0 >= LS || tile * NT + i0 >= nf) break;                  // warp-uniform
+#pragma unroll 1
+            for (int i0 = 4 * hg; i0 < LS && tile * NT + i0 < nf; i0 += 8) {      // warp-uniform
                 float v[ND][4];
                 load_levels(tmem + ((uint32_t)(lq * 32) << 16) + (uint32_t)i0, LS, v);
                 if (!ook) continue;
@@ -351,9 +351,9 @@ __global__ void __launch_bounds__(NTH, 2) k_rsyn64(const RingGeom *__restrict__ 
                 if (tid == 0 && t + 1 < ntile) fetch(t + 1, k0, nk);      // the MMAs have read this tile's block
             }
             {
-                for (int gq = 0; gq < 4; ++gq) {
-                    const int i0 = 16 * hg + 4 * gq, j0 = t * NT + i0;
-                    if (i0 >= LS || j0 >= R.kc) break;                        // warp-uniform
+#pragma unroll 1
+                for (int i0 = 4 * hg; i0 < LS && t * NT + i0 < R.kc; i0 += 8) {       // warp-uniform
+                    const int j0 = t * NT + i0;
                     float v[ND][4];
                     load_levels(tmem + ((uint32_t)(lq * 32) << 16) + (uint32_t)i0, LS, v);
                     if (!ook) continue;
