@@ -24,6 +24,7 @@ namespace sfb {
 
 // alm[lm][c] *= s (m = 0) or s / 2 (m >= 1) (w E above); lm = l (l+1)/2 + m
 __global__ void k_halve_m(double *alm, int64_t lmsize, int64_t ncol, double s) {
+    pdl_entry();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= lmsize * ncol) return;
     const int64_t lm = i / ncol;
@@ -36,10 +37,11 @@ __global__ void k_halve_m(double *alm, int64_t lmsize, int64_t ncol, double s) {
 // Transpose of the radial projection a_nlm = s sum_b c[pair(n,l)][b] A_b[lm]:
 //   Abar[lm][2b + t] = s sum_n c[pair(n,l)][b] abar[noff(n) + lm][t]   (t = re, im)
 // for the basis functions b in [b0, b0 + nbc).
-__global__ void k_proj_adjoint(const double *__restrict__ abar, const double *__restrict__ coef, int64_t nbasis,
-                               const int32_t *__restrict__ pair_index, const int64_t *__restrict__ noff, int lmax,
+__global__ void k_proj_adjoint(const double *abar, const double *coef, int64_t nbasis,
+                               const int32_t *pair_index, const int64_t *noff, int lmax,
                                int nmax, int64_t lmsize, int64_t b0, int64_t nbc, double s,
-                               double *__restrict__ Abar) {
+                               double *Abar) {
+    pdl_entry();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= lmsize * nbc) return;
     const int64_t lm = i / nbc, b = b0 + (i - lm * nbc);
@@ -64,10 +66,11 @@ __global__ void k_proj_adjoint(const double *__restrict__ abar, const double *__
 // with phi_b the piecewise Legendre basis of the deposit (P_k on the galaxy's
 // piece, the constants outside [rmin, rmax]); galaxies are keyed exactly as
 // the deposit keys them.
-__global__ void k_deposit_adjoint(const double *__restrict__ rtp, int64_t ngal, int64_t nside, int64_t npix,
+__global__ void k_deposit_adjoint(const double *rtp, int64_t ngal, int64_t nside, int64_t npix,
                                   double rmin, double rmax, double inv_width, int pieces, int deg, int64_t nbasis,
-                                  const double *__restrict__ Dbar, int64_t sb, int64_t sp, int64_t b0, int64_t nbc,
-                                  double *__restrict__ dw, int *err) {
+                                  const double *Dbar, int64_t sb, int64_t sp, int64_t b0, int64_t nbc,
+                                  double *dw, int *err) {
+    pdl_entry();
     __shared__ double clen[2 * 64];                   // (2k+1)/(k+1), (k+1)/(k+2) for k < 64
     for (int k = threadIdx.x; k <= min(deg, 63); k += blockDim.x) {
         clen[2 * k] = (2.0 * k + 1.0) / (k + 1.0);
@@ -119,7 +122,7 @@ __global__ void k_deposit_adjoint(const double *__restrict__ rtp, int64_t ngal, 
 void launch_halve_m(double *alm, int64_t lmsize, int64_t ncol, double s, cudaStream_t st) {
     const int64_t n = lmsize * ncol;
     if (n <= 0) return;
-    k_halve_m<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(alm, lmsize, ncol, s);
+    launch_pdl(k_halve_m, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, st, alm, lmsize, ncol, s);
     note_launch();
 }
 
@@ -127,15 +130,15 @@ void launch_proj_adjoint(const Plan &p, const double *abar, const int32_t *pair_
                          int64_t nbc, double s, double *Abar, cudaStream_t st) {
     const int64_t n = p.lmsize * nbc;
     if (n <= 0) return;
-    k_proj_adjoint<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(abar, p.d_coef, p.nbasis, pair_index, noff, p.lmax,
-                                                                (int)p.nmax, p.lmsize, b0, nbc, s, Abar);
+    launch_pdl(k_proj_adjoint, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, st, abar, p.d_coef, p.nbasis,
+        pair_index, noff, p.lmax, (int)p.nmax, p.lmsize, b0, nbc, s, Abar);
     note_launch();
 }
 
 void launch_deposit_adjoint(const Plan &p, const double *rtp, int64_t ngal, const double *Dbar, int64_t sb, int64_t sp,
                             int64_t b0, int64_t nbc, double *dw, cudaStream_t st) {
     if (ngal <= 0) return;
-    k_deposit_adjoint<<<(unsigned)((ngal + 255) / 256), 256, 0, st>>>(
+    launch_pdl(k_deposit_adjoint, dim3((unsigned)((ngal + 255) / 256)), dim3(256), 0, st,
         rtp, ngal, p.nside, p.npix, p.rmin, p.rmax, (double)p.pieces / (p.rmax - p.rmin), p.pieces, p.degree,
         p.nbasis, Dbar, sb, sp, b0, nbc, dw, p.d_err);
     note_launch();

@@ -138,11 +138,12 @@ __device__ __forceinline__ int mock_of(const Mocks &mk, int64_t i) {
 // whose pixel the FP32 evaluation cannot settle goes to fb_list with key
 // -2 - slot, and gets its key and rank from k_deposit_keys_fallback (FP64
 // pixel), so no warp runs the FP64 pixel path for one lane.
-__global__ void k_deposit_keys(const double *__restrict__ rtp, const double *__restrict__ wgt, int64_t ngal,
+__global__ void k_deposit_keys(const double *rtp, const double *wgt, int64_t ngal,
                                int64_t gbase, int64_t nside, int64_t npix, double rmin, double rmax,
-                               double inv_width, int pieces, const __grid_constant__ Mocks mk, int32_t *__restrict__ counts,
-                               int32_t *__restrict__ key, int32_t *__restrict__ rank, double *__restrict__ xloc,
-                               int32_t *__restrict__ fb_list, int32_t *__restrict__ fb_count, int *err) {
+                               double inv_width, int pieces, const __grid_constant__ Mocks mk, int32_t *counts,
+                               int32_t *key, int32_t *rank, double *xloc,
+                               int32_t *fb_list, int32_t *fb_count, int *err) {
+    pdl_entry();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= ngal) return;
     const double r = rtp[3 * i], th = rtp[3 * i + 1], ph = rtp[3 * i + 2];
@@ -180,11 +181,12 @@ struct RadialKeyParams {
     float rmin_hi, rmin_lo, invw_hi, invw_lo;
 };
 
-__global__ void k_deposit_keys_mixed(const double *__restrict__ rtp, const double *__restrict__ wgt, int64_t ngal,
+__global__ void k_deposit_keys_mixed(const double *rtp, const double *wgt, int64_t ngal,
                                      int64_t gbase, int64_t nside, int64_t npix, RadialKeyParams rk, int pieces,
-                                     const __grid_constant__ Mocks mk, int32_t *__restrict__ counts, int32_t *__restrict__ key,
-                                     int32_t *__restrict__ rank, float2 *__restrict__ xdf,
-                                     int32_t *__restrict__ fb_list, int32_t *__restrict__ fb_count, int *err) {
+                                     const __grid_constant__ Mocks mk, int32_t *counts, int32_t *key,
+                                     int32_t *rank, float2 *xdf,
+                                     int32_t *fb_list, int32_t *fb_count, int *err) {
+    pdl_entry();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= ngal) return;
     const double r = rtp[3 * i], th = rtp[3 * i + 1], ph = rtp[3 * i + 2];
@@ -238,10 +240,11 @@ __global__ void k_deposit_keys_mixed(const double *__restrict__ rtp, const doubl
 // The galaxies the FP32 pixel evaluation left: exact FP64 pixel, then key and
 // rank as above with the slot the keys pass found (rtp, key, rank indexed
 // globally).
-__global__ void k_deposit_keys_fallback(const double *__restrict__ rtp, int64_t nside, int64_t npix,
-                                        int32_t *__restrict__ counts, int32_t *__restrict__ key,
-                                        int32_t *__restrict__ rank, const int32_t *__restrict__ fb_list,
-                                        const int32_t *__restrict__ fb_count) {
+__global__ void k_deposit_keys_fallback(const double *rtp, int64_t nside, int64_t npix,
+                                        int32_t *counts, int32_t *key,
+                                        int32_t *rank, const int32_t *fb_list,
+                                        const int32_t *fb_count) {
+    pdl_entry();
     const int n = *fb_count;
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
         const int64_t i = fb_list[t];
@@ -257,8 +260,9 @@ __global__ void k_deposit_keys_fallback(const double *__restrict__ rtp, int64_t 
 // Exclusive scan, tile pass: each block scans SCAN_TILE counters in place and
 // writes its total; the block that finishes last (counted in *done, zero on
 // entry) scans the totals, so that step costs no launch of its own.
-__global__ void __launch_bounds__(SCAN_THREADS) k_scan_tiles(int32_t *__restrict__ data, int64_t n,
-                                                             int32_t *__restrict__ tile_sums, int *done) {
+__global__ void __launch_bounds__(SCAN_THREADS) k_scan_tiles(int32_t *data, int64_t n,
+                                                             int32_t *tile_sums, int *done) {
+    pdl_entry();
     __shared__ int32_t warp_tot[SCAN_THREADS / 32];
     __shared__ int32_t carry;
     __shared__ bool last;
@@ -334,14 +338,16 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_tiles(int32_t *__restrict
     }
 }
 
-__global__ void k_scan_add(int32_t *__restrict__ data, int64_t n, const int32_t *__restrict__ tile_sums) {
+__global__ void k_scan_add(int32_t *data, int64_t n, const int32_t *tile_sums) {
+    pdl_entry();
     const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx < n) data[idx] += tile_sums[idx / SCAN_TILE];
 }
 
-__global__ void k_deposit_scatter(const double *__restrict__ wgt, int64_t ngal, const int32_t *__restrict__ key,
-                                  const int32_t *__restrict__ rank, const double *__restrict__ xloc,
-                                  const int32_t *__restrict__ offset, double2 *__restrict__ sorted) {
+__global__ void k_deposit_scatter(const double *wgt, int64_t ngal, const int32_t *key,
+                                  const int32_t *rank, const double *xloc,
+                                  const int32_t *offset, double2 *sorted) {
+    pdl_entry();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= ngal) return;
     const int32_t k = key[i];
@@ -352,10 +358,11 @@ __global__ void k_deposit_scatter(const double *__restrict__ wgt, int64_t ngal, 
 
 // Mixed precision: (x, w) as double-float pairs {x.hi, x.lo, w.hi, w.lo}, w
 // split from the double by integer operations.
-__global__ void k_deposit_scatter_mixed(const double *__restrict__ wgt, int64_t ngal,
-                                        const int32_t *__restrict__ key, const int32_t *__restrict__ rank,
-                                        const float2 *__restrict__ xdf, const int32_t *__restrict__ offset,
-                                        float4 *__restrict__ sorted) {
+__global__ void k_deposit_scatter_mixed(const double *wgt, int64_t ngal,
+                                        const int32_t *key, const int32_t *rank,
+                                        const float2 *xdf, const int32_t *offset,
+                                        float4 *sorted) {
+    pdl_entry();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= ngal) return;
     const int32_t k = key[i];
@@ -377,7 +384,7 @@ constexpr double monic_lead(int k) {
 }
 
 template <int MAXDEG>
-__device__ __forceinline__ void bin_moments(const double2 *__restrict__ sorted, int64_t g0, int64_t g1, int deg,
+__device__ __forceinline__ void bin_moments(const double2 *sorted, int64_t g0, int64_t g1, int deg,
                                             double (&acc)[MAXDEG + 1]) {
 #pragma unroll
     for (int k = 0; k <= MAXDEG; ++k) acc[k] = 0.0;
@@ -434,9 +441,10 @@ __device__ __forceinline__ int rank_bins(int cnt, int *hist) {
 // consecutive threads on consecutive pixels.  Bound: the FP64 pipe, 72 operations a galaxy at degree 24 (with
 // four operations a degree and unsorted bins 274 us for 6e5 galaxies at nside 128; 151 so).
 template <int MAXDEG>
-__global__ void __launch_bounds__(128) k_deposit_moments(const int32_t *__restrict__ offset,
-                                                         const double2 *__restrict__ sorted, int64_t npix, int pieces,
-                                                         int deg, int64_t nbasis, double *__restrict__ maps) {
+__global__ void __launch_bounds__(128) k_deposit_moments(const int32_t *offset,
+                                                         const double2 *sorted, int64_t npix, int pieces,
+                                                         int deg, int64_t nbasis, double *maps) {
+    pdl_entry();
     extern __shared__ double out_s[];                  // [deg + 1][128]
     __shared__ int hist[64];
     __shared__ int perm[128];
@@ -510,7 +518,7 @@ __device__ __forceinline__ void leg_chain(dfl x, dfl q0, dfl q1, dfl (&acc)[MAXD
 // pairs of k_deposit_scatter_mixed; the next galaxy's load overlaps this
 // one's basis.
 template <int MAXDEG>
-__device__ __forceinline__ void bin_moments_df(const float4 *__restrict__ sorted, int64_t g0, int64_t g1, int deg,
+__device__ __forceinline__ void bin_moments_df(const float4 *sorted, int64_t g0, int64_t g1, int deg,
                                                dfl (&acc)[MAXDEG + 1]) {
 #pragma unroll
     for (int k = 0; k <= MAXDEG; ++k) acc[k] = {0.f, 0.f};
@@ -532,9 +540,10 @@ __device__ __forceinline__ void bin_moments_df(const float4 *__restrict__ sorted
 // fluctuation acc - mu_b ref all in double-float (mudf = mu and cdf = ref as
 // hi + lo pairs), stored as normalised double-float pairs.
 template <int MAXDEG>
-__global__ void k_deposit_moments_df(const int32_t *__restrict__ offset, const float4 *__restrict__ sorted,
-                                     int64_t npix, int pieces, int deg, int64_t nbasis, const float2 *__restrict__ cdf,
-                                     const float2 *__restrict__ mudf, float2 *__restrict__ maps) {
+__global__ void k_deposit_moments_df(const int32_t *offset, const float4 *sorted,
+                                     int64_t npix, int pieces, int deg, int64_t nbasis, const float2 *cdf,
+                                     const float2 *mudf, float2 *maps) {
+    pdl_entry();
     // grid.y: mocks
     offset += (int64_t)blockIdx.y * (pieces + 2) * npix;
     maps += (int64_t)blockIdx.y * nbasis * npix;
@@ -586,13 +595,14 @@ __global__ void k_deposit_moments_df(const int32_t *__restrict__ offset, const f
 // and are written with consecutive threads on consecutive pixels.  Needs
 // npix >= 128 (a block spans at most two slots).
 template <int MAXDEG>
-__global__ void __launch_bounds__(128) k_deposit_moments_bal(const int32_t *__restrict__ offset,
-                                                             const float4 *__restrict__ sorted, int64_t npix,
+__global__ void __launch_bounds__(128) k_deposit_moments_bal(const int32_t *offset,
+                                                             const float4 *sorted, int64_t npix,
                                                              int pieces, int deg, int64_t nbasis,
-                                                             const float2 *__restrict__ cdf,
-                                                             const float2 *__restrict__ mudf,
-                                                             float2 *__restrict__ maps, int64_t nside,
-                                                             const int *__restrict__ ring_live) {
+                                                             const float2 *cdf,
+                                                             const float2 *mudf,
+                                                             float2 *maps, int64_t nside,
+                                                             const int *ring_live) {
+    pdl_entry();
     __shared__ int hist[64];
     __shared__ int perm[128];
     __shared__ float2 out[(MAXDEG + 1) * 128];
@@ -713,7 +723,7 @@ __device__ __forceinline__ void leg_chain_sm(dfl x, dfl q0, dfl q1, uint32_t col
 }
 
 template <int MAXDEG>
-__device__ __forceinline__ void bin_moments_sm(const float4 *__restrict__ sorted, int64_t g0, int64_t g1, int deg,
+__device__ __forceinline__ void bin_moments_sm(const float4 *sorted, int64_t g0, int64_t g1, int deg,
                                                uint32_t col) {
 #pragma unroll
     for (int k = 0; k <= MAXDEG; ++k)
@@ -737,13 +747,14 @@ __device__ __forceinline__ void bin_moments_sm(const float4 *__restrict__ sorted
 }
 
 template <int MAXDEG>
-__global__ void __launch_bounds__(128, 8) k_deposit_moments_sm(const int32_t *__restrict__ offset,
-                                                               const float4 *__restrict__ sorted, int64_t npix,
+__global__ void __launch_bounds__(128, 8) k_deposit_moments_sm(const int32_t *offset,
+                                                               const float4 *sorted, int64_t npix,
                                                                int pieces, int deg, int64_t nbasis,
-                                                               const float2 *__restrict__ cdf,
-                                                               const float2 *__restrict__ mudf,
-                                                               float2 *__restrict__ maps, int64_t nside,
-                                                               const int *__restrict__ ring_live) {
+                                                               const float2 *cdf,
+                                                               const float2 *mudf,
+                                                               float2 *maps, int64_t nside,
+                                                               const int *ring_live) {
+    pdl_entry();
     __shared__ int hist[64];
     __shared__ int perm[128];
     __shared__ __align__(16) float2 acc_s[(MAXDEG + 1) * 128];
@@ -842,11 +853,12 @@ constexpr int STATS_STRIDE = 32;
 // block that finishes last (*done zero on entry) forms mu[b] = S[b] / Q[slot(b)]
 // (0 where the sampled reference map is zero) and the same as a double-float pair.
 template <int MAXDEG>
-__global__ void __launch_bounds__(32) k_deposit_stats(const int32_t *__restrict__ offset,
-                                                      const float4 *__restrict__ sorted, int64_t npix, int pieces,
-                                                      int deg, int64_t nbasis, const float2 *__restrict__ cdf,
-                                                      double *S, double *Q, double *__restrict__ mu,
-                                                      float2 *__restrict__ mudf, int *done) {
+__global__ void __launch_bounds__(32) k_deposit_stats(const int32_t *offset,
+                                                      const float4 *sorted, int64_t npix, int pieces,
+                                                      int deg, int64_t nbasis, const float2 *cdf,
+                                                      double *S, double *Q, double *mu,
+                                                      float2 *mudf, int *done) {
+    pdl_entry();
     __shared__ float2 red[32][MAXDEG + 3];
     // grid.y: mocks
     offset += (int64_t)blockIdx.y * (pieces + 2) * npix;
@@ -929,10 +941,11 @@ __global__ void __launch_bounds__(32) k_deposit_stats(const int32_t *__restrict_
 // FP64 value hi + lo (exact) and as the pair itself.
 // ring_live[ring] is set to 1 for every ring holding a galaxy (preset to 0).
 // The window's reference map W01 goes behind the count maps.
-__global__ void k_weight_map_mixed(const int32_t *__restrict__ offset, const float4 *__restrict__ sorted,
-                                   int64_t nside, int64_t npix, int nslots, double *__restrict__ C,
-                                   float2 *__restrict__ cdf, int *__restrict__ ring_live,
-                                   const double *__restrict__ W01) {
+__global__ void k_weight_map_mixed(const int32_t *offset, const float4 *sorted,
+                                   int64_t nside, int64_t npix, int nslots, double *C,
+                                   float2 *cdf, int *ring_live,
+                                   const double *W01) {
+    pdl_entry();
     const int64_t pix = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (pix >= npix) return;
     // grid.y: mocks
@@ -969,23 +982,23 @@ static void launch_moments(const Plan &p, int nmock, const int32_t *counts, cons
     if constexpr (MAXDEG <= 31) {
         if (p.precision == SFB_MIXED && p.npix >= 128) {
             if (p.moments_smem)
-                k_deposit_moments_sm<MAXDEG><<<blocks, 128, 0, st>>>(counts, s4, p.npix, p.pieces, p.degree,
-                                                                     p.nbasis, cdf, mudf, mf, p.nside, ring_live);
+                launch_pdl(k_deposit_moments_sm<MAXDEG>, dim3(blocks), dim3(128), 0, st, counts, s4, p.npix, p.pieces,
+                    p.degree, p.nbasis, cdf, mudf, mf, p.nside, ring_live);
             else
-                k_deposit_moments_bal<MAXDEG><<<blocks, 128, 0, st>>>(counts, s4, p.npix, p.pieces, p.degree,
-                                                                      p.nbasis, cdf, mudf, mf, p.nside, ring_live);
+                launch_pdl(k_deposit_moments_bal<MAXDEG>, dim3(blocks), dim3(128), 0, st, counts, s4, p.npix,
+                    p.pieces, p.degree, p.nbasis, cdf, mudf, mf, p.nside, ring_live);
             done = true;
         }
     }
     if (done) {
     } else if (p.precision == SFB_MIXED)
-        k_deposit_moments_df<MAXDEG><<<blocks, 128, 0, st>>>(counts, s4, p.npix, p.pieces, p.degree, p.nbasis, cdf,
-                                                             mudf, mf);
+        launch_pdl(k_deposit_moments_df<MAXDEG>, dim3(blocks), dim3(128), 0, st, counts, s4, p.npix, p.pieces,
+            p.degree, p.nbasis, cdf, mudf, mf);
     else {
         const size_t smem = (size_t)(p.degree + 1) * 128 * sizeof(double);
         set_smem(k_deposit_moments<MAXDEG>, smem);
-        k_deposit_moments<MAXDEG><<<blocks, 128, smem, st>>>(counts, static_cast<const double2 *>(sorted), p.npix,
-                                                             p.pieces, p.degree, p.nbasis, maps);
+        launch_pdl(k_deposit_moments<MAXDEG>, dim3(blocks), dim3(128), smem, st, counts,
+            static_cast<const double2 *>(sorted), p.npix, p.pieces, p.degree, p.nbasis, maps);
     }
     note_launch();
 }
@@ -995,8 +1008,8 @@ static void launch_stats(const Plan &p, int nmock, const int32_t *counts, const 
                          double *Q, double *mu, float2 *mudf, int *done, cudaStream_t st) {
     const int64_t nkeys = (int64_t)(p.pieces + 2) * p.npix;
     const int64_t blocks = (nkeys + 32 * STATS_STRIDE - 1) / (32 * STATS_STRIDE);
-    k_deposit_stats<MAXDEG><<<dim3((unsigned)blocks, (unsigned)nmock), 32, 0, st>>>(counts, sorted, p.npix, p.pieces, p.degree, p.nbasis,
-                                                              cdf, S, Q, mu, mudf, done);
+    launch_pdl(k_deposit_stats<MAXDEG>, dim3((unsigned)blocks, (unsigned)nmock), dim3(32), 0, st, counts, sorted,
+        p.npix, p.pieces, p.degree, p.nbasis, cdf, S, Q, mu, mudf, done);
     note_launch();
 }
 
@@ -1013,9 +1026,9 @@ int64_t scan_tile_count(int64_t n) { return (n + SCAN_TILE - 1) / SCAN_TILE; }
 
 void launch_exclusive_scan(int32_t *data, int64_t n, int32_t *tile_sums, int *done, cudaStream_t st) {
     const int64_t ntiles = scan_tile_count(n);
-    k_scan_tiles<<<(unsigned)ntiles, SCAN_THREADS, 0, st>>>(data, n, tile_sums, done);
+    launch_pdl(k_scan_tiles, dim3((unsigned)ntiles), dim3(SCAN_THREADS), 0, st, data, n, tile_sums, done);
     note_launch();
-    k_scan_add<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(data, n, tile_sums);
+    launch_pdl(k_scan_add, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, st, data, n, tile_sums);
     note_launch();
 }
 
@@ -1074,33 +1087,34 @@ int deposit_sorted(Plan &p, const DepositArgs &a, cudaStream_t st, const int **r
         if (n <= 0) continue;
         const unsigned nb = (unsigned)((n + 255) / 256);
         if (mixed)
-            k_deposit_keys_mixed<<<nb, 256, 0, st>>>(rtp + 3 * g0, w ? w + g0 : nullptr, n, g0, p.nside, p.npix, rk,
-                                                     p.pieces, a.mocks, counts, key + g0, rank + g0, xdf + g0, fb_list,
-                                                     fb_count, p.d_err);
+            launch_pdl(k_deposit_keys_mixed, dim3(nb), dim3(256), 0, st, rtp + 3 * g0, w ? w + g0 : nullptr, n, g0,
+                p.nside, p.npix, rk, p.pieces, a.mocks, counts, key + g0, rank + g0, xdf + g0, fb_list, fb_count,
+                p.d_err);
         else
-            k_deposit_keys<<<nb, 256, 0, st>>>(rtp + 3 * g0, w ? w + g0 : nullptr, n, g0, p.nside, p.npix, p.rmin,
-                                               p.rmax, inv_width, p.pieces, a.mocks, counts, key + g0, rank + g0, xloc + g0,
-                                               fb_list, fb_count, p.d_err);
+            launch_pdl(k_deposit_keys, dim3(nb), dim3(256), 0, st, rtp + 3 * g0, w ? w + g0 : nullptr, n, g0, p.nside,
+                p.npix, p.rmin, p.rmax, inv_width, p.pieces, a.mocks, counts, key + g0, rank + g0, xloc + g0, fb_list,
+                fb_count, p.d_err);
         note_launch();
     }
     if (ngal > 0) {
-        k_deposit_keys_fallback<<<304, 256, 0, st>>>(rtp, p.nside, p.npix, counts, key, rank, fb_list, fb_count);
+        launch_pdl(k_deposit_keys_fallback, dim3(304), dim3(256), 0, st, rtp, p.nside, p.npix, counts, key, rank,
+            fb_list, fb_count);
         note_launch();
     }
     launch_exclusive_scan(counts, nscan, tsum, scan_done, st);
     if (ngal > 0) {
         if (mixed)
-            k_deposit_scatter_mixed<<<(unsigned)((ngal + 255) / 256), 256, 0, st>>>(w, ngal, key, rank, xdf, counts,
-                                                                                   sorted4);
+            launch_pdl(k_deposit_scatter_mixed, dim3((unsigned)((ngal + 255) / 256)), dim3(256), 0, st, w, ngal, key,
+                rank, xdf, counts, sorted4);
         else
-            k_deposit_scatter<<<(unsigned)((ngal + 255) / 256), 256, 0, st>>>(w, ngal, key, rank, xloc, counts,
-                                                                             static_cast<double2 *>(sorted));
+            launch_pdl(k_deposit_scatter, dim3((unsigned)((ngal + 255) / 256)), dim3(256), 0, st, w, ngal, key, rank,
+                xloc, counts, static_cast<double2 *>(sorted));
         note_launch();
     }
     if (p.degree > 63) return fail(SFB_ENOTSUP, "radial degree above 63 is not supported by the sorted deposit");
     const bool split = ref != nullptr && mixed;
     if (split) {
-        k_weight_map_mixed<<<dim3((unsigned)((p.npix + 255) / 256), (unsigned)nmock), 256, 0, st>>>(
+        launch_pdl(k_weight_map_mixed, dim3((unsigned)((p.npix + 255) / 256), (unsigned)nmock), dim3(256), 0, st,
             counts, sorted4, p.nside, p.npix, p.pieces + 2, ref, cdf, live, a.w01);
         note_launch();
         if (a.ref_ready) SFB_CUDA_TRY(cudaEventRecord(a.ref_ready, st));

@@ -12,6 +12,7 @@ namespace sfb {
 // l = m + parity + 2*li, each row nrn rings long.
 __global__ void k_legendre_table(const RingGeom *rings, int nrn, int lmax, const int64_t *lam_off,
                                  double *lam) {
+    pdl_entry();
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     const int m = blockIdx.y;
     if (r >= nrn || m > lmax) return;
@@ -53,11 +54,12 @@ __global__ void k_legendre_table(const RingGeom *rings, int nrn, int lmax, const
 
 void launch_legendre_table(const Plan &p, cudaStream_t st) {
     dim3 grid((unsigned)((p.nrn + 127) / 128), (unsigned)(p.lmax + 1));
-    k_legendre_table<<<grid, 128, 0, st>>>(p.d_rings, (int)p.nrn, p.lmax, p.d_lam_off, p.d_lam);
+    launch_pdl(k_legendre_table, dim3(grid), dim3(128), 0, st, p.d_rings, (int)p.nrn, p.lmax, p.d_lam_off, p.d_lam);
     note_launch();
 }
 
 __global__ void k_ang2pix(int64_t nside, const double *theta, const double *phi, int64_t n, int64_t *pix) {
+    pdl_entry();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     pix[i] = ang2pix_ring_fast(nside, theta[i], phi[i]);
@@ -66,12 +68,13 @@ __global__ void k_ang2pix(int64_t nside, const double *theta, const double *phi,
 void launch_ang2pix(int64_t nside, const double *theta, const double *phi, int64_t n, int64_t *pix,
                     cudaStream_t st) {
     if (n <= 0) return;
-    k_ang2pix<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(nside, theta, phi, n, pix);
+    launch_pdl(k_ang2pix, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, st, nside, theta, phi, n, pix);
     note_launch();
 }
 
 // out[c][r] = in[r][c]; in is rows x cols row-major.
 __global__ void k_transpose(const double *in, int64_t rows, int64_t cols, double *out) {
+    pdl_entry();
     __shared__ double tile[32][33];
     const int64_t c0 = (int64_t)blockIdx.x * 32;
     for (int64_t r0 = (int64_t)blockIdx.y * 32; r0 < rows; r0 += (int64_t)gridDim.y * 32) {   // grid y <= 65535
@@ -91,7 +94,7 @@ __global__ void k_transpose(const double *in, int64_t rows, int64_t cols, double
 void launch_transpose(const double *in, int64_t rows, int64_t cols, double *out, cudaStream_t st) {
     if (rows <= 0 || cols <= 0) return;
     dim3 grid((unsigned)((cols + 31) / 32), (unsigned)std::min<int64_t>((rows + 31) / 32, 65535));
-    k_transpose<<<grid, dim3(32, 8), 0, st>>>(in, rows, cols, out);
+    launch_pdl(k_transpose, dim3(grid), dim3(32, 8), 0, st, in, rows, cols, out);
     note_launch();
 }
 
@@ -106,6 +109,7 @@ __device__ __forceinline__ TO convert_elem(TI v, TO *) { return (TO)v; }
 // pairs with a zero low word, double -> normalised pairs).
 template <typename TI, typename TO>
 __global__ void k_transpose_ld(const TI *in, int64_t ldi, int64_t rows, int64_t cols, TO *out, int64_t ldo) {
+    pdl_entry();
     __shared__ TI tile[32][33];
     const int64_t c0 = (int64_t)blockIdx.x * 32;
     // row tiles over grid y, which is capped at 65535 (rows are pixels: 98304 tiles at nside 512)
@@ -128,7 +132,7 @@ static void transpose_ld(const TI *in, int64_t ldi, int64_t rows, int64_t cols, 
                          cudaStream_t st) {
     if (rows <= 0 || cols <= 0) return;
     dim3 grid((unsigned)((cols + 31) / 32), (unsigned)std::min<int64_t>((rows + 31) / 32, 65535));
-    k_transpose_ld<TI, TO><<<grid, dim3(32, 8), 0, st>>>(in, ldi, rows, cols, out, ldo);
+    launch_pdl(k_transpose_ld<TI, TO>, dim3(grid), dim3(32, 8), 0, st, in, ldi, rows, cols, out, ldo);
     note_launch();
 }
 
@@ -159,6 +163,7 @@ void launch_transpose_ld(const float *in, int64_t ldi, int64_t rows, int64_t col
 }
 
 __global__ void k_check_finite(const double *x, int64_t n, int *err) {
+    pdl_entry();
     int bad = 0;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         if (!isfinite(x[i])) bad = 1;
@@ -169,7 +174,7 @@ void launch_check_finite(const double *x, int64_t n, int *err, cudaStream_t st) 
     if (n <= 0) return;
     int64_t blocks = (n + 255) / 256;
     if (blocks > 4096) blocks = 4096;
-    k_check_finite<<<(unsigned)blocks, 256, 0, st>>>(x, n, err);
+    launch_pdl(k_check_finite, dim3((unsigned)blocks), dim3(256), 0, st, x, n, err);
     note_launch();
 }
 

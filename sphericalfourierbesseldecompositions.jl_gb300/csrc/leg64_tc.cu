@@ -48,9 +48,10 @@ __device__ __forceinline__ int rows_of(int m, int par, int lmax) {
 // Tiles blockIdx.y < ny0 use task 0, the others task 1 (the Gram update and the aliased rings' synthesis of
 // one refinement pass share a launch: both read the current coefficients).
 template <bool LMROWS>
-__global__ void __launch_bounds__(NTH, 2) k_leg64(const double *__restrict__ data, int64_t ncol, int lmax, int nrn,
-                                                  int klim, const int *__restrict__ nzr, Task64 t0, Task64 t1, int ny0,
+__global__ void __launch_bounds__(NTH, 2) k_leg64(const double *data, int64_t ncol, int lmax, int nrn,
+                                                  int klim, const int *nzr, Task64 t0, Task64 t1, int ny0,
                                                   int *err) {
+    pdl_entry();
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ uint32_t red[2][MTILE];
     __shared__ int ex_s[NT];
@@ -216,9 +217,10 @@ struct TileJob {
 };
 
 template <bool LMROWS>
-__global__ void __launch_bounds__(NTH, 2) k_leg64_short(const double *__restrict__ data, int64_t ncol, int lmax,
+__global__ void __launch_bounds__(NTH, 2) k_leg64_short(const double *data, int64_t ncol, int lmax,
                                                         int nrn, int klim, Task64 t0, Task64 t1, int ny0, int ny1,
                                                         int *err) {
+    pdl_entry();
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ uint32_t red[2][MTILE];
     __shared__ int ex_s[2][NT];
@@ -419,8 +421,9 @@ __device__ __forceinline__ void dims(int kind, int z, int lmax, int nrn, int &N,
 }
 
 // exponent E of every table row, |v| < 2^E (one warp per row)
-__global__ void k64_rowexp(int kind, const double *__restrict__ tab, const int64_t *__restrict__ off64, int64_t sn,
-                           int64_t sk, int lmax, int nrn, int exs, int16_t *__restrict__ ex) {
+__global__ void k64_rowexp(int kind, const double *tab, const int64_t *off64, int64_t sn,
+                           int64_t sk, int lmax, int nrn, int exs, int16_t *ex) {
+    pdl_entry();
     const int z = blockIdx.y, lane = threadIdx.x & 31;
     int N, K;
     dims(kind, z, lmax, nrn, N, K);
@@ -433,11 +436,12 @@ __global__ void k64_rowexp(int kind, const double *__restrict__ tab, const int64
 }
 
 // one block per (tile and chunk, z): the digit planes and the live chunk range of the tile
-__global__ void __launch_bounds__(256) k64_build(int kind, const double *__restrict__ tab,
-                                                 const int64_t *__restrict__ off64, int64_t sn, int64_t sk, int lmax,
-                                                 int nrn, int exs, const int16_t *__restrict__ ex, int ntile,
-                                                 int nkmax, const int64_t *__restrict__ off,
-                                                 uint16_t *__restrict__ dig, int2 *__restrict__ live) {
+__global__ void __launch_bounds__(256) k64_build(int kind, const double *tab,
+                                                 const int64_t *off64, int64_t sn, int64_t sk, int lmax,
+                                                 int nrn, int exs, const int16_t *ex, int ntile,
+                                                 int nkmax, const int64_t *off,
+                                                 uint16_t *dig, int2 *live) {
+    pdl_entry();
     const int z = blockIdx.y, tile = blockIdx.x / nkmax, kc = blockIdx.x % nkmax;
     int N, K;
     dims(kind, z, lmax, nrn, N, K);
@@ -465,6 +469,7 @@ __global__ void __launch_bounds__(256) k64_build(int kind, const double *__restr
 }
 
 __global__ void k64_fill(int2 *r, int64_t n) {
+    pdl_entry();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         r[i] = make_int2(0x7fffffff, -1);
 }
@@ -541,10 +546,11 @@ bool ensure_tc64(Plan &p, cudaStream_t st) {
             return false;
         }
         const int64_t nl = (int64_t)nz * ntile[kind];
-        t64::k64_fill<<<(unsigned)((nl + 255) / 256), 256, 0, st>>>(const_cast<int2 *>(t.live), nl);
-        t64::k64_rowexp<<<dim3(16, (unsigned)nz), 256, 0, st>>>(kind, t.tab64, t.tab64_off, t.sn, t.sk, p.lmax,
-                                                               (int)p.nrn, t.exs, const_cast<int16_t *>(t.ex));
-        t64::k64_build<<<dim3((unsigned)(ntile[kind] * nkmax[kind]), (unsigned)nz), 256, 0, st>>>(
+        launch_pdl(t64::k64_fill, dim3((unsigned)((nl + 255) / 256)), dim3(256), 0, st, const_cast<int2 *>(t.live),
+            nl);
+        launch_pdl(t64::k64_rowexp, dim3(16, (unsigned)nz), dim3(256), 0, st, kind, t.tab64, t.tab64_off, t.sn, t.sk,
+            p.lmax, (int)p.nrn, t.exs, const_cast<int16_t *>(t.ex));
+        launch_pdl(t64::k64_build, dim3((unsigned)(ntile[kind] * nkmax[kind]), (unsigned)nz), dim3(256), 0, st,
             kind, t.tab64, t.tab64_off, t.sn, t.sk, p.lmax, (int)p.nrn, t.exs, t.ex, t.ntile, nkmax[kind], t.off,
             const_cast<uint16_t *>(t.dig), const_cast<int2 *>(t.live));
         note_launch();
@@ -573,14 +579,14 @@ void launch_leg_analysis64(const Plan &p, const double *F, int64_t ncol, double 
     t.mode = accumulate ? 1 : 0;
     if (!nzr && rlim <= t64::RES * t64::KC) {
         set_smem(t64::k_leg64_short<false>, t64::SMEM_RES);
-        t64::k_leg64_short<false><<<grid64(p, ncol, (int)short_split(p, ncol, t.ntile)), t64::NTH, t64::SMEM_RES, st>>>(
-            F, ncol, p.lmax, (int)p.nrn, rlim, t, t, t.ntile, 0, p.d_err);
+        launch_pdl(t64::k_leg64_short<false>, dim3(grid64(p, ncol, (int)short_split(p, ncol, t.ntile))),
+            dim3(t64::NTH), t64::SMEM_RES, st, F, ncol, p.lmax, (int)p.nrn, rlim, t, t, t.ntile, 0, p.d_err);
         note_launch();
         return;
     }
     set_smem(t64::k_leg64<false>, t64::SMEM);
-    t64::k_leg64<false><<<grid64(p, ncol, t.ntile), t64::NTH, t64::SMEM, st>>>(F, ncol, p.lmax, (int)p.nrn, rlim, nzr,
-                                                                              t, t, t.ntile, p.d_err);
+    launch_pdl(t64::k_leg64<false>, dim3(grid64(p, ncol, t.ntile)), dim3(t64::NTH), t64::SMEM, st, F, ncol, p.lmax,
+        (int)p.nrn, rlim, nzr, t, t, t.ntile, p.d_err);
     note_launch();
 }
 
@@ -598,14 +604,14 @@ void launch_leg_synthesis64(const Plan &p, const double *A, int64_t ncol, double
     if (ny0 + ny1 == 0) return;
     if (p.lmax / 2 + 1 <= t64::RES * t64::KC) {
         set_smem(t64::k_leg64_short<true>, t64::SMEM_RES);
-        t64::k_leg64_short<true><<<grid64(p, ncol, (int)short_split(p, ncol, ny0 + ny1)), t64::NTH, t64::SMEM_RES, st>>>(
-            A, ncol, p.lmax, (int)p.nrn, 0, g, s, ny0, ny1, p.d_err);
+        launch_pdl(t64::k_leg64_short<true>, dim3(grid64(p, ncol, (int)short_split(p, ncol, ny0 + ny1))),
+            dim3(t64::NTH), t64::SMEM_RES, st, A, ncol, p.lmax, (int)p.nrn, 0, g, s, ny0, ny1, p.d_err);
         note_launch();
         return;
     }
     set_smem(t64::k_leg64<true>, t64::SMEM);
-    t64::k_leg64<true><<<grid64(p, ncol, ny0 + ny1), t64::NTH, t64::SMEM, st>>>(A, ncol, p.lmax, (int)p.nrn, 0, nullptr,
-                                                                               g, s, ny0, p.d_err);
+    launch_pdl(t64::k_leg64<true>, dim3(grid64(p, ncol, ny0 + ny1)), dim3(t64::NTH), t64::SMEM, st, A, ncol, p.lmax,
+        (int)p.nrn, 0, nullptr, g, s, ny0, p.d_err);
     note_launch();
 }
 

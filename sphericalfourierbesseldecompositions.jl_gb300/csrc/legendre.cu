@@ -29,10 +29,11 @@ __device__ __forceinline__ int nrows_of(int m, int par, int lmax) {
 // [nzr[0], nzr[1]] (F is zero outside them: the ring transform recorded the
 // span of ring pairs holding data; an empty span sums nothing).
 template <typename T>
-__global__ void __launch_bounds__(256) k_leg_analysis(const T *__restrict__ lam, const int64_t *lam_off,
-                                                      int lmax, int nrn, const T *__restrict__ F,
-                                                      int64_t ncol, T *__restrict__ A, int accumulate, int rlim,
-                                                      const int *__restrict__ nzr) {
+__global__ void __launch_bounds__(256) k_leg_analysis(const T *lam, const int64_t *lam_off,
+                                                      int lmax, int nrn, const T *F,
+                                                      int64_t ncol, T *A, int accumulate, int rlim,
+                                                      const int *nzr) {
+    pdl_entry();
     const int z = blockIdx.z;
     const int m = z >> 1, par = z & 1;
     const int nrows = nrows_of(m, par, lmax);
@@ -97,9 +98,10 @@ __global__ void __launch_bounds__(256) k_leg_analysis(const T *__restrict__ lam,
 
 // Only the rings r < rlim are formed.
 template <typename T>
-__global__ void __launch_bounds__(256) k_leg_synthesis(const T *__restrict__ lam, const int64_t *lam_off,
-                                                       int lmax, int nrn, const T *__restrict__ A,
-                                                       int64_t ncol, T *__restrict__ G, int rlim) {
+__global__ void __launch_bounds__(256) k_leg_synthesis(const T *lam, const int64_t *lam_off,
+                                                       int lmax, int nrn, const T *A,
+                                                       int64_t ncol, T *G, int rlim) {
+    pdl_entry();
     const int z = blockIdx.z;
     const int m = z >> 1, par = z & 1;
     const int nrows = nrows_of(m, par, lmax);   // K dimension
@@ -164,8 +166,9 @@ __global__ void __launch_bounds__(256) k_leg_synthesis(const T *__restrict__ lam
 // every phase is +1 or (-1)^t.  G_0 enters through its real part.
 template <typename T>
 __global__ void __launch_bounds__(128) k_fold_residual(const RingGeom *rings, int nrn, int lmax, double w,
-                                                      const T *__restrict__ F, const T *__restrict__ G, int64_t ncplx,
-                                                      T *__restrict__ R) {
+                                                      const T *F, const T *G, int64_t ncplx,
+                                                      T *R) {
+    pdl_entry();
     // one block per (parity, m', ring); threads stride over the complex columns
     const int mp = blockIdx.x;
     const int r = blockIdx.y;
@@ -213,9 +216,10 @@ __global__ void __launch_bounds__(128) k_fold_residual(const RingGeom *rings, in
 // Analysis: one warp per (block z, row li), lanes stride over the rings
 // (coalesced lambda rows), warp-reduced.
 template <typename T, int NC>
-__global__ void __launch_bounds__(256) k_leg_analysis_narrow(const T *__restrict__ lam, const int64_t *lam_off,
-                                                             int lmax, int nrn, int rlim, const T *__restrict__ F,
-                                                             T *__restrict__ A, int accumulate) {
+__global__ void __launch_bounds__(256) k_leg_analysis_narrow(const T *lam, const int64_t *lam_off,
+                                                             int lmax, int nrn, int rlim, const T *F,
+                                                             T *A, int accumulate) {
+    pdl_entry();
     const int z = blockIdx.y;
     const int m = z >> 1, par = z & 1;
     const int nrows = nrows_of(m, par, lmax);
@@ -249,9 +253,10 @@ __global__ void __launch_bounds__(256) k_leg_analysis_narrow(const T *__restrict
 // Synthesis: one thread per (block z, ring r), looping over the rows li
 // (lambda reads coalesced over r, a_lm broadcast).
 template <typename T, int NC>
-__global__ void __launch_bounds__(128) k_leg_synthesis_narrow(const T *__restrict__ lam, const int64_t *lam_off,
-                                                              int lmax, int nrn, int rlim, const T *__restrict__ A,
-                                                              T *__restrict__ G) {
+__global__ void __launch_bounds__(128) k_leg_synthesis_narrow(const T *lam, const int64_t *lam_off,
+                                                              int lmax, int nrn, int rlim, const T *A,
+                                                              T *G) {
+    pdl_entry();
     const int z = blockIdx.y;
     const int m = z >> 1, par = z & 1;
     const int nrows = nrows_of(m, par, lmax);
@@ -278,14 +283,15 @@ static void narrow_analysis(const Plan &p, const T *lam, const T *F, T *A, bool 
                             cudaStream_t st) {
     const int maxrows = p.lmax / 2 + 1;
     dim3 grid((unsigned)((maxrows + 7) / 8), (unsigned)(2 * (p.lmax + 1)));
-    k_leg_analysis_narrow<T, NC><<<grid, 256, 0, st>>>(lam, p.d_lam_off, p.lmax, (int)p.nrn, rlim, F, A,
-                                                       accumulate ? 1 : 0);
+    launch_pdl(k_leg_analysis_narrow<T, NC>, dim3(grid), dim3(256), 0, st, lam, p.d_lam_off, p.lmax, (int)p.nrn, rlim,
+        F, A, accumulate ? 1 : 0);
 }
 
 template <typename T, int NC>
 static void narrow_synthesis(const Plan &p, const T *lam, const T *A, T *G, int rlim, cudaStream_t st) {
     dim3 grid((unsigned)((rlim + 127) / 128), (unsigned)(2 * (p.lmax + 1)));
-    k_leg_synthesis_narrow<T, NC><<<grid, 128, 0, st>>>(lam, p.d_lam_off, p.lmax, (int)p.nrn, rlim, A, G);
+    launch_pdl(k_leg_synthesis_narrow<T, NC>, dim3(grid), dim3(128), 0, st, lam, p.d_lam_off, p.lmax, (int)p.nrn,
+        rlim, A, G);
 }
 
 template <typename T>
@@ -315,13 +321,14 @@ static bool narrow_dispatch(const Plan &p, const T *lam, const T *in, int64_t nc
 // one thread per (block z, output row r, column), D_z = M_z - I from the plan's FP64 Gram tables (element [li][r]
 // at gram_off[z] + li R + r); the others form G on the rings r < ral, one thread per (block z, ring).
 template <int NC>
-__global__ void __launch_bounds__(128) k_refine_narrow64(const double *__restrict__ gram,
-                                                         const int64_t *__restrict__ gram_off, int R,
-                                                         const double *__restrict__ lam,
-                                                         const int64_t *__restrict__ lam_off, int nrn, int ral, int ng,
-                                                         int lmax, const double *__restrict__ Acur,
-                                                         const double *__restrict__ A0, double *__restrict__ Anew,
-                                                         double *__restrict__ G) {
+__global__ void __launch_bounds__(128) k_refine_narrow64(const double *gram,
+                                                         const int64_t *gram_off, int R,
+                                                         const double *lam,
+                                                         const int64_t *lam_off, int nrn, int ral, int ng,
+                                                         int lmax, const double *Acur,
+                                                         const double *A0, double *Anew,
+                                                         double *G) {
+    pdl_entry();
     const int z = blockIdx.y;
     const int m = z >> 1, par = z & 1;
     const int nrows = nrows_of(m, par, lmax);
@@ -364,8 +371,8 @@ bool launch_refine_narrow64(const Plan &p, const double *A, const double *A0, in
     const int maxrows = p.lmax / 2 + 1, ng = (int)((maxrows * ncol + 127) / 128);
     const dim3 grid((unsigned)(ng + (p.ral + 127) / 128), (unsigned)(2 * (p.lmax + 1)));
     auto go = [&](auto kernel) {
-        kernel<<<grid, 128, 0, st>>>(p.d_gram64, p.d_gram_off, p.gram_rows, p.d_lam, p.d_lam_off, (int)p.nrn, p.ral, ng,
-                                     p.lmax, A, A0, Anew, G);
+        launch_pdl(kernel, dim3(grid), dim3(128), 0, st, p.d_gram64, p.d_gram_off, p.gram_rows, p.d_lam, p.d_lam_off,
+            (int)p.nrn, p.ral, ng, p.lmax, A, A0, Anew, G);
     };
     if (ncol == 2) go(k_refine_narrow64<2>);
     else if (ncol == 4) go(k_refine_narrow64<4>);
@@ -376,11 +383,12 @@ bool launch_refine_narrow64(const Plan &p, const double *A, const double *A0, in
 
 // Many columns: the same update as a tiled GEMM per block z (output rows r x
 // columns, K = the rows li), with the update in the epilogue.
-__global__ void __launch_bounds__(256) k_gram_update_wide(const double *__restrict__ gram,
-                                                          const int64_t *__restrict__ gram_off, int R, int lmax,
-                                                          const double *__restrict__ Acur,
-                                                          const double *__restrict__ A0, int64_t ncol,
-                                                          double *__restrict__ Anew) {
+__global__ void __launch_bounds__(256) k_gram_update_wide(const double *gram,
+                                                          const int64_t *gram_off, int R, int lmax,
+                                                          const double *Acur,
+                                                          const double *A0, int64_t ncol,
+                                                          double *Anew) {
+    pdl_entry();
     const int z = blockIdx.z;
     const int m = z >> 1, par = z & 1;
     const int nrows = nrows_of(m, par, lmax);
@@ -459,11 +467,11 @@ void launch_leg_analysis(const Plan &p, const double *F, int64_t ncol, double *A
     }
     dim3 grid((unsigned)((ncol + BN - 1) / BN), (unsigned)((maxrows + BM - 1) / BM), (unsigned)(2 * (p.lmax + 1)));
     if (p.precision == SFB_MIXED)
-        k_leg_analysis<float><<<grid, 256, 0, st>>>(p.d_lam32, p.d_lam_off, p.lmax, (int)p.nrn, (const float *)F,
-                                                    ncol, (float *)A, accumulate ? 1 : 0, rlim, nzr);
+        launch_pdl(k_leg_analysis<float>, dim3(grid), dim3(256), 0, st, p.d_lam32, p.d_lam_off, p.lmax, (int)p.nrn,
+            (const float *)F, ncol, (float *)A, accumulate ? 1 : 0, rlim, nzr);
     else
-        k_leg_analysis<double><<<grid, 256, 0, st>>>(p.d_lam, p.d_lam_off, p.lmax, (int)p.nrn, F, ncol, A,
-                                                     accumulate ? 1 : 0, rlim, nzr);
+        launch_pdl(k_leg_analysis<double>, dim3(grid), dim3(256), 0, st, p.d_lam, p.d_lam_off, p.lmax, (int)p.nrn, F,
+            ncol, A, accumulate ? 1 : 0, rlim, nzr);
     note_launch();
 }
 
@@ -484,10 +492,11 @@ void launch_leg_synthesis(const Plan &p, const double *A, int64_t ncol, double *
     }
     dim3 grid((unsigned)((ncol + BN - 1) / BN), (unsigned)((rlim + BM - 1) / BM), (unsigned)(2 * (p.lmax + 1)));
     if (p.precision == SFB_MIXED)
-        k_leg_synthesis<float><<<grid, 256, 0, st>>>(p.d_lam32, p.d_lam_off, p.lmax, (int)p.nrn, (const float *)A,
-                                                     ncol, (float *)G, rlim);
+        launch_pdl(k_leg_synthesis<float>, dim3(grid), dim3(256), 0, st, p.d_lam32, p.d_lam_off, p.lmax, (int)p.nrn,
+            (const float *)A, ncol, (float *)G, rlim);
     else
-        k_leg_synthesis<double><<<grid, 256, 0, st>>>(p.d_lam, p.d_lam_off, p.lmax, (int)p.nrn, A, ncol, G, rlim);
+        launch_pdl(k_leg_synthesis<double>, dim3(grid), dim3(256), 0, st, p.d_lam, p.d_lam_off, p.lmax, (int)p.nrn, A,
+            ncol, G, rlim);
     note_launch();
 }
 
@@ -512,10 +521,11 @@ __device__ __forceinline__ float2 df_resid(float2 F, float f, float s) {
 }
 
 // Mixed-precision column-major fold (as k_fold_cols): F (nullable) and R double-float, G FP32.
-__global__ void __launch_bounds__(128) k_fold_cols_df(const RingGeom *__restrict__ rings, int nrn, int rlim, int lmax,
-                                                      double w, const float2 *__restrict__ F,
-                                                      const float *__restrict__ G, int64_t ncplx,
-                                                      float2 *__restrict__ R, int *__restrict__ Ecol) {
+__global__ void __launch_bounds__(128) k_fold_cols_df(const RingGeom *rings, int nrn, int rlim, int lmax,
+                                                      double w, const float2 *F,
+                                                      const float *G, int64_t ncplx,
+                                                      float2 *R, int *Ecol) {
+    pdl_entry();
     const int mp = blockIdx.y >> 1, par = blockIdx.y & 1;
     const int rc0 = blockIdx.z * FOLD_RC;
     const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -577,9 +587,10 @@ __global__ void __launch_bounds__(128) k_fold_cols_df(const RingGeom *__restrict
 // F == nullptr: R = -w n cfold Fold(G) (the aliased-ring term of the Gram
 // refinement).  Only rings r < rlim are written.
 template <typename T>
-__global__ void __launch_bounds__(128) k_fold_cols(const RingGeom *__restrict__ rings, int nrn, int rlim, int lmax,
-                                                   double w, const T *__restrict__ F, const T *__restrict__ G,
-                                                   int64_t ncplx, T *__restrict__ R, int *__restrict__ Ecol) {
+__global__ void __launch_bounds__(128) k_fold_cols(const RingGeom *rings, int nrn, int rlim, int lmax,
+                                                   double w, const T *F, const T *G,
+                                                   int64_t ncplx, T *R, int *Ecol) {
+    pdl_entry();
     const int mp = blockIdx.y >> 1, par = blockIdx.y & 1;
     const int rc0 = blockIdx.z * FOLD_RC;
     const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -660,9 +671,10 @@ __device__ __forceinline__ uint32_t recip32(int n) { return (uint32_t)(0x1000000
 __device__ __forceinline__ int div32(int a, uint32_t inv) { return (int)__umulhi((uint32_t)a, inv); }
 
 template <int FC, bool MXREG>
-__global__ void __launch_bounds__(256) k_fold_alias(const RingGeom *__restrict__ rings, int nrn, int ral, int rpb,
-                                                    int nbk, int lmax, double w, const float *__restrict__ G,
-                                                    int64_t ncplx, float2 *__restrict__ R, int *__restrict__ Ecol) {
+__global__ void __launch_bounds__(256) k_fold_alias(const RingGeom *rings, int nrn, int ral, int rpb,
+                                                    int nbk, int lmax, double w, const float *G,
+                                                    int64_t ncplx, float2 *R, int *Ecol) {
+    pdl_entry();
     extern __shared__ float2 fsm[];
     const int par = blockIdx.y;
     const int64_t c0 = (int64_t)blockIdx.x * FC;
@@ -785,9 +797,10 @@ __global__ void __launch_bounds__(256) k_fold_alias(const RingGeom *__restrict__
 // ring's rows are on their way in registers.  Bound: the latency of the steps of one ring; k_fold_cols above
 // reads every aliased G term from memory for every m' (91 us a pass at 101 maps, 41 rings, lmax 82).
 template <int FC>
-__global__ void __launch_bounds__(256) k_fold_alias64(const RingGeom *__restrict__ rings, int nrn, int ral, int rpb,
-                                                      int nbk, int lmax, double w, const double *__restrict__ G,
-                                                      int64_t ncplx, double *__restrict__ R) {
+__global__ void __launch_bounds__(256) k_fold_alias64(const RingGeom *rings, int nrn, int ral, int rpb,
+                                                      int nbk, int lmax, double w, const double *G,
+                                                      int64_t ncplx, double *R) {
+    pdl_entry();
     extern __shared__ double2 fsm64[];
     const int par = blockIdx.y, tid = threadIdx.x;
     const int64_t c0 = (int64_t)blockIdx.x * FC;
@@ -863,9 +876,8 @@ static bool fold_alias64(const Plan &p, const double *G, int64_t ncplx, double *
     const int64_t gx = (ncplx + FC - 1) / FC;
     const int rpb = (int)std::max<int64_t>(1, std::min<int64_t>(4, 2 * gx * rlim / 1216));
     set_smem(k_fold_alias64<FC>, smem);
-    k_fold_alias64<FC><<<dim3((unsigned)((ncplx + FC - 1) / FC), 2, (unsigned)((rlim + rpb - 1) / rpb)), 256, smem,
-                         st>>>(p.d_rings, (int)p.nrn, rlim, rpb, nbk, p.lmax, 4.0 * M_PI / (double)p.npix, G, ncplx,
-                               R);
+    launch_pdl(k_fold_alias64<FC>, dim3((unsigned)((ncplx + FC - 1) / FC), 2, (unsigned)((rlim + rpb - 1) / rpb)),
+        dim3(256), smem, st, p.d_rings, (int)p.nrn, rlim, rpb, nbk, p.lmax, 4.0 * M_PI / (double)p.npix, G, ncplx, R);
     note_launch();
     return true;
 }
@@ -881,9 +893,10 @@ __device__ __forceinline__ float2 resid_of(const float2 *F, int64_t off, float f
 // TF: element type of F and R (double, or the double-float pairs of the mixed transform)
 template <typename T, typename TF>
 __global__ void __launch_bounds__(256) k_fold_residual_narrow(const RingGeom *rings, int nrn, int rlim, int lmax,
-                                                             double w, const TF *__restrict__ F,
-                                                             const T *__restrict__ G, int64_t ncplx,
-                                                             TF *__restrict__ R) {
+                                                             double w, const TF *F,
+                                                             const T *G, int64_t ncplx,
+                                                             TF *R) {
+    pdl_entry();
     const int L1 = lmax + 1;
     const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t total = (int64_t)2 * L1 * rlim * ncplx;     // rings r < rlim only
@@ -931,7 +944,8 @@ bool launch_gram_update_fp64(const Plan &p, const double *Acur, const double *A0
     }
     const int maxrows = p.lmax / 2 + 1;
     dim3 wg((unsigned)((ncol + BN - 1) / BN), (unsigned)((maxrows + BM - 1) / BM), (unsigned)(2 * (p.lmax + 1)));
-    k_gram_update_wide<<<wg, 256, 0, st>>>(p.d_gram64, p.d_gram_off, p.gram_rows, p.lmax, Acur, A0, ncol, Anew);
+    launch_pdl(k_gram_update_wide, dim3(wg), dim3(256), 0, st, p.d_gram64, p.d_gram_off, p.gram_rows, p.lmax, Acur,
+        A0, ncol, Anew);
     note_launch();
     return true;
 }
@@ -959,12 +973,12 @@ void launch_fold_residual(const Plan &p, const double *F, const double *G, int64
                 const double w = 4.0 * M_PI / (double)p.npix;
                 if (mxreg) {
                     set_smem(k_fold_alias<FC, true>, smem);
-                    k_fold_alias<FC, true><<<grid, 256, smem, st>>>(p.d_rings, (int)p.nrn, rlim, rpb, nbk, p.lmax,
-                                                                    w, (const float *)G, ncplx, (float2 *)R, Ecol);
+                    launch_pdl(k_fold_alias<FC, true>, dim3(grid), dim3(256), smem, st, p.d_rings, (int)p.nrn, rlim,
+                        rpb, nbk, p.lmax, w, (const float *)G, ncplx, (float2 *)R, Ecol);
                 } else {
                     set_smem(k_fold_alias<FC, false>, smem);
-                    k_fold_alias<FC, false><<<grid, 256, smem, st>>>(p.d_rings, (int)p.nrn, rlim, rpb, nbk, p.lmax,
-                                                                     w, (const float *)G, ncplx, (float2 *)R, Ecol);
+                    launch_pdl(k_fold_alias<FC, false>, dim3(grid), dim3(256), smem, st, p.d_rings, (int)p.nrn, rlim,
+                        rpb, nbk, p.lmax, w, (const float *)G, ncplx, (float2 *)R, Ecol);
                 }
                 note_launch();
                 return;
@@ -973,8 +987,8 @@ void launch_fold_residual(const Plan &p, const double *F, const double *G, int64
         dim3 grid((unsigned)((ncplx + 127) / 128), (unsigned)(2 * (p.lmax + 1)),
                   (unsigned)((rlim + FOLD_RC - 1) / FOLD_RC));
         const double w = 4.0 * M_PI / (double)p.npix;
-        k_fold_cols_df<<<grid, 128, 0, st>>>(p.d_rings, (int)p.nrn, rlim, p.lmax, w, (const float2 *)F,
-                                             (const float *)G, ncplx, (float2 *)R, Ecol);
+        launch_pdl(k_fold_cols_df, dim3(grid), dim3(128), 0, st, p.d_rings, (int)p.nrn, rlim, p.lmax, w,
+            (const float2 *)F, (const float *)G, ncplx, (float2 *)R, Ecol);
         note_launch();
         return;
     }
@@ -988,8 +1002,8 @@ void launch_fold_residual(const Plan &p, const double *F, const double *G, int64
                   (unsigned)((rlim + FOLD_RC - 1) / FOLD_RC));
         const double w = 4.0 * M_PI / (double)p.npix;
         if (rlim > 0)
-            k_fold_cols<double><<<grid, 128, 0, st>>>(p.d_rings, (int)p.nrn, rlim, p.lmax, w, nullptr, G, ncplx, R,
-                                                      nullptr);
+            launch_pdl(k_fold_cols<double>, dim3(grid), dim3(128), 0, st, p.d_rings, (int)p.nrn, rlim, p.lmax, w,
+                nullptr, G, ncplx, R, nullptr);
         note_launch();
         return;
     }
@@ -998,24 +1012,25 @@ void launch_fold_residual(const Plan &p, const double *F, const double *G, int64
         const unsigned blocks = (unsigned)((total + 255) / 256);
         const double w = 4.0 * M_PI / (double)p.npix;
         if (p.precision == SFB_MIXED)
-            k_fold_residual_narrow<float, float2><<<blocks, 256, 0, st>>>(p.d_rings, (int)p.nrn, rlim, p.lmax, w,
-                                                                         (const float2 *)F, (const float *)G, ncplx,
-                                                                         (float2 *)R);
+            launch_pdl(k_fold_residual_narrow<float, float2>, dim3(blocks), dim3(256), 0, st, p.d_rings, (int)p.nrn,
+                rlim, p.lmax, w, (const float2 *)F, (const float *)G, ncplx, (float2 *)R);
         else
-            k_fold_residual_narrow<double, double><<<blocks, 256, 0, st>>>(p.d_rings, (int)p.nrn, rlim, p.lmax, w, F,
-                                                                          G, ncplx, R);
+            launch_pdl(k_fold_residual_narrow<double, double>, dim3(blocks), dim3(256), 0, st, p.d_rings, (int)p.nrn,
+                rlim, p.lmax, w, F, G, ncplx, R);
         note_launch();
         return;
     }
     // FP64, many columns, full residual (the mixed transform returned above)
     dim3 grid((unsigned)(p.lmax + 1), (unsigned)p.nrn, 2u);
     const double w = 4.0 * M_PI / (double)p.npix;
-    k_fold_residual<double><<<grid, 128, 0, st>>>(p.d_rings, (int)p.nrn, p.lmax, w, F, G, ncplx, R);
+    launch_pdl(k_fold_residual<double>, dim3(grid), dim3(128), 0, st, p.d_rings, (int)p.nrn, p.lmax, w, F, G, ncplx,
+        R);
     note_launch();
 }
 
 // double -> normalised double-float pairs (the mixed transform's map format)
 __global__ void k_to_df(const double *in, int64_t n, float2 *out) {
+    pdl_entry();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const double v = in[i];
         const float h = (float)v;
@@ -1027,11 +1042,12 @@ void launch_to_df(const double *in, int64_t n, float2 *out, cudaStream_t st) {
     if (n <= 0) return;
     int64_t blocks = (n + 255) / 256;
     if (blocks > 8192) blocks = 8192;
-    k_to_df<<<(unsigned)blocks, 256, 0, st>>>(in, n, out);
+    launch_pdl(k_to_df, dim3((unsigned)blocks), dim3(256), 0, st, in, n, out);
     note_launch();
 }
 
 __global__ void k_to_float(const double *in, int64_t n, float *out) {
+    pdl_entry();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         out[i] = (float)in[i];
 }
@@ -1040,7 +1056,7 @@ void launch_to_float(const double *in, int64_t n, float *out, cudaStream_t st) {
     if (n <= 0) return;
     int64_t blocks = (n + 255) / 256;
     if (blocks > 8192) blocks = 8192;
-    k_to_float<<<(unsigned)blocks, 256, 0, st>>>(in, n, out);
+    launch_pdl(k_to_float, dim3((unsigned)blocks), dim3(256), 0, st, in, n, out);
     note_launch();
 }
 

@@ -207,9 +207,10 @@ __device__ __forceinline__ bool lvl_stage_free(const LvlSmem &cs, int kc) {
 // sums (8-bit leading slices of F and lambda, at most 2^14 units a product)
 // stay within 2^24 units.
 // (nzr: F is zero outside the ring pairs [nzr[0], nzr[1]], which are the only ones read)
-__global__ void __launch_bounds__(256) k_colmax(const float2 *__restrict__ F, int64_t ncol, int lmax, int nrn,
-                                                int *__restrict__ Ecol, const int *__restrict__ nzr,
-                                                const int2 *__restrict__ live, int ntile) {
+__global__ void __launch_bounds__(256) k_colmax(const float2 *F, int64_t ncol, int lmax, int nrn,
+                                                int *Ecol, const int *nzr,
+                                                const int2 *live, int ntile) {
+    pdl_entry();
     const int z = blockIdx.y;
     const int m = z >> 1, par = z & 1;
     const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -245,14 +246,15 @@ __global__ void __launch_bounds__(256) k_colmax(const float2 *__restrict__ F, in
 // Analysis: grid (column tiles, row tiles of NMAX, blocks z); warps 0-7
 // produce (thread: column c, half kh of each chunk), warp 8 issues the MMAs.
 // Rings r >= rlim count as zero (the sum over the first rlim rings only).
-__global__ void __launch_bounds__(NTH, 2) k_leg_analysis_tc(const __nv_bfloat16 *__restrict__ lamtc,
-                                                            const int64_t *__restrict__ lamtc_off, int lmax, int nrn,
-                                                            int nchunks, int rlim, const float2 *__restrict__ F,
-                                                            int64_t ncol, const int *__restrict__ Ecol,
-                                                            double *__restrict__ A, float2 *__restrict__ Adf,
-                                                            int accumulate, int *__restrict__ Eout,
-                                                            const int *__restrict__ nzr,
-                                                            const int2 *__restrict__ live, int *err) {
+__global__ void __launch_bounds__(NTH, 2) k_leg_analysis_tc(const __nv_bfloat16 *lamtc,
+                                                            const int64_t *lamtc_off, int lmax, int nrn,
+                                                            int nchunks, int rlim, const float2 *F,
+                                                            int64_t ncol, const int *Ecol,
+                                                            double *A, float2 *Adf,
+                                                            int accumulate, int *Eout,
+                                                            const int *nzr,
+                                                            const int2 *live, int *err) {
+    pdl_entry();
     extern __shared__ __align__(1024) unsigned char smem[];
     const int z = blockIdx.z;
     const int m = z >> 1, par = z & 1;
@@ -441,10 +443,11 @@ struct SynTable {
     int nrn, NT;
 };
 __global__ void __launch_bounds__(NTH, 2) k_leg_synthesis_tc(SynTable gram, SynTable syn, int ny0, int lmax,
-                                                             const float2 *__restrict__ Adf, int64_t ncol,
-                                                             float *__restrict__ G, const float2 *__restrict__ A0,
-                                                             float2 *__restrict__ Adfnew, const int *__restrict__ Ein,
-                                                             int *__restrict__ Eout, int *err) {
+                                                             const float2 *Adf, int64_t ncol,
+                                                             float *G, const float2 *A0,
+                                                             float2 *Adfnew, const int *Ein,
+                                                             int *Eout, int *err) {
+    pdl_entry();
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ float red[2][MTILE];
     const int z = blockIdx.z;
@@ -613,8 +616,9 @@ __global__ void __launch_bounds__(NTH, 2) k_leg_synthesis_tc(SynTable gram, SynT
 
 // Row scales of the lambda tables.  Analysis: per (z, li) over the rings;
 // synthesis: per (z, ring) over the rows.  E with max |lambda| < 2^E.
-__global__ void k_lam_rowexp(const double *__restrict__ lam, const int64_t *lam_off, int lmax, int nrn, int *Ea,
+__global__ void k_lam_rowexp(const double *lam, const int64_t *lam_off, int lmax, int nrn, int *Ea,
                              int *Es) {
+    pdl_entry();
     const int z = blockIdx.y;
     const int m = z >> 1, par = z & 1;
     const int nrows = rows_of(m, par, lmax);
@@ -648,8 +652,9 @@ __device__ __forceinline__ void slices4(double v, int E, __nv_bfloat16 (&o)[4]) 
 
 // Analysis table: block z, chunk kc, plane q, row li < NP, ring k < KC in the
 // core-matrix layout (zero padding), sliced on the row scale Ea.
-__global__ void k_build_lamtc(const double *__restrict__ lam, const int64_t *lam_off, int lmax, int nrn, int nchunks,
-                              const int *__restrict__ Ea, const int64_t *lamtc_off, __nv_bfloat16 *lamtc) {
+__global__ void k_build_lamtc(const double *lam, const int64_t *lam_off, int lmax, int nrn, int nchunks,
+                              const int *Ea, const int64_t *lamtc_off, __nv_bfloat16 *lamtc) {
+    pdl_entry();
     const int z = blockIdx.y;
     const int m = z >> 1, par = z & 1;
     const int nrows = rows_of(m, par, lmax);
@@ -680,8 +685,9 @@ __global__ void k_build_lamtc(const double *__restrict__ lam, const int64_t *lam
 // Synthesis table: block z, ring tile nt, chunk kc, plane q, ring rr < NT,
 // row k < KC in the core-matrix layout (N = rings, K = rows li), sliced on
 // the ring scale Es.
-__global__ void k_build_lamts(const double *__restrict__ lam, const int64_t *lam_off, int lmax, int nrn, int NT,
-                              const int *__restrict__ Es, const int64_t *lamts_off, __nv_bfloat16 *lamts) {
+__global__ void k_build_lamts(const double *lam, const int64_t *lam_off, int lmax, int nrn, int NT,
+                              const int *Es, const int64_t *lamts_off, __nv_bfloat16 *lamts) {
+    pdl_entry();
     const int z = blockIdx.y;
     const int m = z >> 1, par = z & 1;
     const int nrows = rows_of(m, par, lmax);
@@ -715,6 +721,7 @@ __global__ void k_build_lamts(const double *__restrict__ lam, const int64_t *lam
 // Self-test of the bounded waits: one CTA waits on an mbarrier that nothing
 // arrives at; the wait gives up after SPIN_LIMIT polls and records the error.
 __global__ void k_selftest_wait(int *err) {
+    pdl_entry();
     __shared__ __align__(8) uint64_t bar;
     if (threadIdx.x == 0) {
         mbar_init(&bar, 1);
@@ -751,13 +758,13 @@ int64_t tc_table_offsets(const Plan &p, std::vector<int64_t> &off) {
 void launch_build_lamtc(const Plan &p, const int *Ea, const int *Es, cudaStream_t st) {
     {
         dim3 grid(8, (unsigned)(2 * (p.lmax + 1)));
-        tc::k_lam_rowexp<<<grid, 256, 0, st>>>(p.d_lam, p.d_lam_off, p.lmax, (int)p.nrn, const_cast<int *>(Ea),
-                                               const_cast<int *>(Es));
+        launch_pdl(tc::k_lam_rowexp, dim3(grid), dim3(256), 0, st, p.d_lam, p.d_lam_off, p.lmax, (int)p.nrn,
+            const_cast<int *>(Ea), const_cast<int *>(Es));
         note_launch();
     }
     dim3 grid(64, (unsigned)(2 * (p.lmax + 1)));
-    tc::k_build_lamtc<<<grid, 256, 0, st>>>(p.d_lam, p.d_lam_off, p.lmax, (int)p.nrn, tc_chunks(p), Ea,
-                                            p.d_lamtc_off, (__nv_bfloat16 *)p.d_lamtc);
+    launch_pdl(tc::k_build_lamtc, dim3(grid), dim3(256), 0, st, p.d_lam, p.d_lam_off, p.lmax, (int)p.nrn,
+        tc_chunks(p), Ea, p.d_lamtc_off, (__nv_bfloat16 *)p.d_lamtc);
     note_launch();
 }
 
@@ -767,17 +774,16 @@ void launch_leg_analysis_tc(const Plan &p, const float2 *F, int64_t ncol, double
     if (rlim < 0 || rlim > p.nrn) rlim = (int)p.nrn;
     if (!scales_ready) {
         dim3 grid((unsigned)((ncol + 255) / 256), (unsigned)(2 * (p.lmax + 1)));
-        tc::k_colmax<<<grid, 256, 0, st>>>(F, ncol, p.lmax, (int)p.nrn, Ecol, nzr, p.d_lamtc_live,
+        launch_pdl(tc::k_colmax, dim3(grid), dim3(256), 0, st, F, ncol, p.lmax, (int)p.nrn, Ecol, nzr, p.d_lamtc_live,
                                            (tc_np_max(p) + tc::NMAX - 1) / tc::NMAX);
         note_launch();
     }
     set_smem(tc::k_leg_analysis_tc, tc::LEG_SMEM);
     const int ntile = (tc_np_max(p) + tc::NMAX - 1) / tc::NMAX;
     dim3 grid((unsigned)((ncol + tc::MTILE - 1) / tc::MTILE), (unsigned)ntile, (unsigned)(2 * (p.lmax + 1)));
-    tc::k_leg_analysis_tc<<<grid, tc::NTH, tc::LEG_SMEM, st>>>((const __nv_bfloat16 *)p.d_lamtc, p.d_lamtc_off,
-                                                              p.lmax, (int)p.nrn, (rlim + tc::KC - 1) / tc::KC, rlim,
-                                                              F, ncol, Ecol, A, Adf, accumulate ? 1 : 0, Eout,
-                                                              nzr, p.d_lamtc_live, p.d_err);
+    launch_pdl(tc::k_leg_analysis_tc, dim3(grid), dim3(tc::NTH), tc::LEG_SMEM, st, (const __nv_bfloat16 *)p.d_lamtc,
+        p.d_lamtc_off, p.lmax, (int)p.nrn, (rlim + tc::KC - 1) / tc::KC, rlim, F, ncol, Ecol, A, Adf,
+        accumulate ? 1 : 0, Eout, nzr, p.d_lamtc_live, p.d_err);
     note_launch();
 }
 
@@ -816,14 +822,16 @@ namespace tc {
 // per (block z, ring tile) the synthesis table's row chunks.  Ranges [x, y]
 // (x > y: no live chunk), preset to {INT_MAX, -1}.
 __global__ void k_fill_range(int2 *r, int64_t n) {
+    pdl_entry();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         r[i] = make_int2(0x7fffffff, -1);
 }
 
 // grid (z, ring chunk kc); element e of a plane lies at row (core >> 1) * 8 + ((e & 63) >> 3) with
 // core = e >> 6 (core-matrix layout, KC = 16 columns per row group)
-__global__ void k_live_analysis(const uint16_t *__restrict__ tab, const int64_t *__restrict__ off, int lmax,
-                                int nch, int ntile, int2 *__restrict__ live) {
+__global__ void k_live_analysis(const uint16_t *tab, const int64_t *off, int lmax,
+                                int nch, int ntile, int2 *live) {
+    pdl_entry();
     __shared__ int any[64];
     const int z = blockIdx.x, kc = blockIdx.y;
     const int m = z >> 1, par = z & 1;
@@ -848,8 +856,9 @@ __global__ void k_live_analysis(const uint16_t *__restrict__ tab, const int64_t 
 }
 
 // grid (z, ring tile nt x row chunk kc)
-__global__ void k_live_synthesis(const uint16_t *__restrict__ tab, const int64_t *__restrict__ off, int lmax,
-                                 int NT, int ntiles, int nkmax, int2 *__restrict__ live) {
+__global__ void k_live_synthesis(const uint16_t *tab, const int64_t *off, int lmax,
+                                 int NT, int ntiles, int nkmax, int2 *live) {
+    pdl_entry();
     const int z = blockIdx.x, nt = blockIdx.y / nkmax, kc = blockIdx.y % nkmax;
     const int m = z >> 1, par = z & 1;
     const int nrows = rows_of(m, par, lmax);
@@ -867,8 +876,9 @@ __global__ void k_live_synthesis(const uint16_t *__restrict__ tab, const int64_t
 // Ring DFT spectra that no analysis chunk reads: ring pair r and column block u
 // (m in [64 u, 64 u + 63]) are dead when, for every block z of those m and
 // every row tile, the chunk of r lies outside the tile's live range.
-__global__ void k_dft_dead(const int2 *__restrict__ live, int lmax, int nrn, int ntile, int ntn,
-                           unsigned char *__restrict__ dead) {
+__global__ void k_dft_dead(const int2 *live, int lmax, int nrn, int ntile, int ntn,
+                           unsigned char *dead) {
+    pdl_entry();
     const int r = blockIdx.x * blockDim.x + threadIdx.x, u = blockIdx.y;
     if (r >= nrn) return;
     const int kc = r / KC;
@@ -900,12 +910,12 @@ int build_live_ranges(Plan &p, cudaStream_t st) {
     }
     p.device_bytes += (na + ns) * (int64_t)sizeof(int2);
     p.d_lamts_live = p.d_lamtc_live + na;
-    tc::k_fill_range<<<(unsigned)((na + ns + 255) / 256), 256, 0, st>>>(p.d_lamtc_live, na + ns);
+    launch_pdl(tc::k_fill_range, dim3((unsigned)((na + ns + 255) / 256)), dim3(256), 0, st, p.d_lamtc_live, na + ns);
     note_launch();
-    tc::k_live_analysis<<<dim3((unsigned)nz, (unsigned)tc_chunks(p)), 256, 0, st>>>(
+    launch_pdl(tc::k_live_analysis, dim3((unsigned)nz, (unsigned)tc_chunks(p)), dim3(256), 0, st,
         (const uint16_t *)p.d_lamtc, p.d_lamtc_off, p.lmax, tc_chunks(p), ntile_a, p.d_lamtc_live);
     note_launch();
-    tc::k_live_synthesis<<<dim3((unsigned)nz, (unsigned)(ntiles_s * nkmax)), 256, 0, st>>>(
+    launch_pdl(tc::k_live_synthesis, dim3((unsigned)nz, (unsigned)(ntiles_s * nkmax)), dim3(256), 0, st,
         (const uint16_t *)p.d_lamts, p.d_lamts_off, p.lmax, NT, ntiles_s, nkmax, p.d_lamts_live);
     note_launch();
     const int ntn = (p.lmax + 1 + 63) / 64;
@@ -915,7 +925,7 @@ int build_live_ranges(Plan &p, cudaStream_t st) {
         return fail(SFB_ENOMEM, "device allocation failed (ring DFT dead flags)");
     }
     p.device_bytes += p.nrn * ntn;
-    tc::k_dft_dead<<<dim3((unsigned)((p.nrn + 127) / 128), (unsigned)ntn), 128, 0, st>>>(
+    launch_pdl(tc::k_dft_dead, dim3((unsigned)((p.nrn + 127) / 128), (unsigned)ntn), dim3(128), 0, st,
         p.d_lamtc_live, p.lmax, (int)p.nrn, ntile_a, ntn, p.d_dft_dead);
     note_launch();
     return cudaGetLastError() == cudaSuccess ? SFB_OK : fail(SFB_ECUDA, "live chunk ranges failed");
@@ -923,8 +933,8 @@ int build_live_ranges(Plan &p, cudaStream_t st) {
 
 void launch_build_lamts(const Plan &p, const int *Es, cudaStream_t st) {
     dim3 grid(64, (unsigned)(2 * (p.lmax + 1)));
-    tc::k_build_lamts<<<grid, 256, 0, st>>>(p.d_lam, p.d_lam_off, p.lmax, (int)p.nrn, tc_synth_nt(p), Es,
-                                            p.d_lamts_off, (__nv_bfloat16 *)p.d_lamts);
+    launch_pdl(tc::k_build_lamts, dim3(grid), dim3(256), 0, st, p.d_lam, p.d_lam_off, p.lmax, (int)p.nrn,
+        tc_synth_nt(p), Es, p.d_lamts_off, (__nv_bfloat16 *)p.d_lamts);
     note_launch();
 }
 
@@ -943,13 +953,14 @@ void launch_leg_synthesis_tc(const Plan &p, const float2 *Adf, int64_t ncol, flo
     // ring tiles covering the first rlim rings (a tile's rings past rlim are computed as well)
     dim3 grid((unsigned)((ncol + tc::MTILE - 1) / tc::MTILE), (unsigned)(ny0 + (rlim + NT - 1) / NT),
               (unsigned)(2 * (p.lmax + 1)));
-    tc::k_leg_synthesis_tc<<<grid, tc::NTH, tc::LEG_SMEM, st>>>(gram, syn, ny0, p.lmax, Adf, ncol, G, A0, Adfnew, Ein,
-                                                               Eout, p.d_err);
+    launch_pdl(tc::k_leg_synthesis_tc, dim3(grid), dim3(tc::NTH), tc::LEG_SMEM, st, gram, syn, ny0, p.lmax, Adf, ncol,
+        G, A0, Adfnew, Ein, Eout, p.d_err);
     note_launch();
 }
 
 namespace tc {
-__global__ void k_df_to_fp64(const float2 *__restrict__ a, int64_t n, double *__restrict__ out) {
+__global__ void k_df_to_fp64(const float2 *a, int64_t n, double *out) {
+    pdl_entry();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const float2 v = a[i];
         out[i] = (double)v.x + (double)v.y;
@@ -960,7 +971,7 @@ __global__ void k_df_to_fp64(const float2 *__restrict__ a, int64_t n, double *__
 void launch_df_to_fp64(const float2 *a, int64_t n, double *out, cudaStream_t st) {
     if (n <= 0) return;
     const int64_t blocks = std::min<int64_t>((n + 255) / 256, 152 * 16);
-    tc::k_df_to_fp64<<<(unsigned)blocks, 256, 0, st>>>(a, n, out);
+    launch_pdl(tc::k_df_to_fp64, dim3((unsigned)blocks), dim3(256), 0, st, a, n, out);
     note_launch();
 }
 
@@ -971,6 +982,7 @@ void launch_df_to_fp64(const float2 *a, int64_t n, double *out, cudaStream_t st)
 // kernels, then sliced into the synthesis layout with the output rows as rings.
 namespace tc {
 __global__ void k_unit_alm(int lmax, int R, double *E) {
+    pdl_entry();
     const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t lmsize = (int64_t)(lmax + 1) * (lmax + 2) / 2;
     if (idx >= lmsize * R) return;
@@ -983,8 +995,9 @@ __global__ void k_unit_alm(int lmax, int R, double *E) {
     E[idx] = (c == ((l - m) >> 1)) ? 1.0 : 0.0;
 }
 
-__global__ void k_gram_weights(const RingGeom *__restrict__ rings, int nrn, int lmax, int ral, double w, int R,
+__global__ void k_gram_weights(const RingGeom *rings, int nrn, int lmax, int ral, double w, int R,
                                double *G) {
+    pdl_entry();
     const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t total = (int64_t)2 * (lmax + 1) * nrn * R;
     if (idx >= total) return;
@@ -993,8 +1006,9 @@ __global__ void k_gram_weights(const RingGeom *__restrict__ rings, int nrn, int 
     G[idx] = r < ral ? 0.0 : G[idx] * (w * (double)g.nph * g.cfold);
 }
 
-__global__ void k_gram_gather(int lmax, int R, const double *__restrict__ A, const int64_t *__restrict__ gram_off,
-                              double *__restrict__ gram) {
+__global__ void k_gram_gather(int lmax, int R, const double *A, const int64_t *gram_off,
+                              double *gram) {
+    pdl_entry();
     const int z = blockIdx.y;
     const int m = z >> 1, par = z & 1;
     const int nrows = rows_of(m, par, lmax);
@@ -1046,17 +1060,17 @@ int build_gram_tables(Plan &p, cudaStream_t st) {
     cudaMemcpy(d_goff, goff.data(), goff.size() * sizeof(int64_t), cudaMemcpyHostToDevice);
     const int32_t prec = p.precision;
     p.precision = SFB_FP64;
-    tc::k_unit_alm<<<(unsigned)((nE + 255) / 256), 256, 0, st>>>(p.lmax, R, E);
+    launch_pdl(tc::k_unit_alm, dim3((unsigned)((nE + 255) / 256)), dim3(256), 0, st, p.lmax, R, E);
     note_launch();
     launch_leg_synthesis(p, E, R, G, st);
-    tc::k_gram_weights<<<(unsigned)((nG + 255) / 256), 256, 0, st>>>(p.d_rings, (int)p.nrn, p.lmax, p.ral,
-                                                                     4.0 * M_PI / (double)p.npix, R, G);
+    launch_pdl(tc::k_gram_weights, dim3((unsigned)((nG + 255) / 256)), dim3(256), 0, st, p.d_rings, (int)p.nrn,
+        p.lmax, p.ral, 4.0 * M_PI / (double)p.npix, R, G);
     note_launch();
     launch_leg_analysis(p, G, R, A, false, st);
     p.precision = prec;
-    tc::k_gram_gather<<<dim3(16, (unsigned)(2 * L1)), 256, 0, st>>>(p.lmax, R, A, d_goff, gram);
+    launch_pdl(tc::k_gram_gather, dim3(16, (unsigned)(2 * L1)), dim3(256), 0, st, p.lmax, R, A, d_goff, gram);
     note_launch();
-    tc::k_lam_rowexp<<<dim3(8, (unsigned)(2 * L1)), 256, 0, st>>>(gram, d_goff, p.lmax, R, Ea, Es);
+    launch_pdl(tc::k_lam_rowexp, dim3(8, (unsigned)(2 * L1)), dim3(256), 0, st, gram, d_goff, p.lmax, R, Ea, Es);
     note_launch();
     std::vector<int64_t> soff;
     const int64_t ssz = tc_synth_table_offsets(p, soff, R);
@@ -1068,9 +1082,8 @@ int build_gram_tables(Plan &p, cudaStream_t st) {
     } else {
         p.device_bytes += (ssz + 1) * 2 + (int64_t)(soff.size() * sizeof(int64_t));
         cudaMemcpy(p.d_gramts_off, soff.data(), soff.size() * sizeof(int64_t), cudaMemcpyHostToDevice);
-        tc::k_build_lamts<<<dim3(64, (unsigned)(2 * L1)), 256, 0, st>>>(gram, d_goff, p.lmax, R, tc_synth_nt(R), Es,
-                                                                        p.d_gramts_off,
-                                                                        (__nv_bfloat16 *)p.d_gramts);
+        launch_pdl(tc::k_build_lamts, dim3(64, (unsigned)(2 * L1)), dim3(256), 0, st, gram, d_goff, p.lmax, R,
+            tc_synth_nt(R), Es, p.d_gramts_off, (__nv_bfloat16 *)p.d_gramts);
         note_launch();
     }
     if (cudaStreamSynchronize(st) != cudaSuccess && rc == SFB_OK)
@@ -1096,7 +1109,7 @@ extern "C" int sfb_selftest_wait_timeout(void) {
         return sfb::fail(SFB_ECUDA, "no CUDA device available");
     }
     cudaMemset(d, 0, sizeof(int));
-    sfb::tc::k_selftest_wait<<<1, 32>>>(d);
+    sfb::launch_pdl(sfb::tc::k_selftest_wait, dim3(1), dim3(32), 0, 0, d);
     sfb::note_launch();
     int h = 0;
     const cudaError_t e = cudaMemcpy(&h, d, sizeof(int), cudaMemcpyDeviceToHost);

@@ -14,6 +14,12 @@ namespace sfb {
 static thread_local std::string g_last_error;
 static std::atomic<int64_t> g_launches{0};
 
+// one call at a time on a thread decides for the launches it makes
+static thread_local bool t_pdl = false;
+PdlScope::PdlScope(bool on) : before(t_pdl) { t_pdl = on; }
+PdlScope::~PdlScope() { t_pdl = before; }
+bool PdlScope::enabled() { return t_pdl; }
+
 void note_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 
 void set_error(const std::string &msg) { g_last_error = msg; }
@@ -781,6 +787,9 @@ int64_t chunk_pairs(const Plan &p) {
     return c;
 }
 
+// map pixels up to which a mixed catalogue transform uses programmatic dependent launches (PdlScope)
+constexpr int64_t PDL_MAX = int64_t(1) << 24;
+
 // a_nlm of mocks.n catalogues (one, or the mocks of a group: mock j's result at out + 2 j nlmsize).
 // defer_finish (batched calls): the device error word is neither cleared nor read here and the
 // call does not wait for the device; the caller clears it once and checks it at the end.
@@ -819,6 +828,7 @@ int cat2amln_dev(sfb_plan *h, const double *rtp, const double *w, int64_t ngal, 
         const int64_t cp = wk == SFB_WINDOW_DENSE ? chunk_pairs(p) : 0;
         const bool joint = split && cp > 0 && cp >= p.npairs;
         const int64_t nb = p.nbasis, nm = nmock * nb + (mask_map ? 1 : 0) + (joint ? p.npairs : 0);
+        const PdlScope pdl(!split || nm * p.npix <= PDL_MAX);
         double *Cmap = nullptr, *mu = nullptr, *nu = nullptr, *smean = nullptr, *refsq = nullptr;
         const double *ralm = nullptr;             // FP64 a_lm of (C of every mock, W01), [lmsize][2 nmock + 2]
         if (split) {
@@ -1576,6 +1586,7 @@ int sfb_map2alm_adjoint(sfb_plan *h, const double *abar, int64_t nmaps, double *
     SFB_TRY(check_plan(h));
     SFB_TRY(set_device_of(h));
     if (nmaps <= 0 || !abar || !maps_out) return fail(SFB_EINVAL, "bad map2alm adjoint arguments");
+    const PdlScope pdl(true);
     Plan &p = h->p;
     cudaStream_t st = h->stream;
     // abar [nmaps][lmsize] complex (map2alm's output layout) -> [lmsize][2 nmaps] on the device
@@ -1600,6 +1611,7 @@ int sfb_cat2amln_vjp(sfb_plan *h, const double *rtp, int64_t ngal, double nbar, 
     SFB_TRY(set_device_of(h));
     if (ngal < 0 || (ngal > 0 && (!rtp || !dw_out)) || !abar) return fail(SFB_EINVAL, "bad cat2amln vjp arguments");
     if (!(std::isfinite(nbar) && nbar != 0.0)) return fail(SFB_ENONFINITE, "nbar must be finite and non-zero");
+    const PdlScope pdl(true);
     Plan &p = h->p;
     if (p.radial_mode != SFB_RADIAL_POLY)
         return fail(SFB_ENOTSUP, "the cat2amln adjoint needs the piecewise-polynomial radial basis (SFB_RADIAL_POLY)");
@@ -1662,6 +1674,7 @@ static int field2anlm_vjp_impl(sfb_plan *h, const double *abar, int64_t nr, doub
     SFB_TRY(set_device_of(h));
     if (!abar || !df_out || nr < 1 || !(rmin < rmax)) return fail(SFB_EINVAL, "bad field2anlm vjp arguments");
     if (dtype != SFB_F64 && dtype != SFB_F32) return fail(SFB_EINVAL, "unknown field dtype");
+    const PdlScope pdl(true);
     Plan &p = h->p;
     cudaStream_t st = h->stream;
     const double dr = (rmax - rmin) / (double)nr;
@@ -1722,6 +1735,7 @@ static int sfb_map2alm_impl(sfb_plan *h, const double *maps, int64_t nmaps, doub
     SFB_TRY(check_plan(h));
     SFB_TRY(set_device_of(h));
     if (nmaps <= 0 || !maps || !alm_out) return fail(SFB_EINVAL, "bad map2alm arguments");
+    const PdlScope pdl(true);
     Plan &p = h->p;
     cudaStream_t st = h->stream;
     SFB_TRY(grow(p, p.maps, (size_t)nmaps * p.npix));
@@ -1745,6 +1759,7 @@ static int sfb_field2anlm_impl(sfb_plan *h, const void *f, int32_t dtype, int64_
     SFB_TRY(set_device_of(h));
     if (!f || !anlm_out || nr < 1 || !(rmin < rmax)) return fail(SFB_EINVAL, "bad field2anlm arguments");
     if (dtype != SFB_F64 && dtype != SFB_F32) return fail(SFB_EINVAL, "unknown field dtype");
+    const PdlScope pdl(true);
     Plan &p = h->p;
     cudaStream_t st = h->stream;
     const double dr = (rmax - rmin) / (double)nr;
@@ -1803,6 +1818,7 @@ static int sfb_anlm2field_impl(sfb_plan *h, const double *anlm, int64_t nr, doub
     SFB_TRY(check_plan(h));
     SFB_TRY(set_device_of(h));
     if (!anlm || !f_out || nr < 1 || !(rmin < rmax)) return fail(SFB_EINVAL, "bad anlm2field arguments");
+    const PdlScope pdl(true);
     Plan &p = h->p;
     cudaStream_t st = h->stream;
     const double dr = (rmax - rmin) / (double)nr;

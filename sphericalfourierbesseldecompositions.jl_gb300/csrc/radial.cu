@@ -30,10 +30,11 @@ __device__ __forceinline__ bool galaxy_ok(double r, double th, double ph, double
 }
 
 // Spline mode: maps[q][pix] += w * g_{pair0+q}(r) / (nbar dOmega) for a chunk of pairs.
-__global__ void k_deposit_spline(const double *__restrict__ rtp, const double *__restrict__ wgt, int64_t ngal,
+__global__ void k_deposit_spline(const double *rtp, const double *wgt, int64_t ngal,
                                  int64_t nside, int64_t npix, const int64_t *spl_off, const double *sx,
                                  const double *sy, const double *sypp, int64_t pair0, int64_t npair_chunk,
-                                 double scale, double *__restrict__ maps, int *err) {
+                                 double scale, double *maps, int *err) {
+    pdl_entry();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= ngal) return;
     const double r = rtp[3 * i], th = rtp[3 * i + 1], ph = rtp[3 * i + 2];
@@ -53,14 +54,15 @@ void launch_deposit_spline_chunk(const Plan &p, const double *rtp, const double 
     if (ngal <= 0 || npc <= 0) return;
     unsigned gy = (unsigned)(npc < 64 ? npc : 64);
     dim3 grid((unsigned)((ngal + 255) / 256), gy);
-    k_deposit_spline<<<grid, 256, 0, st>>>(rtp, w, ngal, p.nside, p.npix, p.d_spl_off, p.d_spl_x, p.d_spl_y,
-                                           p.d_spl_ypp, pair0, npc, scale, maps, p.d_err);
-                                           note_launch();
+    launch_pdl(k_deposit_spline, dim3(grid), dim3(256), 0, st, rtp, w, ngal, p.nside, p.npix, p.d_spl_off, p.d_spl_x,
+        p.d_spl_y, p.d_spl_ypp, pair0, npc, scale, maps, p.d_err);
+    note_launch();
 }
 
 // maps[q][p] -= dense[p + npix*(l + (lmax+1)*(n-1))] for the chunk's pairs.
 __global__ void k_subtract_dense(double *maps, const double *dense, int64_t npix, int lmax, const int32_t *pair_n,
                                  const int32_t *pair_l, int64_t pair0, int64_t npc) {
+    pdl_entry();
     const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t q = blockIdx.y;
     if (p >= npix || q >= npc) return;
@@ -73,13 +75,15 @@ void launch_subtract_dense_chunk(const Plan &p, double *maps, const double *dens
                                  cudaStream_t st) {
     if (npc <= 0) return;
     dim3 grid((unsigned)((p.npix + 255) / 256), (unsigned)npc);
-    k_subtract_dense<<<grid, 256, 0, st>>>(maps, dense, p.npix, p.lmax, p.d_pair_n, p.d_pair_l, pair0, npc);
+    launch_pdl(k_subtract_dense, dim3(grid), dim3(256), 0, st, maps, dense, p.npix, p.lmax, p.d_pair_n, p.d_pair_l,
+        pair0, npc);
     note_launch();
 }
 
 // maps[q][p] -= mask[p] * W_ln[l + (lmax+1)(n-1)] for the chunk's pairs (separable window).
 __global__ void k_subtract_sep(double *maps, const double *mask, const double *w_ln, int64_t npix, int lmax,
                                const int32_t *pair_n, const int32_t *pair_l, int64_t pair0, int64_t npc) {
+    pdl_entry();
     const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t q = blockIdx.y;
     if (p >= npix || q >= npc) return;
@@ -92,11 +96,13 @@ void launch_subtract_sep_chunk(const Plan &p, double *maps, const double *mask, 
                                int64_t npc, cudaStream_t st) {
     if (npc <= 0) return;
     dim3 grid((unsigned)((p.npix + 255) / 256), (unsigned)npc);
-    k_subtract_sep<<<grid, 256, 0, st>>>(maps, mask, w_ln, p.npix, p.lmax, p.d_pair_n, p.d_pair_l, pair0, npc);
+    launch_pdl(k_subtract_sep, dim3(grid), dim3(256), 0, st, maps, mask, w_ln, p.npix, p.lmax, p.d_pair_n, p.d_pair_l,
+        pair0, npc);
     note_launch();
 }
 
 __global__ void k_axpy(double *y, const double *x, int64_t n) {
+    pdl_entry();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         y[i] += x[i];
 }
@@ -105,13 +111,14 @@ void launch_axpy(double *y, const double *x, int64_t n, cudaStream_t st) {
     if (n <= 0) return;
     int64_t blocks = (n + 255) / 256;
     if (blocks > 8192) blocks = 8192;
-    k_axpy<<<(unsigned)blocks, 256, 0, st>>>(y, x, n);
+    launch_pdl(k_axpy, dim3((unsigned)blocks), dim3(256), 0, st, y, x, n);
     note_launch();
 }
 
 // Gather dense window maps of a chunk of pairs: maps[q] = W[:, l, n].
 __global__ void k_gather_dense(double *maps, const double *dense, int64_t npix, int lmax, const int32_t *pair_n,
                                const int32_t *pair_l, int64_t pair0, int64_t npc) {
+    pdl_entry();
     const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t q = blockIdx.y;
     if (p >= npix || q >= npc) return;
@@ -124,7 +131,8 @@ void launch_gather_dense_chunk(const Plan &p, double *maps, const double *dense,
                                cudaStream_t st) {
     if (npc <= 0) return;
     dim3 grid((unsigned)((p.npix + 255) / 256), (unsigned)npc);
-    k_gather_dense<<<grid, 256, 0, st>>>(maps, dense, p.npix, p.lmax, p.d_pair_n, p.d_pair_l, pair0, npc);
+    launch_pdl(k_gather_dense, dim3(grid), dim3(256), 0, st, maps, dense, p.npix, p.lmax, p.d_pair_n, p.d_pair_l,
+        pair0, npc);
     note_launch();
 }
 
@@ -135,6 +143,7 @@ void launch_gather_dense_chunk(const Plan &p, double *maps, const double *dense,
 __global__ void k_radial_coeffs(const int64_t *spl_off, const double *sx, const double *sy, const double *sypp,
                                 double rmin, double rmax, int pieces, int deg, int64_t nbasis, const double *glx,
                                 const double *pq, int Q, double *coef) {
+    pdl_entry();
     extern __shared__ double gq[];
     const int64_t pr = blockIdx.x;
     const int j = blockIdx.y;
@@ -160,9 +169,9 @@ __global__ void k_radial_coeffs(const int64_t *spl_off, const double *sx, const 
 void launch_radial_coeffs(const Plan &p, const double *gl_x, const double *pq, int Q, double *coef,
                           cudaStream_t st) {
     dim3 grid((unsigned)p.npairs, (unsigned)p.pieces);
-    k_radial_coeffs<<<grid, 128, Q * sizeof(double), st>>>(p.d_spl_off, p.d_spl_x, p.d_spl_y, p.d_spl_ypp, p.rmin,
-                                                          p.rmax, p.pieces, p.degree, p.nbasis, gl_x, pq, Q, coef);
-                                                          note_launch();
+    launch_pdl(k_radial_coeffs, dim3(grid), dim3(128), Q * sizeof(double), st, p.d_spl_off, p.d_spl_x, p.d_spl_y,
+        p.d_spl_ypp, p.rmin, p.rmax, p.pieces, p.degree, p.nbasis, gl_x, pq, Q, coef);
+    note_launch();
 }
 
 // max over knots of |expansion - y| / max|y| per pair; atomicMax on the bit
@@ -170,6 +179,7 @@ void launch_radial_coeffs(const Plan &p, const double *gl_x, const double *pq, i
 __global__ void k_radial_error(const int64_t *spl_off, const double *sx, const double *sy, const double *ymax,
                                double rmin, double rmax, int pieces, int deg, int64_t nbasis, const double *coef,
                                unsigned long long *err_bits) {
+    pdl_entry();
     const int64_t pr = blockIdx.x;
     const int64_t o = spl_off[pr], N = spl_off[pr + 1] - o;
     const double width = (rmax - rmin) / pieces;
@@ -201,17 +211,18 @@ __global__ void k_radial_error(const int64_t *spl_off, const double *sx, const d
 
 void launch_radial_error_impl(const Plan &p, const double *coef, const double *ymax, unsigned long long *err_bits,
                               cudaStream_t st) {
-    k_radial_error<<<(unsigned)p.npairs, 128, 0, st>>>(p.d_spl_off, p.d_spl_x, p.d_spl_y, ymax, p.rmin, p.rmax,
-                                                       p.pieces, p.degree, p.nbasis, coef, err_bits);
-                                                       note_launch();
+    launch_pdl(k_radial_error, dim3((unsigned)p.npairs), dim3(128), 0, st, p.d_spl_off, p.d_spl_x, p.d_spl_y, ymax,
+        p.rmin, p.rmax, p.pieces, p.degree, p.nbasis, coef, err_bits);
+    note_launch();
 }
 
 // a_nlm = scale * sum_b C[pair][b] A[lm][b] - window term.
 template <typename TA>
 __global__ void k_project_poly(const int32_t *out_pair, const int32_t *out_lm, const int32_t *pair_n,
                                const int32_t *pair_l, int64_t nlmsize, int64_t nbasis, const double *coef,
-                               const TA *__restrict__ A, int64_t ldA, double scale, int window_kind,
+                               const TA *A, int64_t ldA, double scale, int window_kind,
                                const double *w_ln, int lmax, int64_t mask_col, double *out) {
+    pdl_entry();
     const int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (o >= nlmsize) return;
     const int pr = out_pair[o];
@@ -241,7 +252,7 @@ void launch_project_poly(const Plan &p, const double *A, int64_t ldA, double sca
     (void)Awin; (void)ldW;
     if (p.nlmsize <= 0) return;
     // a_lm are held in FP64 in both precision modes
-    k_project_poly<double><<<(unsigned)((p.nlmsize + 127) / 128), 128, 0, st>>>(
+    launch_pdl(k_project_poly<double>, dim3((unsigned)((p.nlmsize + 127) / 128)), dim3(128), 0, st,
             p.d_out_pair, p.d_out_lm, p.d_pair_n, p.d_pair_l, p.nlmsize, p.nbasis, p.d_coef, A, ldA, scale,
             window_kind, w_ln, p.lmax, mask_col, out);
         note_launch();
@@ -250,6 +261,7 @@ void launch_project_poly(const Plan &p, const double *A, int64_t ldA, double sca
 // out[o] -= Awin[lm][pair - pair0] for outputs whose pair lies in the chunk.
 __global__ void k_sub_window_chunk(const int32_t *out_pair, const int32_t *out_lm, int64_t nlmsize,
                                    const double *Awin, int64_t ldW, int64_t pair0, int64_t npc, double *out) {
+    pdl_entry();
     const int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (o >= nlmsize) return;
     const int64_t q = (int64_t)out_pair[o] - pair0;
@@ -262,14 +274,15 @@ __global__ void k_sub_window_chunk(const int32_t *out_pair, const int32_t *out_l
 void launch_sub_window_chunk(const Plan &p, const double *Awin, int64_t ldW, int64_t pair0, int64_t npc, double *out,
                              cudaStream_t st) {
     if (p.nlmsize <= 0) return;
-    k_sub_window_chunk<<<(unsigned)((p.nlmsize + 127) / 128), 128, 0, st>>>(p.d_out_pair, p.d_out_lm, p.nlmsize, Awin,
-                                                                           ldW, pair0, npc, out);
-                                                                           note_launch();
+    launch_pdl(k_sub_window_chunk, dim3((unsigned)((p.nlmsize + 127) / 128)), dim3(128), 0, st, p.d_out_pair,
+        p.d_out_lm, p.nlmsize, Awin, ldW, pair0, npc, out);
+    note_launch();
 }
 
 // Spline mode: out[o] = A[lm][pair - pair0] (map already scaled and window-subtracted).
 __global__ void k_extract_spline(const int32_t *out_pair, const int32_t *out_lm, int64_t nlmsize, const double *A,
                                  int64_t ldA, int64_t pair0, int64_t npc, double *out) {
+    pdl_entry();
     const int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (o >= nlmsize) return;
     const int64_t q = (int64_t)out_pair[o] - pair0;
@@ -282,14 +295,15 @@ __global__ void k_extract_spline(const int32_t *out_pair, const int32_t *out_lm,
 void launch_extract_spline_chunk(const Plan &p, const double *A, int64_t ldA, int64_t pair0, int64_t npc, double *out,
                                  cudaStream_t st) {
     if (p.nlmsize <= 0) return;
-    k_extract_spline<<<(unsigned)((p.nlmsize + 127) / 128), 128, 0, st>>>(p.d_out_pair, p.d_out_lm, p.nlmsize, A, ldA,
-                                                                         pair0, npc, out);
-                                                                         note_launch();
+    launch_pdl(k_extract_spline, dim3((unsigned)((p.nlmsize + 127) / 128)), dim3(128), 0, st, p.d_out_pair,
+        p.d_out_lm, p.nlmsize, A, ldA, pair0, npc, out);
+    note_launch();
 }
 
 // gtab[pair][s] = g_pair(r_s) * (with_r2dr ? r_s^2 dr : 1), r_s = rmin + (s+1/2) dr.
 __global__ void k_gtab(const int64_t *spl_off, const double *sx, const double *sy, const double *sypp,
                        int64_t npairs, int64_t nr, double rmin, double dr, int with_r2dr, double *gtab) {
+    pdl_entry();
     const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= nr) return;
     const double r = rmin + dr / 2 + s * dr;
@@ -303,14 +317,15 @@ __global__ void k_gtab(const int64_t *spl_off, const double *sx, const double *s
 
 void launch_gtab(const Plan &p, int64_t nr, double rmin, double dr, int with_r2dr, double *gtab, cudaStream_t st) {
     dim3 grid((unsigned)((nr + 127) / 128), (unsigned)std::min<int64_t>(p.npairs, 65535));
-    k_gtab<<<grid, 128, 0, st>>>(p.d_spl_off, p.d_spl_x, p.d_spl_y, p.d_spl_ypp, p.npairs, nr, rmin, dr, with_r2dr,
-                                 gtab);
+    launch_pdl(k_gtab, dim3(grid), dim3(128), 0, st, p.d_spl_off, p.d_spl_x, p.d_spl_y, p.d_spl_ypp, p.npairs, nr,
+        rmin, dr, with_r2dr, gtab);
                                  note_launch();
 }
 
 // field2anlm radial sum: out[o] = sum_s gtab[pair][s] A[lm][s]  (src/cat2anlm.jl:347-353)
 __global__ void k_project_shells(const int32_t *out_pair, const int32_t *out_lm, int64_t nlmsize, const double *gtab,
-                                 int64_t nr, const double *__restrict__ A, int64_t ldA, double *out) {
+                                 int64_t nr, const double *A, int64_t ldA, double *out) {
+    pdl_entry();
     const int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (o >= nlmsize) return;
     const double *g = gtab + (int64_t)out_pair[o] * nr;
@@ -327,14 +342,15 @@ __global__ void k_project_shells(const int32_t *out_pair, const int32_t *out_lm,
 void launch_project_shells_g(const Plan &p, const double *gtab, int64_t nr, const double *A, int64_t ldA, double *out,
                              cudaStream_t st) {
     if (p.nlmsize <= 0) return;
-    k_project_shells<<<(unsigned)((p.nlmsize + 127) / 128), 128, 0, st>>>(p.d_out_pair, p.d_out_lm, p.nlmsize, gtab, nr,
-                                                                         A, ldA, out);
-                                                                         note_launch();
+    launch_pdl(k_project_shells, dim3((unsigned)((p.nlmsize + 127) / 128)), dim3(128), 0, st, p.d_out_pair,
+        p.d_out_lm, p.nlmsize, gtab, nr, A, ldA, out);
+    note_launch();
 }
 
 // anlm2field radial sum: A[lm][s] = sum_n gtab[pair(n,l)][s] a[idx(n,l,m)] (src/cat2anlm.jl:403-414)
 __global__ void k_shell_alm(const int32_t *pair_index, const int64_t *noff, int nmax, int lmax, const double *gtab,
                             int64_t nr, const double *anlm, double *A, int64_t ldA) {
+    pdl_entry();
     const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= nr) return;
     const int64_t lmsize = (int64_t)(lmax + 1) * (lmax + 2) / 2;
@@ -361,13 +377,14 @@ __global__ void k_shell_alm(const int32_t *pair_index, const int64_t *noff, int 
 void launch_shell_alm_g(const Plan &p, const int32_t *pair_index, const int64_t *noff, const double *gtab, int64_t nr,
                         const double *anlm, double *A, int64_t ldA, cudaStream_t st) {
     dim3 grid((unsigned)((nr + 127) / 128), (unsigned)std::min<int64_t>(p.lmsize, 65535));
-    k_shell_alm<<<grid, 128, 0, st>>>(pair_index, noff, p.nmax, p.lmax, gtab, nr, anlm, A, ldA);
+    launch_pdl(k_shell_alm, dim3(grid), dim3(128), 0, st, pair_index, noff, p.nmax, p.lmax, gtab, nr, anlm, A, ldA);
     note_launch();
 }
 
 // W_ln[l + (lmax+1)(n-1)] = sum_s gtab[pair][s] phi[s]  (gtab includes r^2 dr); NaN off-mode.
 __global__ void k_win_sep(const int32_t *pair_n, const int32_t *pair_l, int64_t npairs, const double *gtab, int64_t nr,
                           const double *phi, int lmax, double *out) {
+    pdl_entry();
     const int64_t pr = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (pr >= npairs) return;
     double acc = 0.0;
@@ -376,14 +393,15 @@ __global__ void k_win_sep(const int32_t *pair_n, const int32_t *pair_l, int64_t 
 }
 
 void launch_win_sep_g(const Plan &p, const double *gtab, int64_t nr, const double *phi, double *out, cudaStream_t st) {
-    k_win_sep<<<(unsigned)((p.npairs + 127) / 128), 128, 0, st>>>(p.d_pair_n, p.d_pair_l, p.npairs, gtab, nr, phi,
-                                                                  p.lmax, out);
-                                                                  note_launch();
+    launch_pdl(k_win_sep, dim3((unsigned)((p.npairs + 127) / 128)), dim3(128), 0, st, p.d_pair_n, p.d_pair_l,
+        p.npairs, gtab, nr, phi, p.lmax, out);
+    note_launch();
 }
 
 // Dense: W[p + npix(l + (lmax+1)(n-1))] = sum_s win[s + nr p] gtab[pair][s]
 __global__ void k_win_dense(const int32_t *pair_n, const int32_t *pair_l, int64_t npairs, const double *gtab, int64_t nr,
                             const double *win, int64_t npix, int lmax, double *out) {
+    pdl_entry();
     const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= npix) return;
     const double *wc = win + p * nr;
@@ -397,16 +415,18 @@ __global__ void k_win_dense(const int32_t *pair_n, const int32_t *pair_l, int64_
 
 void launch_win_dense_g(const Plan &p, const double *gtab, int64_t nr, const double *win, double *out, cudaStream_t st) {
     dim3 grid((unsigned)((p.npix + 127) / 128), (unsigned)std::min<int64_t>(p.npairs, 65535));
-    k_win_dense<<<grid, 128, 0, st>>>(p.d_pair_n, p.d_pair_l, p.npairs, gtab, nr, win, p.npix, p.lmax, out);
+    launch_pdl(k_win_dense, dim3(grid), dim3(128), 0, st, p.d_pair_n, p.d_pair_l, p.npairs, gtab, nr, win, p.npix,
+        p.lmax, out);
     note_launch();
 }
 
 // amln2clnn (src/SphericalFourierBesselDecompositions.jl:114-150): one warp per
 // (l, n1, n2) column of lnn (3 x nlnn, 1-based n), over nbatch coefficient vectors:
 // C = [Re(a1_0 a2_0) + 2 sum_{m>=1} Re(a1_m conj(a2_m))] / (2l + 1).
-__global__ void k_amln2clnn(const double *__restrict__ a1, const double *__restrict__ a2, int64_t nlmsize,
-                            const int64_t *__restrict__ lnn, int64_t nlnn, int64_t nbatch, const int64_t *noff,
-                            double *__restrict__ out) {
+__global__ void k_amln2clnn(const double *a1, const double *a2, int64_t nlmsize,
+                            const int64_t *lnn, int64_t nlnn, int64_t nbatch, const int64_t *noff,
+                            double *out) {
+    pdl_entry();
     const int64_t wid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (wid >= nlnn * nbatch) return;
@@ -427,16 +447,18 @@ void launch_amln2clnn(const double *a1, const double *a2, int64_t nlmsize, const
                       int64_t nbatch, const int64_t *noff, double *out, cudaStream_t st) {
     const int64_t threads = nlnn * nbatch * 32;
     if (threads <= 0) return;
-    k_amln2clnn<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(a1, a2, nlmsize, lnn, nlnn, nbatch, noff, out);
+    launch_pdl(k_amln2clnn, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0, st, a1, a2, nlmsize, lnn, nlnn,
+        nbatch, noff, out);
     note_launch();
 }
 
 // winweights2galweights (src/cat2anlm.jl:218-238): w_i = weights[bin(r_i), pix(theta_i, phi_i)]
 // with bin = nr if r == rmax, else searchsortedlast(rbounds, r) (1-based), over
 // the caller's rbounds[0..nr].  Out-of-range bins set ERR_RANGE_R and give NaN.
-__global__ void k_winweights(const double *__restrict__ weights, int64_t nr, int64_t npix, int64_t nside,
-                             const double *__restrict__ rbounds, double rmax, const double *__restrict__ rtp,
-                             int64_t ngal, double *__restrict__ w, int *err) {
+__global__ void k_winweights(const double *weights, int64_t nr, int64_t npix, int64_t nside,
+                             const double *rbounds, double rmax, const double *rtp,
+                             int64_t ngal, double *w, int *err) {
+    pdl_entry();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= ngal) return;
     const double r = rtp[3 * i], th = rtp[3 * i + 1], ph = rtp[3 * i + 2];
@@ -469,8 +491,8 @@ __global__ void k_winweights(const double *__restrict__ weights, int64_t nr, int
 void launch_winweights(const double *weights, int64_t nr, int64_t nside, const double *rbounds, double rmax,
                        const double *rtp, int64_t ngal, double *w, int *err, cudaStream_t st) {
     if (ngal <= 0) return;
-    k_winweights<<<(unsigned)((ngal + 255) / 256), 256, 0, st>>>(weights, nr, 12 * nside * nside, nside, rbounds, rmax,
-                                                                 rtp, ngal, w, err);
+    launch_pdl(k_winweights, dim3((unsigned)((ngal + 255) / 256)), dim3(256), 0, st, weights, nr, 12 * nside * nside,
+        nside, rbounds, rmax, rtp, ngal, w, err);
     note_launch();
 }
 
@@ -495,8 +517,9 @@ __device__ __forceinline__ df2 dfm(df2 a, df2 b) {
 }
 
 // CT[(l * nbasis + b) * nmax + n - 1] = coef[pair(n, l)][b] as hi + lo (0 where (n, l) is not a mode).
-__global__ void k_coef_df(const double *__restrict__ coef, const int32_t *__restrict__ pair_index, int lmax, int nmax,
-                          int64_t nbasis, float2 *__restrict__ CT) {
+__global__ void k_coef_df(const double *coef, const int32_t *pair_index, int lmax, int nmax,
+                          int64_t nbasis, float2 *CT) {
+    pdl_entry();
     const int64_t total = (int64_t)(lmax + 1) * nbasis * nmax;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
         const int n1 = (int)(i % nmax);
@@ -511,15 +534,16 @@ __global__ void k_coef_df(const double *__restrict__ coef, const int32_t *__rest
 }
 
 void launch_coef_df(const Plan &p, const int32_t *pair_index, float2 *CT, cudaStream_t st) {
-    k_coef_df<<<1024, 256, 0, st>>>(p.d_coef, pair_index, p.lmax, (int)p.nmax, p.nbasis, CT);
+    launch_pdl(k_coef_df, dim3(1024), dim3(256), 0, st, p.d_coef, pair_index, p.lmax, (int)p.nmax, p.nbasis, CT);
     note_launch();
 }
 
 // s[pair] = sum_b coef[pair][b] mu_b (FP64): the mean part of every pair, one
 // warp per pair (lanes over b, coalesced rows).
 // (grid.y: mocks, their mu and s one after another)
-__global__ void k_mean_proj(const double *__restrict__ coef, int64_t npairs, int64_t nbasis,
-                            const double *__restrict__ mu, double *__restrict__ s) {
+__global__ void k_mean_proj(const double *coef, int64_t npairs, int64_t nbasis,
+                            const double *mu, double *s) {
+    pdl_entry();
     mu += blockIdx.y * nbasis;
     s += blockIdx.y * npairs;
     const int64_t pr = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -567,16 +591,17 @@ struct Scales {
 
 // grid.y: mocks (launch_project_mixed says where each one's data lie)
 template <int KS>
-__global__ void __launch_bounds__(32 * KS) k_project_mixed(const float2 *__restrict__ Adf, int64_t ldA,
-                                                              int64_t nbasis, const float2 *__restrict__ CT, int nmax,
-                                                              int lmax, const int3 *__restrict__ tiles,
-                                                              const int64_t *__restrict__ noff,
-                                                              const int32_t *__restrict__ pair_index, Scales scales,
-                                                              const double *__restrict__ smean, int64_t npairs,
-                                                              const double *__restrict__ ralm, int64_t ldR,
+__global__ void __launch_bounds__(32 * KS) k_project_mixed(const float2 *Adf, int64_t ldA,
+                                                              int64_t nbasis, const float2 *CT, int nmax,
+                                                              int lmax, const int3 *tiles,
+                                                              const int64_t *noff,
+                                                              const int32_t *pair_index, Scales scales,
+                                                              const double *smean, int64_t npairs,
+                                                              const double *ralm, int64_t ldR,
                                                               int64_t nlmsize, int window_kind,
-                                                              const double *__restrict__ w_ln,
-                                                              double *__restrict__ out, int *err) {
+                                                              const double *w_ln,
+                                                              double *out, int *err) {
+    pdl_entry();
     __shared__ float4 part[KS - 1][PJ_NPT][32];
     const int mock = blockIdx.y;
     const double scale = scales.v[mock];
@@ -665,8 +690,8 @@ std::vector<int3> project_tiles(const std::vector<int32_t> &pair_index, int lmax
 }
 
 void launch_mean_proj(const Plan &p, const double *mu, int nmock, double *smean, cudaStream_t st) {
-    k_mean_proj<<<dim3((unsigned)((p.npairs + 3) / 4), (unsigned)nmock), 128, 0, st>>>(p.d_coef, p.npairs, p.nbasis, mu,
-                                                                                     smean);
+    launch_pdl(k_mean_proj, dim3((unsigned)((p.npairs + 3) / 4), (unsigned)nmock), dim3(128), 0, st, p.d_coef,
+        p.npairs, p.nbasis, mu, smean);
     note_launch();
 }
 
@@ -677,14 +702,15 @@ void launch_project_mixed(const Plan &p, const float2 *Adf, int64_t ldA, const f
     if (p.n_proj_tiles <= 0) return;
     Scales sc;
     std::copy(scale, scale + nmock, sc.v);
-    k_project_mixed<PJ_KS><<<dim3((unsigned)p.n_proj_tiles, (unsigned)nmock), 32 * PJ_KS, 0, st>>>(
+    launch_pdl(k_project_mixed<PJ_KS>, dim3((unsigned)p.n_proj_tiles, (unsigned)nmock), dim3(32 * PJ_KS), 0, st,
         Adf, ldA, p.nbasis, CT, (int)p.nmax, p.lmax, p.d_proj_tiles, noff, pair_index, sc, smean, p.npairs, ralm, ldR,
         p.nlmsize, window_kind, w_ln, out, err);
     note_launch();
 }
 
 // <ref, ref> of one map, by one block
-__global__ void __launch_bounds__(1024) k_ref_square(const double *__restrict__ ref, int64_t npix, double *refsq) {
+__global__ void __launch_bounds__(1024) k_ref_square(const double *ref, int64_t npix, double *refsq) {
+    pdl_entry();
     __shared__ double red[32];
     double q = 0.0;
 #pragma unroll 4
@@ -699,7 +725,7 @@ __global__ void __launch_bounds__(1024) k_ref_square(const double *__restrict__ 
 }
 
 void launch_ref_square(const double *ref, int64_t npix, double *refsq, cudaStream_t st) {
-    k_ref_square<<<1, 1024, 0, st>>>(ref, npix, refsq);
+    launch_pdl(k_ref_square, dim3(1), dim3(1024), 0, st, ref, npix, refsq);
     note_launch();
 }
 
@@ -707,12 +733,13 @@ void launch_ref_square(const double *ref, int64_t npix, double *refsq, cudaStrea
 // split by integer operations).  The window map is read where the caller's array has it, the second time from L2,
 // and written once.  Bound: the FP64 pipe (two operations a pixel) beside HBM (16 bytes); as a gather, an in-place
 // split with three FP64 operations and a conversion pass it took 446 us for 507 maps of nside 64.
-__global__ void __launch_bounds__(512) k_dense_maps_df(const double *__restrict__ dense, int64_t npix, int lmax,
-                                                       const int32_t *__restrict__ pair_n,
-                                                       const int32_t *__restrict__ pair_l, int64_t pair0,
-                                                       const double *__restrict__ ref,
-                                                       const double *__restrict__ refsq, double *__restrict__ nu,
-                                                       float2 *__restrict__ maps) {
+__global__ void __launch_bounds__(512) k_dense_maps_df(const double *dense, int64_t npix, int lmax,
+                                                       const int32_t *pair_n,
+                                                       const int32_t *pair_l, int64_t pair0,
+                                                       const double *ref,
+                                                       const double *refsq, double *nu,
+                                                       float2 *maps) {
+    pdl_entry();
     __shared__ double red[16];
     const int64_t pr = pair0 + blockIdx.x;
     const double *W = dense + npix * ((int64_t)pair_l[pr] + (int64_t)(lmax + 1) * (pair_n[pr] - 1));
@@ -742,17 +769,18 @@ __global__ void __launch_bounds__(512) k_dense_maps_df(const double *__restrict_
 void launch_dense_maps_df(const Plan &p, const double *dense, const double *ref, const double *refsq, int64_t pair0,
                           int64_t npc, double *nu, float2 *maps, cudaStream_t st) {
     if (npc <= 0) return;
-    k_dense_maps_df<<<(unsigned)npc, 512, 0, st>>>(dense, p.npix, p.lmax, p.d_pair_n, p.d_pair_l, pair0, ref, refsq, nu,
-                                                   maps);
+    launch_pdl(k_dense_maps_df, dim3((unsigned)npc), dim3(512), 0, st, dense, p.npix, p.lmax, p.d_pair_n, p.d_pair_l,
+        pair0, ref, refsq, nu, maps);
     note_launch();
 }
 
 // The window's part of every coefficient of the chunk's pairs, from the double-float a_lm (the rows l of pair (n,
 // l) only) and the reference map's FP64 ones.
-__global__ void k_sub_window_df(const int32_t *__restrict__ out_pair, const int32_t *__restrict__ out_lm,
-                                int64_t nlmsize, const float2 *__restrict__ Adf, int64_t ldA, int64_t pair0, int64_t npc,
-                                const double *__restrict__ nu, const double *__restrict__ rref, int64_t ldR,
-                                double *__restrict__ out, int *err) {
+__global__ void k_sub_window_df(const int32_t *out_pair, const int32_t *out_lm,
+                                int64_t nlmsize, const float2 *Adf, int64_t ldA, int64_t pair0, int64_t npc,
+                                const double *nu, const double *rref, int64_t ldR,
+                                double *out, int *err) {
+    pdl_entry();
     const int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (o >= nlmsize) return;
     const int64_t q = (int64_t)out_pair[o] - pair0;
@@ -769,12 +797,13 @@ __global__ void k_sub_window_df(const int32_t *__restrict__ out_pair, const int3
 
 void launch_sub_window_df(const Plan &p, const float2 *Adf, int64_t ldA, int64_t pair0, int64_t npc, const double *nu,
                           const double *rref, int64_t ldR, double *out, int *err, cudaStream_t st) {
-    k_sub_window_df<<<(unsigned)((p.nlmsize + 127) / 128), 128, 0, st>>>(p.d_out_pair, p.d_out_lm, p.nlmsize, Adf, ldA,
-                                                                        pair0, npc, nu, rref, ldR, out, err);
+    launch_pdl(k_sub_window_df, dim3((unsigned)((p.nlmsize + 127) / 128)), dim3(128), 0, st, p.d_out_pair, p.d_out_lm,
+        p.nlmsize, Adf, ldA, pair0, npc, nu, rref, ldR, out, err);
     note_launch();
 }
 
 __global__ void k_fill(double *x, int64_t n, double v) {
+    pdl_entry();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         x[i] = v;
 }
@@ -783,7 +812,7 @@ void launch_fill(double *x, int64_t n, double v, cudaStream_t st) {
     if (n <= 0) return;
     int64_t blocks = (n + 255) / 256;
     if (blocks > 8192) blocks = 8192;
-    k_fill<<<(unsigned)blocks, 256, 0, st>>>(x, n, v);
+    launch_pdl(k_fill, dim3((unsigned)blocks), dim3(256), 0, st, x, n, v);
     note_launch();
 }
 
@@ -793,22 +822,24 @@ namespace sfb {
 
 // w00[s] = Re a_00 of map s of an FP64 a_lm set (row lm = 0, columns 2 s / 2 s + 1)
 __global__ void k_extract_a00(const double *alm, int64_t nm, double *w00) {
+    pdl_entry();
     const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (s < nm) w00[s] = alm[2 * s];
 }
 
 void launch_extract_a00(const double *alm, int64_t ldA, int64_t nm, double *w00, cudaStream_t st) {
     (void)ldA;
-    k_extract_a00<<<(unsigned)((nm + 127) / 128), 128, 0, st>>>(alm, nm, w00);
+    launch_pdl(k_extract_a00, dim3((unsigned)((nm + 127) / 128)), dim3(128), 0, st, alm, nm, w00);
     note_launch();
 }
 
 // win_lnn radial integrals (reference calc_intr_gg_fn, src/windows.jl:394-422, trapezoidal
 // nodes = shell midpoints, weights = dr, f = W00 / sqrt(4 pi)): one warp per column i of lnn,
 //   out[i] = sum_s (g_nl(r_s) r_s sqrt(dr) sqrt(f_s)) (g_n'l(r_s) r_s sqrt(dr) sqrt(f_s)).
-__global__ void k_win_lnn(const int32_t *__restrict__ pair_index, int lmax, const double *__restrict__ gtab,
-                          int64_t nr, double rmin, double dr, const double *__restrict__ w00,
-                          const int64_t *__restrict__ lnn, int64_t nlnn, double *__restrict__ out) {
+__global__ void k_win_lnn(const int32_t *pair_index, int lmax, const double *gtab,
+                          int64_t nr, double rmin, double dr, const double *w00,
+                          const int64_t *lnn, int64_t nlnn, double *out) {
+    pdl_entry();
     const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (i >= nlnn) return;
@@ -828,8 +859,8 @@ __global__ void k_win_lnn(const int32_t *__restrict__ pair_index, int lmax, cons
 
 void launch_win_lnn(const Plan &p, const int32_t *pair_index, const double *gtab, int64_t nr, double rmin, double dr,
                     const double *w00, const int64_t *lnn, int64_t nlnn, double *out, cudaStream_t st) {
-    k_win_lnn<<<(unsigned)((nlnn * 32 + 127) / 128), 128, 0, st>>>(pair_index, p.lmax, gtab, nr, rmin, dr, w00, lnn,
-                                                                    nlnn, out);
+    launch_pdl(k_win_lnn, dim3((unsigned)((nlnn * 32 + 127) / 128)), dim3(128), 0, st, pair_index, p.lmax, gtab, nr,
+        rmin, dr, w00, lnn, nlnn, out);
     note_launch();
 }
 

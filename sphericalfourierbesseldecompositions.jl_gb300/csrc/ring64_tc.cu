@@ -68,10 +68,11 @@ __device__ __forceinline__ int64_t fixed53(double x, int emax) {
 // Folded sums of a ring pair: one warp per map.  Q[ring][combination][parity nm + map][kp], ex[ring][map] the
 // exponent field of the pair's largest magnitude (0: the pair is zero and its Q not written; 2047: not finite).
 // Two passes over the pair's pixels, the second from L1.  Bound: 8 bytes read and about 9 written a pixel.
-__global__ void __launch_bounds__(256) k_fold64(const RingGeom *__restrict__ rings, int ns, int64_t npix,
-                                                const double *__restrict__ maps, int64_t nm,
-                                                const int64_t *__restrict__ qoff, int64_t *__restrict__ Q,
-                                                int *__restrict__ ex, int *nzr, int z0) {
+__global__ void __launch_bounds__(256) k_fold64(const RingGeom *rings, int ns, int64_t npix,
+                                                const double *maps, int64_t nm,
+                                                const int64_t *qoff, int64_t *Q,
+                                                int *ex, int *nzr, int z0) {
+    pdl_entry();
     const int r = ring_at(z0 + blockIdx.y, ns), lane = threadIdx.x & 31;
     const int64_t b = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (b >= nm) return;
@@ -128,11 +129,12 @@ __global__ void __launch_bounds__(256) k_fold64(const RingGeom *__restrict__ rin
 
 // F of 128 rows (parity nm + map) x one tile of 32 frequencies of one combination and ring.
 // Bound: MMA issue (about 450 cycles a chunk and tile) beside forming the digits (about 350).
-__global__ void __launch_bounds__(NTH, 2) k_rdft64(const RingGeom *__restrict__ rings, int ns, int lmax, int64_t nm,
-                                                   const int64_t *__restrict__ qoff, const int64_t *__restrict__ Q,
-                                                   const int *__restrict__ ex, const uint16_t *__restrict__ dig,
-                                                   const int64_t *__restrict__ off, int Ew, double *__restrict__ F,
+__global__ void __launch_bounds__(NTH, 2) k_rdft64(const RingGeom *rings, int ns, int lmax, int64_t nm,
+                                                   const int64_t *qoff, const int64_t *Q,
+                                                   const int *ex, const uint16_t *dig,
+                                                   const int64_t *off, int Ew, double *F,
                                                    int z0, int *err) {
+    pdl_entry();
     extern __shared__ __align__(1024) unsigned char smem[];
     const int r = ring_at(z0 + blockIdx.z, ns), cb = blockIdx.y & 3, tile = blockIdx.y >> 2;
     const int e = cb & 1, isS = cb >> 1;
@@ -229,11 +231,12 @@ __global__ void __launch_bounds__(NTH, 2) k_rdft64(const RingGeom *__restrict__ 
 // Y[ring][combination][row][kp] += the integers of sum_m c_m G_m cos / sin, shifted right by sh, on the unit of
 // gex[ring][combination][row] (the exponent field of the row's largest coefficient).
 // Bound: forming the integers (about 45 operations an output) beside the MMAs.
-__global__ void __launch_bounds__(NTH, 2) k_rsyn64(const RingGeom *__restrict__ rings, int ns, int lmax, int64_t nm,
-                                                   const double *__restrict__ G, const uint16_t *__restrict__ dig,
-                                                   const int64_t *__restrict__ off, const int64_t *__restrict__ qoff,
-                                                   int64_t *__restrict__ Y, int *__restrict__ gex, int kbmax, int sh,
+__global__ void __launch_bounds__(NTH, 2) k_rsyn64(const RingGeom *rings, int ns, int lmax, int64_t nm,
+                                                   const double *G, const uint16_t *dig,
+                                                   const int64_t *off, const int64_t *qoff,
+                                                   int64_t *Y, int *gex, int kbmax, int sh,
                                                    int z0, int *err) {
+    pdl_entry();
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ uint32_t red[2][MTILE];
     __shared__ __align__(8) uint64_t bars[2];
@@ -383,10 +386,11 @@ __global__ void __launch_bounds__(NTH, 2) k_rsyn64(const RingGeom *__restrict__ 
 // The pixels of ring pair r: one thread per map and four j.  PIXMAJOR: out[pix ld + map] (lanes over maps),
 // else out[map ld + pix] (lanes over j).
 template <typename T, bool PIXMAJOR>
-__global__ void __launch_bounds__(256) k_unfold64(const RingGeom *__restrict__ rings, int ns, int64_t nm,
-                                                  const int64_t *__restrict__ qoff, const int64_t *__restrict__ Y,
-                                                  const int *__restrict__ gex, int sh, T *__restrict__ out,
+__global__ void __launch_bounds__(256) k_unfold64(const RingGeom *rings, int ns, int64_t nm,
+                                                  const int64_t *qoff, const int64_t *Y,
+                                                  const int *gex, int sh, T *out,
                                                   int64_t ld, int z0) {
+    pdl_entry();
     const int r = ring_at(z0 + blockIdx.z, ns);
     const RingGeom g = rings[r];
     const Ring R = ring_of(g, r, ns);
@@ -466,8 +470,9 @@ __device__ __forceinline__ double trig(int64_t t, int n, bool sine) {
 // Table of class cls and combination cb: SYN: rows n = j, columns k = coefficient m = e + 2 k (half weight for
 // m = 0); else rows n = frequency e + 2 n, columns k = j, times wm (the quadrature weight's significand).
 template <bool SYN>
-__global__ void __launch_bounds__(256) k_ring_tab(const RingGeom *__restrict__ rings, int ns, int lmax, double wm,
-                                                  const int64_t *__restrict__ off, uint16_t *__restrict__ dig) {
+__global__ void __launch_bounds__(256) k_ring_tab(const RingGeom *rings, int ns, int lmax, double wm,
+                                                  const int64_t *off, uint16_t *dig) {
+    pdl_entry();
     const int cls = blockIdx.z, cb = blockIdx.y, e = cb & 1;
     const bool sine = cb >> 1;
     int r = cls;
@@ -558,8 +563,10 @@ static bool ensure_ring64(Plan &p, int dir, cudaStream_t st) {
     const double wm = std::frexp(4.0 * M_PI / (double)p.npix, &Ew);
     p.ring64_ew = Ew;
     const dim3 grid(64, 4, (unsigned)(ns + 1));
-    if (dir) r64::k_ring_tab<true><<<grid, 256, 0, st>>>(p.d_rings, ns, p.lmax, 1.0, doff, p.ring64_dig[1]);
-    else r64::k_ring_tab<false><<<grid, 256, 0, st>>>(p.d_rings, ns, p.lmax, wm, doff, p.ring64_dig[0]);
+    if (dir) launch_pdl(r64::k_ring_tab<true>, dim3(grid), dim3(256), 0, st, p.d_rings, ns, p.lmax, 1.0, doff,
+        p.ring64_dig[1]);
+    else launch_pdl(r64::k_ring_tab<false>, dim3(grid), dim3(256), 0, st, p.d_rings, ns, p.lmax, wm, doff,
+        p.ring64_dig[0]);
     note_launch();
     if (cudaGetLastError() != cudaSuccess) return false;
     p.ring64_state[dir] = 1;
@@ -581,13 +588,14 @@ bool launch_ring_analysis64(Plan &p, const double *maps, int64_t nm, double *F, 
     if (!ensure_ring64(p, 0, st) || !ring64_room(p, nm, ex)) return false;
     const int ns = (int)p.nside;
     int64_t *Q = reinterpret_cast<int64_t *>(p.ring64.ptr);
-    r64::k_fold64<<<dim3((unsigned)((nm + 7) / 8), (unsigned)nz), 256, 0, st>>>(p.d_rings, ns, p.npix, maps, nm,
-                                                                             p.ring64_qoff[0], Q, ex, nzr, z0);
+    launch_pdl(r64::k_fold64, dim3((unsigned)((nm + 7) / 8), (unsigned)nz), dim3(256), 0, st, p.d_rings, ns, p.npix,
+        maps, nm, p.ring64_qoff[0], Q, ex, nzr, z0);
     const int ntile = (r64::nfreq(4 * ns, p.lmax, 0) + t64::NT - 1) / t64::NT;
     set_smem(r64::k_rdft64, t64::SMEM);
-    r64::k_rdft64<<<dim3((unsigned)((2 * nm + t64::MTILE - 1) / t64::MTILE), (unsigned)(4 * ntile), (unsigned)nz),
-                    t64::NTH, t64::SMEM, st>>>(p.d_rings, ns, p.lmax, nm, p.ring64_qoff[0], Q, ex, p.ring64_dig[0],
-                                               p.ring64_off[0], p.ring64_ew, F, z0, p.d_err);
+    launch_pdl(r64::k_rdft64,
+        dim3((unsigned)((2 * nm + t64::MTILE - 1) / t64::MTILE), (unsigned)(4 * ntile), (unsigned)nz), dim3(t64::NTH),
+        t64::SMEM, st, p.d_rings, ns, p.lmax, nm, p.ring64_qoff[0], Q, ex, p.ring64_dig[0], p.ring64_off[0],
+        p.ring64_ew, F, z0, p.d_err);
     note_launch();
     note_launch();
     return true;
@@ -608,21 +616,22 @@ bool launch_ring_synthesis64(Plan &p, const double *G, int64_t nm, void *out, in
     while (K >= (64 << sh)) ++sh;
     const size_t smem = (size_t)kb * t64::ND * (t64::PLANE_A + t64::NT * t64::KC * 2);
     set_smem(r64::k_rsyn64, smem);
-    r64::k_rsyn64<<<dim3((unsigned)((2 * nm + t64::MTILE - 1) / t64::MTILE), 4, (unsigned)nz), t64::NTH, smem, st>>>(
-        p.d_rings, ns, p.lmax, nm, G, p.ring64_dig[1], p.ring64_off[1], p.ring64_qoff[1], Y, ex, kb, sh, z0, p.d_err);
+    launch_pdl(r64::k_rsyn64, dim3((unsigned)((2 * nm + t64::MTILE - 1) / t64::MTILE), 4, (unsigned)nz),
+        dim3(t64::NTH), smem, st, p.d_rings, ns, p.lmax, nm, G, p.ring64_dig[1], p.ring64_off[1], p.ring64_qoff[1], Y,
+        ex, kb, sh, z0, p.d_err);
     const int kcmax = ns + 1;
     if (pixmajor) {
         const dim3 grid((unsigned)((nm + 31) / 32), (unsigned)((kcmax + 31) / 32), (unsigned)nz);
         if (f32)
-            r64::k_unfold64<float, true><<<grid, 256, 0, st>>>(p.d_rings, ns, nm, p.ring64_qoff[1], Y, ex, sh,
-                                                               (float *)out, ld, z0);
+            launch_pdl(r64::k_unfold64<float, true>, dim3(grid), dim3(256), 0, st, p.d_rings, ns, nm,
+                p.ring64_qoff[1], Y, ex, sh, (float *)out, ld, z0);
         else
-            r64::k_unfold64<double, true><<<grid, 256, 0, st>>>(p.d_rings, ns, nm, p.ring64_qoff[1], Y, ex, sh,
-                                                                (double *)out, ld, z0);
+            launch_pdl(r64::k_unfold64<double, true>, dim3(grid), dim3(256), 0, st, p.d_rings, ns, nm,
+                p.ring64_qoff[1], Y, ex, sh, (double *)out, ld, z0);
     } else {
         const dim3 grid((unsigned)((nm + 7) / 8), (unsigned)((kcmax + 127) / 128), (unsigned)nz);
-        r64::k_unfold64<double, false><<<grid, 256, 0, st>>>(p.d_rings, ns, nm, p.ring64_qoff[1], Y, ex, sh,
-                                                             (double *)out, ld, z0);
+        launch_pdl(r64::k_unfold64<double, false>, dim3(grid), dim3(256), 0, st, p.d_rings, ns, nm, p.ring64_qoff[1],
+            Y, ex, sh, (double *)out, ld, z0);
     }
     note_launch();
     note_launch();

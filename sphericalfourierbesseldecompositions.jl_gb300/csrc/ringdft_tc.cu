@@ -114,10 +114,11 @@ __device__ __forceinline__ void st_shared_v4(unsigned char *p, const uint32_t (&
 // nzr[0] / nzr[1] get the first / last ring pair with a non-zero row (preset
 // to a large value / -1).  With live, rows on the rings marked 0 there are zero by
 // construction and are not read.
-__global__ void __launch_bounds__(128) k_ring_rowexp(const float2 *__restrict__ maps, int64_t npix, int64_t nmaps,
-                                                     const RingGeom *__restrict__ rings, int nrn, int *erow,
+__global__ void __launch_bounds__(128) k_ring_rowexp(const float2 *maps, int64_t npix, int64_t nmaps,
+                                                     const RingGeom *rings, int nrn, int *erow,
                                                      int *nzr, LiveRings live,
                                                      int nrings, int r0) {
+    pdl_entry();
     const int r = r0 + blockIdx.x;
     const int64_t b = (int64_t)blockIdx.y * 4 + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
@@ -164,12 +165,13 @@ __global__ void __launch_bounds__(128) k_ring_rowexp(const float2 *__restrict__ 
 // Grid (tiles, classes, groups of SLICE_CPG chunks), one thread per (row,
 // 16-pixel half) as the DFT's imaged producers.
 constexpr int SLICE_CPG = 4;
-__global__ void __launch_bounds__(NPROD) k_dft_slice_a(const float2 *__restrict__ maps, int64_t npix, int64_t nmaps,
-                                                        const RingGeom *__restrict__ rings, int nrn,
-                                                        const int32_t *__restrict__ cls_rings,
-                                                        const int32_t *__restrict__ cls_off,
-                                                        const int *__restrict__ erow, const int64_t *__restrict__ aoff,
-                                                        unsigned char *__restrict__ aimg) {
+__global__ void __launch_bounds__(NPROD) k_dft_slice_a(const float2 *maps, int64_t npix, int64_t nmaps,
+                                                        const RingGeom *rings, int nrn,
+                                                        const int32_t *cls_rings,
+                                                        const int32_t *cls_off,
+                                                        const int *erow, const int64_t *aoff,
+                                                        unsigned char *aimg) {
+    pdl_entry();
     const int cls = blockIdx.y;
     const int rb = cls_off[cls];
     const int64_t npairs = (int64_t)(cls_off[cls + 1] - rb) * nmaps;
@@ -240,18 +242,19 @@ __global__ void __launch_bounds__(NPROD) k_dft_slice_a(const float2 *__restrict_
 // stage in one transaction, and the producers only release the stages and run the epilogue; without
 // IMG warps 4-7 gather the B planes from the ring's table meanwhile).
 template <bool IMG, bool AIMG>
-__global__ void __launch_bounds__(NTHR, 1) k_ring_dft_tc(const float2 *__restrict__ maps, int64_t npix, int64_t nmaps,
-                                                         const RingGeom *__restrict__ rings, int nrn, int lmax,
-                                                         const int32_t *__restrict__ cls_rings,
-                                                         const int32_t *__restrict__ cls_off,
-                                                         const int *__restrict__ erow, const uint2 *__restrict__ dtw,
-                                                         const int64_t *__restrict__ dtw_off,
-                                                         const unsigned char *__restrict__ img,
-                                                         const int64_t *__restrict__ img_off, float2 *__restrict__ F,
+__global__ void __launch_bounds__(NTHR, 1) k_ring_dft_tc(const float2 *maps, int64_t npix, int64_t nmaps,
+                                                         const RingGeom *rings, int nrn, int lmax,
+                                                         const int32_t *cls_rings,
+                                                         const int32_t *cls_off,
+                                                         const int *erow, const uint2 *dtw,
+                                                         const int64_t *dtw_off,
+                                                         const unsigned char *img,
+                                                         const int64_t *img_off, float2 *F,
                                                          int64_t ldF, float2 wdf, const unsigned char *dead,
                                                          int ntn, const int *span, int rev,
-                                                         const int64_t *__restrict__ aoff,
-                                                         const unsigned char *__restrict__ aimg, int *err) {
+                                                         const int64_t *aoff,
+                                                         const unsigned char *aimg, int *err) {
+    pdl_entry();
     extern __shared__ __align__(1024) unsigned char smem[];
     // grid (column blocks u, row tiles, classes): the column blocks of one row tile are launched
     // together and read its map rows through L2 once; rev: classes in reverse order (the polar
@@ -614,13 +617,14 @@ __global__ void __launch_bounds__(NTHR, 1) k_ring_dft_tc(const float2 *__restric
 // the same bits the gather variant builds (chunk (c, u, kc) at img_off[c] +
 // u nch_c + kc, 32 KB each).  Grid (max chunks, classes, column blocks), 128
 // threads (one per column).
-__global__ void __launch_bounds__(NROW) k_build_dft_image(const RingGeom *__restrict__ rings, int lmax,
-                                                          const int32_t *__restrict__ cls_rings,
-                                                          const int32_t *__restrict__ cls_off,
-                                                          const uint2 *__restrict__ dtw,
-                                                          const int64_t *__restrict__ dtw_off,
-                                                          const int64_t *__restrict__ img_off,
-                                                          unsigned char *__restrict__ img) {
+__global__ void __launch_bounds__(NROW) k_build_dft_image(const RingGeom *rings, int lmax,
+                                                          const int32_t *cls_rings,
+                                                          const int32_t *cls_off,
+                                                          const uint2 *dtw,
+                                                          const int64_t *dtw_off,
+                                                          const int64_t *img_off,
+                                                          unsigned char *img) {
+    pdl_entry();
     const int kc = blockIdx.x, cls = blockIdx.y, u = blockIdx.z, ti = threadIdx.x;
     if (img_off[cls] < 0) return;
     const int ring0 = cls_rings[cls_off[cls]];
@@ -682,8 +686,8 @@ void launch_build_dft_image(const Plan &p, int max_nch, cudaStream_t st) {
     const int ncls = p.n_polar + p.n_eq_cls;
     if (ncls <= 0 || !p.d_dtimg) return;
     dim3 grid((unsigned)max_nch, (unsigned)ncls, (unsigned)((p.lmax + 1 + 63) / 64));
-    dft::k_build_dft_image<<<grid, dft::NROW, 0, st>>>(p.d_rings, p.lmax, p.d_cls_rings, p.d_cls_off, p.d_dtw,
-                                                       p.d_dtw_off, p.d_dtimg_off, p.d_dtimg);
+    launch_pdl(dft::k_build_dft_image, dim3(grid), dim3(dft::NROW), 0, st, p.d_rings, p.lmax, p.d_cls_rings,
+        p.d_cls_off, p.d_dtw, p.d_dtw_off, p.d_dtimg_off, p.d_dtimg);
     note_launch();
 }
 
@@ -708,7 +712,7 @@ uint2 dft_slices(double v, int EB) {
 
 static void ring_rowexp(const Plan &p, const float2 *maps, int64_t nmaps, int *erow, int *nzr, const LiveRings &live,
                         int r0, int nr, cudaStream_t st) {
-    dft::k_ring_rowexp<<<dim3((unsigned)nr, (unsigned)((nmaps + 3) / 4)), 128, 0, st>>>(
+    launch_pdl(dft::k_ring_rowexp, dim3((unsigned)nr, (unsigned)((nmaps + 3) / 4)), dim3(128), 0, st,
         maps, p.npix, nmaps, p.d_rings, (int)p.nrn, erow, nzr, live, (int)(4 * p.nside - 1), r0);
     note_launch();
 }
@@ -765,15 +769,15 @@ static void ring_tc_dft(const Plan &p, const float2 *maps, int64_t nmaps, float2
     if (ai) {
         // chunk groups: the longest ring (4 nside pixels) in groups of SLICE_CPG chunks
         const unsigned ngrp = (unsigned)((4 * p.nside + dft::KC * dft::SLICE_CPG - 1) / (dft::KC * dft::SLICE_CPG));
-        dft::k_dft_slice_a<<<dim3(tiles, ncls, ngrp), dft::NPROD, 0, st>>>(
-            maps, p.npix, nmaps, p.d_rings, (int)p.nrn, p.d_cls_rings, p.d_cls_off + c0, erow, p.d_aimg_off + c0, aimg);
+        launch_pdl(dft::k_dft_slice_a, dim3(tiles, ncls, ngrp), dim3(dft::NPROD), 0, st, maps, p.npix, nmaps,
+            p.d_rings, (int)p.nrn, p.d_cls_rings, p.d_cls_off + c0, erow, p.d_aimg_off + c0, aimg);
         note_launch();
     }
     auto go = [&](auto kernel) {
-        kernel<<<dim3(ntn, tiles, ncls), dft::NTHR, dft::SMEM, st>>>(
-            maps, p.npix, nmaps, p.d_rings, (int)p.nrn, p.lmax, p.d_cls_rings, p.d_cls_off + c0, erow, p.d_dtw,
-            p.d_dtw_off, img ? p.d_dtimg : nullptr, img ? p.d_dtimg_off + c0 : nullptr, F, 2 * nmaps, wdf, dead, (int)ntn,
-            span, eq ? 0 : 1, ai ? p.d_aimg_off + c0 : nullptr, ai ? aimg : nullptr, p.d_err);
+        launch_pdl(kernel, dim3(ntn, tiles, ncls), dim3(dft::NTHR), dft::SMEM, st, maps, p.npix, nmaps, p.d_rings,
+            (int)p.nrn, p.lmax, p.d_cls_rings, p.d_cls_off + c0, erow, p.d_dtw, p.d_dtw_off,
+            img ? p.d_dtimg : nullptr, img ? p.d_dtimg_off + c0 : nullptr, F, 2 * nmaps, wdf, dead, (int)ntn, span,
+            eq ? 0 : 1, ai ? p.d_aimg_off + c0 : nullptr, ai ? aimg : nullptr, p.d_err);
     };
     if (img && ai) go(dft::k_ring_dft_tc<true, true>);
     else if (ai) go(dft::k_ring_dft_tc<false, true>);

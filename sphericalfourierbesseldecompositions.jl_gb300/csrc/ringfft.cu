@@ -159,7 +159,7 @@ __device__ void four_step(cx<T> *buf, cx<T> *src, const cx<T> *tw, int n, int o,
 // Twiddles W_n^t = e^{dir 2 pi i t / n} from the plan's FP64 table of
 // e^{-2 pi i t / n} (one block of n entries per ring, offset twoff).
 template <typename T>
-__device__ void fill_twiddles(cx<T> *tw, const double2 *__restrict__ tab, int n, int dir) {
+__device__ void fill_twiddles(cx<T> *tw, const double2 *tab, int n, int dir) {
     for (int t = threadIdx.x; t < n; t += blockDim.x) {
         const double2 v = tab[t];
         tw[t] = {(T)v.x, (T)(dir < 0 ? v.y : -v.y)};
@@ -174,9 +174,10 @@ template <typename T, typename TI, typename TW>
 __global__ void __launch_bounds__(256) k_ring_analysis(const RingGeom *rings, int nrn, int lmax,
                                                        int64_t npix, const TI *maps, int64_t nmaps,
                                                        int MT, T *F, int64_t ldF, int r0,
-                                                       const TW *__restrict__ twtab,
-                                                       const int64_t *__restrict__ twoff,
-                                                       const TW *__restrict__ wphase, int *nzr) {
+                                                       const TW *twtab,
+                                                       const int64_t *twoff,
+                                                       const TW *wphase, int *nzr) {
+    pdl_entry();
     extern __shared__ unsigned char smem_raw[];
     const int r = r0 + blockIdx.x;
     const int64_t b0 = (int64_t)blockIdx.y * MT;
@@ -295,9 +296,10 @@ template <typename T>
 __global__ void __launch_bounds__(256) k_ring_synthesis(const RingGeom *rings, int nrn, int lmax,
                                                         const T *G, int64_t ldG, int64_t nmaps, int MT,
                                                         int64_t npix, double *maps, int r0,
-                                                        const double2 *__restrict__ twtab,
-                                                        const int64_t *__restrict__ twoff,
-                                                        const double2 *__restrict__ phase) {
+                                                        const double2 *twtab,
+                                                        const int64_t *twoff,
+                                                        const double2 *phase) {
+    pdl_entry();
     extern __shared__ unsigned char smem_raw[];
     const int r = r0 + blockIdx.x;
     const int64_t b0 = (int64_t)blockIdx.y * MT;
@@ -391,8 +393,8 @@ static void ring_analysis_t(const Plan &p, const TI *maps, int64_t nmaps, T *F, 
         const size_t smem = ring_smem(n, sizeof(cx<T>), two, MT);
         set_smem(k_ring_analysis<T, TI, TW>, smem);
         dim3 grid((unsigned)nr, (unsigned)((nmaps + MT - 1) / MT));
-        k_ring_analysis<T, TI, TW><<<grid, 256, smem, st>>>(p.d_rings, (int)p.nrn, p.lmax, p.npix, maps, nmaps, MT,
-                                                            F, 2 * nmaps, r0, tw, p.d_twoff, wph, nzr);
+        launch_pdl(k_ring_analysis<T, TI, TW>, dim3(grid), dim3(256), smem, st, p.d_rings, (int)p.nrn, p.lmax, p.npix,
+            maps, nmaps, MT, F, 2 * nmaps, r0, tw, p.d_twoff, wph, nzr);
         note_launch();
     };
     // two maps or fewer leave most of the chip to the other group: both in one launch (the mixed transform's
@@ -427,8 +429,8 @@ void launch_ring_synthesis(Plan &p, const double *G, int64_t nmaps, double *maps
         const size_t smem = ring_smem(gr.n, sizeof(cx<double>), gr.two, MT);
         set_smem(k_ring_synthesis<double>, smem);
         dim3 grid((unsigned)gr.nr, (unsigned)((nmaps + MT - 1) / MT));
-        k_ring_synthesis<double><<<grid, 256, smem, st>>>(p.d_rings, (int)p.nrn, p.lmax, G, 2 * nmaps, nmaps, MT,
-                                                          p.npix, maps, gr.r0, p.d_twtab, p.d_twoff, p.d_phase);
+        launch_pdl(k_ring_synthesis<double>, dim3(grid), dim3(256), smem, st, p.d_rings, (int)p.nrn, p.lmax, G,
+            2 * nmaps, nmaps, MT, p.npix, maps, gr.r0, p.d_twtab, p.d_twoff, p.d_phase);
         note_launch();
     }
 }

@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/sfb_gpu.h"
@@ -210,6 +211,44 @@ template <typename K>
 inline void set_smem(K kernel, size_t bytes) {
     if (bytes > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
+
+// Programmatic dependent launch: in a call that wants it (PdlScope) a kernel's blocks may be brought onto the SMs
+// while the last blocks of the kernel before it on the stream still run, and every kernel begins by waiting for that
+// kernel's completion (pdl_entry), so the launch latency between dependent kernels is hidden.  Nothing of a kernel
+// runs before its wait: a block that came early holds no TMEM and has written nothing.  The kernels' pointers carry
+// no __restrict__: loads through const restrict pointers count as read-only for the kernel's lifetime, and the
+// compiler may move them above the wait.
+// Chains of short kernels gain (us a call without and with: 231 and 190 at nside 16, 300 and 262 at nside 32, 583 and
+// 537 for field_f64's field); where the FP64 reference transform on the side stream competes for the SMs the blocks
+// that wait are in its way (594 and 607 at nside 128 with 104 maps), so the caller decides.
+struct PdlScope {
+    explicit PdlScope(bool on);
+    ~PdlScope();
+    static bool enabled();
+
+  private:
+    bool before;
+};
+#ifdef __CUDACC__
+__device__ __forceinline__ void pdl_entry() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <typename... P, typename... A>
+inline void launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A &&...args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = PdlScope::enabled() ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);      // (errors: the callers' cudaGetLastError)
+}
+#endif
 
 // ---------------------------------------------------------------------------
 // kernels (launch wrappers; all enqueue on `st`)

@@ -42,7 +42,8 @@ __device__ __forceinline__ double double_of_ord(unsigned long long o) {
 
 // mx: order image of max(win) (preset to 0, below every image); err |= ERR_NONFINITE_INPUT
 // for a NaN entry
-__global__ void k_window_max(const double *__restrict__ win, int64_t n, unsigned long long *mx, int *err) {
+__global__ void k_window_max(const double *win, int64_t n, unsigned long long *mx, int *err) {
+    pdl_entry();
     unsigned long long best = 0;
     bool bad = false;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -55,10 +56,11 @@ __global__ void k_window_max(const double *__restrict__ win, int64_t n, unsigned
     if (bad) atomicOr(err, ERR_NONFINITE_INPUT);
 }
 
-__global__ void k_window_flags(const double *__restrict__ rtp, int64_t ngal, const double *__restrict__ win,
+__global__ void k_window_flags(const double *rtp, int64_t ngal, const double *win,
                                int64_t nr, int64_t nside, double rmin, double rmax, double dr,
-                               const double *__restrict__ uniform, uint64_t seed,
-                               const unsigned long long *__restrict__ mx, int32_t *__restrict__ flags, int *err) {
+                               const double *uniform, uint64_t seed,
+                               const unsigned long long *mx, int32_t *flags, int *err) {
+    pdl_entry();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= ngal) return;
     const double r = rtp[3 * i], th = rtp[3 * i + 1], ph = rtp[3 * i + 2];
@@ -83,8 +85,9 @@ __global__ void k_window_flags(const double *__restrict__ rtp, int64_t ngal, con
 }
 
 // off: exclusive scan of the flags (off[ngal] = number kept)
-__global__ void k_window_scatter(const double *__restrict__ rtp, int64_t ngal, const int32_t *__restrict__ off,
-                                 double *__restrict__ out) {
+__global__ void k_window_scatter(const double *rtp, int64_t ngal, const int32_t *off,
+                                 double *out) {
+    pdl_entry();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= ngal) return;
     const int32_t o = off[i];
@@ -113,14 +116,14 @@ int run(int64_t nside, const double *win, int64_t nr, double rmin, double rmax, 
     unsigned long long *mx = reinterpret_cast<unsigned long long *>(ws + (((ngal + 1 + ntiles) * 4 + 15) / 16) * 16);
     int *err = reinterpret_cast<int *>(mx + 1);
     SFB_CUDA_TRY(cudaMemsetAsync(mx, 0, sizeof(unsigned long long) + 2 * sizeof(int), st));
-    k_window_max<<<608, 256, 0, st>>>(win, nr * npix, mx, err);
+    launch_pdl(k_window_max, dim3(608), dim3(256), 0, st, win, nr * npix, mx, err);
     note_launch();
-    k_window_flags<<<(unsigned)((ngal + 255) / 256), 256, 0, st>>>(rtp, ngal, win, nr, nside, rmin, rmax, dr, uniform,
-                                                                   seed, mx, flags, err);
+    launch_pdl(k_window_flags, dim3((unsigned)((ngal + 255) / 256)), dim3(256), 0, st, rtp, ngal, win, nr, nside,
+        rmin, rmax, dr, uniform, seed, mx, flags, err);
     note_launch();
     SFB_CUDA_TRY(cudaMemsetAsync(flags + ngal, 0, sizeof(int32_t), st));
     launch_exclusive_scan(flags, ngal + 1, tsum, err + 1, st);
-    k_window_scatter<<<(unsigned)((ngal + 255) / 256), 256, 0, st>>>(rtp, ngal, flags, out);
+    launch_pdl(k_window_scatter, dim3((unsigned)((ngal + 255) / 256)), dim3(256), 0, st, rtp, ngal, flags, out);
     note_launch();
     int32_t h[2] = {0, 0};
     SFB_CUDA_TRY(cudaMemcpyAsync(&h[0], flags + ngal, sizeof(int32_t), cudaMemcpyDeviceToHost, st));

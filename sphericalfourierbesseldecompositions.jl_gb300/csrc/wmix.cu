@@ -99,11 +99,12 @@ __device__ int w3j_family(int j2, int j3, int m2, int m3, double *f, int *nf) {
     return jmin;
 }
 
-__global__ void __launch_bounds__(256) k_wmix(const int32_t *__restrict__ pair_n, const int32_t *__restrict__ pair_l,
-                                              int64_t npairs, const int64_t *__restrict__ noff,
-                                              const double *__restrict__ gtab, int64_t nr, double rmin, double dr,
-                                              const double *__restrict__ WT, int64_t ldW, int LW, int neg_m,
-                                              int64_t nlmsize, double *__restrict__ out) {
+__global__ void __launch_bounds__(256) k_wmix(const int32_t *pair_n, const int32_t *pair_l,
+                                              int64_t npairs, const int64_t *noff,
+                                              const double *gtab, int64_t nr, double rmin, double dr,
+                                              const double *WT, int64_t ldW, int LW, int neg_m,
+                                              int64_t nlmsize, double *out) {
+    pdl_entry();
     extern __shared__ double sm[];
     const int64_t P = blockIdx.x, Q = blockIdx.y;
     const int l = pair_l[P], n = pair_n[P], lp = pair_l[Q], np = pair_n[Q];
@@ -196,8 +197,8 @@ void launch_wmix(const Plan &p, const int64_t *noff, const double *gtab, int64_t
                  const double *WT, int64_t ldW, int LW, int neg_m, double *out, size_t smem, cudaStream_t st) {
     set_smem(k_wmix, smem);
     dim3 grid((unsigned)p.npairs, (unsigned)p.npairs);
-    k_wmix<<<grid, 256, smem, st>>>(p.d_pair_n, p.d_pair_l, p.npairs, noff, gtab, nr, rmin, dr, WT, ldW, LW, neg_m,
-                                    p.nlmsize, out);
+    launch_pdl(k_wmix, dim3(grid), dim3(256), smem, st, p.d_pair_n, p.d_pair_l, p.npairs, noff, gtab, nr, rmin, dr,
+        WT, ldW, LW, neg_m, p.nlmsize, out);
     note_launch();
 }
 

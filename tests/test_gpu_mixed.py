@@ -226,3 +226,39 @@ def test_partial_sky_after_other_map_counts(zlim):
     sfbgpu.field2anlm(f, wm, b, precision="mixed")
     got = sfbgpu.cat2amln(rtp, b, 1e-5, None, None, precision="mixed")
     assert rel_err(got, fresh) < 1e-9
+
+
+@pytest.mark.parametrize("precision,nside", [("mixed", 16), ("mixed", 64), ("fp64", 32)])
+def test_calls_queued_without_waiting_equal_waited_calls(precision, nside):
+    """Device-pointer calls on alternating inputs with nothing waited for in between: a kernel's blocks may
+    be on the SMs before the kernel in front of it has ended, and must not read what that one still writes
+    or what an earlier call left.  Same kernels on the same inputs: the deposit's run-to-run rounding, 1e-9."""
+    import ctypes
+
+    import torch
+    from sfbgpu import _capi as capi
+    from sfbgpu.cat2anlm import GPUPlan
+
+    plan = GPUPlan(sfbgpu.AnlmModes(0.03, 500.0, 1000.0, nside=nside), precision=precision)
+    ptr = lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
+    sets, waited = [], []
+
+    def call(rtp):
+        out = torch.empty(2 * plan.nlmsize, dtype=torch.float64, device="cuda")
+        capi.check(capi.lib.sfb_cat2amln_device(plan.handle, ptr(rtp), None, rtp.shape[0], 1e-5, ctypes.byref(capi.Window()), ptr(out),
+                                                ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+        return out
+
+    for seed in range(2):
+        rng = np.random.default_rng(80 + seed)
+        n = 20_000 + 3_001 * seed
+        r = np.cbrt(500.0 ** 3 + rng.random(n) * (1000.0 ** 3 - 500.0 ** 3))
+        rtp = np.stack([r, np.arccos(rng.uniform(-0.5, 1.0, n)), rng.uniform(0, 2 * np.pi, n)], axis=1)
+        sets.append(torch.from_numpy(rtp).cuda())
+        out = call(sets[-1])
+        torch.cuda.synchronize()
+        waited.append(out.cpu().numpy())
+    queued = [call(sets[i % 2]) for i in range(40)]
+    torch.cuda.synchronize()
+    for i, got in enumerate(queued):
+        assert rel_err(got.cpu().numpy(), waited[i % 2]) < 1e-9
