@@ -41,6 +41,17 @@ constexpr int SCAN_THREADS = 256;
 constexpr int SCAN_ITEMS = 16;                    // per thread
 constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
 
+// Bin offsets as the scan leaves them: a prefix within the bin's tile and the tile's own.  The readers add the two
+// (the tiles' few values stay in L1), which spares a pass over the counters (48 us for 11.8 million).
+struct Offsets {
+    const int32_t *in_tile, *tile;
+    int64_t first;
+    __device__ __forceinline__ int32_t operator[](int64_t i) const {
+        const uint64_t k = (uint64_t)(first + i);
+        return in_tile[k] + tile[k / SCAN_TILE];
+    }
+};
+
 // Double-float arithmetic (value = hi + lo, |lo| <= ulp(hi)/2): ~48
 // significant bits from FP32 operations, whose throughput on this GPU is
 // many times that of FP64.  TwoSum / TwoProd with FMA (Dekker, Knuth).
@@ -267,14 +278,19 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_tiles(int32_t *data, int6
     __shared__ int32_t carry;
     __shared__ bool last;
     const int64_t base = (int64_t)blockIdx.x * SCAN_TILE + (int64_t)threadIdx.x * SCAN_ITEMS;
-    int32_t v[SCAN_ITEMS];
+    alignas(16) int32_t v[SCAN_ITEMS];
     int32_t s = 0;
+    const bool whole = base + SCAN_ITEMS <= n;             // (the counters start on a 16-byte boundary)
+    if (whole) {
 #pragma unroll
-    for (int j = 0; j < SCAN_ITEMS; ++j) {
-        const int64_t idx = base + j;
-        v[j] = idx < n ? data[idx] : 0;
-        s += v[j];
+        for (int j = 0; j < SCAN_ITEMS; j += 4)
+            *reinterpret_cast<int4 *>(v + j) = *reinterpret_cast<const int4 *>(data + base + j);
+    } else {
+#pragma unroll
+        for (int j = 0; j < SCAN_ITEMS; ++j) v[j] = base + j < n ? data[base + j] : 0;
     }
+#pragma unroll
+    for (int j = 0; j < SCAN_ITEMS; ++j) s += v[j];
     // exclusive scan of thread sums across the block
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     int32_t inc = s;
@@ -294,11 +310,20 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_tiles(int32_t *data, int6
     }
     __syncthreads();
     int32_t run = inc - s + (wid > 0 ? warp_tot[wid - 1] : 0);
+    alignas(16) int32_t o[SCAN_ITEMS];
 #pragma unroll
     for (int j = 0; j < SCAN_ITEMS; ++j) {
-        const int64_t idx = base + j;
-        if (idx < n) data[idx] = run;
+        o[j] = run;
         run += v[j];
+    }
+    if (whole) {
+#pragma unroll
+        for (int j = 0; j < SCAN_ITEMS; j += 4)
+            *reinterpret_cast<int4 *>(data + base + j) = *reinterpret_cast<const int4 *>(o + j);
+    } else {
+#pragma unroll
+        for (int j = 0; j < SCAN_ITEMS; ++j)
+            if (base + j < n) data[base + j] = o[j];
     }
     if (threadIdx.x == SCAN_THREADS - 1) {
         tile_sums[blockIdx.x] = run;
@@ -346,7 +371,7 @@ __global__ void k_scan_add(int32_t *data, int64_t n, const int32_t *tile_sums) {
 
 __global__ void k_deposit_scatter(const double *wgt, int64_t ngal, const int32_t *key,
                                   const int32_t *rank, const double *xloc,
-                                  const int32_t *offset, double2 *sorted) {
+                                  Offsets offset, double2 *sorted) {
     pdl_entry();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= ngal) return;
@@ -360,7 +385,7 @@ __global__ void k_deposit_scatter(const double *wgt, int64_t ngal, const int32_t
 // split from the double by integer operations.
 __global__ void k_deposit_scatter_mixed(const double *wgt, int64_t ngal,
                                         const int32_t *key, const int32_t *rank,
-                                        const float2 *xdf, const int32_t *offset,
+                                        const float2 *xdf, Offsets offset,
                                         float4 *sorted) {
     pdl_entry();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -441,7 +466,7 @@ __device__ __forceinline__ int rank_bins(int cnt, int *hist) {
 // consecutive threads on consecutive pixels.  Bound: the FP64 pipe, 72 operations a galaxy at degree 24 (with
 // four operations a degree and unsorted bins 274 us for 6e5 galaxies at nside 128; 151 so).
 template <int MAXDEG>
-__global__ void __launch_bounds__(128) k_deposit_moments(const int32_t *offset,
+__global__ void __launch_bounds__(128) k_deposit_moments(Offsets offset,
                                                          const double2 *sorted, int64_t npix, int pieces,
                                                          int deg, int64_t nbasis, double *maps) {
     pdl_entry();
@@ -449,7 +474,7 @@ __global__ void __launch_bounds__(128) k_deposit_moments(const int32_t *offset,
     __shared__ int hist[64];
     __shared__ int perm[128];
     // grid.y: mocks
-    offset += (int64_t)blockIdx.y * (pieces + 2) * npix;
+    offset.first += (int64_t)blockIdx.y * (pieces + 2) * npix;
     maps += (int64_t)blockIdx.y * nbasis * npix;
     const int t = threadIdx.x;
     const int64_t nkeys = (int64_t)(pieces + 2) * npix;
@@ -540,12 +565,12 @@ __device__ __forceinline__ void bin_moments_df(const float4 *sorted, int64_t g0,
 // fluctuation acc - mu_b ref all in double-float (mudf = mu and cdf = ref as
 // hi + lo pairs), stored as normalised double-float pairs.
 template <int MAXDEG>
-__global__ void k_deposit_moments_df(const int32_t *offset, const float4 *sorted,
+__global__ void k_deposit_moments_df(Offsets offset, const float4 *sorted,
                                      int64_t npix, int pieces, int deg, int64_t nbasis, const float2 *cdf,
                                      const float2 *mudf, float2 *maps) {
     pdl_entry();
     // grid.y: mocks
-    offset += (int64_t)blockIdx.y * (pieces + 2) * npix;
+    offset.first += (int64_t)blockIdx.y * (pieces + 2) * npix;
     maps += (int64_t)blockIdx.y * nbasis * npix;
     if (cdf) {
         cdf += blockIdx.y * npix;
@@ -595,7 +620,7 @@ __global__ void k_deposit_moments_df(const int32_t *offset, const float4 *sorted
 // and are written with consecutive threads on consecutive pixels.  Needs
 // npix >= 128 (a block spans at most two slots).
 template <int MAXDEG>
-__global__ void __launch_bounds__(128) k_deposit_moments_bal(const int32_t *offset,
+__global__ void __launch_bounds__(128) k_deposit_moments_bal(Offsets offset,
                                                              const float4 *sorted, int64_t npix,
                                                              int pieces, int deg, int64_t nbasis,
                                                              const float2 *cdf,
@@ -607,7 +632,7 @@ __global__ void __launch_bounds__(128) k_deposit_moments_bal(const int32_t *offs
     __shared__ int perm[128];
     __shared__ float2 out[(MAXDEG + 1) * 128];
     // grid.y: mocks
-    offset += (int64_t)blockIdx.y * (pieces + 2) * npix;
+    offset.first += (int64_t)blockIdx.y * (pieces + 2) * npix;
     maps += (int64_t)blockIdx.y * nbasis * npix;
     if (cdf) {
         cdf += blockIdx.y * npix;
@@ -747,7 +772,7 @@ __device__ __forceinline__ void bin_moments_sm(const float4 *sorted, int64_t g0,
 }
 
 template <int MAXDEG>
-__global__ void __launch_bounds__(128, 8) k_deposit_moments_sm(const int32_t *offset,
+__global__ void __launch_bounds__(128, 8) k_deposit_moments_sm(Offsets offset,
                                                                const float4 *sorted, int64_t npix,
                                                                int pieces, int deg, int64_t nbasis,
                                                                const float2 *cdf,
@@ -759,7 +784,7 @@ __global__ void __launch_bounds__(128, 8) k_deposit_moments_sm(const int32_t *of
     __shared__ int perm[128];
     __shared__ __align__(16) float2 acc_s[(MAXDEG + 1) * 128];
     // grid.y: mocks
-    offset += (int64_t)blockIdx.y * (pieces + 2) * npix;
+    offset.first += (int64_t)blockIdx.y * (pieces + 2) * npix;
     maps += (int64_t)blockIdx.y * nbasis * npix;
     if (cdf) {
         cdf += blockIdx.y * npix;
@@ -853,7 +878,7 @@ constexpr int STATS_STRIDE = 32;
 // block that finishes last (*done zero on entry) forms mu[b] = S[b] / Q[slot(b)]
 // (0 where the sampled reference map is zero) and the same as a double-float pair.
 template <int MAXDEG>
-__global__ void __launch_bounds__(32) k_deposit_stats(const int32_t *offset,
+__global__ void __launch_bounds__(32) k_deposit_stats(Offsets offset,
                                                       const float4 *sorted, int64_t npix, int pieces,
                                                       int deg, int64_t nbasis, const float2 *cdf,
                                                       double *S, double *Q, double *mu,
@@ -861,7 +886,7 @@ __global__ void __launch_bounds__(32) k_deposit_stats(const int32_t *offset,
     pdl_entry();
     __shared__ float2 red[32][MAXDEG + 3];
     // grid.y: mocks
-    offset += (int64_t)blockIdx.y * (pieces + 2) * npix;
+    offset.first += (int64_t)blockIdx.y * (pieces + 2) * npix;
     cdf += blockIdx.y * npix;
     double *const S0 = S, *const Q0 = Q;
     S += blockIdx.y * nbasis;
@@ -941,7 +966,7 @@ __global__ void __launch_bounds__(32) k_deposit_stats(const int32_t *offset,
 // FP64 value hi + lo (exact) and as the pair itself.
 // ring_live[ring] is set to 1 for every ring holding a galaxy (preset to 0).
 // The window's reference map W01 goes behind the count maps.
-__global__ void k_weight_map_mixed(const int32_t *offset, const float4 *sorted,
+__global__ void k_weight_map_mixed(Offsets offset, const float4 *sorted,
                                    int64_t nside, int64_t npix, int nslots, double *C,
                                    float2 *cdf, int *ring_live,
                                    const double *W01) {
@@ -950,7 +975,7 @@ __global__ void k_weight_map_mixed(const int32_t *offset, const float4 *sorted,
     if (pix >= npix) return;
     // grid.y: mocks
     if (W01 && blockIdx.y == 0) C[gridDim.y * npix + pix] = W01[pix];
-    offset += (int64_t)blockIdx.y * nslots * npix;
+    offset.first += (int64_t)blockIdx.y * nslots * npix;
     C += blockIdx.y * npix;
     cdf += blockIdx.y * npix;
     ring_live += blockIdx.y * (4 * nside - 1);
@@ -972,7 +997,7 @@ __global__ void k_weight_map_mixed(const int32_t *offset, const float4 *sorted,
 
 // FP64 path: double (x, w); mixed: double-float pairs and the count map as cdf
 template <int MAXDEG>
-static void launch_moments(const Plan &p, int nmock, const int32_t *counts, const void *sorted, const float2 *cdf,
+static void launch_moments(const Plan &p, int nmock, Offsets offset, const void *sorted, const float2 *cdf,
                            const float2 *mudf, double *maps, cudaStream_t st, const int *ring_live) {
     const int64_t nkeys = (int64_t)(p.pieces + 2) * p.npix;
     const dim3 blocks((unsigned)((nkeys + 127) / 128), (unsigned)nmock);
@@ -982,33 +1007,33 @@ static void launch_moments(const Plan &p, int nmock, const int32_t *counts, cons
     if constexpr (MAXDEG <= 31) {
         if (p.precision == SFB_MIXED && p.npix >= 128) {
             if (p.moments_smem)
-                launch_pdl(k_deposit_moments_sm<MAXDEG>, dim3(blocks), dim3(128), 0, st, counts, s4, p.npix, p.pieces,
+                launch_pdl(k_deposit_moments_sm<MAXDEG>, dim3(blocks), dim3(128), 0, st, offset, s4, p.npix, p.pieces,
                     p.degree, p.nbasis, cdf, mudf, mf, p.nside, ring_live);
             else
-                launch_pdl(k_deposit_moments_bal<MAXDEG>, dim3(blocks), dim3(128), 0, st, counts, s4, p.npix,
+                launch_pdl(k_deposit_moments_bal<MAXDEG>, dim3(blocks), dim3(128), 0, st, offset, s4, p.npix,
                     p.pieces, p.degree, p.nbasis, cdf, mudf, mf, p.nside, ring_live);
             done = true;
         }
     }
     if (done) {
     } else if (p.precision == SFB_MIXED)
-        launch_pdl(k_deposit_moments_df<MAXDEG>, dim3(blocks), dim3(128), 0, st, counts, s4, p.npix, p.pieces,
+        launch_pdl(k_deposit_moments_df<MAXDEG>, dim3(blocks), dim3(128), 0, st, offset, s4, p.npix, p.pieces,
             p.degree, p.nbasis, cdf, mudf, mf);
     else {
         const size_t smem = (size_t)(p.degree + 1) * 128 * sizeof(double);
         set_smem(k_deposit_moments<MAXDEG>, smem);
-        launch_pdl(k_deposit_moments<MAXDEG>, dim3(blocks), dim3(128), smem, st, counts,
+        launch_pdl(k_deposit_moments<MAXDEG>, dim3(blocks), dim3(128), smem, st, offset,
             static_cast<const double2 *>(sorted), p.npix, p.pieces, p.degree, p.nbasis, maps);
     }
     note_launch();
 }
 
 template <int MAXDEG>
-static void launch_stats(const Plan &p, int nmock, const int32_t *counts, const float4 *sorted, const float2 *cdf, double *S,
+static void launch_stats(const Plan &p, int nmock, Offsets offset, const float4 *sorted, const float2 *cdf, double *S,
                          double *Q, double *mu, float2 *mudf, int *done, cudaStream_t st) {
     const int64_t nkeys = (int64_t)(p.pieces + 2) * p.npix;
     const int64_t blocks = (nkeys + 32 * STATS_STRIDE - 1) / (32 * STATS_STRIDE);
-    launch_pdl(k_deposit_stats<MAXDEG>, dim3((unsigned)blocks, (unsigned)nmock), dim3(32), 0, st, counts, sorted,
+    launch_pdl(k_deposit_stats<MAXDEG>, dim3((unsigned)blocks, (unsigned)nmock), dim3(32), 0, st, offset, sorted,
         p.npix, p.pieces, p.degree, p.nbasis, cdf, S, Q, mu, mudf, done);
     note_launch();
 }
@@ -1101,32 +1126,34 @@ int deposit_sorted(Plan &p, const DepositArgs &a, cudaStream_t st, const int **r
             fb_list, fb_count);
         note_launch();
     }
-    launch_exclusive_scan(counts, nscan, tsum, scan_done, st);
+    launch_pdl(k_scan_tiles, dim3((unsigned)ntiles), dim3(SCAN_THREADS), 0, st, counts, nscan, tsum, scan_done);
+    note_launch();
+    const Offsets offset{counts, tsum, 0};
     if (ngal > 0) {
         if (mixed)
             launch_pdl(k_deposit_scatter_mixed, dim3((unsigned)((ngal + 255) / 256)), dim3(256), 0, st, w, ngal, key,
-                rank, xdf, counts, sorted4);
+                rank, xdf, offset, sorted4);
         else
             launch_pdl(k_deposit_scatter, dim3((unsigned)((ngal + 255) / 256)), dim3(256), 0, st, w, ngal, key, rank,
-                xloc, counts, static_cast<double2 *>(sorted));
+                xloc, offset, static_cast<double2 *>(sorted));
         note_launch();
     }
     if (p.degree > 63) return fail(SFB_ENOTSUP, "radial degree above 63 is not supported by the sorted deposit");
     const bool split = ref != nullptr && mixed;
     if (split) {
         launch_pdl(k_weight_map_mixed, dim3((unsigned)((p.npix + 255) / 256), (unsigned)nmock), dim3(256), 0, st,
-            counts, sorted4, p.nside, p.npix, p.pieces + 2, ref, cdf, live, a.w01);
+            offset, sorted4, p.nside, p.npix, p.pieces + 2, ref, cdf, live, a.w01);
         note_launch();
         if (a.ref_ready) SFB_CUDA_TRY(cudaEventRecord(a.ref_ready, st));
         by_degree(p.degree, [&](auto D) {
-            launch_stats<decltype(D)::value>(p, (int)nmock, counts, sorted4, cdf, S, Q, mu, mudf, stats_done, st);
+            launch_stats<decltype(D)::value>(p, (int)nmock, offset, sorted4, cdf, S, Q, mu, mudf, stats_done, st);
         });
         if (a.mu_ready) SFB_CUDA_TRY(cudaEventRecord(a.mu_ready, st));
     }
     // moments in FP64 (FP64 path) or double-float (mixed); stored in the transform's precision
     const bool skip_empty = split && p.npix >= 128 && p.degree <= 31;                 // the balanced kernel
     by_degree(p.degree, [&](auto D) {
-        launch_moments<decltype(D)::value>(p, (int)nmock, counts, sorted, split ? cdf : nullptr, mudf, a.maps, st,
+        launch_moments<decltype(D)::value>(p, (int)nmock, offset, sorted, split ? cdf : nullptr, mudf, a.maps, st,
                                            skip_empty ? live : nullptr);
     });
     if (skip_empty) *ring_live = live;
