@@ -75,10 +75,11 @@ void launch_sub_window_chunk(const Plan &p, const double *Awin, int64_t ldW, int
 void launch_extract_spline_chunk(const Plan &p, const double *A, int64_t ldA, int64_t pair0, int64_t npc, double *out,
                                  cudaStream_t st);
 void launch_gtab(const Plan &p, int64_t nr, double rmin, double dr, int with_r2dr, double *gtab, cudaStream_t st);
-void launch_project_shells_g(const Plan &p, const double *gtab, int64_t nr, const double *A, int64_t ldA, double *out,
-                             cudaStream_t st);
-void launch_shell_alm_g(const Plan &p, const int32_t *pair_index, const int64_t *noff, const double *gtab, int64_t nr,
-                        const double *anlm, double *A, int64_t ldA, cudaStream_t st);
+void launch_project_shells_g(const Plan &p, const int32_t *pair_index, const int64_t *noff, const double *gtab,
+                             int64_t ldg, int64_t nr, const double *A, const float2 *Adf, bool add, double *out,
+                             int *err, cudaStream_t st);
+void launch_shell_alm_g(const Plan &p, const int32_t *pair_index, const int64_t *noff, const double *gtab, int64_t ldg,
+                        int64_t nr, const double *anlm, double *A, int64_t ldA, cudaStream_t st);
 void launch_win_sep_g(const Plan &p, const double *gtab, int64_t nr, const double *phi, double *out, cudaStream_t st);
 void launch_win_dense_g(const Plan &p, const double *gtab, int64_t nr, const double *win, double *out, cudaStream_t st);
 void launch_fill(double *x, int64_t n, double v, cudaStream_t st);
@@ -463,6 +464,9 @@ int field_ring_stage(sfb_plan *h, const FieldSrc &s, double *maps, double *F, in
     return SFB_OK;
 }
 
+// whether the mixed transform of nm maps refines by the Gram tables
+static bool gram_mixed(const Plan &p, int64_t nm) { return nm > 4 && p.d_gramts && p.niter > 0; }
+
 // fp64_out: the FP64 a_lm (alm) is wanted besides the double-float copy (almdf, mixed precision); the
 // Gram refinement carries only the double-float one and converts at the end when asked.
 // src: the maps are still to be made in `maps` from a field in host memory (field_ring_stage).
@@ -502,7 +506,7 @@ int sht_analysis(sfb_plan *h, const double *maps, int64_t nm, cudaStream_t st, b
         Stage s(h, stage(SFB_STAGE_RING_FFT), st);
         // the Gram refinement and niter = 0 read the spectra only in the first analysis pass (over the
         // span with data and the live chunks); the full refinement passes fold them over every ring
-        const bool skip_unread = (nm > 4 && p.d_gramts && p.niter > 0) || p.niter == 0;
+        const bool skip_unread = gram_mixed(p, nm) || p.niter == 0;
         if (src)
             SFB_TRY(field_ring_stage(h, *src, const_cast<double *>(maps), fbuf.ptr, reinterpret_cast<int *>(p.erow.ptr),
                                      nzr, skip_unread, st));
@@ -534,7 +538,7 @@ int sht_analysis(sfb_plan *h, const double *maps, int64_t nm, cudaStream_t st, b
                                        acc ? nullptr : nzr);
         else launch_leg_analysis(p, src, ncol, alm.ptr, acc, st);
     };
-    if (tc && ncol / 2 > 4 && p.d_gramts && p.niter > 0) {
+    if (tc && gram_mixed(p, nm)) {
         // Gram refinement: a <- a + (a0 - M a) - A_al(Fold(S_al a)) = a0 - D a - A_al(Fold(S_al a)),
         // M the Gram matrix of the alias-free rings (fold = identity there), D = M - I as the
         // tables store it, S_al / A_al the synthesis and analysis over the aliased rings r < ral.
@@ -896,9 +900,9 @@ int cat2amln_dev(sfb_plan *h, const double *rtp, const double *w, int64_t ngal, 
                                      h->d_pair_index, nmock, scale, smean, ralm, 2 * (nmock + 1), wk, win->w_ln, out,
                                      wk == SFB_WINDOW_DENSE ? nullptr : p.d_err, st);
             else
-                for (int j = 0; j < nmock; ++j)
-                    launch_project_poly(p, p.alm.ptr + 2 * nb * j, 2 * nm, scale[j], wk, win->w_ln, nb * (nmock - j),
-                                        nullptr, 0, out + 2 * p.nlmsize * j, st);
+                launch_project_poly(p, h->d_pair_index, h->d_noff, p.alm.ptr, nm, nmock, scale,
+                                    wk == SFB_WINDOW_SEPARABLE ? win->w_ln : nullptr, out,
+                                    wk == SFB_WINDOW_DENSE ? nullptr : p.d_err, st);
         }
         const float2 *adf = reinterpret_cast<const float2 *>(p.almdf.ptr);
         if (joint) {
@@ -937,8 +941,8 @@ int cat2amln_dev(sfb_plan *h, const double *rtp, const double *w, int64_t ngal, 
         }
     }
     SFB_CUDA_TRY(cudaGetLastError());
-    // the mixed projection, or the subtraction of a dense window after it, has checked what it wrote
-    const bool checked = p.radial_mode == SFB_RADIAL_POLY && p.precision == SFB_MIXED;
+    // the projection, or the mixed subtraction of a dense window after it, has checked what it wrote
+    const bool checked = p.radial_mode == SFB_RADIAL_POLY && (p.precision == SFB_MIXED || wk != SFB_WINDOW_DENSE);
     if (defer_finish) {
         Stage s(h, SFB_STAGE_OTHER, st);
         if (!checked) launch_check_finite(out, 2 * p.nlmsize * nmock, p.d_err, st);
@@ -1683,21 +1687,18 @@ static int field2anlm_vjp_impl(sfb_plan *h, const double *abar, int64_t nr, doub
     const bool resident = field_resident(p, nr, es, &cs);
     const int64_t fld = ((resident ? nr : cs) * p.npix * (int64_t)es + 7) / 8;     // field / staging, in doubles
     // [abar 2 nlmsize][gtab npairs x nr][Abar lmsize x 2 cs][field or staging]
-    SFB_TRY(grow(p, p.scratch, (size_t)(2 * p.nlmsize + p.npairs * nr + p.lmsize * 2 * cs + fld)));
-    double *d_ab = p.scratch.ptr, *d_g = d_ab + 2 * p.nlmsize, *d_A = d_g + p.npairs * nr;
+    SFB_TRY(grow(p, p.scratch, (size_t)(2 * p.nlmsize + p.npairs * nr + p.lmsize * 2 * cs + fld + 2)));
+    double *d_ab = p.scratch.ptr, *d_g = d_ab + 2 * p.nlmsize, *d_A = d_g + (p.npairs * nr + 1) / 2 * 2;
     double *d_f = d_A + p.lmsize * 2 * cs;
     SFB_CUDA_TRY(cudaMemcpyAsync(d_ab, abar, 2 * p.nlmsize * sizeof(double), cudaMemcpyHostToDevice, st));
     SFB_TRY(clear_err(p, st));
     bool copied = false;
     launch_gtab(p, nr, rmin, dr, 1, d_g, st);                // g_nl(r_s) r_s^2 dr, the field2anlm weights
-    SFB_TRY(grow(p, p.scratch2, (size_t)cs * p.npairs));
     SFB_TRY(grow(p, p.maps, (size_t)cs * p.npix));
     for (int64_t s0 = 0; s0 < nr; s0 += cs) {
         const int64_t nsc = std::min(cs, nr - s0);
-        SFB_CUDA_TRY(cudaMemcpy2DAsync(p.scratch2.ptr, nsc * sizeof(double), d_g + s0, nr * sizeof(double),
-                                       nsc * sizeof(double), p.npairs, cudaMemcpyDeviceToDevice, st));
         // Abar_s[lm] = sum_n g_nl(r_s) r_s^2 dr abar_nlm (the transpose of the radial sum)
-        launch_shell_alm_g(p, h->d_pair_index, h->d_noff, p.scratch2.ptr, nsc, d_ab, d_A, 2 * nsc, st);
+        launch_shell_alm_g(p, h->d_pair_index, h->d_noff, d_g + s0, nr, nsc, d_ab, d_A, 2 * nsc, st);
         // shells s0 .. s0+nsc of df: (ir, p) at ir + nr p (resident) or ir - s0 + nsc p (staging)
         const int64_t ld = resident ? nr : nsc, off = resident ? s0 : 0;
         const bool f32 = dtype == SFB_F32;
@@ -1767,20 +1768,17 @@ static int sfb_field2anlm_impl(sfb_plan *h, const void *f, int32_t dtype, int64_
     const size_t es = dtype == SFB_F32 ? sizeof(float) : sizeof(double);
     const bool resident = field_resident(p, nr, es, &cs);
     const int64_t fld = ((resident ? nr : cs) * p.npix * (int64_t)es + 7) / 8;     // field / staging, in doubles
-    // [gtab npairs*nr][out 2*nlmsize][acc 2*nlmsize][field or staging]
-    SFB_TRY(grow(p, p.scratch, (size_t)(p.npairs * nr + 4 * p.nlmsize + fld)));
-    double *d_g = p.scratch.ptr;
-    double *d_out = d_g + p.npairs * nr;
-    double *d_acc = d_out + 2 * p.nlmsize;
-    double *d_f = d_acc + 2 * p.nlmsize;
+    // [field or staging][acc 2*nlmsize][gtab npairs*nr]
+    SFB_TRY(grow(p, p.scratch, (size_t)(2 * p.nlmsize + p.npairs * nr + fld)));
+    double *d_f = p.scratch.ptr;
+    double *d_acc = d_f + fld;
+    double *d_g = d_acc + 2 * p.nlmsize;
     // all shells in one transform: the copy runs beside its ring stage
     const bool one = resident && cs >= nr && belt_groups(nr * p.npix * (int64_t)es) > 0;
     const FieldSrc src{static_cast<const char *>(f), reinterpret_cast<char *>(d_f), dtype, nr};
     if (resident && !one) SFB_CUDA_TRY(cudaMemcpyAsync(d_f, f, (size_t)nr * p.npix * es, cudaMemcpyHostToDevice, st));
     launch_gtab(p, nr, rmin, dr, 1, d_g, st);
-    SFB_CUDA_TRY(cudaMemsetAsync(d_acc, 0, 2 * p.nlmsize * sizeof(double), st));
     SFB_TRY(clear_err(p, st));
-    SFB_TRY(grow(p, p.scratch2, (size_t)cs * p.npairs));
     const bool mixed = p.precision == SFB_MIXED;
     for (int64_t s0 = 0; s0 < nr; s0 += cs) {
         const int64_t nsc = std::min(cs, nr - s0);
@@ -1801,14 +1799,14 @@ static int sfb_field2anlm_impl(sfb_plan *h, const void *f, int32_t dtype, int64_
                 else launch_transpose_ld(q, ld, p.npix, nsc, p.maps.ptr, p.npix, st);
             }
         }
-        SFB_TRY(sht_analysis(h, p.maps.ptr, nsc, st, false, -1, nullptr, true, LiveRings(), one ? &src : nullptr));
-        // gtab for this chunk: rows pair, cols nsc (copy sub-block)
-        SFB_CUDA_TRY(cudaMemcpy2DAsync(p.scratch2.ptr, nsc * sizeof(double), d_g + s0, nr * sizeof(double),
-                                       nsc * sizeof(double), p.npairs, cudaMemcpyDeviceToDevice, st));
-        launch_project_shells_g(p, p.scratch2.ptr, nsc, p.alm.ptr, 2 * nsc, d_out, st);
-        launch_axpy(d_acc, d_out, 2 * p.nlmsize, st);  // d_acc += d_out
+        // the Gram refinement leaves double-float pairs, which the projection reads as they are
+        const bool df = mixed && gram_mixed(p, nsc);
+        SFB_TRY(sht_analysis(h, p.maps.ptr, nsc, st, false, -1, nullptr, !df, LiveRings(), one ? &src : nullptr));
+        launch_project_shells_g(p, h->d_pair_index, h->d_noff, d_g + s0, nr, nsc, p.alm.ptr,
+                                df ? reinterpret_cast<const float2 *>(p.almdf.ptr) : nullptr, s0 > 0, d_acc,
+                                s0 + nsc == nr ? p.d_err : nullptr, st);
     }
-    SFB_TRY(finish(h, d_acc, st));
+    SFB_TRY(finish(h, d_acc, st, p.nlmsize > 0));
     SFB_CUDA_TRY(cudaMemcpyAsync(anlm_out, d_acc, 2 * p.nlmsize * sizeof(double), cudaMemcpyDeviceToHost, st));
     SFB_CUDA_TRY(cudaStreamSynchronize(st));
     return SFB_OK;
@@ -1822,15 +1820,14 @@ static int sfb_anlm2field_impl(sfb_plan *h, const double *anlm, int64_t nr, doub
     Plan &p = h->p;
     cudaStream_t st = h->stream;
     const double dr = (rmax - rmin) / (double)nr;
-    // [anlm 2*nlmsize][gtab npairs*nr][field nr*npix]
+    // [field nr*npix][anlm 2*nlmsize][gtab npairs*nr]
     SFB_TRY(grow(p, p.scratch, (size_t)(2 * p.nlmsize + p.npairs * nr + nr * p.npix)));
-    double *d_a = p.scratch.ptr;
+    double *d_f = p.scratch.ptr;
+    double *d_a = d_f + nr * p.npix;
     double *d_g = d_a + 2 * p.nlmsize;
-    double *d_f = d_g + p.npairs * nr;
     SFB_CUDA_TRY(cudaMemcpyAsync(d_a, anlm, 2 * p.nlmsize * sizeof(double), cudaMemcpyHostToDevice, st));
     launch_gtab(p, nr, rmin, dr, 0, d_g, st);
     const int64_t cs = std::max<int64_t>(1, std::min<int64_t>(nr, chunk_pairs(p)));
-    SFB_TRY(grow(p, p.scratch2, (size_t)cs * p.npairs));
     const size_t fsz = (size_t)2 * (p.lmax + 1) * p.nrn * 2 * cs;
     SFB_TRY(grow(p, p.gbuf, fsz));
     SFB_TRY(grow(p, p.alm, (size_t)p.lmsize * 2 * cs));
@@ -1840,9 +1837,7 @@ static int sfb_anlm2field_impl(sfb_plan *h, const double *anlm, int64_t nr, doub
     if (2 * cs > 8) ensure_tc64(p, st);
     for (int64_t s0 = 0; s0 < nr; s0 += cs) {
         const int64_t nsc = std::min(cs, nr - s0);
-        SFB_CUDA_TRY(cudaMemcpy2DAsync(p.scratch2.ptr, nsc * sizeof(double), d_g + s0, nr * sizeof(double),
-                                       nsc * sizeof(double), p.npairs, cudaMemcpyDeviceToDevice, st));
-        launch_shell_alm_g(p, h->d_pair_index, h->d_noff, p.scratch2.ptr, nsc, d_a, p.alm.ptr, 2 * nsc, st);
+        launch_shell_alm_g(p, h->d_pair_index, h->d_noff, d_g + s0, nr, nsc, d_a, p.alm.ptr, 2 * nsc, st);
         launch_leg_synthesis(p, p.alm.ptr, 2 * nsc, p.gbuf.ptr, st);
         // f[s0+s + nr p], written so by the tensor-core transform; else transposed from maps[s][p]
         bool pm = false;

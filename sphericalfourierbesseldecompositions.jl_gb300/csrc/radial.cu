@@ -216,46 +216,169 @@ void launch_radial_error_impl(const Plan &p, const double *coef, const double *y
     note_launch();
 }
 
-// a_nlm = scale * sum_b C[pair][b] A[lm][b] - window term.
-template <typename TA>
-__global__ void k_project_poly(const int32_t *out_pair, const int32_t *out_lm, const int32_t *pair_n,
-                               const int32_t *pair_l, int64_t nlmsize, int64_t nbasis, const double *coef,
-                               const TA *A, int64_t ldA, double scale, int window_kind,
-                               const double *w_ln, int lmax, int64_t mask_col, double *out) {
-    pdl_entry();
-    const int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (o >= nlmsize) return;
-    const int pr = out_pair[o];
-    const int64_t lm = out_lm[o];
-    const double *C = coef + (int64_t)pr * nbasis;
-    const TA *Ar = A + lm * ldA;
-    double re = 0.0, im = 0.0;
-    for (int64_t b = 0; b < nbasis; ++b) {
-        const double c = C[b];
-        re = fma(c, (double)Ar[2 * b], re);
-        im = fma(c, (double)Ar[2 * b + 1], im);
-    }
-    re *= scale;
-    im *= scale;
-    if (window_kind == SFB_WINDOW_SEPARABLE) {
-        const double wl = w_ln[pair_l[pr] + (int64_t)(lmax + 1) * (pair_n[pr] - 1)];
-        re -= wl * (double)Ar[2 * mask_col];
-        im -= wl * (double)Ar[2 * mask_col + 1];
-    }
-    out[2 * o] = re;
-    out[2 * o + 1] = im;
+// The FP64 radial projection of the FP64 catalogue transform and of fields,
+//   out[n,l,m] (+)= scale (sum_s T[pair(n,l)][s] A[lm][s] - w_ln[l,n] A[lm][mask])   (src/cat2anlm.jl:347-353)
+// with A in FP64 or as double-float pairs.  The outputs are few (25,295 at lmax 82) and the FP64 pipe bounds the sums
+// (205 shells: 10.4 million FMAs, about 20 us), if rows come in coalesced and the quarters of the SMs get equal work:
+// a block takes 16 orders of one degree and 2 PS_J radial indices, and its four warps each a quarter of the terms, 16
+// at a time through its own part of the shared memory, the next ones' loads in flight meanwhile.  FP64 rows: PS_J = 1,
+// small blocks, as most degrees have few radial indices (77 functions: 35 us as one thread an output, its rows
+// uncoalesced; 22 now).  Double-float rows: PS_J = 4, so that a value is widened once for eight indices (205 shells:
+// 73 us and 11 for a pass that widened all; 70 now).
+constexpr int PS_M = 16, PS_S = 16, PS_W = 4;
+
+struct Scales {
+    double v[MOCKS_MAX];
+};
+
+__device__ __forceinline__ double2 ps_value(double2 a) { return a; }
+// a float as a double in integer operations: the conversion instructions share the FP64 pipe with the sums
+__device__ __forceinline__ double widen(float f) {
+    const unsigned u = __float_as_uint(f), e = u << 1;
+    if (e - 0x01000000u >= 0xfe000000u) return e ? (double)f : 0.0;          // zero; subnormal, infinite, NaN
+    return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(u << 29));
+}
+__device__ __forceinline__ double2 ps_value(float4 a) {
+    return make_double2(widen(a.x) + widen(a.y), widen(a.z) + widen(a.w));
 }
 
-void launch_project_poly(const Plan &p, const double *A, int64_t ldA, double scale, int window_kind,
-                         const double *w_ln, int64_t mask_col, const double *Awin, int64_t ldW, double *out,
-                         cudaStream_t st) {
-    (void)Awin; (void)ldW;
+// grid: (degree and 16 orders, 2 PS_J radial indices, mocks); mock j's columns start at j * mcols, the mask's is the last
+template <typename TA, int PS_J>
+__global__ void __launch_bounds__(32 * PS_W) k_project64(const int32_t *pair_index, int nmax, int lmax,
+                                                         const int64_t *noff, const double *T, int64_t ldT, int K,
+                                                         const TA *A, int64_t ldA,
+                                                         const __grid_constant__ Scales scales, int64_t mcols,
+                                                         const double *w_ln, int add, int64_t nlmsize, double *out,
+                                                         int *err) {
+    pdl_entry();
+    constexpr int PS_N = 2 * PS_J;
+    __shared__ double2 As[PS_W][PS_M][PS_S + 1];
+    __shared__ double Ts[PS_W][PS_N][PS_S];
+    __shared__ double2 part[PS_W - 1][PS_J][32];
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, mock = blockIdx.z;
+    const int i = lane % PS_M, w = lane / PS_M;
+    // degrees 16 q .. 16 q + 15 have q + 1 blocks of orders each, 8 q (q + 1) blocks before them
+    const int x = blockIdx.x;
+    int q = (int)sqrtf((float)x * 0.125f);
+    while (8 * q * (q + 1) > x) --q;
+    while (8 * (q + 1) * (q + 2) <= x) ++q;
+    const int rem = x - 8 * q * (q + 1), l = PS_M * q + rem / (q + 1), m0 = PS_M * (rem % (q + 1));
+    const int n0 = blockIdx.y * PS_N + w, m = m0 + i;
+    int pr[PS_J];                                                         // lane (i, w): radial indices n0 + 2 j
+    bool any = false;
+#pragma unroll
+    for (int j = 0; j < PS_J; ++j) {
+        pr[j] = n0 + 2 * j < nmax ? pair_index[(int64_t)(n0 + 2 * j) * (lmax + 1) + l] : -1;
+        any |= pr[j] >= 0;
+    }
+    if (!__any_sync(0xffffffffu, any)) return;                            // (the same in every warp)
+    bool live[PS_J];
+#pragma unroll
+    for (int j = 0; j < PS_J; ++j) live[j] = __any_sync(0xffffffffu, pr[j] >= 0);
+    const int64_t lm0 = (int64_t)l * (l + 1) / 2;
+    A += mock * mcols;
+    // lane (i, w) loads column i of the rows w, w + 2, .. and of its own radial indices' rows of T
+    constexpr int NA = PS_M * PS_S / 32;
+    TA av[NA];
+    double tv[PS_J];
+    const TA *Ab = A + (lm0 + m0 + w) * ldA + i;
+    const int k0 = (int)((int64_t)K * wp / PS_W), k1 = (int)((int64_t)K * (wp + 1) / PS_W);
+    const int rows = l + 1 - m0 - w;                                      // row w + 2 j is there if 2 j < rows
+    auto load = [&](int s0) {
+        const bool in = s0 + i < k1;
+#pragma unroll
+        for (int j = 0; j < NA; ++j) {
+            av[j] = TA{};
+            if (in && 2 * j < rows) av[j] = Ab[2 * j * ldA + s0];
+        }
+#pragma unroll
+        for (int j = 0; j < PS_J; ++j) tv[j] = in && pr[j] >= 0 ? T[pr[j] * ldT + s0 + i] : 0.0;
+    };
+    double re[PS_J], im[PS_J];
+#pragma unroll
+    for (int j = 0; j < PS_J; ++j) re[j] = im[j] = 0.0;
+    if (k0 < k1) load(k0);
+    for (int s0 = k0; s0 < k1; s0 += PS_S) {
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < NA; ++j) As[wp][2 * j + w][i] = ps_value(av[j]);
+#pragma unroll
+        for (int j = 0; j < PS_J; ++j) Ts[wp][w + 2 * j][i] = tv[j];
+        __syncwarp();
+        if (s0 + PS_S < k1) load(s0 + PS_S);
+        const int ns = min(PS_S, k1 - s0);
+#pragma unroll 4
+        for (int s = 0; s < ns; ++s) {
+            const double2 a = As[wp][i][s];
+#pragma unroll
+            for (int j = 0; j < PS_J; ++j)
+                if (live[j]) {
+                    const double t = Ts[wp][w + 2 * j][s];
+                    re[j] = fma(t, a.x, re[j]);
+                    im[j] = fma(t, a.y, im[j]);
+                }
+        }
+    }
+    if (wp > 0)
+#pragma unroll
+        for (int j = 0; j < PS_J; ++j) part[wp - 1][j][lane] = make_double2(re[j], im[j]);
+    __syncthreads();
+    if (wp > 0 || m > l) return;
+#pragma unroll
+    for (int j = 0; j < PS_J; ++j) {
+        if (pr[j] < 0) continue;
+        const int n1 = n0 + 2 * j;
+        double vr = (re[j] + part[0][j][lane].x) + (part[1][j][lane].x + part[2][j][lane].x);
+        double vi = (im[j] + part[0][j][lane].y) + (part[1][j][lane].y + part[2][j][lane].y);
+        vr *= scales.v[mock];
+        vi *= scales.v[mock];
+        if (w_ln) {
+            const double wl = w_ln[l + (int64_t)(lmax + 1) * n1];
+            const double2 a = ps_value(A[(lm0 + m) * ldA + mcols * (gridDim.z - mock)]);
+            vr -= wl * a.x;
+            vi -= wl * a.y;
+        }
+        double *o = out + 2 * (mock * nlmsize + noff[n1] + lm0 + m);      // (a caller's pointer: eight-byte aligned)
+        if (add) {
+            vr += o[0];
+            vi += o[1];
+        }
+        o[0] = vr;
+        o[1] = vi;
+        if (err && !(isfinite(vr) && isfinite(vi))) atomicOr(err, ERR_NONFINITE_OUTPUT);
+    }
+}
+
+template <int PS_J, typename TA>
+static void project64(const Plan &p, const int32_t *pair_index, const int64_t *noff, const double *T, int64_t ldT,
+                      int64_t K, const TA *A, int64_t ldA, int nmock, const double *scale, int64_t mcols,
+                      const double *w_ln, bool add, double *out, int *err, cudaStream_t st) {
     if (p.nlmsize <= 0) return;
-    // a_lm are held in FP64 in both precision modes
-    launch_pdl(k_project_poly<double>, dim3((unsigned)((p.nlmsize + 127) / 128)), dim3(128), 0, st,
-            p.d_out_pair, p.d_out_lm, p.d_pair_n, p.d_pair_l, p.nlmsize, p.nbasis, p.d_coef, A, ldA, scale,
-            window_kind, w_ln, p.lmax, mask_col, out);
-        note_launch();
+    Scales sc;
+    std::copy(scale, scale + nmock, sc.v);
+    const unsigned full = (unsigned)((p.lmax + 1) / PS_M), rest = (unsigned)((p.lmax + 1) % PS_M);
+    dim3 grid(8 * full * (full + 1) + rest * (full + 1), (unsigned)((p.nmax + 2 * PS_J - 1) / (2 * PS_J)), (unsigned)nmock);
+    launch_pdl(k_project64<TA, PS_J>, grid, dim3(32 * PS_W), 0, st, pair_index, (int)p.nmax, (int)p.lmax, noff, T, ldT,
+               (int)K, A, ldA, sc, mcols, w_ln, (int)add, p.nlmsize, out, err);
+    note_launch();
+}
+
+void launch_project_poly(const Plan &p, const int32_t *pair_index, const int64_t *noff, const double *A, int64_t ncplx,
+                         int nmock, const double *scale, const double *w_ln, double *out, int *err, cudaStream_t st) {
+    project64<1>(p, pair_index, noff, p.d_coef, p.nbasis, p.nbasis, reinterpret_cast<const double2 *>(A), ncplx, nmock,
+              scale, p.nbasis, w_ln, false, out, err, st);
+}
+
+void launch_project_shells_g(const Plan &p, const int32_t *pair_index, const int64_t *noff, const double *gtab,
+                             int64_t ldg, int64_t nr, const double *A, const float2 *Adf, bool add, double *out,
+                             int *err, cudaStream_t st) {
+    const double one = 1.0;
+    if (Adf)
+        project64<4>(p, pair_index, noff, gtab, ldg, nr, reinterpret_cast<const float4 *>(Adf), nr, 1, &one, 0, nullptr,
+                  add, out, err, st);
+    else
+        project64<1>(p, pair_index, noff, gtab, ldg, nr, reinterpret_cast<const double2 *>(A), nr, 1, &one, 0, nullptr,
+                  add, out, err, st);
 }
 
 // out[o] -= Awin[lm][pair - pair0] for outputs whose pair lies in the chunk.
@@ -322,62 +445,71 @@ void launch_gtab(const Plan &p, int64_t nr, double rmin, double dr, int with_r2d
                                  note_launch();
 }
 
-// field2anlm radial sum: out[o] = sum_s gtab[pair][s] A[lm][s]  (src/cat2anlm.jl:347-353)
-__global__ void k_project_shells(const int32_t *out_pair, const int32_t *out_lm, int64_t nlmsize, const double *gtab,
-                                 int64_t nr, const double *A, int64_t ldA, double *out) {
+// anlm2field radial sum: A[lm][s] = sum_n gtab[pair(n,l)][s] a[idx(n,l,m)] (src/cat2anlm.jl:403-414).  A block takes
+// 128 shells of four orders of one degree: a shell's radial functions are read once for the four orders, whose
+// coefficients wait in shared memory (each sum in the order of n, one thread).
+// 128 shells at lmax 82: 46 us as one thread a coefficient, which found its degree by an FP64 root; 24 now.
+constexpr int SA_M = 4, SA_N = 64;
+__global__ void __launch_bounds__(128) k_shell_alm(const int32_t *pair_index, const int64_t *noff, int nmax, int lmax,
+                                                   const double *gtab, int64_t ldg, int64_t nr, const double *anlm,
+                                                   double *A, int64_t ldA) {
     pdl_entry();
-    const int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (o >= nlmsize) return;
-    const double *g = gtab + (int64_t)out_pair[o] * nr;
-    const double *Ar = A + (int64_t)out_lm[o] * ldA;
-    double re = 0.0, im = 0.0;
-    for (int64_t s = 0; s < nr; ++s) {
-        re = fma(g[s], Ar[2 * s], re);
-        im = fma(g[s], Ar[2 * s + 1], im);
-    }
-    out[2 * o] = re;
-    out[2 * o + 1] = im;
-}
-
-void launch_project_shells_g(const Plan &p, const double *gtab, int64_t nr, const double *A, int64_t ldA, double *out,
-                             cudaStream_t st) {
-    if (p.nlmsize <= 0) return;
-    launch_pdl(k_project_shells, dim3((unsigned)((p.nlmsize + 127) / 128)), dim3(128), 0, st, p.d_out_pair,
-        p.d_out_lm, p.nlmsize, gtab, nr, A, ldA, out);
-    note_launch();
-}
-
-// anlm2field radial sum: A[lm][s] = sum_n gtab[pair(n,l)][s] a[idx(n,l,m)] (src/cat2anlm.jl:403-414)
-__global__ void k_shell_alm(const int32_t *pair_index, const int64_t *noff, int nmax, int lmax, const double *gtab,
-                            int64_t nr, const double *anlm, double *A, int64_t ldA) {
-    pdl_entry();
-    const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= nr) return;
-    const int64_t lmsize = (int64_t)(lmax + 1) * (lmax + 2) / 2;
-    for (int64_t lm = blockIdx.y; lm < lmsize; lm += gridDim.y) {        // grid y is capped at 65535
-        // recover (l, m) from lm = l(l+1)/2 + m
-        int l = (int)((sqrt(8.0 * (double)lm + 1.0) - 1.0) / 2.0);
-        while ((int64_t)(l + 1) * (l + 2) / 2 <= lm) ++l;
-        while ((int64_t)l * (l + 1) / 2 > lm) --l;
-        const int m = (int)(lm - (int64_t)l * (l + 1) / 2);
-        double re = 0.0, im = 0.0;
-        for (int n = 1; n <= nmax; ++n) {
-            const int pr = pair_index[(int64_t)(n - 1) * (lmax + 1) + l];
-            if (pr < 0) continue;
-            const int64_t idx = noff[n - 1] + (int64_t)l * (l + 1) / 2 + m;
-            const double g = gtab[(int64_t)pr * nr + s];
-            re = fma(g, anlm[2 * idx], re);
-            im = fma(g, anlm[2 * idx + 1], im);
+    __shared__ double2 an[SA_N][SA_M];
+    __shared__ int prs[SA_N];
+    // degrees 4 q .. 4 q + 3 have q + 1 blocks of orders each, 2 q (q + 1) blocks before them
+    const int x = blockIdx.x;
+    int q = (int)sqrtf((float)x * 0.5f);
+    while (2 * q * (q + 1) > x) --q;
+    while (2 * (q + 1) * (q + 2) <= x) ++q;
+    const int rem = x - 2 * q * (q + 1), l = SA_M * q + rem / (q + 1), m0 = SA_M * (rem % (q + 1));
+    const int64_t lm0 = (int64_t)l * (l + 1) / 2;
+    const int nm = min(SA_M, l + 1 - m0);
+    for (int64_t s0 = (int64_t)blockIdx.y * 128; s0 < nr; s0 += (int64_t)gridDim.y * 128) {
+        const int64_t s = s0 + threadIdx.x;
+        double re[SA_M], im[SA_M];
+#pragma unroll
+        for (int j = 0; j < SA_M; ++j) re[j] = im[j] = 0.0;
+        for (int n0 = 0; n0 < nmax; n0 += SA_N) {
+            const int nn = min(SA_N, nmax - n0);
+            __syncthreads();
+            for (int i = threadIdx.x; i < nn; i += 128) prs[i] = pair_index[(int64_t)(n0 + i) * (lmax + 1) + l];
+            __syncthreads();
+            for (int i = threadIdx.x; i < nn * SA_M; i += 128) {
+                const int n = i / SA_M, j = i % SA_M;
+                if (prs[n] < 0 || j >= nm) continue;
+                const double *a = anlm + 2 * (noff[n0 + n] + lm0 + m0 + j);
+                an[n][j] = make_double2(a[0], a[1]);
+            }
+            __syncthreads();
+            if (s >= nr) continue;
+#pragma unroll 4
+            for (int n = 0; n < nn; ++n) {
+                const int pr = prs[n];
+                if (pr < 0) continue;
+                const double g = gtab[(int64_t)pr * ldg + s];
+#pragma unroll
+                for (int j = 0; j < SA_M; ++j)
+                    if (j < nm) {
+                        re[j] = fma(g, an[n][j].x, re[j]);
+                        im[j] = fma(g, an[n][j].y, im[j]);
+                    }
+            }
         }
-        A[lm * ldA + 2 * s] = re;
-        A[lm * ldA + 2 * s + 1] = (m == 0) ? 0.0 : im;
+        if (s >= nr) continue;
+#pragma unroll
+        for (int j = 0; j < SA_M; ++j)
+            if (j < nm)
+                *reinterpret_cast<double2 *>(A + (lm0 + m0 + j) * ldA + 2 * s) =
+                    make_double2(re[j], m0 + j == 0 ? 0.0 : im[j]);
     }
 }
 
-void launch_shell_alm_g(const Plan &p, const int32_t *pair_index, const int64_t *noff, const double *gtab, int64_t nr,
-                        const double *anlm, double *A, int64_t ldA, cudaStream_t st) {
-    dim3 grid((unsigned)((nr + 127) / 128), (unsigned)std::min<int64_t>(p.lmsize, 65535));
-    launch_pdl(k_shell_alm, dim3(grid), dim3(128), 0, st, pair_index, noff, p.nmax, p.lmax, gtab, nr, anlm, A, ldA);
+void launch_shell_alm_g(const Plan &p, const int32_t *pair_index, const int64_t *noff, const double *gtab, int64_t ldg,
+                        int64_t nr, const double *anlm, double *A, int64_t ldA, cudaStream_t st) {
+    const unsigned full = (unsigned)((p.lmax + 1) / SA_M), rest = (unsigned)((p.lmax + 1) % SA_M);
+    dim3 grid(2 * full * (full + 1) + rest * (full + 1), (unsigned)std::min<int64_t>((nr + 127) / 128, 65535));
+    launch_pdl(k_shell_alm, grid, dim3(128), 0, st, pair_index, noff, (int)p.nmax, (int)p.lmax, gtab, ldg, nr, anlm, A,
+               ldA);
     note_launch();
 }
 
@@ -585,17 +717,14 @@ __device__ __forceinline__ void pj_mac(pacc &a, float2 c, float xh, float xl) {
     a.lo = fmaf(c.y, xh, fmaf(c.x, xl, (a.lo + err) + e));
 }
 
-struct Scales {
-    double v[MOCKS_MAX];
-};
-
 // grid.y: mocks (launch_project_mixed says where each one's data lie)
 template <int KS>
 __global__ void __launch_bounds__(32 * KS) k_project_mixed(const float2 *Adf, int64_t ldA,
                                                               int64_t nbasis, const float2 *CT, int nmax,
                                                               int lmax, const int3 *tiles,
                                                               const int64_t *noff,
-                                                              const int32_t *pair_index, Scales scales,
+                                                              const int32_t *pair_index,
+                                                              const __grid_constant__ Scales scales,
                                                               const double *smean, int64_t npairs,
                                                               const double *ralm, int64_t ldR,
                                                               int64_t nlmsize, int window_kind,
@@ -628,7 +757,7 @@ __global__ void __launch_bounds__(32 * KS) k_project_mixed(const float2 *Adf, in
 #pragma unroll
         for (int j = 0; j < PJ_NPT; ++j) {
             if (j < npt) {
-                const float2 c = __ldg(cb + j);
+                const float2 c = __ldg(cb + j);   // (a table of the plan)
                 pj_mac(re[j], c, a.x, a.y);
                 pj_mac(im[j], c, a.z, a.w);
             }

@@ -362,9 +362,8 @@ void launch_fold_residual(const Plan &p, const double *F, const double *G, int64
                           int *Ecol = nullptr, int rlim = -1, bool ecol_preset = false);
 void launch_radial_coeffs(const Plan &p, const double *gl_x, const double *pq, int Q, double *coef,
                           cudaStream_t st);
-void launch_project_poly(const Plan &p, const double *A, int64_t ldA, double scale, int window_kind,
-                         const double *w_ln, int64_t mask_col, const double *Awin, int64_t ldW,
-                         double *out, cudaStream_t st);
+void launch_project_poly(const Plan &p, const int32_t *pair_index, const int64_t *noff, const double *A, int64_t ncplx,
+                         int nmock, const double *scale, const double *w_ln, double *out, int *err, cudaStream_t st);
 void launch_to_float(const double *in, int64_t n, float *out, cudaStream_t st);
 // double -> normalised double-float pairs (maps of the mixed-precision transform)
 void launch_to_df(const double *in, int64_t n, float2 *out, cudaStream_t st);
