@@ -50,6 +50,7 @@
 // the row-exponent pass with ZERO_ROW_E) are never read.  A tile with no live
 // row writes zero spectra without MMAs.  Two tiles whose southern rows are all
 // zero run as one tile of 128 northern rows (F+ = F- = F_N).  Both are exact.
+#include <algorithm>
 #include <cuda_bf16.h>
 
 #include <cmath>
@@ -123,31 +124,40 @@ __global__ void __launch_bounds__(128) k_ring_rowexp(const float2 *maps, int64_t
     const int64_t b = (int64_t)blockIdx.y * 4 + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     const RingGeom g = rings[r];
+    // both hemispheres' rows together: their loads are in flight at once (104 maps of nside 128: 25 -> 20 us)
     bool any = false;
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        if (b >= nmaps) break;
-        if (b < live.n && !live.ring[(b / live.per) * nrings + (h ? nrings - 1 - r : r)]) {
-            if (lane == 0) erow[((int64_t)h * nrn + r) * nmaps + b] = ZERO_ROW_E;
-            continue;
+    if (b < nmaps) {
+        bool on[2] = {true, true};
+        if (b < live.n) {
+            const int *lr = live.ring + (b / live.per) * nrings;
+            on[0] = lr[r] != 0;
+            on[1] = lr[nrings - 1 - r] != 0;
         }
-        const float2 *x = maps + b * npix + (h ? g.start_s : g.start_n);
-        float mx = 0.f;
-        bool fin = true;
+        const float2 *x = maps + b * npix;
+        float mx[2] = {0.f, 0.f};
+        bool fin[2] = {true, true};
+#pragma unroll 2
         for (int j = lane; j < g.nph; j += 32) {
-            const float2 v = x[j];                       // |hi + lo| < 2^E when |hi| < 2^E
-            fin &= isfinite(v.x) && isfinite(v.y);
-            mx = fmaxf(mx, fabsf(v.x));
+            float2 v[2];
+            v[0] = on[0] ? x[g.start_n + j] : make_float2(0.f, 0.f);      // |hi + lo| < 2^E when |hi| < 2^E
+            v[1] = on[1] ? x[g.start_s + j] : make_float2(0.f, 0.f);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                fin[h] &= isfinite(v[h].x) && isfinite(v[h].y);
+                mx[h] = fmaxf(mx[h], fabsf(v[h].x));
+            }
         }
-        for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-        fin = __all_sync(0xffffffffu, fin);
-        int E = scale_exp(mx);
-        const int lg = 32 - __clz(g.nph - 1);              // ceil(log2 n)
-        E += max(0, lg - 10);
-        E = max(-90, min(E, 100));
-        if (mx == 0.f && fin) E = ZERO_ROW_E;
-        else any = true;
-        if (lane == 0) erow[((int64_t)h * nrn + r) * nmaps + b] = E;
+        const int lg = 32 - __clz(g.nph - 1);                  // ceil(log2 n)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            for (int off = 16; off > 0; off >>= 1) mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], off));
+            fin[h] = __all_sync(0xffffffffu, fin[h]);
+            int E = scale_exp(mx[h]) + max(0, lg - 10);
+            E = max(-90, min(E, 100));
+            if (mx[h] == 0.f && fin[h]) E = ZERO_ROW_E;
+            else any = true;
+            if (lane == 0) erow[((int64_t)h * nrn + r) * nmaps + b] = E;
+        }
     }
     // the ring-pair range: one thread per block, and an atomic only where it moves a bound
     if (__syncthreads_or(any) && threadIdx.x == 0) {
@@ -165,18 +175,23 @@ __global__ void __launch_bounds__(128) k_ring_rowexp(const float2 *maps, int64_t
 // Grid (tiles, classes, groups of SLICE_CPG chunks), one thread per (row,
 // 16-pixel half) as the DFT's imaged producers.
 constexpr int SLICE_CPG = 4;
+// Row tiles [t0, t1) of each (equatorial) class that one launch takes, in whole pairs; the grid counts from t0.
+struct Tiles {
+    int t0[2], t1[2];
+};
 __global__ void __launch_bounds__(NPROD) k_dft_slice_a(const float2 *maps, int64_t npix, int64_t nmaps,
                                                         const RingGeom *rings, int nrn,
                                                         const int32_t *cls_rings,
                                                         const int32_t *cls_off,
                                                         const int *erow, const int64_t *aoff,
-                                                        unsigned char *aimg) {
+                                                        unsigned char *aimg, Tiles tiles) {
     pdl_entry();
     const int cls = blockIdx.y;
     const int rb = cls_off[cls];
     const int64_t npairs = (int64_t)(cls_off[cls + 1] - rb) * nmaps;
-    const int ty = blockIdx.x;
+    const int ty = tiles.t0[cls & 1] + blockIdx.x;
     const int64_t pair0 = (int64_t)ty * NPAIR;
+    if (ty >= tiles.t1[cls & 1]) return;
     if (pair0 >= npairs || (int)blockIdx.z * SLICE_CPG * KC >= rings[cls_rings[rb]].nph) return;
     const int tid = threadIdx.x;
     bool snz = false;
@@ -253,7 +268,7 @@ __global__ void __launch_bounds__(NTHR, 1) k_ring_dft_tc(const float2 *maps, int
                                                          int64_t ldF, float2 wdf, const unsigned char *dead,
                                                          int ntn, const int *span, int rev,
                                                          const int64_t *aoff,
-                                                         const unsigned char *aimg, int *err) {
+                                                         const unsigned char *aimg, Tiles tiles, int *err) {
     pdl_entry();
     extern __shared__ __align__(1024) unsigned char smem[];
     // grid (column blocks u, row tiles, classes): the column blocks of one row tile are launched
@@ -262,9 +277,9 @@ __global__ void __launch_bounds__(NTHR, 1) k_ring_dft_tc(const float2 *maps, int
     const int cls = rev ? (int)(gridDim.z - 1 - blockIdx.z) : (int)blockIdx.z;
     const int rb = cls_off[cls];
     const int64_t npairs = (int64_t)(cls_off[cls + 1] - rb) * nmaps;
-    const int ty = blockIdx.y;
+    const int ty = tiles.t0[cls & 1] + blockIdx.y;
     const int64_t pair0 = (int64_t)ty * NPAIR;
-    if (pair0 >= npairs) return;
+    if (ty >= tiles.t1[cls & 1] || pair0 >= npairs) return;
     const int u = blockIdx.x;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // dead: the spectra of ring r and column block u that no analysis chunk reads (lambda is zero in
@@ -751,17 +766,32 @@ int ring_tc_begin(Plan &p, int64_t nmaps, int *nzr, cudaStream_t st) {
     return grow(p, p.aimg, (size_t)(p.h_aimg_off[ncls] * (4 * dft::PLANE) / sizeof(double)));
 }
 
-// Slicing pass and DFT of the equatorial classes (eq) or the polar rings, after their row exponents.
+// Slicing pass and DFT of the equatorial rings [r0, r1) (eq) or the polar rings [r0, r1), after their row exponents.
+// A tile pair of an equatorial class that holds rows of rings before and after r0 or r1 goes with its last ring, so
+// launches over successive ranges take every tile once, when all of its rows are there.
 static void ring_tc_dft(const Plan &p, const float2 *maps, int64_t nmaps, float2 *F, const int *erow,
-                        const unsigned char *dead, const int *span, bool eq, cudaStream_t st) {
+                        const unsigned char *dead, const int *span, bool eq, int r0, int r1, cudaStream_t st) {
     const unsigned ntn = (unsigned)((p.lmax + 1 + 63) / 64);
     const double wq = 4.0 * M_PI / (double)p.npix;
     const float2 wdf = make_float2((float)wq, (float)(wq - (double)(float)wq));
-    const unsigned mtiles = (unsigned)((nmaps + dft::NPAIR - 1) / dft::NPAIR);
-    const int64_t eq_tiles = ((int64_t)p.eq_max_rings * nmaps + dft::NPAIR - 1) / dft::NPAIR;
-    const unsigned tiles = eq ? (unsigned)eq_tiles : mtiles, ncls = (unsigned)(eq ? p.n_eq_cls : p.n_polar);
-    if (ncls == 0) return;
-    const int c0 = eq ? p.n_polar : 0;
+    const int c0 = eq ? p.n_polar : r0;              // polar ring r is class r
+    const unsigned ncls = (unsigned)(eq ? p.n_eq_cls : r1 - r0);
+    dft::Tiles range{{0, 0}, {0x7fffffff, 0x7fffffff}};
+    unsigned tiles = (unsigned)((nmaps + dft::NPAIR - 1) / dft::NPAIR);
+    if (eq) {
+        tiles = 0;
+        for (unsigned c = 0; c < ncls; ++c) {
+            const int32_t *first = p.h_cls_rings.data() + p.h_cls_off[c0 + c], *end = p.h_cls_rings.data() + p.h_cls_off[c0 + c + 1];
+            auto upto = [&](int r) {                  // tiles of the rings below r: whole pairs, or all
+                const int64_t rows = (std::lower_bound(first, end, r) - first) * nmaps;
+                return (int)(r >= p.nrn ? (rows + dft::NPAIR - 1) / dft::NPAIR : rows / (2 * dft::NPAIR) * 2);
+            };
+            range.t0[c] = upto(r0);
+            range.t1[c] = upto(r1);
+            tiles = std::max(tiles, (unsigned)(range.t1[c] - range.t0[c]));
+        }
+    }
+    if (ncls == 0 || tiles == 0) return;
     const bool ai = eq ? aimg_eq(p) : aimg_polar(p);
     // imaged classes read B from the image, the others gather it from the ring table
     const bool img = eq ? p.d_dtimg != nullptr : p.dtimg_polar && !(ai && p.dft_polar_gather);
@@ -770,14 +800,14 @@ static void ring_tc_dft(const Plan &p, const float2 *maps, int64_t nmaps, float2
         // chunk groups: the longest ring (4 nside pixels) in groups of SLICE_CPG chunks
         const unsigned ngrp = (unsigned)((4 * p.nside + dft::KC * dft::SLICE_CPG - 1) / (dft::KC * dft::SLICE_CPG));
         launch_pdl(dft::k_dft_slice_a, dim3(tiles, ncls, ngrp), dim3(dft::NPROD), 0, st, maps, p.npix, nmaps,
-            p.d_rings, (int)p.nrn, p.d_cls_rings, p.d_cls_off + c0, erow, p.d_aimg_off + c0, aimg);
+            p.d_rings, (int)p.nrn, p.d_cls_rings, p.d_cls_off + c0, erow, p.d_aimg_off + c0, aimg, range);
         note_launch();
     }
     auto go = [&](auto kernel) {
         launch_pdl(kernel, dim3(ntn, tiles, ncls), dim3(dft::NTHR), dft::SMEM, st, maps, p.npix, nmaps, p.d_rings,
             (int)p.nrn, p.lmax, p.d_cls_rings, p.d_cls_off + c0, erow, p.d_dtw, p.d_dtw_off,
             img ? p.d_dtimg : nullptr, img ? p.d_dtimg_off + c0 : nullptr, F, 2 * nmaps, wdf, dead, (int)ntn, span,
-            eq ? 0 : 1, ai ? p.d_aimg_off + c0 : nullptr, ai ? aimg : nullptr, p.d_err);
+            eq ? 0 : 1, ai ? p.d_aimg_off + c0 : nullptr, ai ? aimg : nullptr, range, p.d_err);
     };
     if (img && ai) go(dft::k_ring_dft_tc<true, true>);
     else if (ai) go(dft::k_ring_dft_tc<false, true>);
@@ -786,15 +816,14 @@ static void ring_tc_dft(const Plan &p, const float2 *maps, int64_t nmaps, float2
     note_launch();
 }
 
-// The equatorial rings (eq) or the polar rings of a transform begun with ring_tc_begin, alone: their maps arrive
-// apart (a field that is still being copied).  The span of ring pairs with data is not known yet, so the spectra
-// outside it are written too.
+// The ring pairs [r0, r1) of a transform begun with ring_tc_begin, alone, either all equatorial or all polar: their
+// maps arrive apart (a field that is still being copied).  Ranges of equatorial rings come in ascending order.  The
+// span of ring pairs with data is not known yet, so the spectra outside it are written too.
 void ring_tc_part(const Plan &p, const float2 *maps, int64_t nmaps, float2 *F, int *erow, int *nzr, bool skip_unread,
-                  bool eq, cudaStream_t st) {
-    const int r0 = eq ? p.n_polar : 0, nr = eq ? (int)p.nrn - p.n_polar : p.n_polar;
-    if (nr <= 0) return;
-    ring_rowexp(p, maps, nmaps, erow, nzr, LiveRings(), r0, nr, st);
-    ring_tc_dft(p, maps, nmaps, F, erow, skip_unread ? p.d_dft_dead : nullptr, nullptr, eq, st);
+                  int r0, int r1, cudaStream_t st) {
+    if (r1 <= r0) return;
+    ring_rowexp(p, maps, nmaps, erow, nzr, LiveRings(), r0, r1 - r0, st);
+    ring_tc_dft(p, maps, nmaps, F, erow, skip_unread ? p.d_dft_dead : nullptr, nullptr, r0 >= p.n_polar, r0, r1, st);
 }
 
 int launch_ring_analysis_tc(Plan &p, const float2 *maps, int64_t nmaps, float2 *F, int *erow, int *nzr,
@@ -814,8 +843,8 @@ int launch_ring_analysis_tc(Plan &p, const float2 *maps, int64_t nmaps, float2 *
         cudaEventRecord(p.dft_fork, st);
         cudaStreamWaitEvent(p.dft_side, p.dft_fork, 0);
     }
-    ring_tc_dft(p, maps, nmaps, F, erow, dead, span, true, two ? p.dft_side : st);
-    ring_tc_dft(p, maps, nmaps, F, erow, dead, span, false, st);
+    ring_tc_dft(p, maps, nmaps, F, erow, dead, span, true, p.n_polar, (int)p.nrn, two ? p.dft_side : st);
+    ring_tc_dft(p, maps, nmaps, F, erow, dead, span, false, 0, p.n_polar, st);
     if (two) {
         cudaEventRecord(p.dft_join, p.dft_side);
         cudaStreamWaitEvent(st, p.dft_join, 0);

@@ -379,7 +379,7 @@ int launch_ring_analysis_tc(Plan &p, const float2 *maps, int64_t nmaps, float2 *
                             cudaStream_t st, const LiveRings &live = LiveRings(), bool skip_unread = false);
 int ring_tc_begin(Plan &p, int64_t nmaps, int *nzr, cudaStream_t st);
 void ring_tc_part(const Plan &p, const float2 *maps, int64_t nmaps, float2 *F, int *erow, int *nzr, bool skip_unread,
-                  bool eq, cudaStream_t st);
+                  int r0, int r1, cudaStream_t st);
 uint2 dft_slices(double v, int EB);
 int64_t dft_image_offsets(const Plan &p, const std::vector<int32_t> &crings, const std::vector<int32_t> &coff,
                           bool with_polar, std::vector<int64_t> &off, int &max_nch);
