@@ -20,7 +20,7 @@ using namespace tc;
 constexpr int ND = 7;                                  // digits, and levels kept
 constexpr int KC = 16;                                 // K per chunk (one MMA K step)
 constexpr int MTILE = 128;                             // data columns per CTA
-constexpr int NT = 32;                                 // table rows per CTA
+constexpr int NT = LEG64_TILE;                         // table rows per CTA
 constexpr int SBK = 16;                                // chunks per exact K block (256 values)
 // eight warps: a ninth for the MMAs would leave 96 registers a thread at two CTAs per SM instead of 128
 constexpr int NTH = 256;

@@ -58,7 +58,7 @@ __global__ void __launch_bounds__(NTH, 2) k_leg64(const double *data, int64_t nc
     const int z = blockIdx.z, m = z >> 1, par = z & 1;
     const bool first_task = (int)blockIdx.y < ny0;
     const Task64 &t = first_task ? t0 : t1;
-    const int tile = first_task ? blockIdx.y : blockIdx.y - ny0;
+    const int tile = (first_task ? blockIdx.y : blockIdx.y - ny0) + (first_task ? t0.tile0 : t1.tile0);
     const int nrows = rows_of(m, par, lmax);
     const int N = t.n_is_rows ? nrows : t.nout;                  // table rows of the block
     const int nwrite = t.n_is_rows ? nrows : t.nlim;             // rows written
@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(NTH, 2) k_leg64_short(const double *data, int6
     auto job_at = [&](int i, TileJob &j) -> bool {
         j.task = i < ny0 ? 0 : 1;
         const Task64 &t = j.task ? t1 : t0;
-        j.tile = j.task ? i - ny0 : i;
+        j.tile = (j.task ? i - ny0 : i) + t.tile0;
         const int N = t.n_is_rows ? nrows : t.nout;
         j.nwrite = t.n_is_rows ? nrows : t.nlim;
         if (j.tile * NT >= j.nwrite || (t.n_is_rows && nrows == 0)) return false;
@@ -590,6 +590,21 @@ void launch_leg_analysis64(const Plan &p, const double *F, int64_t ncol, double 
     note_launch();
 }
 
+static void leg_synthesis64(const Plan &p, const double *A, int64_t ncol, const Task64 &g, const Task64 &s, int ny0,
+                            int ny1, cudaStream_t st) {
+    if (ny0 + ny1 == 0) return;
+    if (p.lmax / 2 + 1 <= t64::RES * t64::KC) {
+        set_smem(t64::k_leg64_short<true>, t64::SMEM_RES);
+        launch_pdl(t64::k_leg64_short<true>, dim3(grid64(p, ncol, (int)short_split(p, ncol, ny0 + ny1))),
+            dim3(t64::NTH), t64::SMEM_RES, st, A, ncol, p.lmax, (int)p.nrn, 0, g, s, ny0, ny1, p.d_err);
+    } else {
+        set_smem(t64::k_leg64<true>, t64::SMEM);
+        launch_pdl(t64::k_leg64<true>, dim3(grid64(p, ncol, ny0 + ny1)), dim3(t64::NTH), t64::SMEM, st, A, ncol,
+            p.lmax, (int)p.nrn, 0, nullptr, g, s, ny0, p.d_err);
+    }
+    note_launch();
+}
+
 // G of the rings r < rlim (G may be null) and, with Anew, the Gram update Anew = A0 - D A.
 void launch_leg_synthesis64(const Plan &p, const double *A, int64_t ncol, double *G, cudaStream_t st, int rlim,
                             const double *A0, double *Anew) {
@@ -600,19 +615,19 @@ void launch_leg_synthesis64(const Plan &p, const double *A, int64_t ncol, double
     s.out = G;
     s.mode = 0;
     s.nlim = rlim;
-    const int ny0 = Anew ? g.ntile : 0, ny1 = G && rlim > 0 ? (rlim + t64::NT - 1) / t64::NT : 0;
-    if (ny0 + ny1 == 0) return;
-    if (p.lmax / 2 + 1 <= t64::RES * t64::KC) {
-        set_smem(t64::k_leg64_short<true>, t64::SMEM_RES);
-        launch_pdl(t64::k_leg64_short<true>, dim3(grid64(p, ncol, (int)short_split(p, ncol, ny0 + ny1))),
-            dim3(t64::NTH), t64::SMEM_RES, st, A, ncol, p.lmax, (int)p.nrn, 0, g, s, ny0, ny1, p.d_err);
-        note_launch();
-        return;
-    }
-    set_smem(t64::k_leg64<true>, t64::SMEM);
-    launch_pdl(t64::k_leg64<true>, dim3(grid64(p, ncol, ny0 + ny1)), dim3(t64::NTH), t64::SMEM, st, A, ncol, p.lmax,
-        (int)p.nrn, 0, nullptr, g, s, ny0, p.d_err);
-    note_launch();
+    leg_synthesis64(p, A, ncol, g, s, Anew ? g.ntile : 0, G && rlim > 0 ? (rlim + t64::NT - 1) / t64::NT : 0, st);
+}
+
+// G of the tiles of LEG64_TILE rings that hold the rings [r0, r1).
+void launch_leg_synthesis64_rings(const Plan &p, const double *A, int64_t ncol, double *G, int r0, int r1,
+                                  cudaStream_t st) {
+    Task64 s = p.t64[1];
+    s.out = G;
+    s.mode = 0;
+    s.tile0 = r0 / t64::NT;
+    const int t1 = (r1 + t64::NT - 1) / t64::NT;
+    s.nlim = std::min((int)p.nrn, t1 * t64::NT);
+    if (r1 > r0) leg_synthesis64(p, A, ncol, s, s, 0, t1 - s.tile0, st);
 }
 
 }  // namespace sfb

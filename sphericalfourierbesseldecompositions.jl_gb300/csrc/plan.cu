@@ -692,26 +692,49 @@ int reference_alm(sfb_plan *h, const double *ref, int64_t nref, cudaStream_t st)
     return rc;
 }
 
-// Pixel-major ring synthesis into out[pixel ld + map] of nm maps on the device; with host, which has the same layout,
-// each ring group's pixels go there on the side stream while the next group is formed (the caller's stream waits
-// for the copies at the end).  *done: false when the plan's tensor-core transform is not available (nothing done).
+// The Legendre synthesis of A into G, and the pixel-major ring synthesis of G into out[pixel ld + map] of nm maps on the
+// device; with host, which has the same layout, ring group by ring group, each group's pixels going there on the side
+// stream while the next one is formed (the caller's stream waits for the copies at the end).  The copy bounds these
+// calls (201 MB at 193 GB/s: 1040 us), so what is done before it begins counts: the rings of the first group only, not
+// all (128 shells of nside 128: 1345 -> 1235 us a call).  *done: false when out is null or the plan's tensor-core transform is not available (then G is
+// all there is).
 // *copied: the field is on its way to host.
-int synthesis_pixmajor(sfb_plan *h, const double *G, int64_t nm, void *out, int64_t ld, bool f32, void *host,
+int synthesis_pixmajor(sfb_plan *h, const double *A, double *G, int64_t nm, void *out, int64_t ld, bool f32, void *host,
                        cudaStream_t st, bool *done, bool *copied) {
     Plan &p = h->p;
     *done = *copied = false;
-    if (nm < RING64_MIN) return SFB_OK;
+    const int64_t ncol = 2 * nm;
     const size_t row = (size_t)ld * (f32 ? sizeof(float) : sizeof(double));
     const int belt = belt_groups((int64_t)row * p.npix);
-    if (!host || belt == 0) {
+    const bool groups = out && host && belt > 0 && nm >= RING64_MIN;
+    // The Legendre synthesis in parts too where a part fills the SMs (two CTAs each) and the copy, not the ring
+    // transform, is what the rest waits for: each part forms the columns' digits again (128 FP64 maps: 1328 -> 1241 us
+    // a call; 64 maps into FP32: 704 -> 717).
+    const int64_t ctas = (ncol + 127) / 128 * 2 * (p.lmax + 1);
+    const bool parts = groups && p.tc64_state > 0 && !f32 && ctas >= 304;
+    if (!parts) launch_leg_synthesis(p, A, ncol, G, st);
+    if (!out || nm < RING64_MIN) return SFB_OK;
+    if (!groups) {
         *done = launch_ring_synthesis64(p, G, nm, out, ld, true, f32, st);
         return SFB_OK;
     }
     const std::vector<PixGroup> gs = pix_groups(p, belt);
+    const int tile_first = p.n_polar / LEG64_TILE;
+    int tile_next = tile_first;
     for (size_t i = 0; i < gs.size(); ++i) {
         const PixGroup &g = gs[i];
+        if (parts) {
+            // the belt from the caps to the equator, then the caps up to the belt's first tile
+            const int end = g.r0 < p.n_polar ? tile_first * LEG64_TILE : g.r1;
+            const int beg = g.r0 < p.n_polar ? 0 : tile_next * LEG64_TILE;
+            launch_leg_synthesis64_rings(p, A, ncol, G, beg, end, st);
+            if (g.r0 >= p.n_polar) tile_next = std::max(tile_next, (end + LEG64_TILE - 1) / LEG64_TILE);
+        }
         if (!launch_ring_synthesis64(p, G, nm, out, ld, true, f32, st, g.z0, g.nz)) {
-            if (i == 0) return SFB_OK;
+            if (i == 0) {
+                if (parts) launch_leg_synthesis(p, A, ncol, G, st);
+                return SFB_OK;
+            }
             return fail(SFB_ENOMEM, "ring synthesis workspace lost");
         }
         SFB_CUDA_TRY(cudaEventRecord(h->ev_copy[i], st));
@@ -780,9 +803,8 @@ int sht_analysis_adjoint(sfb_plan *h, double *abar, int64_t nm, double *maps_out
         }
         x = p.alm.ptr;
     }
-    launch_leg_synthesis(p, x, ncol, p.gbuf.ptr, st);
     bool pm = false, cp = false;
-    if (pix_out) SFB_TRY(synthesis_pixmajor(h, p.gbuf.ptr, nm, pix_out, pix_ld, pix_f32, pix_host, st, &pm, &cp));
+    SFB_TRY(synthesis_pixmajor(h, x, p.gbuf.ptr, nm, pix_out, pix_ld, pix_f32, pix_host, st, &pm, &cp));
     if (copied) *copied = cp;
     if (pixmajor) *pixmajor = pm;
     if (!pm) launch_ring_synthesis(p, p.gbuf.ptr, nm, maps_out, st);
@@ -1846,10 +1868,9 @@ static int sfb_anlm2field_impl(sfb_plan *h, const double *anlm, int64_t nr, doub
     for (int64_t s0 = 0; s0 < nr; s0 += cs) {
         const int64_t nsc = std::min(cs, nr - s0);
         launch_shell_alm_g(p, h->d_pair_index, h->d_noff, d_g + s0, nr, nsc, d_a, p.alm.ptr, 2 * nsc, st);
-        launch_leg_synthesis(p, p.alm.ptr, 2 * nsc, p.gbuf.ptr, st);
         // f[s0+s + nr p], written so by the tensor-core transform; else transposed from maps[s][p]
         bool pm = false;
-        SFB_TRY(synthesis_pixmajor(h, p.gbuf.ptr, nsc, d_f + s0, nr, false, nsc == nr ? f_out : nullptr, st, &pm, &copied));
+        SFB_TRY(synthesis_pixmajor(h, p.alm.ptr, p.gbuf.ptr, nsc, d_f + s0, nr, false, nsc == nr ? f_out : nullptr, st, &pm, &copied));
         if (!pm) {
             launch_ring_synthesis(p, p.gbuf.ptr, nsc, p.maps.ptr, st);
             launch_transpose_ld(p.maps.ptr, p.npix, nsc, p.npix, d_f + s0, nr, st);

@@ -73,6 +73,7 @@ struct Task64 {
     int exs = 0, ntile = 0;
     int n_is_rows = 0;                 // table rows are coefficients l = m + parity + 2 n (else rings)
     int nout = 0, nlim = 0;            // rings of the output's layout, and those written
+    int tile0 = 0;                     // the first tile of the launch
     const double *tab64 = nullptr;
     const int64_t *tab64_off = nullptr;
     int64_t sn = 0, sk = 0;
@@ -356,6 +357,9 @@ void launch_leg_analysis64(const Plan &p, const double *F, int64_t ncol, double 
                            int rlim, const int *nzr);
 void launch_leg_synthesis64(const Plan &p, const double *A, int64_t ncol, double *G, cudaStream_t st, int rlim,
                             const double *A0, double *Anew);
+void launch_leg_synthesis64_rings(const Plan &p, const double *A, int64_t ncol, double *G, int r0, int r1,
+                                  cudaStream_t st);
+constexpr int LEG64_TILE = 32;
 // rlim: only rings r < rlim (-1: all); F == nullptr (Gram refinement): R = -w n cfold Fold(G)
 // Ecol: preset here below every exponent, unless ecol_preset (the caller did)
 void launch_fold_residual(const Plan &p, const double *F, const double *G, int64_t ncol, double *R, cudaStream_t st,
