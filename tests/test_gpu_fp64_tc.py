@@ -147,3 +147,35 @@ def test_rings_nonfinite(bad, monkeypatch):
     g = map2alm(f, a, radial="spline"), map2alm_adjoint(y, a, radial="spline")
     assert not np.isfinite(g[0][2]).any() and np.isfinite(np.delete(g[0], 2, 0)).all()
     assert not np.isfinite(g[1][4]).any() and np.isfinite(np.delete(g[1], 4, 0)).all()
+
+
+# 50 MB in three belt groups and the caps; the caps and the belt share a table tile, or (nside 65) just do not
+@pytest.mark.parametrize("nside,nr", [(64, 129), (65, 129)])
+def test_large_synthesis_in_ring_groups(nside, nr, monkeypatch):
+    """anlm2field with the Legendre synthesis ring group by ring group against the FP64 units in one launch."""
+    out = []
+    for v in ("1", "0"):
+        monkeypatch.setenv("SFBGPU_TC64", v)
+        a = sfbgpu.AnlmModes(0.054, 500.0, 1500.0, nside=nside)
+        assert 2 * (a.lmax + 1) * ((2 * nr + 127) // 128) >= 304
+        wm = sfbgpu.ConfigurationSpaceModes(a.rmin, a.rmax, nr, nside)
+        c = np.random.default_rng(16).normal(size=(sfbgpu.getnlmsize(a), 2)) @ np.array([1.0, 1j])
+        out.append(sfbgpu.anlm2field(c, wm, a))
+    assert rel_err(out[0], out[1]) < TOL
+
+
+# shells below, at and above the four warps' terms and the chunks of 16 they stage, in one chunk and in several
+@pytest.mark.parametrize("nr", [1, 2, 3, 5, 63, 64, 65, 70])
+def test_few_shells_vs_map2alm(nr):
+    """The radial sum over few shells: sum_s r_s^2 dr g_nl(r_s) a_lm(s) of the shells' own transforms, FP64.
+    A different grouping of at most 70 FP64 terms: 1e-12."""
+    a = sfbgpu.AnlmModes(0.03, 500.0, 1000.0, nside=16)
+    wm = sfbgpu.ConfigurationSpaceModes(a.rmin, a.rmax, nr, 16)
+    f = np.asfortranarray(np.random.default_rng(17).normal(size=(nr, wm.npix)))
+    whole = sfbgpu.field2anlm(f, wm, a, precision="fp64")
+    parts = np.zeros_like(whole)
+    for s in range(nr):                                # linear in the shells
+        one = np.zeros_like(f)
+        one[s] = f[s]
+        parts += sfbgpu.field2anlm(one, wm, a, precision="fp64")
+    assert rel_err(whole, parts) < 1e-12

@@ -262,3 +262,19 @@ def test_calls_queued_without_waiting_equal_waited_calls(precision, nside):
     torch.cuda.synchronize()
     for i, got in enumerate(queued):
         assert rel_err(got.cpu().numpy(), waited[i % 2]) < 1e-9
+
+
+# 33 MB (two belt groups) to 51 MB (three), the caps in two; ring groups that end within a tile pair
+@pytest.mark.parametrize("nside,nr", [(64, 172), (65, 251)])
+def test_large_fields_in_ring_groups(nside, nr, monkeypatch):
+    """A field whose ring transform follows its copy in ring groups, against the same field in two chunks of
+    shells, each transformed at once: the same sums but for the grouping of the radial one (1e-12)."""
+    rng = np.random.default_rng(18)
+    f = np.asfortranarray(rng.normal(size=(nr, 12 * nside * nside)).astype(np.float32))
+    out = []
+    for budget in ("0", str(4 * (nr // 2 + 1) * 12 * nside * nside)):
+        monkeypatch.setenv("SFBGPU_FIELD_MAX_BYTES", budget)
+        a = sfbgpu.AnlmModes(0.03, 500.0, 1000.0, nside=nside)
+        wm = sfbgpu.ConfigurationSpaceModes(a.rmin, a.rmax, nr, nside)
+        out.append(sfbgpu.field2anlm(f, wm, a, precision="mixed"))
+    assert rel_err(out[0], out[1]) < 1e-12
