@@ -692,12 +692,12 @@ int reference_alm(sfb_plan *h, const double *ref, int64_t nref, cudaStream_t st)
     return rc;
 }
 
-// The Legendre synthesis of A into G, and the pixel-major ring synthesis of G into out[pixel ld + map] of nm maps on the
-// device; with host, which has the same layout, ring group by ring group, each group's pixels going there on the side
-// stream while the next one is formed (the caller's stream waits for the copies at the end).  The copy bounds these
-// calls (201 MB at 193 GB/s: 1040 us), so what is done before it begins counts: the rings of the first group only, not
-// all (128 shells of nside 128: 1345 -> 1235 us a call).  *done: false when out is null or the plan's tensor-core transform is not available (then G is
-// all there is).
+// The Legendre synthesis of A into G, and the pixel-major ring synthesis of G into out[pixel ld + map] of nm maps on
+// the device; with host, which has the same layout, ring group by ring group, each group's pixels going there on the
+// side stream while the next one is formed (the caller's stream waits for the copies at the end).  The copy bounds
+// these calls (201 MB at 193 GB/s: 1040 us), so what is done before it begins counts: the rings of the first group
+// only, not all (128 shells of nside 128: 1345 -> 1235 us a call).  *done: false when out is null or the plan's
+// tensor-core transform is not available (then G is all there is).
 // *copied: the field is on its way to host.
 int synthesis_pixmajor(sfb_plan *h, const double *A, double *G, int64_t nm, void *out, int64_t ld, bool f32, void *host,
                        cudaStream_t st, bool *done, bool *copied) {
