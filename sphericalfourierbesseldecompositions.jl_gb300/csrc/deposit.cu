@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_tiles(int32_t *data, int6
     const int64_t base = (int64_t)blockIdx.x * SCAN_TILE + (int64_t)threadIdx.x * SCAN_ITEMS;
     alignas(16) int32_t v[SCAN_ITEMS];
     int32_t s = 0;
-    const bool whole = base + SCAN_ITEMS <= n;             // (the counters start on a 16-byte boundary)
+    const bool whole = base + SCAN_ITEMS <= n;             // (data is on a 16-byte boundary: launch_exclusive_scan)
     if (whole) {
 #pragma unroll
         for (int j = 0; j < SCAN_ITEMS; j += 4)

@@ -325,7 +325,8 @@ constexpr int WMIX_LMAX = 128;
 size_t wmix_smem_bytes(int l, int lp, int64_t nr, int neg_m);
 void launch_wmix(const Plan &p, const int64_t *noff, const double *gtab, int64_t nr, double rmin, double dr,
                  const double *WT, int64_t ldW, int LW, int neg_m, double *out, size_t smem, cudaStream_t st);
-// Exclusive prefix sum of n int32 counters in place; tile_sums holds scan_tile_count(n) ints, *done is zero.
+// Exclusive prefix sum of n int32 counters in place; data is on a 16-byte boundary (whole tiles are read as int4),
+// tile_sums holds scan_tile_count(n) ints, *done is zero.
 int64_t scan_tile_count(int64_t n);
 void launch_exclusive_scan(int32_t *data, int64_t n, int32_t *tile_sums, int *done, cudaStream_t st);
 void launch_ring_analysis(Plan &p, const double *maps, int64_t nmaps, double *F, cudaStream_t st, int *nzr = nullptr);

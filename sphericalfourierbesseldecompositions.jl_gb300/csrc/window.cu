@@ -106,7 +106,8 @@ int check_args(int64_t nside, const double *win, int64_t nr, double rmin, double
     return SFB_OK;
 }
 
-// Device-pointer core: workspace ws holds [flags ngal + 1][tile sums][max: 1 u64][err: 1 int][scan counter: 1 int].
+// Device-pointer core: workspace ws (on a 16-byte boundary) holds [flags ngal + 1][tile sums][max: 1 u64][err: 1
+// int][scan counter: 1 int].
 int run(int64_t nside, const double *win, int64_t nr, double rmin, double rmax, double dr, const double *rtp,
         int64_t ngal, const double *uniform, uint64_t seed, double *out, int64_t *nkept, char *ws, cudaStream_t st) {
     const int64_t npix = 12 * nside * nside;
@@ -161,11 +162,12 @@ extern "C" int sfb_apply_window(int64_t nside, const double *win, int64_t nr, do
         cudaGetLastError();
         return fail(SFB_ENOMEM, "device allocation failed");
     }
-    double *dwin = reinterpret_cast<double *>(d);
-    double *drtp = reinterpret_cast<double *>(d + wb);
-    double *dout = reinterpret_cast<double *>(d + wb + gb);
-    double *du = uniform ? reinterpret_cast<double *>(d + wb + 2 * gb) : nullptr;
-    char *ws = d + wb + 2 * gb + ub;
+    // the workspace first: its counters need the allocation's alignment (the draws may be an odd number of doubles)
+    char *ws = d, *e = d + workspace_bytes(ngal);
+    double *dwin = reinterpret_cast<double *>(e);
+    double *drtp = reinterpret_cast<double *>(e + wb);
+    double *dout = reinterpret_cast<double *>(e + wb + gb);
+    double *du = uniform ? reinterpret_cast<double *>(e + wb + 2 * gb) : nullptr;
     int st = SFB_OK;
     do {
         if (cudaMemcpy(dwin, win, wb, cudaMemcpyHostToDevice) != cudaSuccess ||

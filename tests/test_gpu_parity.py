@@ -389,6 +389,21 @@ def test_apply_window_vs_oracle(draws):
     assert gpu.shape == ref.shape and np.array_equal(gpu, ref)
 
 
+# below one thread's 16 counters, one more, one tile of 4096 counters less one, many tiles: every odd size leaves the
+# draws, which lie beside the counters, an odd number of doubles long
+@pytest.mark.parametrize("n", [15, 17, 4095, 300_001])
+def test_apply_window_odd_sizes(n):
+    nside, nr, rmin, rmax = 16, 20, 500.0, 1000.0
+    wm = sfbgpu.ConfigurationSpaceModes(rmin, rmax, nr, nside)
+    rng = np.random.default_rng(n)
+    win = rng.uniform(0.2, 1.0, (nr, wm.npix))
+    rtp, _ = catalogue(n, rmin, rmax, seed=n)
+    u = rng.random(n)
+    gpu = sfbgpu.apply_window(rtp, win, wm, uniform=u)
+    ref = osfb.apply_window(rtp, win, rmin, rmax, wm.dr, nside, u)
+    assert gpu.shape == ref.shape and np.array_equal(gpu, ref)
+
+
 def test_apply_window_edges():
     nside, nr = 4, 5
     wm = sfbgpu.ConfigurationSpaceModes(500.0, 1000.0, nr, nside)
