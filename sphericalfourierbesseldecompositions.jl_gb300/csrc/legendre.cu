@@ -307,6 +307,10 @@ static bool narrow_dispatch(const Plan &p, const T *lam, const T *in, int64_t nc
         if (analysis) narrow_analysis<T, 4>(p, lam, in, out, accumulate, rlim, st);
         else narrow_synthesis<T, 4>(p, lam, in, out, rlim, st);
         return true;
+    case 6:
+        if (analysis) narrow_analysis<T, 6>(p, lam, in, out, accumulate, rlim, st);
+        else narrow_synthesis<T, 6>(p, lam, in, out, rlim, st);
+        return true;
     case 8:
         if (analysis) narrow_analysis<T, 8>(p, lam, in, out, accumulate, rlim, st);
         else narrow_synthesis<T, 8>(p, lam, in, out, rlim, st);
@@ -367,7 +371,7 @@ __global__ void __launch_bounds__(128) k_refine_narrow64(const double *gram,
 
 bool launch_refine_narrow64(const Plan &p, const double *A, const double *A0, int64_t ncol, double *G, double *Anew,
                             cudaStream_t st) {
-    if (!p.d_gram64 || p.precision != SFB_FP64 || (ncol != 2 && ncol != 4 && ncol != 8)) return false;
+    if (!p.d_gram64 || p.precision != SFB_FP64 || ncol > 8 || (ncol & 1)) return false;
     const int maxrows = p.lmax / 2 + 1, ng = (int)((maxrows * ncol + 127) / 128);
     const dim3 grid((unsigned)(ng + (p.ral + 127) / 128), (unsigned)(2 * (p.lmax + 1)));
     auto go = [&](auto kernel) {
@@ -376,6 +380,7 @@ bool launch_refine_narrow64(const Plan &p, const double *A, const double *A0, in
     };
     if (ncol == 2) go(k_refine_narrow64<2>);
     else if (ncol == 4) go(k_refine_narrow64<4>);
+    else if (ncol == 6) go(k_refine_narrow64<6>);
     else go(k_refine_narrow64<8>);
     note_launch();
     return true;

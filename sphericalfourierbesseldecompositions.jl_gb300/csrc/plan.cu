@@ -334,7 +334,7 @@ struct ShtWork {
 };
 
 // One FP64 Gram refinement step's products of the current coefficients: G on the aliased rings and
-// Anew = A0 - D A (one launch for many columns on the tensor cores, and for 2, 4 or 8).
+// Anew = A0 - D A (one launch for many columns on the tensor cores, and for up to 8).
 void synthesis_and_gram64(const Plan &p, const double *A, const double *A0, int64_t ncol, double *G, double *Anew,
                           cudaStream_t st) {
     if (p.tc64_state > 0 && ncol > 8) {
@@ -599,7 +599,7 @@ int sht_analysis(sfb_plan *h, const double *maps, int64_t nm, cudaStream_t st, b
         return SFB_OK;
     }
     if (!tc && p.d_gram64 && p.niter > 0) {
-        // FP64 Gram refinement: the same identity as above, in FP64 (narrow kernels for 2, 4 or 8
+        // FP64 Gram refinement: the same identity as above, in FP64 (narrow kernels for up to 8
         // columns: reference maps, small map2alm batches; tiled GEMMs for more, the first pass over
         // the ring pairs with data).  alm holds [result | other | first pass]; step it writes one of the
         // first two, the last step the first.

@@ -345,7 +345,7 @@ constexpr int64_t RING64_MIN = 5;      // maps from which they are used (launch_
 void launch_leg_analysis(const Plan &p, const double *F, int64_t ncol, double *A, bool accumulate,
                          cudaStream_t st, int rlim = -1, const int *nzr = nullptr);
 void launch_leg_synthesis(const Plan &p, const double *A, int64_t ncol, double *G, cudaStream_t st, int rlim = -1);
-// Gram update and aliased rings' synthesis of one FP64 refinement step for 2, 4 or 8 columns (else false).
+// Gram update and aliased rings' synthesis of one FP64 refinement step for up to 8 columns (else false).
 bool launch_refine_narrow64(const Plan &p, const double *A, const double *A0, int64_t ncol, double *G, double *Anew,
                             cudaStream_t st);
 // FP64 Gram refinement step (any column count); false when the plan has no Gram tables

@@ -107,3 +107,22 @@ def test_groups_of_mocks_equal_single_calls(precision, window):
             assert not np.any(batch[k])
             continue
         assert rel_err(batch[k], single) < (1e-12 if precision == "fp64" else 1e-9), k
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("nmocks", [2, 3, 4, 18])
+def test_small_and_last_groups(precision, nmocks):
+    """Groups of two (the whole batch, or its last group), three and four mocks: six, eight and ten reference columns
+    in the mixed path.  Tolerances as above."""
+    a = sfbgpu.AnlmModes(0.03, 500.0, 1000.0, nside=16)
+    wm, phi, mask = _window(a)
+    sep = sfbgpu.SeparableArray(phi, mask, "phi", "mask")
+    win = sfbgpu.win_rhat_ln(sep, wm, a)
+    veff = sfbgpu.integrate_window(sep, wm)
+    sizes = [2000 + 97 * k for k in range(nmocks)]
+    cats, ws = _mocks(a, sizes, 53)
+    nbars = [n / veff for n in sizes]
+    batch = sfbgpu.cat2amln_batched(cats, a, nbars, win, ws, precision=precision)
+    for k in range(nmocks):
+        single = sfbgpu.cat2amln(cats[k], a, nbars[k], win, ws[k], precision=precision)
+        assert rel_err(batch[k], single) < (1e-12 if precision == "fp64" else 1e-9), k

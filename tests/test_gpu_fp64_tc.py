@@ -70,6 +70,24 @@ def test_adjoint_vs_fp64_units(nside, lmax, nmaps, niter, monkeypatch):
     assert e < TOL
 
 
+@pytest.mark.parametrize("nmaps", [1, 2, 3, 4])
+@pytest.mark.parametrize("nside,lmax", [(16, 24), (32, 60), (12, 30)])
+def test_few_maps(nside, lmax, nmaps):
+    """Up to eight columns take their own kernels (the oracle, as above), whatever the plan has done before: the
+    same bits before and after a call of many columns."""
+    a = _modes(lmax, nside)
+    f = _maps(nmaps, nside, 8)
+    first = map2alm(f, a, radial="spline")
+    ref = SHT(nside, lmax).map2alm(f, niter=3)
+    ref = np.stack([ref[:, l, m] for l in range(lmax + 1) for m in range(l + 1)], axis=1)
+    assert rel_err(first, ref) < TOL
+    y = np.random.default_rng(9).normal(size=(nmaps, ref.shape[1], 2)) @ np.array([1.0, 1j])
+    back = map2alm_adjoint(y, a, radial="spline")
+    map2alm(_maps(9, nside, 8), a, radial="spline")
+    assert np.array_equal(map2alm(f, a, radial="spline"), first)
+    assert np.array_equal(map2alm_adjoint(y, a, radial="spline"), back)
+
+
 @pytest.mark.parametrize("scale", [1e-25, 1e30])
 def test_scales(scale):
     """Magnitudes far from one (the ring transform's odd factors run in double-float, which bounds them)."""
