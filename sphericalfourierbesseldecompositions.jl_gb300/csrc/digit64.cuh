@@ -55,7 +55,7 @@ __device__ __forceinline__ int64_t fixed55(double x, int emax) {
     int e = (int)(hi >> 20) & 0x7ff;
     uint64_t mant = ((uint64_t)((hi & 0xfffffu) | (e ? 0x100000u : 0u)) << 32) | lo;
     e = max(e, 1);
-    const int s = min(emax - e, 63);
+    const uint32_t s = min((uint32_t)(emax - e), 63u);       // (a zero may come with e above emax)
     const int64_t q = (int64_t)((((mant << 3) >> s) + 1) >> 1);
     return (int32_t)hi < 0 ? -q : q;
 }
@@ -157,9 +157,9 @@ __device__ __forceinline__ void issue(uint32_t tmem, uint32_t sa, uint32_t sb, i
 }
 
 // One exact K block, chunks [k0, k1) of nch (k0 even), up to its last MMA's issue: every warp turns its values
-// into digits (load(kc, buf): this thread's eight values of chunk kc, row tid % 128, k = 8 (tid / 128)..; fix: a
-// value as the integer), the table digits of chunk kc come from tab + kc ND LS KC, and the last warp issues a
-// chunk's MMAs once all have written theirs.  pre holds the values of chunks k0 and k0 + 1 on entry.  end_block
+// into digits (load(kc, buf, i): this thread's eight values of chunk kc, row tid % 128, k = 8 (tid / 128)..; fix(v, i,
+// j): value j of them as the integer; i is the buffer, pre[i]), the table digits of chunk kc come from tab + kc ND LS
+// KC, and the last warp issues a chunk's MMAs once all have written theirs.  pre holds the values of chunks k0 and k0 + 1 on entry.  end_block
 // waits for the MMAs.
 template <typename T, typename Load, typename Fix>
 __device__ __forceinline__ void run_block(const Smem &cs, uint32_t tmem, int k0, int k1, int nch, int LS,
@@ -167,7 +167,7 @@ __device__ __forceinline__ void run_block(const Smem &cs, uint32_t tmem, int k0,
     const int tid = threadIdx.x, lane = tid & 31;
     const uint32_t bytesB = (uint32_t)ND * LS * KC * 2;
     const uint32_t off = core_off(tid & (MTILE - 1), 8 * (tid >> 7));
-    auto chunk = [&](int kc, T (&cur)[8]) -> bool {
+    auto chunk = [&](int kc, T (&cur)[8], int i) -> bool {
         const int s = kc % NSTAGE;
         if (kc >= NSTAGE) {
             if (*(volatile int *)cs.bad) return false;
@@ -185,14 +185,14 @@ __device__ __forceinline__ void run_block(const Smem &cs, uint32_t tmem, int k0,
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             uint32_t v[ND];
-            digits2(fix(cur[2 * j]), fix(cur[2 * j + 1]), v);
+            digits2(fix(cur[2 * j], i, 2 * j), fix(cur[2 * j + 1], i, 2 * j + 1), v);
 #pragma unroll
             for (int q = 0; q < ND; ++q) w[q][j] = v[q];
         }
 #pragma unroll
         for (int q = 0; q < ND; ++q)
             *reinterpret_cast<uint4 *>(sa + q * PLANE_A + off) = make_uint4(w[q][0], w[q][1], w[q][2], w[q][3]);
-        if (kc + 2 < nch) load(kc + 2, cur);
+        if (kc + 2 < nch) load(kc + 2, cur, i);
         fence_proxy_async();
         __syncwarp();
         if (lane == 0) {
@@ -213,8 +213,8 @@ __device__ __forceinline__ void run_block(const Smem &cs, uint32_t tmem, int k0,
         return true;
     };
     for (int kc = k0; kc < k1; kc += 2) {
-        if (!chunk(kc, pre[0])) break;
-        if (kc + 1 < k1 && !chunk(kc + 1, pre[1])) break;
+        if (!chunk(kc, pre[0], 0)) break;
+        if (kc + 1 < k1 && !chunk(kc + 1, pre[1], 1)) break;
     }
     if (tid == 32 * MMA_WARP) mma_commit(cs.done);          // arrives once every MMA issued above has completed
     __syncwarp();

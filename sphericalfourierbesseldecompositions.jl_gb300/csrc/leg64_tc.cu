@@ -44,6 +44,30 @@ namespace t64 {
 __device__ __forceinline__ int rows_of(int m, int par, int lmax) {
     return (m + par <= lmax) ? (lmax - m - par) / 2 + 1 : 0;
 }
+
+// Exponents in which the rings of the analysis differ: a ring's values are held on the scale of its largest lambda in
+// the block (2^(kx - KXR), kx = KXR for the ring with the largest of all), down to 2^-KXR, and its table column on the
+// inverse.  The scale of a data column is then that of its largest contribution, not of its largest value: a
+// bright pixel on the short polar rings, whose spectra reach every m, costs the m bits only that it contributes to,
+// for contrasts up to 2^KXR between the rings (1e8 near a pole on unit noise, nside 64, lmax 120, each m on its own
+// scale: 2e-10 with one scale for all rings, 3e-16 so; an FP64 sum 2e-15).  The sums over l (synthesis, Gram) keep the
+// scale of the largest coefficient of an m and parity.
+constexpr int KXR = 40;
+// Largest value of a column: the key orders the magnitudes on the rings' scales by exponent (its bits 20..); `all`
+// also the values that do not enter a product.  A column with a value that is not finite gets the key BAD.
+constexpr uint32_t BAD = 0xffffffffu;
+struct ColMax {
+    uint32_t key = 0, all = 0;
+    __device__ __forceinline__ void add(double v, int kx, bool live) {
+        const uint32_t hi = (uint32_t)__double2hiint(v) & 0x7fffffffu;
+        all = max(all, hi);
+        if (live && (hi | (uint32_t)__double2loint(v))) key = max(key, max(hi, 0x100000u) + ((uint32_t)kx << 20));
+    }
+    __device__ __forceinline__ uint32_t get() const { return all >= 0x7ff00000u ? BAD : key; }
+};
+// value j of eight packed bytes
+__device__ __forceinline__ int byte_of(uint2 w, int j) { return (int)(((j < 4 ? w.x : w.y) >> (8 * (j & 3))) & 0xffu); }
+
 // One CTA: data columns [128 blockIdx.x, +128) x table rows of one tile of block z = (m, parity).
 // LMROWS: the data rows are coefficients l = m + parity + 2 k (synthesis, Gram); else rings k (analysis).
 // Tiles blockIdx.y < ny0 use task 0, the others task 1 (the Gram update and the aliased rings' synthesis of
@@ -100,6 +124,7 @@ __global__ void __launch_bounds__(NTH, 2) k_leg64(const double *data, int64_t nc
     // The column's values: largest magnitude over every chunk (the high word orders the magnitudes by exponent);
     // those of the first two chunks to be worked stay in registers.
     double pre[2][8];
+    uint2 kxs[2];                             // their rings' scales
     bool use = cok;
     auto load_at = [&](int c16, double (&buf)[8]) {
 #pragma unroll
@@ -108,38 +133,44 @@ __global__ void __launch_bounds__(NTH, 2) k_leg64(const double *data, int64_t nc
             buf[j] = (use && k >= kbeg && k < kend) ? D[row_at(k)] : 0.0;
         }
     };
-    auto load = [&](int kc, double (&buf)[8]) { load_at(lo + kc, buf); };
-    uint32_t mx = 0;
-    auto top = [&](const double (&buf)[8]) {
+    auto kx_at = [&](int c16) -> uint2 {
+        if constexpr (LMROWS) return make_uint2(0u, 0u);
+        return *reinterpret_cast<const uint2 *>(t.kx + (int64_t)z * t.nkx + c16 * KC + 8 * kh);
+    };
+    auto load = [&](int kc, double (&buf)[8], int i) {
+        load_at(lo + kc, buf);
+        kxs[i] = kx_at(lo + kc);
+    };
+    ColMax mx;
+    auto top = [&](const double (&buf)[8], uint2 kx, bool in) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
-            mx = max(mx, ((uint32_t)__double2hiint(buf[j]) & 0x7fffffffu) | (__double2loint(buf[j]) != 0 ? 1u : 0u));
+        for (int j = 0; j < 8; ++j) mx.add(buf[j], LMROWS ? 0 : byte_of(kx, j), in);
     };
     if (tid < NT && tile * NT + tid < nwrite) ex_s[tid] = t.ex[(int64_t)z * t.exs + tile * NT + tid];
     {
-        if (nch > 0) load(0, pre[0]);
-        if (nch > 1) load(1, pre[1]);
+        if (nch > 0) load(0, pre[0], 0);
+        if (nch > 1) load(1, pre[1], 1);
         const int skip0 = nch > 0 ? lo : -1, skip1 = nch > 1 ? lo + 1 : -1;
         for (int c16 = kbeg / KC; c16 * KC < kend; ++c16) {
             if (c16 == skip0 || c16 == skip1) continue;
             double buf[8];
             load_at(c16, buf);
-            top(buf);
+            top(buf, kx_at(c16), c16 >= lo && c16 <= hi);
         }
-        if (nch > 0) top(pre[0]);
-        if (nch > 1) top(pre[1]);
-        red[kh][c] = mx;
+        if (nch > 0) top(pre[0], kxs[0], true);
+        if (nch > 1) top(pre[1], kxs[1], true);
+        red[kh][c] = mx.get();
     }
     Smem cs;
     const uint32_t tmem = setup(cs, smem);    // includes a __syncthreads
     const uint32_t cmx = max(red[0][c], red[1][c]);
     const int emax = max(1, (int)(cmx >> 20));
-    if (cmx == 0 || emax == 2047) {           // no digits: zero or non-finite columns
+    if (cmx == 0 || cmx == BAD) {             // no digits: zero or non-finite columns
         use = false;
 #pragma unroll
         for (int j = 0; j < 8; ++j) pre[0][j] = pre[1][j] = 0.0;
     }
-    auto fix = [&](double v) { return fixed55(v, emax); };
+    auto fix = [&](double v, int i, int j) { return fixed55(v, LMROWS ? emax : emax - byte_of(kxs[i], j)); };
 
     // warp w of the epilogue: TMEM lanes 32 (w % 4).. (columns), every other group of four table rows of the tile
     const int lq = warp & 3, hg = warp >> 2;
@@ -148,7 +179,7 @@ __global__ void __launch_bounds__(NTH, 2) k_leg64(const double *data, int64_t nc
     const int64_t cc = col0 + cl;
     const bool ook = cc < ncol;
     const uint32_t lmx = max(red[0][cl], red[1][cl]);
-    const int lemax = max(1, (int)(lmx >> 20));
+    const int lemax = max(1, (int)(lmx >> 20)) - (LMROWS ? 0 : KXR);
     auto at = [&](int i) -> int64_t {                       // output row i of the tile, this lane's column; rows < 2^31
         const int n = tile * NT + i, l = m + par + 2 * n;
         const uint32_t row = t.n_is_rows ? (uint32_t)(l * (l + 1) / 2 + m) : (uint32_t)((par * (lmax + 1) + m) * t.nout + n);
@@ -181,7 +212,7 @@ __global__ void __launch_bounds__(NTH, 2) k_leg64(const double *data, int64_t nc
                     const int n = tile * NT + i0 + i;
                     if (n >= nwrite) break;
                     double val = 0.0;
-                    if (lemax == 2047) {                  // non-finite data: the plain FP64 sum
+                    if (lmx == BAD) {                     // non-finite data: the plain FP64 sum
                         if (sb == 0)
                             for (int k = kbeg; k < kend; ++k)
                                 val = fma(t.tab64[t.tab64_off[z] + n * t.sn + k * t.sk],
@@ -272,20 +303,23 @@ __global__ void __launch_bounds__(NTH, 2) k_leg64_short(const double *data, int6
     if (cur < 0) return;
 
     double v[RES][8];
-    uint32_t mx = 0;
+    uint2 kxs[RES];                                           // the rings' scales
+    ColMax mx;
 #pragma unroll
-    for (int q = 0; q < RES; ++q)
+    for (int q = 0; q < RES; ++q) {
+        if constexpr (!LMROWS)
+            if (q < nK) kxs[q] = *reinterpret_cast<const uint2 *>(t0.kx + (int64_t)z * t0.nkx + q * KC + 8 * kh);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             const int k = q * KC + 8 * kh + j;
             v[q][j] = (cok && k < K) ? D[row_at(k) + col0 + c] : 0.0;
         }
+    }
 #pragma unroll
     for (int q = 0; q < RES; ++q)
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
-            mx = max(mx, ((uint32_t)__double2hiint(v[q][j]) & 0x7fffffffu) | (__double2loint(v[q][j]) != 0 ? 1u : 0u));
-    red[kh][c] = mx;
+        for (int j = 0; j < 8; ++j) mx.add(v[q][j], LMROWS || q >= nK ? 0 : byte_of(kxs[q], j), true);
+    red[kh][c] = mx.get();
     uint64_t *full_b = &bars[0], *done = &bars[1];
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&slot)),
@@ -312,7 +346,7 @@ __global__ void __launch_bounds__(NTH, 2) k_leg64_short(const double *data, int6
     {
         const uint32_t cmx = max(red[0][c], red[1][c]);
         const int emax = max(1, (int)(cmx >> 20));
-        const bool dead = cmx == 0 || emax == 2047;              // no digits: zero or non-finite columns
+        const bool dead = cmx == 0 || cmx == BAD;                // no digits: zero or non-finite columns
         const uint32_t off = core_off(c, 8 * kh);
 #pragma unroll
         for (int q = 0; q < RES; ++q) {
@@ -321,7 +355,9 @@ __global__ void __launch_bounds__(NTH, 2) k_leg64_short(const double *data, int6
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 uint32_t u[ND];
-                digits2(dead ? 0 : fixed55(v[q][2 * j], emax), dead ? 0 : fixed55(v[q][2 * j + 1], emax), u);
+                const int e0 = LMROWS ? emax : emax - byte_of(kxs[q], 2 * j);
+                const int e1 = LMROWS ? emax : emax - byte_of(kxs[q], 2 * j + 1);
+                digits2(dead ? 0 : fixed55(v[q][2 * j], e0), dead ? 0 : fixed55(v[q][2 * j + 1], e1), u);
 #pragma unroll
                 for (int d = 0; d < ND; ++d) w[d][j] = u[d];
             }
@@ -337,7 +373,8 @@ __global__ void __launch_bounds__(NTH, 2) k_leg64_short(const double *data, int6
     const int cl = lq * 32 + lane;
     const int64_t cc = col0 + cl;
     const bool ook = cc < ncol;
-    const int lemax = max(1, (int)(max(red[0][cl], red[1][cl]) >> 20));
+    const uint32_t lmx = max(red[0][cl], red[1][cl]);
+    const int lemax = max(1, (int)(lmx >> 20)) - (LMROWS ? 0 : KXR);
     int uses = 0;                                             // tiles whose digits were fetched: barrier phases
     for (int step = 0; cur >= 0; ++step) {
         const Task64 &t = job.task ? t1 : t0;
@@ -390,7 +427,7 @@ __global__ void __launch_bounds__(NTH, 2) k_leg64_short(const double *data, int6
                     const int n = job.tile * NT + i0 + i;
                     if (n >= job.nwrite) break;
                     double val = 0.0;
-                    if (lemax == 2047) {                      // non-finite data: the plain FP64 sum
+                    if (lmx == BAD) {                         // non-finite data: the plain FP64 sum
                         for (int k = 0; k < K; ++k)
                             val = fma(t.tab64[t.tab64_off[z] + n * t.sn + k * t.sk], D[row_at(k) + cc], val);
                     } else if (job.nch > 0) {
@@ -421,16 +458,40 @@ __device__ __forceinline__ void dims(int kind, int z, int lmax, int nrn, int &N,
     K = kind == 0 ? nrn : nrows;
 }
 
+// the analysis table's ring scales kx (KXR above), one block per (m, parity)
+__global__ void __launch_bounds__(256) k64_ringexp(const double *tab, const int64_t *off64, int lmax, int nrn, int nkx,
+                                                   uint8_t *kx) {
+    pdl_entry();
+    __shared__ int most;
+    const int z = blockIdx.x, nrows = rows_of(z >> 1, z & 1, lmax);
+    if (threadIdx.x == 0) most = -(1 << 20);
+    __syncthreads();
+    auto exponent = [&](int r) {
+        double mx = 0.0;
+        for (int n = 0; n < nrows; ++n) mx = fmax(mx, fabs(tab[off64[z] + (int64_t)n * nrn + r]));
+        return mx > 0.0 && isfinite(mx) ? ilogb(mx) : -(1 << 20);
+    };
+    for (int r = threadIdx.x; r < nrn; r += 256) atomicMax(&most, exponent(r));
+    __syncthreads();
+    for (int r = threadIdx.x; r < nkx; r += 256)
+        kx[(int64_t)z * nkx + r] = (uint8_t)(r < nrn ? max(0, KXR + exponent(r) - most) : 0);
+}
+// element (n, k) of a table on its column's scale
+__device__ __forceinline__ double element(const double *tab, int64_t at, const uint8_t *kx, int64_t k) {
+    return kx ? ldexp(tab[at], KXR - (int)kx[k]) : tab[at];
+}
+
 // exponent E of every table row, |v| < 2^E (one warp per row)
 __global__ void k64_rowexp(int kind, const double *tab, const int64_t *off64, int64_t sn,
-                           int64_t sk, int lmax, int nrn, int exs, int16_t *ex) {
+                           int64_t sk, int lmax, int nrn, int exs, int16_t *ex, const uint8_t *kx, int nkx) {
     pdl_entry();
     const int z = blockIdx.y, lane = threadIdx.x & 31;
     int N, K;
     dims(kind, z, lmax, nrn, N, K);
     for (int n = blockIdx.x * 8 + (threadIdx.x >> 5); n < N; n += gridDim.x * 8) {
         double mx = 0.0;
-        for (int k = lane; k < K; k += 32) mx = fmax(mx, fabs(tab[off64[z] + n * sn + k * sk]));
+        for (int k = lane; k < K; k += 32)
+            mx = fmax(mx, fabs(element(tab, off64[z] + n * sn + k * sk, kx, (int64_t)z * nkx + k)));
         for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
         if (lane == 0) ex[(int64_t)z * exs + n] = (int16_t)(mx > 0.0 && isfinite(mx) ? ilogb(mx) + 1 : 0);
     }
@@ -441,7 +502,7 @@ __global__ void __launch_bounds__(256) k64_build(int kind, const double *tab,
                                                  const int64_t *off64, int64_t sn, int64_t sk, int lmax,
                                                  int nrn, int exs, const int16_t *ex, int ntile,
                                                  int nkmax, const int64_t *off,
-                                                 uint16_t *dig, int2 *live) {
+                                                 uint16_t *dig, int2 *live, const uint8_t *kx, int nkx) {
     pdl_entry();
     const int z = blockIdx.y, tile = blockIdx.x / nkmax, kc = blockIdx.x % nkmax;
     int N, K;
@@ -456,7 +517,8 @@ __global__ void __launch_bounds__(256) k64_build(int kind, const double *tab,
         const int n = tile * NT + nn, kk = kc * KC + k;
         int64_t q = 0;
         if (n < N && kk < K)
-            q = llrint(ldexp(tab[off64[z] + n * sn + kk * sk], 55 - (int)ex[(int64_t)z * exs + n]));
+            q = llrint(ldexp(element(tab, off64[z] + n * sn + kk * sk, kx, (int64_t)z * nkx + kk),
+                             55 - (int)ex[(int64_t)z * exs + n]));
         any |= q != 0;
         uint32_t w[ND];
         digits2(q, 0, w);
@@ -517,22 +579,26 @@ bool ensure_tc64(Plan &p, cudaStream_t st) {
         return false;
     }
     for (int kind = 0; kind < nkind; ++kind) {
-        // one allocation: [digits][offsets][live ranges][exponents], each part 256-byte aligned
+        // one allocation: [digits][offsets][live ranges][exponents][ring scales], each part 256-byte aligned
         auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
         const size_t b0 = up(bytes[kind] + 16), b1 = up(nz * sizeof(int64_t)),
                      b2 = up((size_t)nz * ntile[kind] * sizeof(int2)), b3 = up((size_t)nz * exs[kind] * sizeof(int16_t));
+        const int nkx = kind == 0 ? nkmax[0] * t64::KC : 0;
+        const size_t b4 = up((size_t)nz * nkx);
         unsigned char *d = nullptr;
-        if (cudaMalloc(&d, b0 + b1 + b2 + b3) != cudaSuccess) {
+        if (cudaMalloc(&d, b0 + b1 + b2 + b3 + b4) != cudaSuccess) {
             cudaGetLastError();
             return false;                     // the tables made so far stay owned by the plan
         }
-        p.device_bytes += (int64_t)(b0 + b1 + b2 + b3);
+        p.device_bytes += (int64_t)(b0 + b1 + b2 + b3 + b4);
         Task64 &t = p.t64[kind];
         p.t64_mem[kind] = d;
         t.dig = reinterpret_cast<uint16_t *>(d);
         t.off = reinterpret_cast<int64_t *>(d + b0);
         t.live = reinterpret_cast<int2 *>(d + b0 + b1);
         t.ex = reinterpret_cast<int16_t *>(d + b0 + b1 + b2);
+        t.kx = kind == 0 ? d + b0 + b1 + b2 + b3 : nullptr;
+        t.nkx = nkx;
         t.exs = exs[kind];
         t.ntile = ntile[kind];
         t.n_is_rows = kind != 1;
@@ -549,11 +615,16 @@ bool ensure_tc64(Plan &p, cudaStream_t st) {
         const int64_t nl = (int64_t)nz * ntile[kind];
         launch_pdl(t64::k64_fill, dim3((unsigned)((nl + 255) / 256)), dim3(256), 0, st, const_cast<int2 *>(t.live),
             nl);
+        if (kind == 0) {
+            launch_pdl(t64::k64_ringexp, dim3((unsigned)nz), dim3(256), 0, st, t.tab64, t.tab64_off, p.lmax,
+                (int)p.nrn, nkx, const_cast<uint8_t *>(t.kx));
+            note_launch();
+        }
         launch_pdl(t64::k64_rowexp, dim3(16, (unsigned)nz), dim3(256), 0, st, kind, t.tab64, t.tab64_off, t.sn, t.sk,
-            p.lmax, (int)p.nrn, t.exs, const_cast<int16_t *>(t.ex));
+            p.lmax, (int)p.nrn, t.exs, const_cast<int16_t *>(t.ex), t.kx, nkx);
         launch_pdl(t64::k64_build, dim3((unsigned)(ntile[kind] * nkmax[kind]), (unsigned)nz), dim3(256), 0, st,
             kind, t.tab64, t.tab64_off, t.sn, t.sk, p.lmax, (int)p.nrn, t.exs, t.ex, t.ntile, nkmax[kind], t.off,
-            const_cast<uint16_t *>(t.dig), const_cast<int2 *>(t.live));
+            const_cast<uint16_t *>(t.dig), const_cast<int2 *>(t.live), t.kx, nkx);
         note_launch();
         note_launch();
         note_launch();

@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(NTH, 2) k_rdft64(const RingGeom *rings, int ns
     const int nch = R.kp / KC;
     const uint16_t *tab = dig + off[4 * R.cls + cb] + (int64_t)tile * nch * ND * NT * KC;
     int64_t pre[2][8];
-    auto load = [&](int kc, int64_t (&buf)[8]) {
+    auto load = [&](int kc, int64_t (&buf)[8], int) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const longlong2 v = use ? *reinterpret_cast<const longlong2 *>(q + kc * KC + 2 * j) : make_longlong2(0, 0);
@@ -190,14 +190,15 @@ __global__ void __launch_bounds__(NTH, 2) k_rdft64(const RingGeom *rings, int ns
             buf[2 * j + 1] = v.y;
         }
     };
-    load(0, pre[0]);
-    if (nch > 1) load(1, pre[1]);
+    load(0, pre[0], 0);
+    if (nch > 1) load(1, pre[1], 1);
     Smem cs;
     const uint32_t tmem = setup(cs, smem);
     const int oem = ook ? ex[(int64_t)r * nm + ob] : 0;
     const int nsb = (nch + SBR - 1) / SBR;
     for (int sb = 0; sb < nsb; ++sb) {
-        run_block(cs, tmem, sb * SBR, min(nch, (sb + 1) * SBR), nch, LS, tab, pre, load, [](int64_t v) { return v; });
+        run_block(cs, tmem, sb * SBR, min(nch, (sb + 1) * SBR), nch, LS, tab, pre, load,
+                  [](int64_t v, int, int) { return v; });
         if (!end_block(cs, sb)) {
             if (tid == 0) atomicOr(err, ERR_TC_TIMEOUT);
             break;

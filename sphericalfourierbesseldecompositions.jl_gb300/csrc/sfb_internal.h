@@ -70,6 +70,8 @@ struct Task64 {
     const int64_t *off = nullptr;
     const int16_t *ex = nullptr;       // [z][exs]
     const int2 *live = nullptr;        // [z][ntile]
+    const uint8_t *kx = nullptr;       // analysis: [z][nkx], value k of a sum is held on the scale 2^(kx - KXR)
+    int nkx = 0;
     int exs = 0, ntile = 0;
     int n_is_rows = 0;                 // table rows are coefficients l = m + parity + 2 n (else rings)
     int nout = 0, nlim = 0;            // rings of the output's layout, and those written
