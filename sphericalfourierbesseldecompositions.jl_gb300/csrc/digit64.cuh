@@ -1,9 +1,9 @@
-// FP64 products on the tensor cores by error-free 8-bit digits: the pieces that
+// FP64 products on the tensor cores by 8-bit digits: the pieces that
 // the Legendre (leg64_tc.cu) and ring (ring64_tc.cu) contractions share.
 //
 // A value is a 55-bit integer on a common scale, written as seven signed 8-bit
 // digits that BF16 holds exactly; the digit products of level v = a + b (v =
-// 0..6) are summed in one FP32 TMEM accumulator per level, exactly for v <= 3
+// 0..6) are summed in one FP32 TMEM accumulator per level, exactly for v <= 5
 // over at most SBK chunks of K, and the levels are joined as a 62-bit integer.
 #pragma once
 
@@ -21,7 +21,12 @@ constexpr int ND = 7;                                  // digits, and levels kep
 constexpr int KC = 16;                                 // K per chunk (one MMA K step)
 constexpr int MTILE = 128;                             // data columns per CTA
 constexpr int NT = LEG64_TILE;                         // table rows per CTA
-constexpr int SBK = 16;                                // chunks per exact K block (256 values)
+constexpr int SBK = 10;                                // chunks per exact K block (160 values)
+// A digit product is at most 2^14 and level v joins v + 1 of them: levels 0..5 of a block stay within the 2^24 up to
+// which FP32 holds every integer.  A unit of level v is 2^(-14 - 8 v) of the scales, so level 4 and 5 have to be exact
+// (2^-46, 2^-54); a rounding in level 6 is below 2^-57.
+static_assert(6 * SBK * KC <= 1 << 10, "levels 0..5 of a block must be exact");
+static_assert(SBK % 2 == 0, "a block begins with the first of the two buffers");
 // eight warps: a ninth for the MMAs would leave 96 registers a thread at two CTAs per SM instead of 128
 constexpr int NTH = 256;
 constexpr int MMA_WARP = NTH / 32 - 1;
@@ -156,11 +161,11 @@ __device__ __forceinline__ void issue(uint32_t tmem, uint32_t sa, uint32_t sb, i
     }
 }
 
-// One exact K block, chunks [k0, k1) of nch (k0 even), up to its last MMA's issue: every warp turns its values
+// One exact K block, chunks [k0, k1) of nch, up to its last MMA's issue: every warp turns its values
 // into digits (load(kc, buf, i): this thread's eight values of chunk kc, row tid % 128, k = 8 (tid / 128)..; fix(v, i,
 // j): value j of them as the integer; i is the buffer, pre[i]), the table digits of chunk kc come from tab + kc ND LS
-// KC, and the last warp issues a chunk's MMAs once all have written theirs.  pre holds the values of chunks k0 and k0 + 1 on entry.  end_block
-// waits for the MMAs.
+// KC, and the last warp issues a chunk's MMAs once all have written theirs.  pre holds the values of chunks k0 and k0 + 1 on entry (in this
+// order: an odd block swaps them at its end).  end_block waits for the MMAs.
 template <typename T, typename Load, typename Fix>
 __device__ __forceinline__ void run_block(const Smem &cs, uint32_t tmem, int k0, int k1, int nch, int LS,
                                           const uint16_t *tab, T (&pre)[2][8], const Load &load, const Fix &fix) {
@@ -218,6 +223,14 @@ __device__ __forceinline__ void run_block(const Smem &cs, uint32_t tmem, int k0,
     }
     if (tid == 32 * MMA_WARP) mma_commit(cs.done);          // arrives once every MMA issued above has completed
     __syncwarp();
+    if (k1 < nch && ((k1 - k0) & 1)) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const T v = pre[0][j];
+            pre[0][j] = pre[1][j];
+            pre[1][j] = v;
+        }
+    }
 }
 
 // Every MMA of block sb is complete; false when a wait gave up.

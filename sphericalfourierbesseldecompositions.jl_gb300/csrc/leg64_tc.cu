@@ -1,6 +1,6 @@
 // FP64 Legendre and Gram contractions on the tensor cores (tcgen05), many
 // columns: the analysis, the synthesis and the Gram update of the FP64
-// transform, as error-free products of 8-bit digits.
+// transform, as products of 8-bit digits.
 //
 // GB300 does about 2 FP64 FMA per clock and SM, so a tiled FP64 GEMM of these
 // contractions is bound by the FP64 pipe at 0.6 TFMA/s.  The BF16 tensor cores
@@ -9,15 +9,15 @@
 // K range (per data column, per table row) and written as seven signed 8-bit
 // digits, which BF16 holds exactly (Ozaki, Ogita, Oishi, Rump, Numer.
 // Algorithms 59, 2012).  The digit products of level v = a + b (v = 0..6, 28
-// of the 49 products; the others are below 2^-56 of the scales) are summed in
-// one FP32 TMEM accumulator per level.  A product is at most 2^14, so the sum
-// of level v over 256 values of K is at most (v + 1) 2^22: levels 0..3 are
-// exact whatever the tensor cores' accumulation order or rounding, and a
-// rounding in level v >= 4 is below 2^-56 of the scales.  K is therefore
-// worked in blocks of SBK chunks; after each the levels are joined as a 62-bit
-// integer, rounded once to FP64 and added to the output.  The result is as
-// close to the exact sum as an FP64 accumulation (the whole FP64 field2anlm
-// against 64-bit references: 3.6e-15 before, 3.5e-15 now).
+// of the 49 products; each of the others is below 2^-56 of the scales) are
+// summed in one FP32 TMEM accumulator per level.  Their sums over a block of SBK
+// chunks are exact in all levels that matter, whatever the tensor cores'
+// accumulation order or rounding (SBK says why); after each block the levels are
+// joined as a 62-bit integer, rounded once to FP64 and added to the output.  The
+// result is as close to the exact sum as an FP64 accumulation in the norm of the
+// scales (the whole FP64 field2anlm against 64-bit references: 3.6e-15 on the
+// FP64 units, 2.4e-15 so); a value far below its column's largest one keeps
+// fewer bits than in FP64, which the ring scales (KXR) make up for in the analysis.
 //
 // MMA shape: M = 128 data columns, N = table rows (<= 32 a tile), K = 16 a
 // step.  Data digit a multiplies the table digits 0..6-a in as few MMAs as N <=
@@ -241,6 +241,7 @@ __global__ void __launch_bounds__(NTH, 2) k_leg64(const double *data, int64_t nc
 // aliased synthesis, 40 so).  Bound: the epilogue's integer operations (about 80 an output), a third of the issue
 // slots at four warps a scheduler.
 constexpr int RES = 3;
+static_assert(RES <= SBK, "a short sum is one exact block");
 constexpr size_t SMEM_RES = (size_t)RES * ND * (PLANE_A + NT * KC * 2);
 
 struct TileJob {

@@ -1,5 +1,5 @@
 // FP64 ring Fourier transforms of many maps on the tensor cores, in both
-// directions, as error-free digit products (digit64.cuh).
+// directions, as digit products (digit64.cuh).
 //
 // The FFT kernels (ringfft.cu) are bound by the FP64 pipe: about 45 FP64
 // operations a pixel at 2 per clock and SM, and 40 percent of them for
@@ -32,8 +32,11 @@ namespace r64 {
 
 using namespace t64;
 
-constexpr int SBR = 12;        // chunks per exact block: the folded sums' leading digit reaches 256 (192 values)
-constexpr int KBMAX = 6;       // synthesis: coefficient chunks held at a time
+// chunks per exact block (144 values): the folded sums' leading digit reaches 256, so level v sums v + 2 times 2^14
+constexpr int SBR = 9;
+static_assert(7 * SBR * KC <= 1 << 10, "levels 0..5 of a block must be exact");
+constexpr int KBMAX = 6;       // synthesis: coefficient chunks held at a time (exact as SBK)
+static_assert(KBMAX <= SBK, "a block of the synthesis must be exact");
 
 struct Ring {
     int n, shifted, kc, kp, cls;
