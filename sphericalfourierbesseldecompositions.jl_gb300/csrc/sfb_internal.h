@@ -215,15 +215,19 @@ inline void set_smem(K kernel, size_t bytes) {
     if (bytes > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
-// Programmatic dependent launch: in a call that wants it (PdlScope) a kernel's blocks may be brought onto the SMs
-// while the last blocks of the kernel before it on the stream still run, and every kernel begins by waiting for that
-// kernel's completion (pdl_entry), so the launch latency between dependent kernels is hidden.  Nothing of a kernel
-// runs before its wait: a block that came early holds no TMEM and has written nothing.  The kernels' pointers carry
-// no __restrict__: loads through const restrict pointers count as read-only for the kernel's lifetime, and the
-// compiler may move them above the wait.
-// Chains of short kernels gain (us a call without and with: 231 and 190 at nside 16, 300 and 262 at nside 32, 583 and
-// 537 for field_f64's field); where the FP64 reference transform on the side stream competes for the SMs the blocks
-// that wait are in its way (594 and 607 at nside 128 with 104 maps), so the caller decides.
+// Programmatic dependent launch: in a call that wants it (PdlScope) a kernel's launch is prepared while the kernel
+// before it on the stream still runs, its blocks come onto the SMs once every block of that kernel has exited, and
+// every kernel begins by waiting for that kernel's completion (pdl_entry).  Nothing of a kernel runs before its wait: a
+// block that came early holds no TMEM and has written nothing.  The kernels' pointers carry no __restrict__: loads
+// through const restrict pointers count as read-only for the kernel's lifetime, and the compiler may move them above
+// the wait.
+// No kernel triggers its dependents itself (griddepcontrol.launch_dependents).  With a trigger at their entry the next
+// kernel's blocks came while the kernel ran and were packed onto the SMs that had room just then: 72 blocks of the
+// FP64 moments on a few SMs, whose FP64 pipe then bounded the call (300,000 galaxies in a cap at nside 16: 4860 us,
+// 1150 without the trigger and 1180 as plain launches; weight_gradient's call 525 and 489).
+// Chains of short kernels gain (us a call as plain and as dependent launches: 231 and 190 at nside 16, 300 and 262 at
+// nside 32, 583 and 537 for field_f64's field); where the FP64 reference transform on the side stream competes for
+// the SMs they did not (594 and 607 at nside 128 with 104 maps, measured with the trigger), so the caller decides.
 struct PdlScope {
     explicit PdlScope(bool on);
     ~PdlScope();
@@ -235,7 +239,6 @@ struct PdlScope {
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_entry() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 template <typename... P, typename... A>
 inline void launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A &&...args) {
