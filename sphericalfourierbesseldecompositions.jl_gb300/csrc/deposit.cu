@@ -899,18 +899,20 @@ __global__ void __launch_bounds__(32) k_deposit_stats(Offsets offset,
     const int64_t pix = valid ? idx - (int64_t)slot * npix : 0;
     const float2 c = valid ? cdf[pix] : make_float2(0.f, 0.f);
     const dfl rv = {c.x, c.y};
+    const unsigned full = 0xffffffffu;
+    const bool any = __any_sync(full, c.x != 0.f);  // (a group whose reference is zero adds nothing)
     dfl acc[MAXDEG + 1];
-    if (valid) {
+    if (any && valid) {
         bin_moments_df<MAXDEG>(sorted, offset[idx], offset[idx + 1], slot < pieces ? deg : 0, acc);
     } else {
 #pragma unroll
         for (int k = 0; k <= MAXDEG; ++k) acc[k] = {0.f, 0.f};
     }
     const int nk = slot < 0 ? 0 : (slot < pieces ? deg + 1 : 1);
-    const unsigned full = 0xffffffffu;
     const int slot0 = __shfl_sync(full, slot, 0);
     auto to_d = [](dfl a) { return (double)a.hi + (double)a.lo; };
-    if (__all_sync(full, slot == slot0)) {          // (a group is never without a valid bin)
+    if (!any) {
+    } else if (__all_sync(full, slot == slot0)) {   // (a group is never without a valid bin)
 #pragma unroll
         for (int k = 0; k <= MAXDEG; ++k)
             if (k < nk) {

@@ -124,7 +124,8 @@ __global__ void __launch_bounds__(128) k_ring_rowexp(const float2 *maps, int64_t
     const int64_t b = (int64_t)blockIdx.y * 4 + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     const RingGeom g = rings[r];
-    // both hemispheres' rows together: their loads are in flight at once (104 maps of nside 128: 25 -> 20 us)
+    // both hemispheres' rows together: their loads are in flight at once (104 maps of nside 128: 25 -> 20 us).  One
+    // hemisphere alone where the other has no data (328 maps of nside 256 in a cap: 131 us with both in one loop, 93 so)
     bool any = false;
     if (b < nmaps) {
         bool on[2] = {true, true};
@@ -136,16 +137,25 @@ __global__ void __launch_bounds__(128) k_ring_rowexp(const float2 *maps, int64_t
         const float2 *x = maps + b * npix;
         float mx[2] = {0.f, 0.f};
         bool fin[2] = {true, true};
+        auto take = [&](float2 v, float &m, bool &f) {                    // |hi + lo| < 2^E when |hi| < 2^E
+            f &= isfinite(v.x) && isfinite(v.y);
+            m = fmaxf(m, fabsf(v.x));
+        };
+        if (on[0] && on[1]) {
 #pragma unroll 2
-        for (int j = lane; j < g.nph; j += 32) {
-            float2 v[2];
-            v[0] = on[0] ? x[g.start_n + j] : make_float2(0.f, 0.f);      // |hi + lo| < 2^E when |hi| < 2^E
-            v[1] = on[1] ? x[g.start_s + j] : make_float2(0.f, 0.f);
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                fin[h] &= isfinite(v[h].x) && isfinite(v[h].y);
-                mx[h] = fmaxf(mx[h], fabsf(v[h].x));
+            for (int j = lane; j < g.nph; j += 32) {
+                const float2 n = x[g.start_n + j], s = x[g.start_s + j];
+                take(n, mx[0], fin[0]);
+                take(s, mx[1], fin[1]);
             }
+        } else if (on[0] || on[1]) {                                      // a survey on one side of the equator
+            const float2 *y = x + (on[0] ? g.start_n : g.start_s);
+            float m = 0.f;
+            bool f = true;
+#pragma unroll 4
+            for (int j = lane; j < g.nph; j += 32) take(y[j], m, f);
+            mx[on[0] ? 0 : 1] = m;
+            fin[on[0] ? 0 : 1] = f;
         }
         const int lg = 32 - __clz(g.nph - 1);                  // ceil(log2 n)
 #pragma unroll
