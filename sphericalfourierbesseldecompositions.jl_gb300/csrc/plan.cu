@@ -812,12 +812,24 @@ int sht_analysis_adjoint(sfb_plan *h, double *abar, int64_t nm, double *maps_out
     return SFB_OK;
 }
 
-int64_t chunk_pairs(const Plan &p) {
-    // keep the per-chunk SHT workspace near 2 GB
+// maps of one transform that keep its SHT workspace near 2 GB
+int64_t chunk_maps(const Plan &p) {
     const double per_map = 8.0 * (p.npix + 3.0 * 2 * (p.lmax + 1) * p.nrn * 2 + 2.0 * p.lmsize);
-    int64_t c = (int64_t)(2.0e9 / per_map);
-    c = std::max<int64_t>(1, std::min<int64_t>(c, p.npairs));
-    return c;
+    return std::max<int64_t>(1, (int64_t)(2.0e9 / per_map));
+}
+int64_t chunk_pairs(const Plan &p) { return std::min<int64_t>(chunk_maps(p), p.npairs); }
+
+// whether the mixed path transforms the maps of a dense window together with the basis maps
+bool joint_window(const Plan &p) { return p.precision == SFB_MIXED && p.npairs + p.nbasis <= chunk_maps(p); }
+
+// The transforms' workspaces, to be made again by the next call (freeing them waits for the device).
+void release_workspace(Plan &p) {
+    for (DevBuf<double> *b : {&p.maps, &p.fbuf, &p.gbuf, &p.rbuf, &p.alm, &p.almdf, &p.almdf2, &p.adf0, &p.ecoef, &p.erow,
+                              &p.maps32, &p.dep, &p.ref, &p.rf, &p.rg, &p.rr, &p.ralm, &p.aimg, &p.ring64, &p.nzr64}) {
+        if (b->ptr) cudaFree(b->ptr);
+        p.device_bytes -= (int64_t)(b->n * sizeof(double));
+        *b = DevBuf<double>();
+    }
 }
 
 // map pixels up to which a mixed catalogue transform uses programmatic dependent launches (PdlScope)
@@ -826,9 +838,10 @@ constexpr int64_t PDL_MAX = int64_t(1) << 24;
 // a_nlm of mocks.n catalogues (one, or the mocks of a group: mock j's result at out + 2 j nlmsize).
 // defer_finish (batched calls): the device error word is neither cleared nor read here and the
 // call does not wait for the device; the caller clears it once and checks it at the end.
-int cat2amln_dev(sfb_plan *h, const double *rtp, const double *w, int64_t ngal, const Mocks &mocks, const double *nbar,
-                 const sfb_window *win, double *out, cudaStream_t st, const cudaEvent_t *chunk_ready = nullptr,
-                 int nchunks = 0, bool defer_finish = false) {
+// joint_ok: a dense window's maps may share the transform of the basis maps (joint_window).
+int cat2amln_run(sfb_plan *h, const double *rtp, const double *w, int64_t ngal, const Mocks &mocks, const double *nbar,
+                 const sfb_window *win, double *out, cudaStream_t st, const cudaEvent_t *chunk_ready, int nchunks,
+                 bool defer_finish, bool joint_ok) {
     Plan &p = h->p;
     if (ngal < 0) return fail(SFB_EINVAL, "ngal < 0");
     if (!win) return fail(SFB_EINVAL, "window descriptor is NULL");
@@ -859,7 +872,7 @@ int cat2amln_dev(sfb_plan *h, const double *rtp, const double *w, int64_t ngal, 
         // dense windows: pairs per window transform; where all pairs fit, the mixed path transforms their maps
         // together with the basis maps
         const int64_t cp = wk == SFB_WINDOW_DENSE ? chunk_pairs(p) : 0;
-        const bool joint = split && cp > 0 && cp >= p.npairs;
+        const bool joint = split && cp > 0 && joint_ok && joint_window(p);
         const int64_t nb = p.nbasis, nm = nmock * nb + (mask_map ? 1 : 0) + (joint ? p.npairs : 0);
         const PdlScope pdl(!split || nm * p.npix <= PDL_MAX);
         double *Cmap = nullptr, *mu = nullptr, *nu = nullptr, *smean = nullptr, *refsq = nullptr;
@@ -980,14 +993,25 @@ int cat2amln_dev(sfb_plan *h, const double *rtp, const double *w, int64_t ngal, 
     return finish(h, out, st, checked);
 }
 
+int cat2amln_dev(sfb_plan *h, const double *rtp, const double *w, int64_t ngal, const Mocks &mocks, const double *nbar,
+                 const sfb_window *win, double *out, cudaStream_t st, const cudaEvent_t *chunk_ready = nullptr,
+                 int nchunks = 0, bool defer_finish = false) {
+    const int rc = cat2amln_run(h, rtp, w, ngal, mocks, nbar, win, out, st, chunk_ready, nchunks, defer_finish, true);
+    if (rc != SFB_ENOMEM || win->kind != SFB_WINDOW_DENSE || !joint_window(h->p)) return rc;
+    // no room for the window's maps beside the basis maps: one after the other
+    release_workspace(h->p);
+    return cat2amln_run(h, rtp, w, ngal, mocks, nbar, win, out, st, chunk_ready, nchunks, defer_finish, false);
+}
+
 // Mocks of [k, nmocks) that go through the kernels together.  Light mocks leave the chip idle and cost their
 // launches' latencies each; the limit is where one mock's maps fill it anyway (2^25 map pixels a group: twelve of
-// the mocks of nside 64 and 53 basis maps, one of nside 256), and 2^23 galaxies, whose copy the next group's
-// transform has to cover.
+// the mocks of nside 64 and 53 basis maps, one of nside 256), the workspace of one transform, and 2^23 galaxies,
+// whose copy the next group's transform has to cover.
 int mock_group(const Plan &p, const int64_t *offsets, int64_t k, int64_t nmocks, int window_kind) {
     if (p.radial_mode != SFB_RADIAL_POLY || window_kind == SFB_WINDOW_DENSE) return 1;
     const int64_t most = std::min<int64_t>(
-        {MOCKS_MAX, (int64_t(1) << 25) / (p.nbasis * p.npix), 0x7fffffff / ((p.pieces + 2) * p.npix) - 1, nmocks - k});
+        {MOCKS_MAX, (int64_t(1) << 25) / (p.nbasis * p.npix), chunk_maps(p) / (p.nbasis + 1),
+         0x7fffffff / ((p.pieces + 2) * p.npix) - 1, nmocks - k});
     int n = 1;
     while (n < most && offsets[k + n + 1] - offsets[k] <= (int64_t(1) << 23)) ++n;
     return n;
@@ -1499,22 +1523,34 @@ int sfb_cat2amln_batched(sfb_plan *h, const double *rtp, const double *weight, c
     }
     if (offsets[nmocks] > 0 && !rtp) return fail(SFB_EINVAL, "rtp is NULL");
     Plan &p = h->p;
-    std::vector<int64_t> first{0};                 // first mock of every group, then nmocks
+    std::vector<int64_t> first;                    // first mock of every group, then nmocks
     int64_t nmax_gal = 0, most = 0;
-    while (first.back() < nmocks) {
-        const int64_t k = first.back();
-        const int n = mock_group(p, offsets, k, nmocks, window->kind);
-        nmax_gal = std::max(nmax_gal, offsets[k + n] - offsets[k]);
-        most = std::max<int64_t>(most, n);
-        first.push_back(k + n);
-    }
-    const int64_t ngroups = (int64_t)first.size() - 1;
+    auto group_up = [&](bool singles) {
+        first.assign(1, 0);
+        nmax_gal = most = 0;
+        while (first.back() < nmocks) {
+            const int64_t k = first.back();
+            const int n = singles ? 1 : mock_group(p, offsets, k, nmocks, window->kind);
+            nmax_gal = std::max(nmax_gal, offsets[k + n] - offsets[k]);
+            most = std::max<int64_t>(most, n);
+            first.push_back(k + n);
+        }
+    };
     cudaStream_t st = h->stream;
     const int64_t wlen = window->kind == SFB_WINDOW_SEPARABLE ? p.npix + (int64_t)(p.lmax + 1) * p.nmax
                        : window->kind == SFB_WINDOW_DENSE ? p.npix * (int64_t)(p.lmax + 1) * p.nmax : 0;
     // [window][2 x (rtp 3 nmax_gal, w nmax_gal, out 2 nlmsize per mock)]
-    const int64_t per_buf = 3 * nmax_gal + (weight ? nmax_gal : 0) + 2 * p.nlmsize * most;
-    SFB_TRY(grow(p, p.scratch, (size_t)(wlen + 2 * per_buf + 1)));
+    int64_t per_buf = 0;
+    auto stage = [&](bool singles) {
+        group_up(singles);
+        per_buf = 3 * nmax_gal + (weight ? nmax_gal : 0) + 2 * p.nlmsize * most;
+        return grow(p, p.scratch, (size_t)(wlen + 2 * per_buf + 1));
+    };
+    int staged = stage(false);
+    if (staged == SFB_ENOMEM && most > 1) staged = stage(true);
+    SFB_TRY(staged);
+    const int64_t ngroups = (int64_t)first.size() - 1;
+    bool singles = false;                          // a group's workspace found no room
     double *d_win = p.scratch.ptr;
     sfb_window dw = *window;
     if (window->kind == SFB_WINDOW_SEPARABLE) {
@@ -1592,8 +1628,20 @@ int sfb_cat2amln_batched(sfb_plan *h, const double *rtp, const double *weight, c
         Mocks mk;
         mk.n = (int)(first[g + 1] - k);
         for (int j = 0; j <= mk.n; ++j) mk.off[j] = (int32_t)(mk.n > 1 ? offsets[k + j] - offsets[k] : 0);
-        rc = cat2amln_dev(h, ngal > 0 ? d_rtp : nullptr, d_w, ngal, mk, nbar + k, &dw, d_out, st, ev[b], sfb_plan::NCOPY,
-                          true);
+        if (!singles || mk.n == 1)
+            rc = cat2amln_dev(h, ngal > 0 ? d_rtp : nullptr, d_w, ngal, mk, nbar + k, &dw, d_out, st, ev[b],
+                              sfb_plan::NCOPY, true);
+        if (mk.n > 1 && (singles || rc == SFB_ENOMEM)) {          // its mocks one by one
+            if (!singles) release_workspace(p);
+            singles = true;
+            rc = SFB_OK;
+            for (int c = 0; c < sfb_plan::NCOPY && rc == SFB_OK; ++c)
+                if (cudaStreamWaitEvent(st, ev[b][c], 0) != cudaSuccess) rc = fail(SFB_ECUDA, "stream wait failed");
+            for (int j = 0; j < mk.n && rc == SFB_OK; ++j)
+                rc = cat2amln_dev(h, mk.off[j + 1] > mk.off[j] ? d_rtp + 3 * (int64_t)mk.off[j] : nullptr,
+                                  d_w ? d_w + mk.off[j] : nullptr, mk.off[j + 1] - mk.off[j], Mocks(), nbar + k + j, &dw,
+                                  d_out + 2 * p.nlmsize * j, st, nullptr, 0, true);
+        }
         if (rc != SFB_OK) break;
         if (cudaEventRecord(ev[b][sfb_plan::NCOPY], st) != cudaSuccess ||
             cudaMemcpyAsync(anlm_out + 2 * p.nlmsize * k, d_out, 2 * p.nlmsize * mk.n * sizeof(double),
