@@ -540,14 +540,16 @@ __global__ void k64_fill(int2 *r, int64_t n) {
 
 }  // namespace t64
 
-// Digit tables of the plan, built at the first FP64 transform of many columns.  14 bytes a table element
-// against 8 in FP64: above a sixteenth of the free device memory (or SFBGPU_TC64=0) the plan keeps the
-// FP64 units instead (state -1).
+// Digit tables of the plan, built at the first FP64 transform of many columns that finds the memory for them: 14 bytes
+// a table element against 8 in FP64, at most a sixteenth of the free device memory.  Without it the call runs on the
+// FP64 units and the next one asks again; SFBGPU_TC64=0 keeps the plan on them (state -1).
 bool ensure_tc64(Plan &p, cudaStream_t st) {
     if (p.tc64_state) return p.tc64_state > 0;
-    p.tc64_state = -1;
     if (const char *e = std::getenv("SFBGPU_TC64"))
-        if (e[0] == '0') return false;
+        if (e[0] == '0') {
+            p.tc64_state = -1;
+            return false;
+        }
     const int nz = 2 * (p.lmax + 1);
     const int nrows0 = p.lmax / 2 + 1;
     constexpr int NT = t64::NT;
@@ -579,6 +581,16 @@ bool ensure_tc64(Plan &p, cudaStream_t st) {
         cudaGetLastError();
         return false;
     }
+    auto give_back = [&] {
+        cudaGetLastError();
+        for (int kind = 0; kind < nkind; ++kind) {
+            if (p.t64_mem[kind]) cudaFree(p.t64_mem[kind]);
+            p.t64_mem[kind] = nullptr;
+            p.device_bytes -= p.t64_bytes[kind];
+            p.t64_bytes[kind] = 0;
+        }
+        return false;
+    };
     for (int kind = 0; kind < nkind; ++kind) {
         // one allocation: [digits][offsets][live ranges][exponents][ring scales], each part 256-byte aligned
         auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
@@ -587,13 +599,11 @@ bool ensure_tc64(Plan &p, cudaStream_t st) {
         const int nkx = kind == 0 ? nkmax[0] * t64::KC : 0;
         const size_t b4 = up((size_t)nz * nkx);
         unsigned char *d = nullptr;
-        if (cudaMalloc(&d, b0 + b1 + b2 + b3 + b4) != cudaSuccess) {
-            cudaGetLastError();
-            return false;                     // the tables made so far stay owned by the plan
-        }
-        p.device_bytes += (int64_t)(b0 + b1 + b2 + b3 + b4);
+        if (cudaMalloc(&d, b0 + b1 + b2 + b3 + b4) != cudaSuccess) return give_back();
         Task64 &t = p.t64[kind];
         p.t64_mem[kind] = d;
+        p.t64_bytes[kind] = (int64_t)(b0 + b1 + b2 + b3 + b4);
+        p.device_bytes += p.t64_bytes[kind];
         t.dig = reinterpret_cast<uint16_t *>(d);
         t.off = reinterpret_cast<int64_t *>(d + b0);
         t.live = reinterpret_cast<int2 *>(d + b0 + b1);
@@ -609,10 +619,8 @@ bool ensure_tc64(Plan &p, cudaStream_t st) {
         t.sn = kind == 0 ? p.nrn : 1;
         t.sk = kind == 0 ? 1 : kind == 1 ? p.nrn : p.gram_rows;
         if (cudaMemcpyAsync(d + b0, off[kind].data(), nz * sizeof(int64_t), cudaMemcpyHostToDevice, st) != cudaSuccess ||
-            cudaStreamSynchronize(st) != cudaSuccess) {
-            cudaGetLastError();
-            return false;
-        }
+            cudaStreamSynchronize(st) != cudaSuccess)
+            return give_back();
         const int64_t nl = (int64_t)nz * ntile[kind];
         launch_pdl(t64::k64_fill, dim3((unsigned)((nl + 255) / 256)), dim3(256), 0, st, const_cast<int2 *>(t.live),
             nl);
@@ -630,7 +638,7 @@ bool ensure_tc64(Plan &p, cudaStream_t st) {
         note_launch();
         note_launch();
     }
-    if (cudaGetLastError() != cudaSuccess) return false;
+    if (cudaGetLastError() != cudaSuccess) return give_back();
     p.tc64_state = 1;
     return true;
 }

@@ -512,15 +512,17 @@ __global__ void __launch_bounds__(256) k_ring_tab(const RingGeom *rings, int ns,
 
 }  // namespace r64
 
-// Digit tables of the ring transforms (dir 0: analysis, 1: synthesis), made at first use; false: the FFT
-// kernels stay (tables above a sixteenth of the free device memory, an nside below 2, or SFBGPU_RING64=0).
+// Digit tables of the ring transforms (dir 0: analysis, 1: synthesis), made at the first use that finds the memory;
+// false: the FFT kernels do this call (tables above a sixteenth of the free device memory) or every one (an nside
+// below 2, or SFBGPU_RING64=0).
 static bool ensure_ring64(Plan &p, int dir, cudaStream_t st) {
     if (p.ring64_state[dir]) return p.ring64_state[dir] > 0;
-    p.ring64_state[dir] = -1;
-    if (const char *e = std::getenv("SFBGPU_RING64"))
-        if (e[0] == '0') return false;
     const int ns = (int)p.nside;
-    if (ns < 2) return false;
+    const char *e = std::getenv("SFBGPU_RING64");
+    if (ns < 2 || (e && e[0] == '0')) {
+        p.ring64_state[dir] = -1;
+        return false;
+    }
     std::vector<int64_t> off;
     int64_t o = 0;
     for (int cls = 0; cls <= ns; ++cls) {
@@ -551,15 +553,16 @@ static bool ensure_ring64(Plan &p, int dir, cudaStream_t st) {
         cudaGetLastError();
         return false;
     }
-    p.ring64_mem[dir] = d;
-    p.device_bytes += (int64_t)(bt + bo);
+    auto give_back = [&] {
+        cudaGetLastError();
+        cudaFree(d);
+        return false;
+    };
     int64_t *doff = reinterpret_cast<int64_t *>(d + bt), *dq = doff + off.size();
     if (cudaMemcpyAsync(doff, off.data(), off.size() * sizeof(int64_t), cudaMemcpyHostToDevice, st) != cudaSuccess ||
         cudaMemcpyAsync(dq, qoff.data(), qoff.size() * sizeof(int64_t), cudaMemcpyHostToDevice, st) != cudaSuccess ||
-        cudaStreamSynchronize(st) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
+        cudaStreamSynchronize(st) != cudaSuccess)
+        return give_back();
     p.ring64_dig[dir] = reinterpret_cast<uint16_t *>(d);
     p.ring64_off[dir] = doff;
     p.ring64_qoff[dir] = dq;
@@ -572,7 +575,9 @@ static bool ensure_ring64(Plan &p, int dir, cudaStream_t st) {
     else launch_pdl(r64::k_ring_tab<false>, dim3(grid), dim3(256), 0, st, p.d_rings, ns, p.lmax, wm, doff,
         p.ring64_dig[0]);
     note_launch();
-    if (cudaGetLastError() != cudaSuccess) return false;
+    if (cudaGetLastError() != cudaSuccess) return give_back();
+    p.ring64_mem[dir] = d;
+    p.device_bytes += (int64_t)(bt + bo);
     p.ring64_state[dir] = 1;
     return true;
 }

@@ -186,10 +186,11 @@ struct Plan {
     DevBuf<double> ecoef;           // Gram refinement: column exponents of both a_lm sets (ints)
     DevBuf<double> erow;            // ring DFT row exponents [2][nrn][nmaps] (int)
     DevBuf<double> maps32;          // FP32 copy of FP64 maps (mixed precision, spline / dense-window paths)
-    // digit tables of the FP64 tensor-core contractions (analysis, synthesis, Gram): 0 not made yet, 1 made,
-    // -1 not used (memory); made by ensure_tc64
+    // digit tables of the FP64 tensor-core contractions (analysis, synthesis, Gram): 0 not made (yet, or for want of
+    // memory), 1 made, -1 not wanted; made by ensure_tc64
     Task64 t64[3];
     void *t64_mem[3] = {};
+    int64_t t64_bytes[3] = {};
     int tc64_state = 0;
     // FP64 ring transforms on the tensor cores (ring64_tc.cu), [0] analysis, [1] synthesis: digit tables
     // (state as tc64_state), integers of the folded rings per map (ring64_row values a row)
@@ -357,7 +358,7 @@ bool launch_refine_narrow64(const Plan &p, const double *A, const double *A0, in
 bool launch_gram_update_fp64(const Plan &p, const double *Acur, const double *A0, int64_t ncol, double *Anew,
                              cudaStream_t st);
 // FP64 contractions of many columns on the tensor cores (leg64_tc.cu).  ensure_tc64 makes the plan's digit
-// tables (once); false: the plan keeps the FP64 units.  The launches need a plan whose tables are made.
+// tables (once); false: this call runs on the FP64 units.  The launches need a plan whose tables are made.
 bool ensure_tc64(Plan &p, cudaStream_t st);
 void launch_leg_analysis64(const Plan &p, const double *F, int64_t ncol, double *A, bool accumulate, cudaStream_t st,
                            int rlim, const int *nzr);

@@ -7,6 +7,7 @@ import pytest
 
 import sfbgpu
 from helpers import rel_err
+from sfbgpu.cat2anlm import map2alm, map2alm_adjoint
 from test_gpu_batched import _mocks, _window
 
 pytestmark = pytest.mark.gpu
@@ -76,3 +77,25 @@ def test_group_of_mocks():
     one, two = _roomy_and_tight(lambda m: sfbgpu.cat2amln_batched(cats, m, nbars, win, ws, precision="mixed"), 0.05)
     for x, y in zip(one, two):
         assert rel_err(y, x) < 1e-9 or not np.any(x)
+
+
+def test_tables_are_made_when_there_is_memory():
+    """A plan whose first calls find no memory for the digit tables runs them on the FP64 units (1e-13, as the
+    tensor-core tests) and later ones as any other plan: the same bits."""
+    def modes():
+        return sfbgpu.AnlmModes.from_nmax_lmax(1, 60, 500.0, 1000.0, nside=64, cache=True)
+
+    f = np.random.default_rng(5).normal(size=(6, 12 * 64 * 64))
+    y = np.random.default_rng(6).normal(size=(6, 61 * 62 // 2, 2)) @ np.array([1.0, 1j])
+    a, b = modes(), modes()
+    fresh = map2alm(f, b, radial="spline"), map2alm_adjoint(y, b, radial="spline")
+    before = sfbgpu.get_plan(a, radial="spline").info()["device_bytes"]
+    held = _leave(60e6)                                # the tables take more than a sixteenth of this
+    short = map2alm(f, a, radial="spline"), map2alm_adjoint(y, a, radial="spline")
+    small = sfbgpu.get_plan(a, radial="spline").info()["device_bytes"]
+    del held
+    _free()
+    later = map2alm(f, a, radial="spline"), map2alm_adjoint(y, a, radial="spline")
+    assert sfbgpu.get_plan(a, radial="spline").info()["device_bytes"] > small > before
+    for s, l, g in zip(short, later, fresh):
+        assert rel_err(s, g) < 1e-13 and np.array_equal(l, g)
