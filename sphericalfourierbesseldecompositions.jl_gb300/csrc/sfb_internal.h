@@ -211,9 +211,15 @@ void note_launch();
 
 // Opt a kernel into `bytes` of dynamic shared memory (only above the 48 KB
 // default).  A failure is left for the caller's cudaGetLastError check.
+// The limit is the kernel's, not the launch's: every caller sets the same one
+// (227 KB less the static part), or a smaller plan on another thread would
+// lower it between this call and its launch.
+constexpr size_t SMEM_LIMIT = 223 * 1024;
 template <typename K>
 inline void set_smem(K kernel, size_t bytes) {
-    if (bytes > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (bytes > 48 * 1024)
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)(bytes > SMEM_LIMIT ? bytes : SMEM_LIMIT));
 }
 
 // Programmatic dependent launch: in a call that wants it (PdlScope) a kernel's launch is prepared while the kernel
