@@ -29,9 +29,10 @@
 // ends (one CTA of 64 rows a SM was slower at every size: field_f64's four
 // analyses 150 us against 117, an lmax 189 call 22.4 ms against 21.5).
 //
-// Measured at 200 columns, nside 64, lmax 58: first analysis 36 us, a Gram update
-// with the aliased synthesis 23, an aliased analysis 15 (the transform of these 100
-// shells took 2332 us a call with tiled FP64 kernels and 1043 with this file's alone).
+// Measured at 200 columns, nside 64, lmax 58: first analysis 39 us (36 with one scale
+// for all rings), a Gram update with the aliased synthesis 22, an aliased analysis 15
+// (the transform of these 100 shells took 2332 us a call with tiled FP64 kernels and 1043
+// with this file's alone).
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
