@@ -24,7 +24,7 @@ constexpr int NT = LEG64_TILE;                         // table rows per CTA
 constexpr int SBK = 10;                                // chunks per exact K block (160 values)
 // A digit product is at most 2^14 and level v joins v + 1 of them: levels 0..5 of a block stay within the 2^24 up to
 // which FP32 holds every integer.  A unit of level v is 2^(-14 - 8 v) of the scales, so level 4 and 5 have to be exact
-// (2^-46, 2^-54); a rounding in level 6 is below 2^-57.
+// (2^-46, 2^-54); the roundings of level 6 (2^-61 each) stay below 2^-54 together.
 static_assert(6 * SBK * KC <= 1 << 10, "levels 0..5 of a block must be exact");
 static_assert(SBK % 2 == 0, "a block begins with the first of the two buffers");
 // eight warps: a ninth for the MMAs would leave 96 registers a thread at two CTAs per SM instead of 128
